@@ -131,41 +131,89 @@ def _wire(codec, n, k, gen, lead=(), std=None):
     return pool.cuda()[pick].reshape(tuple(lead) + (n, k // wpb * bpb))
 
 
-def _linear(codec, n, k, gen):
-    with torch.device("cuda"):
-        layer = KQuantLinear(k, n, False, codec)
-    layer.weight = _wire(codec, n, k, gen)
-    return layer
+class _Package:
+    """The path's steps as this package offers them."""
+
+    @staticmethod
+    def linear(codec, w, k):
+        with torch.device("cuda"):
+            layer = KQuantLinear(k, w.shape[0], False, codec)
+        layer.weight = w
+        return layer
+
+    @staticmethod
+    def heads(codec, w, k):
+        with torch.device("cuda"):
+            layer = KQuantMultiLinear(k, w.shape[1], w.shape[0], codec)
+        layer.weight = w
+        return layer
+
+    norm = staticmethod(lambda x: torch.nn.functional.rms_norm(x, (x.shape[-1],)))
+    swiglu = staticmethod(moe.swiglu)
+    dequantize = staticmethod(kq.dequantize)
+
+    @staticmethod
+    def block(x, logits, top_k, gate, up, down, codec):
+        gate_up = moe.fuse_gate_up(gate, up)
+
+        def block(x, logits):
+            ids, probs = moe.route_topk(logits, top_k)
+            return moe.moe_glu(x, None, None, down, codec, ids, probs, w_gate_up=gate_up)
+        return [x, logits], block
 
 
-def _heads(codec, heads, n, k, gen):
-    with torch.device("cuda"):
-        layer = KQuantMultiLinear(k, n, heads, codec)
-    # used in both orientations: n inputs one way, k the other
-    layer.weight = _wire(codec, n, k, gen, lead=(heads,), std=(n * k) ** -0.25)
-    return layer
+class _Double:
+    """The same steps in plain torch and float64, no value rounded between them."""
+
+    @staticmethod
+    def linear(codec, w, k):
+        return lambda x: x.double() @ _decode(codec, w).T
+
+    @staticmethod
+    def heads(codec, w, k):
+        def product(x, transpose=True):
+            d = _decode(codec, w)
+            return torch.einsum("bhlk,hnk->bhln" if transpose else "bhln,hnk->bhlk", x.double(), d)
+        return product
+
+    @staticmethod
+    def norm(x):
+        eps = torch.finfo(torch.float32).eps   # what rms_norm takes for rows of 16-bit and 32-bit floats
+        return x * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + eps)
+
+    swiglu = staticmethod(lambda gate, up: torch.nn.functional.silu(gate) * up)
+    dequantize = staticmethod(lambda w, scales, codec, dtype: _decode(codec, w))
+
+    @staticmethod
+    def block(x, logits, top_k, gate, up, down, codec):
+        def block(x, logits):
+            x, scores = x.double(), torch.softmax(logits.double(), -1)
+            scores, ids = scores.topk(top_k, dim=-1)
+            scores = scores / scores.sum(-1, keepdim=True)
+            y = torch.zeros_like(x)
+            for e in range(gate.shape[0]):
+                t, slot = (ids == e).nonzero(as_tuple=True)
+                h = _Double.swiglu(x[t] @ _decode(codec, gate[e]).T, x[t] @ _decode(codec, up[e]).T)
+                y.index_add_(0, t, h @ _decode(codec, down[e]).T * scores[t, slot, None])
+            return y
+        return [x, logits], block
 
 
 def _randn(shape, dtype, gen):
     return torch.randn(shape, generator=gen, device="cuda").to(DTYPES[dtype])
 
 
-def _norm(x):
-    return torch.nn.functional.rms_norm(x, (x.shape[-1],))
-
-
-def _mlp(gate, up, down, x):
-    return down(moe.swiglu(gate(x), up(x)))
-
-
-def _step_fn(case, gen):
-    """(inputs, fn): fn(*inputs) is one pass."""
+def _step_fn(case, gen, lib):
+    """(inputs, fn): fn(*inputs) is one pass; lib: whose steps it is made of."""
     kind, codec, dtype = case["kind"], case["codec"], case["dtype"]
+
+    def linear(codec, n, k):
+        return lib.linear(codec, _wire(codec, n, k, gen), k)
     if kind == "linear":
-        layer = _linear(codec, case["n"], case["k"], gen)
+        layer = linear(codec, case["n"], case["k"])
         return [_randn((case["m"], case["k"]), dtype, gen)], layer
     if kind == "chain":
-        layers = [_linear(codec, case["k"], case["k"], gen) for _ in range(case["layers"])]
+        layers = [linear(codec, case["k"], case["k"]) for _ in range(case["layers"])]
 
         def chain(x):
             for layer in layers:
@@ -174,46 +222,57 @@ def _step_fn(case, gen):
         return [_randn((case["m"], case["k"]), dtype, gen)], chain
     if kind in ("layer", "mlp"):
         h, f, down = case["hidden"], case["ffn"], case["codec_down"]
-        blocks = [(_linear(codec, h, h, gen) if kind == "layer" else None, _linear(codec, f, h, gen),
-                   _linear(codec, f, h, gen), _linear(down, h, f, gen)) for _ in range(case.get("layers", 1))]
+        blocks = [(linear(codec, h, h) if kind == "layer" else None, linear(codec, f, h), linear(codec, f, h),
+                   linear(down, h, f)) for _ in range(case.get("layers", 1))]
+
+        def feed_forward(gate, up, down, x):
+            return down(lib.swiglu(gate(x), up(x)))
 
         def mlp(x):
-            return _mlp(*blocks[0][1:], x)
+            return feed_forward(*blocks[0][1:], x)
 
         def decoder(x):
-            for out_proj, gate, up, down_proj in blocks:
-                x = x + out_proj(_norm(x))
-                x = x + _mlp(gate, up, down_proj, _norm(x))
+            for out_proj, *ffn in blocks:
+                x = x + out_proj(lib.norm(x))
+                x = x + feed_forward(*ffn, lib.norm(x))
             return x
         return [_randn((case["m"], h), dtype, gen)], decoder if kind == "layer" else mlp
     if kind == "dequant":
         w = _wire(codec, case["n"], case["k"], gen)
-        return [w], lambda w: kq.dequantize(w, None, codec, DTYPES[dtype])
+        return [w], lambda w: lib.dequantize(w, None, codec, DTYPES[dtype])
     if kind == "heads":
         nh, d, r, b = case["heads"], case["head_dim"], case["rank"], case["batch"]
-        layers = [(_heads(codec, nh, d, r, gen), _heads(codec, nh, d, r, gen)) for _ in range(case["layers"])]
 
-        def heads(q):
+        def heads():   # used in both orientations: d inputs one way, r the other
+            return lib.heads(codec, _wire(codec, d, r, gen, lead=(nh,), std=(d * r) ** -0.25), r)
+        layers = [(heads(), heads()) for _ in range(case["layers"])]
+
+        def attention(q):
             for q_up, v_down in layers:   # the attention between the two is not this package's work
                 q = v_down(q_up(q, transpose=False))
             return q
-        return [_randn((b, nh, 1, d), dtype, gen)], heads
-    h, f, e, top_k = case["hidden"], case["ffn"], case["experts"], case["top_k"]
-    gate_up = moe.fuse_gate_up(_wire(codec, f, h, gen, lead=(e,)), _wire(codec, f, h, gen, lead=(e,)))
+        return [_randn((b, nh, 1, d), dtype, gen)], attention
+    h, f, e = case["hidden"], case["ffn"], case["experts"]
+    gate, up = _wire(codec, f, h, gen, lead=(e,)), _wire(codec, f, h, gen, lead=(e,))
     down = _wire(codec, h, f, gen, lead=(e,))
+    x, logits = _randn((case["tokens"], h), dtype, gen), torch.randn((case["tokens"], e), generator=gen, device="cuda")
+    return lib.block(x, logits, case["top_k"], gate, up, down, codec)
 
-    def block(x, logits):
-        ids, probs = moe.route_topk(logits, top_k)
-        return moe.moe_glu(x, None, None, down, codec, ids, probs, w_gate_up=gate_up)
-    return [_randn((case["tokens"], h), dtype, gen), torch.randn((case["tokens"], e), generator=gen, device="cuda")], block
+
+def _inputs(case, seed, lib):
+    """(the inputs of every step, fn): a case that is replayed from a graph has two steps, any other one."""
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    inputs, fn = _step_fn(case, gen, lib)
+    if not (case["kind"] in ("chain", "layer", "heads") or case.get("graph")):
+        return [inputs], fn
+    return [inputs, [torch.randn(x.shape, generator=gen, device="cuda").to(x.dtype) for x in inputs]], fn
 
 
 def prepare(case, seed):
-    gen = torch.Generator(device="cuda").manual_seed(seed)
-    inputs, fn = _step_fn(case, gen)
-    if not (case["kind"] in ("chain", "layer", "heads") or case.get("graph")):
+    steps, fn = _inputs(case, seed, _Package)
+    inputs = steps[0]
+    if len(steps) == 1:
         return {"inputs": inputs, "fn": fn}
-    second = [torch.randn(x.shape, generator=gen, device="cuda").to(x.dtype) for x in inputs]
     static = [x.clone() for x in inputs]
     side = torch.cuda.Stream()
     side.wait_stream(torch.cuda.current_stream())
@@ -225,7 +284,7 @@ def prepare(case, seed):
     with torch.cuda.graph(graph):
         output = fn(*static)
     # fn holds the weights, which the graph reads
-    return {"steps": [inputs, second], "static": static, "graph": graph, "output": output, "fn": fn,
+    return {"steps": steps, "static": static, "graph": graph, "output": output, "fn": fn,
             "results": [torch.empty_like(output) for _ in range(TOKENS)]}
 
 
@@ -295,3 +354,90 @@ def tolerance(case):
     if kind == "mlp":                                                  # seen: 3.0e-3 / 1.3e-2, f16 9.3e-4 / 4.7e-3
         return {"rel": 4e-3, "max": 2e-2} if half else {"rel": 1.2e-2, "max": 5e-2}
     return {"rel": 2.5e-3, "max": 1e-2} if half else {"rel": 1.5e-2, "max": 0.1}   # seen: 4.7e-3 / 2.5e-2, f16 6e-4
+
+
+def _half(b, at):
+    """The float16 at byte `at` of every block, as [blocks, 1] float64."""
+    return b[:, at:at + 2].contiguous().view(torch.float16).double()
+
+
+def _nibbles(q, run):
+    """Bytes [blocks, n] -> [blocks, n / run, 2, run]: the low nibbles of every run of bytes, then its high ones."""
+    q = q.reshape(q.shape[0], -1, 1, run)
+    return torch.cat((q & 15, q >> 4), 2)
+
+
+def _bits(q, at, count, width):
+    """`count` fields of `width` bits from bit `at` upwards of every byte: [blocks, count, bytes]."""
+    shift = torch.arange(at, at + count * width, width, device=q.device)
+    return (q[:, None] >> shift[:, None]) & ((1 << width) - 1)
+
+
+IQ4 = (-127, -104, -83, -65, -49, -35, -22, -10, 1, 13, 25, 38, 53, 69, 89, 113)
+
+
+def _scales_mins(b):
+    """q4_k / q5_k: the eight 6-bit scales and mins of a block's twelve packed bytes, [blocks, 8, 1] each."""
+    lo, mid, hi = b[:, 0:4], b[:, 4:8], b[:, 8:12]
+    sc = torch.cat((lo & 63, (hi & 15) | (lo >> 6 << 4)), 1)
+    mn = torch.cat((mid & 63, (hi >> 4) | (mid >> 6 << 4)), 1)
+    return sc[..., None].double(), mn[..., None].double()
+
+
+def _decode(codec, wire):
+    """Wire bytes -> float64 weights, from the block formats' definitions. iq2_xxs (a lattice of 256 points that no
+    formula gives) has no decoder here: exact() says None for it."""
+    wpb, bpb, _, _ = kq.codec_geometry(codec)
+    b = wire.reshape(-1, bpb)
+    n = b.shape[0]
+    i = b.int()
+    if codec == "q8_0":
+        v = _half(b, 0) * b[:, 2:].contiguous().view(torch.int8).double()
+    elif codec == "q4_0":
+        v = _half(b, 0) * (_nibbles(i[:, 2:], 16).reshape(n, 32) - 8)
+    elif codec == "q4_1":
+        v = _half(b, 0) * _nibbles(i[:, 4:], 16).reshape(n, 32) + _half(b, 2)
+    elif codec in ("q5_0", "q5_1"):
+        at = 2 if codec == "q5_0" else 4
+        high = _bits(i[:, at:at + 4], 0, 8, 1).transpose(1, 2).reshape(n, 32)
+        q = _nibbles(i[:, at + 4:], 16).reshape(n, 32) | high << 4
+        v = _half(b, 0) * (q - 16) if codec == "q5_0" else _half(b, 0) * q + _half(b, 2)
+    elif codec in ("iq4_nl", "iq4_xs"):
+        levels = torch.tensor(IQ4, device=b.device, dtype=torch.float64)
+        v = levels[_nibbles(i[:, 2 if codec == "iq4_nl" else 8:], 16).long()].reshape(n, -1, 32)
+        if codec == "iq4_xs":
+            low = torch.stack((i[:, 4:8] & 15, i[:, 4:8] >> 4), 2).reshape(n, 8)
+            high = _bits(i[:, 2:4], 0, 4, 2).transpose(1, 2).reshape(n, 8)
+            v = v * ((low | high << 4) - 32)[..., None]
+        v = v * _half(b, 0)[..., None]
+    elif codec == "q4_k":
+        sc, mn = _scales_mins(i[:, 4:16])
+        v = _half(b, 0)[..., None] * sc * _nibbles(i[:, 16:], 32).reshape(n, 8, 32) - _half(b, 2)[..., None] * mn
+    elif codec == "q5_k":
+        sc, mn = _scales_mins(i[:, 4:16])
+        q = _nibbles(i[:, 48:], 32).reshape(n, 8, 32) | _bits(i[:, 16:48], 0, 8, 1) << 4
+        v = _half(b, 0)[..., None] * sc * q - _half(b, 2)[..., None] * mn
+    elif codec == "q6_k":
+        q = torch.cat([_nibbles(i[:, 64 * h:64 * h + 64], 64).reshape(n, 4, 32)
+                       | _bits(i[:, 128 + 32 * h:160 + 32 * h], 0, 4, 2) << 4 for h in (0, 1)], 1) - 32
+        sc = b[:, 192:208].contiguous().view(torch.int8).double()
+        v = _half(b, 208)[..., None] * sc[..., None] * q.reshape(n, 16, 16)
+    elif codec == "q3_k":
+        q = torch.cat([_bits(i[:, 32 + 32 * h:64 + 32 * h], 0, 4, 2) for h in (0, 1)], 1)
+        q = q + 4 * _bits(i[:, :32], 0, 8, 1) - 4
+        sc = torch.cat((i[:, 96:104] & 15, i[:, 96:104] >> 4), 1) | _bits(i[:, 104:108], 0, 4, 2).reshape(n, 16) << 4
+        v = _half(b, 108)[..., None] * (sc - 32)[..., None] * q.reshape(n, 16, 16)
+    elif codec == "q2_k":
+        q = torch.cat([_bits(i[:, 16 + 32 * h:48 + 32 * h], 0, 4, 2) for h in (0, 1)], 1).reshape(n, 16, 16)
+        v = _half(b, 80)[..., None] * (i[:, :16] & 15)[..., None] * q - _half(b, 82)[..., None] * (i[:, :16] >> 4)[..., None]
+    else:
+        raise NotImplementedError(codec)
+    return v.reshape(wire.shape[:-1] + (wire.shape[-1] // bpb * wpb,))
+
+
+def exact(case, seed):
+    if "iq2_xxs" in (case["codec"], case.get("codec_down")):
+        return None
+    steps, fn = _inputs(case, seed, _Double)
+    outputs = [fn(*inputs) for inputs in steps]
+    return outputs if len(steps) > 1 else outputs[0]
