@@ -186,12 +186,15 @@ int kq_quantized_matmul(const void* x, int x_dtype, long long rows, int K, long 
     a.N = N;
     a.K = K;
     a.M = (int)rows;
-    // q4_k, 2-16 rows of bf16 / f32 activations, scratch at hand: exact fp16 copy of the rows (per-row
-    // power-of-two factor), then the fp16 tensor-core decode kernel writing bf16(sum * factor) - several
-    // times faster than the path that takes bf16 rows directly. Without scratch that path still serves.
+    // 2-16 rows the row kernel (kq_rows.cu) does not take as they are - f32 rows, and bf16 rows of q4_k matrices of
+    // a form it does not cover - with scratch at hand: exact fp16 copy of the rows (per-row power-of-two factor),
+    // then the fp16 kernel writing bf16(sum * factor), several times faster than the kernels that take such rows
+    // directly. Without scratch those still serve.
     const size_t need = kq::gemm_workspace_bytes(x_dtype, rows, K);
     int eff_dtype = x_dtype;
-    if (ci == kq::Q4_K && x_dtype != KQ_F16 && rows >= 2 && a.w_align16 && (w_row_bytes & 15) == 0 &&
+    const bool direct = rows >= 2 && kq::gemv_rows_supported(ci, x_dtype, a);
+    const bool q4k = ci == kq::Q4_K && a.w_align16 && (w_row_bytes & 15) == 0;
+    if (x_dtype != KQ_F16 && rows >= 2 && !direct && (q4k || kq::gemv_rows_supported(ci, KQ_F16, a)) &&
         workspace != nullptr && workspace_bytes >= need && need > 0 &&
         (reinterpret_cast<uintptr_t>(workspace) & 255) == 0) {
       float* rs = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) +

@@ -57,6 +57,10 @@ cudaError_t launch_gemv(int codec, int x_dtype, const GemvArgs& a, cudaStream_t 
 bool gemv_dp4a_supported(int codec, int x_dtype, const GemvArgs& a);
 cudaError_t launch_gemv_dp4a(int codec, int x_dtype, const GemvArgs& a, cudaStream_t st);
 
+// 1 to 16 dense rows of fp16 / bf16 on mma.sync over the integers themselves (kq_rows.cu).
+bool gemv_rows_supported(int codec, int x_dtype, const GemvArgs& a);
+cudaError_t launch_gemv_rows(int codec, int x_dtype, const GemvArgs& a, cudaStream_t st);
+
 // Prefill (M > 16) tile kernel on tcgen05 tensor cores with TMEM accumulators.
 // bf16 / f32 activations need gemm_workspace_bytes() of scratch for their fp16 copy.
 size_t gemm_workspace_bytes(int x_dtype, long long rows, int K);

@@ -1,0 +1,660 @@
+// Decode product of a few activation rows: y[M, N] = x[M, K] . dequant(W)^T for 1 <= M <= 16, on mma.sync with the
+// quantized integers themselves as the A operand (sixteen weight rows x sixteen weights an instruction), the
+// activations in their own 16-bit type as the B operand, float32 accumulation. Reference: qmv_fused_rows,
+// src/kquant_cpu_decode.cpp:1032-1065.
+//
+// What bounds it: a tile product is a chain of shared-memory loads, permutes and matrix instructions some 2500 cycles
+// long, with 16 warps on an SM to hide it (without any weight copy [28672, 8192] x 1 row takes 40 of 48 us; without any
+// product 26); HBM is the next bound. Measured [14336, 4096] x 8 bf16 rows: q4_k 17.2 us, q5_k 19.5, q6_k 31 (25.3, 80,
+// 68 on the kernels before it). What it is built around:
+//   * No value is rounded: a weight is scale x integer (- min), the integer goes into the tensor core as it is and
+//     the scale is applied in float32 to the sum over its 16- or 32-weight sub-block. The bytes become operands
+//     with one byte permute per two weights: for bf16 rows byte q becomes the bf16 number (128 + q) * 2^-24
+//     (0x3700 | q), for fp16 rows the subnormal q * 2^-24 (the power of two keeps the sums of the largest finite bf16
+//     rows finite); what the constant offset adds (and the min term of the codecs that have one) is coefficient_j *
+//     (sum of the activations of sub-block j), a product of its own with tf32 instructions over the float32 sums
+//     split in two parts. The sums of a stage are made once per CTA by a helper warp.
+//   * One CTA per SM owns N / SM count consecutive weight rows (rows are independent, so tiles need not be whole) and
+//     walks K in stages of WK superblocks: four producer warps bring the stage's bytes of every row, and the
+//     activations of that K range, into shared memory with 16-byte asynchronous copies, three or more stages in
+//     flight (one bulk copy per row instead was four times slower: a bulk copy costs the SM some 80 cycles); the consumer warps are RT row tiles x WK superblocks, so that a stage is one tile product per warp.
+//   * The weight copies of the first stages are issued before griddepcontrol.wait.
+// Blocks that are not whole numbers of 16 bytes (q6_k) are copied as the 16-byte aligned window around a row's
+// bytes; a block then starts on an even byte, and where that is not a multiple of four the words are taken from the
+// next aligned position, with the sub-block's weights handed to the lanes in another order (the sum over a
+// sub-block does not care, the activations are read in the same order).
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <cstdlib>
+#include <type_traits>
+
+#include "kq_common.cuh"
+#include "kq_imma_q4k.cuh"
+#include "kq_launch.h"
+#include "kq_tcgen05.cuh"
+
+namespace kq {
+
+namespace {
+
+constexpr int kRwMaxSmem = 227 * 1024 - 1024;
+constexpr int kRwMaxStages = 6;
+constexpr int kRwProducers = 4, kRwHelpers = 4;  // warps
+
+// sub-blocks of a superblock, min term, 16-byte blocks
+__host__ __device__ constexpr int rw_nsub(int c) { return c == Q6_K ? 16 : 8; }
+__host__ __device__ constexpr bool rw_min(int c) { return c == Q4_K || c == Q5_K; }
+__host__ __device__ constexpr bool rw_al16(int c) { return c == Q4_K || c == Q5_K; }
+// what the operand of integer 0 stands for, to be subtracted: the bf16 pattern's 128, and the codec's own offset
+template <int C, bool BF>
+__host__ __device__ constexpr int rw_base() { return (BF ? 128 : 0) + (C == Q6_K ? 32 : 0); }
+template <int C, bool BF>
+__host__ __device__ constexpr bool rw_sums() { return rw_min(C) || rw_base<C, BF>() != 0; }
+// words per (superblock, activation row) of the sums: heads, tails, padding against bank conflicts
+__host__ __device__ constexpr int rw_sum_pitch(int c) { return 2 * rw_nsub(c) + 4; }
+
+struct RowsPlan {
+  int R;       // weight rows of a row block
+  int rt, wk;  // row tiles of 16, warps to a row tile: rt * wk consumer warps work
+  int cs;      // superblocks of a stage; warp column k takes k, k + wk, ...
+  int stages, wpitch, xpitch, stage_bytes, x_off, sum_off, red_off, smem;
+  int n_blocks;
+};
+
+__device__ __forceinline__ void rw_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                       uint32_t b1, __half) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void rw_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                       uint32_t b1, __nv_bfloat16) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void rw_mma_tf32(float (&c)[4], const float (&a)[4], float b0, float b1) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])),
+        "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
+}
+__device__ __forceinline__ void rw_cp16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void rw_cp16_upto(uint32_t dst, const void* src, int bytes) {  // the rest is filled with zeros
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+// byte j of v as a float (the integer sits in the low mantissa bits of 2^23); j may be a lane value
+__device__ __forceinline__ float rw_byte(uint32_t v, int j, float minus = 8388608.f) {
+  return __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7440u + j)) - minus;
+}
+__device__ __forceinline__ uint32_t rw_lds(const uint8_t* p) { return *reinterpret_cast<const uint32_t*>(p); }
+
+// One unit of work: sixteen weight rows (this lane: r0 = row g, r1 = row g + 8) x one superblock, all activation rows.
+// xb: this lane's activation row (nt = 0) at the superblock; sums: the stage's sums at the superblock.
+template <int C, typename XT, int NT>
+struct RowsUnit {
+  static constexpr bool kBf = std::is_same<XT, __nv_bfloat16>::value;
+  static constexpr uint32_t kMagic = kBf ? 0x37373737u : 0u;
+  static constexpr float kUp = 16777216.f;                     // operands are scaled by 2^-24
+  static constexpr float kSumUp = kBf ? 16777216.f : 1.f;      // and so are the sums of bf16 rows
+  static constexpr int kBase = rw_base<C, kBf>();
+  static constexpr int kP = rw_sum_pitch(C);
+
+  // y += d * (up * acc - base * sum_j sc_j xs_j) - dmin * sum_j mn_j xs_j
+  static __device__ __forceinline__ void finish(float (&y)[NT][4], const float (&acc)[NT][4], float d0, float d1) {
+#pragma unroll
+    for (int n = 0; n < NT; n++) {
+      y[n][0] = fmaf(d0 * kUp, acc[n][0], y[n][0]);
+      y[n][1] = fmaf(d0 * kUp, acc[n][1], y[n][1]);
+      y[n][2] = fmaf(d1 * kUp, acc[n][2], y[n][2]);
+      y[n][3] = fmaf(d1 * kUp, acc[n][3], y[n][3]);
+    }
+  }
+  // y += f * sum_j a_j xs_j over the NS sub-blocks; a: coefficients of this lane's (row, sub-block) operand places
+  template <int NS>
+  static __device__ __forceinline__ void sum_term(float (&y)[NT][4], const float (&a)[NS / 8][4], const float* sums,
+                                                  int g, int t, float f0, float f1) {
+#pragma unroll
+    for (int n = 0; n < NT; n++) {
+      const float* s = sums + (n * 8 + g) * kP + t;
+      float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int i = 0; i < NS / 8; i++) {
+        rw_mma_tf32(c, a[i], s[8 * i], s[8 * i + 4]);
+        rw_mma_tf32(c, a[i], s[NS + 8 * i], s[NS + 8 * i + 4]);
+      }
+      y[n][0] = fmaf(f0, c[0], y[n][0]);
+      y[n][1] = fmaf(f0, c[1], y[n][1]);
+      y[n][2] = fmaf(f1, c[2], y[n][2]);
+      y[n][3] = fmaf(f1, c[3], y[n][3]);
+    }
+  }
+  // four weights of either row (one byte each) against b[n] = four activations of column n
+  static __device__ __forceinline__ void four(float (&c)[NT][4], uint32_t qa, uint32_t qb, const uint32_t (&b)[NT][2]) {
+    const uint32_t a0 = __byte_perm(qa, kMagic, 0x4140), a2 = __byte_perm(qa, kMagic, 0x4342);
+    const uint32_t a1 = __byte_perm(qb, kMagic, 0x4140), a3 = __byte_perm(qb, kMagic, 0x4342);
+#pragma unroll
+    for (int n = 0; n < NT; n++) rw_mma(c[n], a0, a1, a2, a3, b[n][0], b[n][1], XT());
+  }
+  static __device__ __forceinline__ void scale_add(float (&acc)[NT][4], const float (&c)[NT][4], float s0, float s1) {
+#pragma unroll
+    for (int n = 0; n < NT; n++) {
+      acc[n][0] = fmaf(s0, c[n][0], acc[n][0]);
+      acc[n][1] = fmaf(s0, c[n][1], acc[n][1]);
+      acc[n][2] = fmaf(s1, c[n][2], acc[n][2]);
+      acc[n][3] = fmaf(s1, c[n][3], acc[n][3]);
+    }
+  }
+
+  // q4_k / q5_k: 32 quant bytes hold sub-blocks 2 p (low nibbles) and 2 p + 1 (high); a lane takes bytes 8 t .. 8 t + 7
+  static __device__ __forceinline__ void run_k4(float (&y)[NT][4], const uint8_t* r0, const uint8_t* r1,
+                                                const uint8_t* (&xb)[NT], const float* sums, int g, int t) {
+    const uint4 h0 = *reinterpret_cast<const uint4*>(r0), h1 = *reinterpret_cast<const uint4*>(r1);
+    const StScales s0 = st_unpack(h0), s1 = st_unpack(h1);
+    constexpr int kQs = C == Q5_K ? 48 : 16;
+    uint2 u0 = make_uint2(0u, 0u), u1 = u0;  // q5_k: bit j of byte l is the fifth bit of weight l of sub-block j
+    if constexpr (C == Q5_K) {
+      u0 = *reinterpret_cast<const uint2*>(r0 + 16 + 8 * t);
+      u1 = *reinterpret_cast<const uint2*>(r1 + 16 + 8 * t);
+    }
+    float acc[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; n++) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+      const uint2 wa = *reinterpret_cast<const uint2*>(r0 + kQs + 32 * p + 8 * t);
+      const uint2 wb = *reinterpret_cast<const uint2*>(r1 + kQs + 32 * p + 8 * t);
+#pragma unroll
+      for (int hi = 0; hi < 2; hi++) {
+        const int j = 2 * p + hi;
+        uint32_t b0[NT][2], b1[NT][2];
+#pragma unroll
+        for (int n = 0; n < NT; n++) {
+          const uint4 b = *reinterpret_cast<const uint4*>(xb[n] + 64 * j + 16 * t);
+          b0[n][0] = b.x, b0[n][1] = b.y, b1[n][0] = b.z, b1[n][1] = b.w;
+        }
+        auto nib = [&](uint32_t w, uint32_t u) {
+          uint32_t q = (hi ? w >> 4 : w) & 0x0f0f0f0fu;
+          if constexpr (C == Q5_K) q |= (j <= 4 ? u << (4 - j) : u >> (j - 4)) & 0x10101010u;
+          return q;
+        };
+        float c[NT][4];
+#pragma unroll
+        for (int n = 0; n < NT; n++) c[n][0] = c[n][1] = c[n][2] = c[n][3] = 0.f;
+        four(c, nib(wa.x, u0.x), nib(wb.x, u1.x), b0);
+        four(c, nib(wa.y, u0.y), nib(wb.y, u1.y), b1);
+        scale_add(acc, c, rw_byte(p < 2 ? s0.scl : s0.sch, j & 3), rw_byte(p < 2 ? s1.scl : s1.sch, j & 3));
+      }
+    }
+    const float2 dd0 = __half22float2(*reinterpret_cast<const __half2*>(&h0.x));  // (d, dmin)
+    const float2 dd1 = __half22float2(*reinterpret_cast<const __half2*>(&h1.x));
+    finish(y, acc, dd0.x, dd1.x);
+    const float m[1][4] = {{rw_byte(s0.mnl, t), rw_byte(s1.mnl, t), rw_byte(s0.mnh, t), rw_byte(s1.mnh, t)}};
+    sum_term<8>(y, m, sums, g, t, -kSumUp * dd0.y, -kSumUp * dd1.y);
+    if constexpr (kBase != 0) {
+      const float s[1][4] = {{rw_byte(s0.scl, t), rw_byte(s1.scl, t), rw_byte(s0.sch, t), rw_byte(s1.sch, t)}};
+      sum_term<8>(y, s, sums, g, t, -kSumUp * kBase * dd0.x, -kSumUp * kBase * dd1.x);
+    }
+  }
+
+  // q6_k (src/kquant_cpu_decode.cpp:238-280): sub-block j = 8 h + 2 quarter + s of sixteen weights is one instruction.
+  // PH: the block starts two bytes past a multiple of four. The aligned words around a group of sixteen bytes then
+  // are bytes 2 + 4 t .. 5 + 4 t for t < 3, and for t = 3 bytes 14, 15 and the first two of the next group: lane 3
+  // takes bytes 0, 1 (from the word before) and 14, 15.
+  template <int PH>
+  static __device__ __forceinline__ void run_q6(float (&y)[NT][4], const uint8_t* r0, const uint8_t* r1,
+                                                const uint8_t* (&xb)[NT], const float* sums, int g, int t) {
+    float acc[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; n++) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+    const uint32_t sel = t == 3 ? 0x5432u : 0x7654u;
+    const int xo0 = PH ? (t == 3 ? 0 : 4 + 8 * t) : 8 * t, xo1 = PH ? (t == 3 ? 28 : 8 + 8 * t) : 0;
+    uint32_t sc0[4], sc1[4];  // the sixteen signed scales of either row, biased by 128
+    {
+      if constexpr (PH == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) sc0[i] = rw_lds(r0 + 192 + 4 * i) ^ 0x80808080u, sc1[i] = rw_lds(r1 + 192 + 4 * i) ^ 0x80808080u;
+      } else {
+        uint32_t a[5], b[5];
+#pragma unroll
+        for (int i = 0; i < 5; i++) a[i] = rw_lds(r0 + 190 + 4 * i), b[i] = rw_lds(r1 + 190 + 4 * i);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          sc0[i] = __byte_perm(a[i], a[i + 1], 0x5432) ^ 0x80808080u;
+          sc1[i] = __byte_perm(b[i], b[i + 1], 0x5432) ^ 0x80808080u;
+        }
+      }
+    }
+    auto group = [&](const uint8_t* p, uint32_t& prev) {  // this lane's four bytes of the sixteen at p
+      if constexpr (PH == 0) {
+        return rw_lds(p + 4 * t);
+      } else {
+        const uint32_t w = rw_lds(p + 2 + 4 * t);
+        const uint32_t r = __byte_perm(prev, w, sel);
+        prev = w;
+        return r;
+      }
+    };
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      uint32_t L[2][4], H[2][2];
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        const uint8_t* p = r ? r1 : r0;
+        uint32_t pl = 0u, ph = 0u;
+        if constexpr (PH) {
+          const int po = t == 3 ? -2 : 2;  // only lane 3 uses it
+          pl = rw_lds(p + 64 * h + po);
+          ph = rw_lds(p + 128 + 32 * h + po);
+        }
+#pragma unroll
+        for (int s = 0; s < 4; s++) L[r][s] = group(p + 64 * h + 16 * s, pl);
+#pragma unroll
+        for (int s = 0; s < 2; s++) H[r][s] = group(p + 128 + 32 * h + 16 * s, ph);
+      }
+#pragma unroll
+      for (int s = 0; s < 2; s++) {
+#pragma unroll
+        for (int qd = 0; qd < 4; qd++) {
+          const int j = 8 * h + 2 * qd + s;
+          uint32_t q[2];
+#pragma unroll
+          for (int r = 0; r < 2; r++) {
+            const uint32_t l = L[r][2 * (qd & 1) + s], u = H[r][s];
+            const uint32_t hb = qd == 0 ? u << 4 : (qd == 1 ? u << 2 : (qd == 2 ? u : u >> 2));
+            q[r] = ((qd & 2 ? l >> 4 : l) & 0x0f0f0f0fu) | (hb & 0x30303030u);
+          }
+          uint32_t b[NT][2];
+#pragma unroll
+          for (int n = 0; n < NT; n++) {
+            if constexpr (PH == 0) {
+              const uint2 v = *reinterpret_cast<const uint2*>(xb[n] + 32 * j + xo0);
+              b[n][0] = v.x, b[n][1] = v.y;
+            } else {
+              b[n][0] = rw_lds(xb[n] + 32 * j + xo0);
+              b[n][1] = rw_lds(xb[n] + 32 * j + xo1);
+            }
+          }
+          float c[NT][4];
+#pragma unroll
+          for (int n = 0; n < NT; n++) c[n][0] = c[n][1] = c[n][2] = c[n][3] = 0.f;
+          four(c, q[0], q[1], b);
+          scale_add(acc, c, rw_byte(sc0[j >> 2], j & 3, 8388736.f), rw_byte(sc1[j >> 2], j & 3, 8388736.f));
+        }
+      }
+    }
+    const float d0 = __half2float(*reinterpret_cast<const __half*>(r0 + 208));
+    const float d1 = __half2float(*reinterpret_cast<const __half*>(r1 + 208));
+    finish(y, acc, d0, d1);
+    float s[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      s[i][0] = rw_byte(sc0[2 * i], t, 8388736.f), s[i][1] = rw_byte(sc1[2 * i], t, 8388736.f);
+      s[i][2] = rw_byte(sc0[2 * i + 1], t, 8388736.f), s[i][3] = rw_byte(sc1[2 * i + 1], t, 8388736.f);
+    }
+    sum_term<16>(y, s, sums, g, t, -kSumUp * kBase * d0, -kSumUp * kBase * d1);
+  }
+
+  static __device__ __forceinline__ void run(float (&y)[NT][4], const uint8_t* r0, const uint8_t* r1,
+                                             const uint8_t* (&xb)[NT], const float* sums, int g, int t) {
+    if constexpr (C == Q6_K) {
+      if ((smem_u32(r0) & 2) == 0) run_q6<0>(y, r0, r1, xb, sums, g, t);
+      else run_q6<1>(y, r0, r1, xb, sums, g, t);
+    } else {
+      run_k4(y, r0, r1, xb, sums, g, t);
+    }
+  }
+};
+
+// The sums of one superblock's sub-blocks for eight activation rows (columns), by ones x activations; lanes 0..3 hold
+// columns 2 t, 2 t + 1 and store them as a tf32 head and the rest.
+template <int C, typename XT>
+__device__ __forceinline__ void rows_sums(const uint8_t* xrow, float* out, int lane) {
+  constexpr int NS = rw_nsub(C), P = rw_sum_pitch(C);
+  constexpr uint32_t one = std::is_same<XT, __half>::value ? 0x3C003C00u : 0x33803380u;
+  const int t = lane & 3;
+  uint2 b[16];  // all loads before the first store: the compiler cannot tell that they do not overlap
+#pragma unroll
+  for (int i = 0; i < 16; i++) {
+    if constexpr (NS == 8) {
+      if (i & 1) continue;
+      const uint4 v = *reinterpret_cast<const uint4*>(xrow + 32 * i + 16 * t);
+      b[i] = make_uint2(v.x, v.y), b[i + 1] = make_uint2(v.z, v.w);
+    } else {
+      b[i] = *reinterpret_cast<const uint2*>(xrow + 32 * i + 8 * t);
+    }
+  }
+  float c[NS][4];
+#pragma unroll
+  for (int j = 0; j < NS; j++) {
+    c[j][0] = c[j][1] = c[j][2] = c[j][3] = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16 / NS; i++) rw_mma(c[j], one, one, one, one, b[j * (16 / NS) + i].x, b[j * (16 / NS) + i].y, XT());
+  }
+  if (lane < 4) {
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      float* o = out + (2 * t + i) * P;
+#pragma unroll
+      for (int j = 0; j < NS; j += 4) {
+        float4 h, l;
+        float* hp = &h.x;
+        float* lp = &l.x;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          hp[q] = __uint_as_float(__float_as_uint(c[j + q][i]) & 0xffffe000u);
+          lp[q] = c[j + q][i] - hp[q];
+        }
+        *reinterpret_cast<float4*>(o + j) = h;
+        *reinterpret_cast<float4*>(o + NS + j) = l;
+      }
+    }
+  }
+}
+
+constexpr int kRwWarps = 16;  // consumer warps
+
+template <int C, typename XT, int NT>
+__global__ void __launch_bounds__(32 * (kRwWarps + kRwHelpers + kRwProducers), 1)
+rows_kernel(const GemvArgs a, const RowsPlan pl, int* __restrict__ error_word) {
+  constexpr int NW = kRwWarps, BPB = bpb_of(C);
+  constexpr bool kBf = std::is_same<XT, __nv_bfloat16>::value;
+  constexpr bool kSums = rw_sums<C, kBf>();
+  extern __shared__ __align__(128) uint8_t rw_dyn[];
+  __shared__ uint64_t full[kRwMaxStages], ready[kRwMaxStages], empty[kRwMaxStages];
+  __shared__ int abort_s;
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int S = pl.stages, M = a.M;
+  const int nsb = a.K >> 8, nst = (nsb + pl.cs - 1) / pl.cs;
+  const int live = pl.rt * pl.wk;  // consumer warps with work
+  if (threadIdx.x == 0) {
+    abort_s = 0;
+    for (int s = 0; s < S; s++) {
+      mbar_init(&full[s], 32 * kRwProducers);
+      mbar_init(&ready[s], kRwHelpers);
+      mbar_init(&empty[s], live + (kSums ? kRwHelpers : 0));
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  __syncthreads();
+  volatile int* abort_flag = &abort_s;
+  auto wait = [&](uint64_t* bar, int parity) { return mbar_wait_err(bar, parity, abort_flag, 0x100, error_word); };
+
+  if (warp >= NW + kRwHelpers) {
+    // ================= producers =================
+    const int pw = warp - NW - kRwHelpers;
+    const int my_blocks = (pl.n_blocks - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;
+    const int total = my_blocks * nst;
+    const uint8_t* wend = a.w + (long long)a.N * a.row_bytes;
+    int blk_w = blockIdx.x, st_w = 0, slot_w = 0, st_x = 0, slot_x = 0;
+    // Pieces of sixteen bytes, piece q of a stage: row q / per_row, place q % per_row. A thread takes every 128th:
+    // both numbers advance by a constant, no division in the loop.
+    const int tid = pw * 32 + lane;
+    constexpr int kThreads = 32 * kRwProducers;
+    auto copy_w = [&]() {
+      const int row0 = blk_w * pl.R, rows = min(pl.R, a.N - row0), len = min(pl.cs, nsb - st_w * pl.cs) * BPB;
+      const uint32_t dst = smem_u32(rw_dyn + slot_w * pl.stage_bytes);
+      const uint8_t* src = a.w + (long long)row0 * a.row_bytes + (long long)st_w * pl.cs * BPB;
+      const int rb = (int)a.row_bytes;
+      const int per_row = rw_al16(C) ? len >> 4 : (len + 30) >> 4;  // a window holds at most that many
+      const int dr = kThreads / per_row, dc = kThreads - dr * per_row;
+      int r = tid / per_row, c = tid - r * per_row;
+      if constexpr (rw_al16(C)) {
+        const int n = rows * per_row;
+#pragma unroll 4
+        for (int q = tid; q < n; q += kThreads) {
+          rw_cp16(dst + r * pl.wpitch + 16 * c, src + ((long long)r * rb + 16 * c));
+          r += dr, c += dc;
+          if (c >= per_row) c -= per_row, r++;
+        }
+      } else {  // the aligned window around the row's bytes; the matrix may end inside it
+        const int n = rows * per_row;
+#pragma unroll 4
+        for (int q = tid; q < n; q += kThreads) {
+          const uint8_t* p = src + (long long)r * rb;
+          const int ph = (int)(reinterpret_cast<uintptr_t>(p) & 15);
+          p += 16 * c - ph;
+          if (16 * c < len + ph) {
+            const long long left = wend - p;
+            rw_cp16_upto(dst + r * pl.wpitch + 16 * c, p, left < 16 ? (int)left : 16);
+          }
+          r += dr, c += dc;
+          if (c >= per_row) c -= per_row, r++;
+        }
+      }
+      if (++st_w == nst) st_w = 0, blk_w += gridDim.x;
+      if (++slot_w == S) slot_w = 0;
+    };
+    auto copy_x = [&]() {  // and the arrival of this thread once all its copies of the stage have landed
+      const int per_row = min(pl.cs, nsb - st_x * pl.cs) * 32;
+      const uint32_t dst = smem_u32(rw_dyn + slot_x * pl.stage_bytes + pl.x_off);
+      const XT* src = static_cast<const XT*>(a.x) + st_x * pl.cs * 256;
+      const int dr = kThreads / per_row, dc = kThreads - dr * per_row;
+      int r = tid / per_row, c = tid - r * per_row;
+#pragma unroll 4
+      for (int q = tid; q < M * per_row; q += kThreads) {
+        rw_cp16(dst + r * pl.xpitch + 16 * c, src + ((long long)r * a.x_row_stride + 8 * c));
+        r += dr, c += dc;
+        if (c >= per_row) c -= per_row, r++;
+      }
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(smem_u32(&full[slot_x])) : "memory");
+      if (++st_x == nst) st_x = 0;
+      if (++slot_x == S) slot_x = 0;
+    };
+    const int first = min(S, total);
+    for (int i = 0; i < first; i++) copy_w();
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the activations may come from the kernel before this one
+    for (int i = 0; i < first; i++) copy_x();
+    int parity = 0;
+    for (int i = first; i < total; i++) {
+      if (!wait(&empty[slot_w], parity)) break;
+      if (slot_w == S - 1) parity ^= 1;
+      copy_w();
+      copy_x();
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+  } else if (warp >= NW) {
+    // ================= helpers: the stage's activation sums =================
+    if constexpr (kSums) {
+      const int my_blocks = (pl.n_blocks - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;
+      int s = 0, parity = 0, st = 0;
+      for (int i = 0; i < my_blocks * nst; i++) {
+        const int here = min(pl.cs, nsb - st * pl.cs);
+        if (!wait(&full[s], parity)) break;
+        const uint8_t* xs = rw_dyn + (long long)s * pl.stage_bytes + pl.x_off;
+        float* sums = reinterpret_cast<float*>(rw_dyn + (long long)s * pl.stage_bytes + pl.sum_off);
+        for (int e = warp - NW; e < here * NT; e += kRwHelpers) {
+          const int k = e / NT, n = e % NT;
+          rows_sums<C, XT>(xs + min(8 * n + (lane >> 2), M - 1) * pl.xpitch + 512 * k,
+                           sums + (k * NT + n) * 8 * rw_sum_pitch(C), lane);
+        }
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(&ready[s]);
+          mbar_arrive(&empty[s]);
+        }
+        if (++st == nst) st = 0;
+        if (++s == S) s = 0, parity ^= 1;
+      }
+    }
+  } else if (warp < live) {
+    // ================= consumers: warp = (row tile, superblock of the stage) =================
+    const int tile = warp % pl.rt, ks = warp / pl.rt;
+    const int g = lane >> 2, t = lane & 3;
+    float* red = reinterpret_cast<float*>(rw_dyn + pl.red_off);
+    constexpr int kRedPitch = 8 * NT + 2;
+    bool ok = true;
+    int s = 0, parity = 0;
+    for (int blk = blockIdx.x; blk < pl.n_blocks; blk += gridDim.x) {
+      const int row0 = blk * pl.R, rows = min(pl.R, a.N - row0);
+      const int l0 = min(16 * tile + g, rows - 1), l1 = min(16 * tile + g + 8, rows - 1);
+      float y[NT][4];
+#pragma unroll
+      for (int n = 0; n < NT; n++) y[n][0] = y[n][1] = y[n][2] = y[n][3] = 0.f;
+      for (int st = 0; st < nst; st++) {
+        if (ok) ok = wait(kSums ? &ready[s] : &full[s], parity);
+        const uint8_t* base = rw_dyn + s * pl.stage_bytes;
+        const int here = ok ? min(pl.cs, nsb - st * pl.cs) : 0;
+        for (int k = ks; k < here; k += pl.wk) {
+          const uint8_t *r0 = base + l0 * pl.wpitch + k * BPB, *r1 = base + l1 * pl.wpitch + k * BPB;
+          if constexpr (!rw_al16(C)) {  // the bytes of a row start at their offset within a 16-byte word
+            const long long o0 = (long long)(row0 + l0) * a.row_bytes + (long long)st * pl.cs * BPB;
+            const long long o1 = (long long)(row0 + l1) * a.row_bytes + (long long)st * pl.cs * BPB;
+            r0 += (int)(o0 & 15), r1 += (int)(o1 & 15);
+          }
+          const uint8_t* xb[NT];
+#pragma unroll
+          for (int n = 0; n < NT; n++) xb[n] = base + pl.x_off + min(8 * n + g, M - 1) * pl.xpitch + 512 * k;
+          const float* sums = reinterpret_cast<const float*>(base + pl.sum_off) + k * NT * 8 * rw_sum_pitch(C);
+          RowsUnit<C, XT, NT>::run(y, r0, r1, xb, sums, g, t);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[s]);
+        if (++s == S) s = 0, parity ^= 1;
+      }
+      // the superblock columns of a row meet in shared memory, in a fixed order
+      float* mine = red + (long long)(ks * pl.rt * 16 + 16 * tile + g) * kRedPitch + 2 * t;
+#pragma unroll
+      for (int n = 0; n < NT; n++) {
+        *reinterpret_cast<float2*>(mine + 8 * n) = make_float2(y[n][0], y[n][1]);
+        *reinterpret_cast<float2*>(mine + 8 * kRedPitch + 8 * n) = make_float2(y[n][2], y[n][3]);
+      }
+      asm volatile("bar.sync 1, %0;\n" ::"r"(live * 32) : "memory");
+      if (ok) {
+        const int rp = pl.rt * 16;
+        for (int e = threadIdx.x; e < rp * M; e += live * 32) {
+          const int r = e % rp, m = e / rp;
+          if (r < rows) {
+            float v = 0.f;
+            for (int k = 0; k < pl.wk; k++) v += red[(long long)(k * rp + r) * kRedPitch + m];
+            if (a.row_scale != nullptr) v *= a.row_scale[m];
+            const long long o = (long long)m * a.y_row_stride + row0 + r;
+            if (kBf || a.out_bf16) static_cast<__nv_bfloat16*>(a.y)[o] = __float2bfloat16_rn(v);
+            else static_cast<__half*>(a.y)[o] = __float2half_rn(v);
+          }
+        }
+      }
+      asm volatile("bar.sync 1, %0;\n" ::"r"(live * 32) : "memory");
+    }
+  }
+}
+
+int rows_sm_count() {
+  static int sms[16] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 16) return 0;
+  if (sms[dev] == 0) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 0;
+    sms[dev] = n;
+  }
+  return sms[dev];
+}
+
+// Row blocks as even as the SM count allows, one per SM and pass; a stage as deep as the warps left over by the
+// row tiles can take, shortened until three stages (or all of K) fit shared memory.
+template <int C, bool BF, int NT>
+bool rows_plan(const GemvArgs& a, RowsPlan& p) {
+  constexpr int NW = kRwWarps, BPB = bpb_of(C);
+  const int sms = rows_sm_count();
+  if (sms <= 0) return false;
+  const int nsb = a.K >> 8;
+  const int passes = (a.N + sms * 16 * NW - 1) / (sms * 16 * NW);
+  p.R = std::max(8, (a.N + sms * passes - 1) / (sms * passes));
+  p.n_blocks = (a.N + p.R - 1) / p.R;
+  p.rt = (p.R + 15) / 16;
+  p.wk = std::min(NW / p.rt, nsb);
+  for (p.cs = std::min(2 * p.wk, nsb); p.cs >= 1; p.cs--) {
+    p.wk = std::min(p.wk, p.cs);
+    int wb = p.cs * BPB;
+    if (!rw_al16(C)) wb = (wb + 30 + 15) & ~15;
+    // 8-byte reads of four rows, or 4-byte reads of eight, in different banks
+    while (rw_al16(C) ? (wb & 63) != 32 : (wb & 31) != 16) wb += 16;
+    p.wpitch = wb;
+    p.xpitch = p.cs * 512 + (rw_nsub(C) == 8 ? 64 : 32);
+    p.x_off = (p.R * p.wpitch + 127) & ~127;
+    p.sum_off = (p.x_off + a.M * p.xpitch + 15) & ~15;
+    p.stage_bytes = (p.sum_off + (rw_sums<C, BF>() ? p.cs * NT * 8 * rw_sum_pitch(C) * 4 : 0) + 127) & ~127;
+    const int red = p.wk * p.rt * 16 * (8 * NT + 2) * 4;
+    const int nst = (nsb + p.cs - 1) / p.cs * ((p.n_blocks + sms - 1) / sms);
+    p.stages = std::min({kRwMaxStages, nst, (kRwMaxSmem - red) / p.stage_bytes});
+    if (p.stages >= std::min(3, nst)) {
+      p.red_off = p.stages * p.stage_bytes;
+      p.smem = p.red_off + red;
+      return true;
+    }
+  }
+  return false;
+}
+
+template <int C, typename XT, int NT>
+cudaError_t launch_rows_nt(const GemvArgs& a, cudaStream_t st) {
+  RowsPlan p;
+  if (!rows_plan<C, std::is_same<XT, __nv_bfloat16>::value, NT>(a, p)) return cudaErrorInvalidConfiguration;
+  static bool attr_set[16] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 16) return cudaErrorInvalidDevice;
+  if (!attr_set[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(rows_kernel<C, XT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRwMaxSmem);
+    if (e != cudaSuccess) return e;
+    attr_set[dev] = true;
+  }
+  int* err = device_error_word();
+  if (err == nullptr) return cudaErrorUnknown;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(std::min(p.n_blocks, rows_sm_count()), 1, 1);
+  cfg.blockDim = dim3(32 * (kRwWarps + kRwHelpers + kRwProducers));
+  cfg.dynamicSmemBytes = p.smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  static const bool no_pdl = std::getenv("KQ_NO_PDL") != nullptr;  // A/B lever
+  cfg.numAttrs = no_pdl ? 0 : 1;
+  return cudaLaunchKernelEx(&cfg, rows_kernel<C, XT, NT>, a, p, err);
+}
+
+template <int C, typename XT>
+cudaError_t launch_rows_c(const GemvArgs& a, cudaStream_t st) {
+  if (a.M <= 8) return launch_rows_nt<C, XT, 1>(a, st);
+  return launch_rows_nt<C, XT, 2>(a, st);
+}
+
+}  // namespace
+
+bool gemv_rows_supported(int codec, int x_dtype, const GemvArgs& a) {
+  if (codec != Q4_K && codec != Q5_K && codec != Q6_K) return false;
+  if (!(x_dtype == F16 || x_dtype == BF16) || a.tasks != nullptr || a.bias != nullptr || a.M < 1 || a.M > 16 || a.N < 8 ||
+      a.K < 256 || (a.K & 255) != 0 || a.w_align16 == 0 || a.row_bytes != (long long)(a.K >> 8) * bpb_of(codec))
+    return false;
+  // q6_k: every row starts on the same phase modulo four
+  if (codec == Q6_K && (a.row_bytes & 3) != 0) return false;
+  return (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && (a.x_row_stride & 7) == 0;
+}
+
+cudaError_t launch_gemv_rows(int codec, int x_dtype, const GemvArgs& a, cudaStream_t st) {
+  if (x_dtype == F16) {
+    switch (codec) {
+      case Q4_K: return launch_rows_c<Q4_K, __half>(a, st);
+      case Q5_K: return launch_rows_c<Q5_K, __half>(a, st);
+      case Q6_K: return launch_rows_c<Q6_K, __half>(a, st);
+    }
+  } else {
+    switch (codec) {
+      case Q4_K: return launch_rows_c<Q4_K, __nv_bfloat16>(a, st);
+      case Q5_K: return launch_rows_c<Q5_K, __nv_bfloat16>(a, st);
+      case Q6_K: return launch_rows_c<Q6_K, __nv_bfloat16>(a, st);
+    }
+  }
+  return cudaErrorInvalidValue;
+}
+
+}  // namespace kq

@@ -1,0 +1,56 @@
+"""Two to sixteen rows of q4_k, q5_k and q6_k (kq_rows.cu) against float64 products of the oracle's weights."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import x_to_torch, y_to_f32
+from oracle.kq_oracle import Oracle
+
+pytestmark = pytest.mark.gpu
+
+# (m, n, k): row tiles and row blocks with remainders, one superblock, stages with remainders, rows of q6_k that do
+# not start on 16-byte boundaries and a matrix whose last byte does not end on one (k = 512 * odd, odd n), more rows
+# than one pass of the SMs holds, both column tiles
+SHAPES = [(2, 8, 512), (3, 333, 512), (8, 2049, 1536), (9, 257, 1024), (16, 40, 4096), (5, 4099, 2560), (12, 3000, 512),
+          (2, 38000, 512)]
+
+
+def _rel(y, ref, out_eps):
+    """Relative Frobenius error after the one rounding of the output (uniform in half a unit: eps / sqrt 3 at most)."""
+    err = np.linalg.norm(y - ref) / np.linalg.norm(ref)
+    assert err < out_eps / np.sqrt(3) + 2e-5, err
+
+
+@pytest.mark.parametrize("codec", ["q4_k", "q5_k", "q6_k"])
+@pytest.mark.parametrize("dt", ["f16", "bf16", "f32"])
+@pytest.mark.parametrize("m,n,k", SHAPES)
+def test_rows_against_float64(codec, dt, m, n, k):
+    import mlx_kquant_b200 as kq
+
+    rng = np.random.default_rng(m * 1000003 + n * 101 + k)
+    some = rng.standard_normal((min(n, 64), k)).astype(np.float32) * 0.05
+    wire = kq.quantize(torch.from_numpy(some), codec)[0].numpy()
+    wire = wire[rng.integers(0, len(wire), n)]
+    x_f32 = rng.standard_normal((m, k)).astype(np.float32)
+    x_f32[0] *= 1e-3
+    x_f32[-1] *= 300.0
+    x, _ = x_to_torch(x_f32, dt)
+    xr = (x.bfloat16() if dt == "f32" else x).double().cpu().numpy()
+    ref = xr @ Oracle().dequantize(wire, codec, "f32").astype(np.float64).T
+    w = torch.from_numpy(wire).cuda()
+    y = y_to_f32(kq.quantized_matmul(x, w, None, codec)).astype(np.float64)
+    for r in range(m):  # rows of very different magnitude
+        _rel(y[r], ref[r], 2.0 ** -11 if dt == "f16" else 2.0 ** -8)
+
+
+def test_rows_largest_finite_bf16():
+    """Rows near the largest bf16 number: the operands' power of two keeps every partial sum finite."""
+    import mlx_kquant_b200 as kq
+
+    rng = np.random.default_rng(5)
+    for codec in ("q4_k", "q6_k"):
+        w = kq.quantize(torch.from_numpy(rng.standard_normal((64, 512)).astype(np.float32) * 1e-3), codec)[0]
+        x = (torch.from_numpy(rng.standard_normal((4, 512))).clamp(-3, 3) * 1e38).bfloat16()
+        ref = x.double().numpy() @ Oracle().dequantize(w.numpy(), codec, "f32").astype(np.float64).T
+        y = kq.quantized_matmul(x.cuda(), w.cuda(), None, codec).double().cpu().numpy()
+        _rel(y, ref, 2.0 ** -8)
