@@ -4,9 +4,13 @@ from __future__ import annotations
 import numpy as np
 import torch
 
+import mlx_kquant_b200 as kq
 from oracle import kq_oracle
 from oracle.kq_oracle import GEOMETRY
 
+# codecs with a host encoder in this package
+HOST_ENCODED = {"q2_k", "q3_k", "q4_k", "q5_k", "q6_k", "q4_0", "q4_1", "q5_0", "q5_1", "q8_0", "iq4_nl", "iq4_xs",
+                "iq2_xxs"}
 TORCH_DT = {"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16}
 
 
@@ -44,9 +48,13 @@ synthetic_wire = kq_oracle.synthetic_wire
 def mint_wire(codec: str, W: np.ndarray, imatrix=None) -> np.ndarray:
     """Really-encoded wire bytes from the reference encoder when its library is
     present (and the codec has an encoder: mxfp4 / nvfp4 are decode-only in the
-    reference, src/kquant_codec.cpp:33-34), else synthetic valid bytes of the same shape."""
+    reference, src/kquant_codec.cpp:33-34), else from this package's host encoder (byte-identical with it,
+    tests/test_quantize.py), else synthetic valid bytes of the same shape."""
     if kq_oracle.Ref.available() and codec not in kq_oracle.DECODE_ONLY:
         if imatrix is None and GEOMETRY[codec][3]:
             imatrix = np.ones(W.shape[-1], np.float32)
         return kq_oracle.Ref().quantize(W, codec, imatrix)
+    if codec in HOST_ENCODED:
+        im = torch.from_numpy(imatrix) if imatrix is not None else (torch.ones(W.shape[-1]) if GEOMETRY[codec][3] else None)
+        return kq.quantize(torch.from_numpy(np.ascontiguousarray(W, np.float32)), codec, im)[0].numpy()
     return synthetic_wire(codec, W.shape[0], W.shape[1], seed=int(abs(W[0, 0]) * 1e6) % 9973)
