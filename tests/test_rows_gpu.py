@@ -15,10 +15,11 @@ SHAPES = [(2, 8, 512), (3, 333, 512), (8, 2049, 1536), (9, 257, 1024), (16, 40, 
           (2, 38000, 512)]
 
 
-def _rel(y, ref, out_eps):
-    """Relative Frobenius error after the one rounding of the output (uniform in half a unit: eps / sqrt 3 at most)."""
-    err = np.linalg.norm(y - ref) / np.linalg.norm(ref)
-    assert err < out_eps / np.sqrt(3) + 2e-5, err
+def _close(y, ref, out_eps):
+    """Every output within half a unit of the output type (out_eps, relative; at least the 2^-25 of fp16 subnormals)
+    plus the sums in float32: 2e-5 of the outputs' root mean square, some hundred units of float32."""
+    off = np.abs(y - ref) - np.maximum(out_eps * np.abs(ref), 2.0 ** -25)
+    assert off.max() < 2e-5 * np.sqrt(np.mean(ref ** 2)), off.max()
 
 
 @pytest.mark.parametrize("codec", ["q4_k", "q5_k", "q6_k"])
@@ -40,7 +41,7 @@ def test_rows_against_float64(codec, dt, m, n, k):
     w = torch.from_numpy(wire).cuda()
     y = y_to_f32(kq.quantized_matmul(x, w, None, codec)).astype(np.float64)
     for r in range(m):  # rows of very different magnitude
-        _rel(y[r], ref[r], 2.0 ** -11 if dt == "f16" else 2.0 ** -8)
+        _close(y[r], ref[r], 2.0 ** -11 if dt == "f16" else 2.0 ** -8)
 
 
 def test_rows_largest_finite_bf16():
@@ -53,4 +54,4 @@ def test_rows_largest_finite_bf16():
         x = (torch.from_numpy(rng.standard_normal((4, 512))).clamp(-3, 3) * 1e38).bfloat16()
         ref = x.double().numpy() @ Oracle().dequantize(w.numpy(), codec, "f32").astype(np.float64).T
         y = kq.quantized_matmul(x.cuda(), w.cuda(), None, codec).double().cpu().numpy()
-        _rel(y, ref, 2.0 ** -8)
+        _close(y, ref, 2.0 ** -8)
