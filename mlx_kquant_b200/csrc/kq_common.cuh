@@ -447,4 +447,36 @@ __device__ __forceinline__ IqTables stage_iq_tables(uint8_t* smem, int tid, int 
   return t;
 }
 
+// The entries i of a gather call that multiply by matrix e, with an activation row in range, as (row of x, i) in the
+// order of i; all threads of the CTA take part, `count` (shared) starts at 0. n at most 4 * TH.
+template <int TH>
+__device__ __forceinline__ int collect_entries(const uint32_t* __restrict__ rhs, const uint32_t* __restrict__ lhs, int n,
+                                               long long x_batch, uint32_t e, int2* list, int* count) {
+  for (int i = threadIdx.x; i < n; i += TH) {
+    if (rhs[i] != e) continue;
+    const uint32_t l = lhs[i];
+    if ((long long)l < x_batch) list[atomicAdd(count, 1)] = make_int2((int)l, i);
+  }
+  __syncthreads();
+  const int c = *count;
+  int2 mine[4];
+  int rank[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {  // the atomics leave any order: a place is the number of smaller entries
+    const int at = threadIdx.x + q * TH;
+    rank[q] = -1;
+    if (at < c) {
+      mine[q] = list[at];
+      rank[q] = 0;
+      for (int j = 0; j < c; j++) rank[q] += list[j].y < mine[q].y;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+    if (rank[q] >= 0) list[rank[q]] = mine[q];
+  __syncthreads();
+  return c;
+}
+
 }  // namespace kq

@@ -366,6 +366,9 @@ cudaError_t launch_gather(int codec, int x_dtype, const void* x, long long x_bat
                           cudaStream_t st) {
   if (n_entries <= 0 || M <= 0) return cudaSuccess;
   const GatherLayout L = gather_layout(n_entries, M, n_experts, allow_grouped ? K : 0);
+  if (!L.grouped && gather_rows_supported(codec, x_dtype, x, M, K, w, expert_stride, row_bytes, N, n_entries, n_experts))
+    return launch_gather_rows(codec, x_dtype, x, x_batch, K, w, n_experts, expert_stride, row_bytes, N, lhs, rhs,
+                              n_entries, y, st);
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   int* counts = reinterpret_cast<int*>(ws + L.counts);
   int* cursor = reinterpret_cast<int*>(ws + L.cursor);

@@ -61,6 +61,13 @@ cudaError_t launch_gemv_dp4a(int codec, int x_dtype, const GemvArgs& a, cudaStre
 bool gemv_rows_supported(int codec, int x_dtype, const GemvArgs& a);
 cudaError_t launch_gemv_rows(int codec, int x_dtype, const GemvArgs& a, cudaStream_t st);
 
+// gather_qmm with one row per entry on the same kernel, up to 1024 entries.
+bool gather_rows_supported(int codec, int x_dtype, const void* x, int M, int K, const uint8_t* w, long long expert_stride,
+                           long long row_bytes, int N, long long n_entries, int n_experts);
+cudaError_t launch_gather_rows(int codec, int x_dtype, const void* x, long long x_batch, int K, const uint8_t* w,
+                               int n_experts, long long expert_stride, long long row_bytes, int N, const uint32_t* lhs,
+                               const uint32_t* rhs, long long n_entries, void* y, cudaStream_t st);
+
 // Prefill (M > 16) tile kernel on tcgen05 tensor cores with TMEM accumulators.
 // bf16 / f32 activations need gemm_workspace_bytes() of scratch for their fp16 copy.
 size_t gemm_workspace_bytes(int x_dtype, long long rows, int K);

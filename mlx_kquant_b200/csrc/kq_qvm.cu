@@ -10,6 +10,7 @@
 // further passes over the weights (grid.z): correct for any M, efficient for decode-sized M only.
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "kq_common.cuh"
@@ -124,10 +125,118 @@ qvm_kernel(const XT* __restrict__ x, long long x_row_stride, void* __restrict__ 
   cluster.sync();  // peers may still be reading this CTA's partial sums
 }
 
+// The gather form for calls whose entries share matrices (absorbed attention: every sequence multiplies by the head's
+// matrix): a CTA owns one matrix and 128 output columns, collects the matrix's entries from the index arrays by itself
+// and multiplies up to eight of them per pass over the weights, so a weight is decoded once for eight rows where the
+// kernel above decodes it for each. A warp's halves take two rows of W at a time, a lane eight columns; the partial
+// sums meet by one shuffle and in shared memory. Bound by the decode arithmetic and the latency of its byte loads;
+// 64 heads [128, 512] q6_k, eight rows each: 39.7 -> 6 us a launch.
+constexpr int kRowCols = 128, kRowM = 8;
+constexpr int kRowEntries = 512;  // every CTA looks through all entries
+template <int C, int A, typename XT>
+__global__ void __launch_bounds__(kThreads, 2)
+qvm_rows_kernel(const XT* __restrict__ x, void* __restrict__ y, const uint8_t* __restrict__ w, long long row_bytes,
+                int N, int K, QvmGather gq, int n_entries) {
+  using OT = typename std::conditional<std::is_same<XT, __half>::value, __half, __nv_bfloat16>::type;
+  constexpr int BPB = bpb_of(C), kChunk = 256;
+  constexpr bool kIq = (C == IQ4_NL || C == IQ4_XS || C == IQ2_XXS);
+  __shared__ __align__(16) float xs[kChunk][kRowM];          // activations of a K chunk
+  __shared__ float red[kWarps][kRowM][kRowCols];
+  __shared__ __align__(16) uint8_t s_tabs[kIq ? kIqSmemBytes : 16];
+  __shared__ int2 list[kRowEntries];                         // (row of x, row of y)
+  __shared__ int count_s;
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  IqTables tabs = global_iq_tables();
+  if constexpr (kIq) tabs = stage_iq_tables(s_tabs, threadIdx.x, kThreads);
+  if (threadIdx.x == 0) count_s = 0;
+  __syncthreads();
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  const uint32_t e = blockIdx.y;
+  const int count = collect_entries<kThreads>(gq.rhs, gq.lhs, n_entries, gq.x_batch, e, list, &count_s);
+  if (count == 0) return;
+  w += (long long)e * gq.expert_stride;
+
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4, oc = lane & 15;
+  const int c0 = blockIdx.x * kRowCols + 8 * oc;
+  const bool live = c0 < N;  // N is a whole number of blocks: eight columns exist or none
+  const long long blk_off = live ? block_of<C>(c0) * BPB : 0;
+  const int oct = octet_of<C>(live ? c0 : 0);
+  for (int e0 = kRowM * blockIdx.z; e0 < count; e0 += kRowM * gridDim.z) {  // grid.z CTAs share the entries
+    const int m = min(kRowM, count - e0);
+    float acc[kRowM][8];
+#pragma unroll
+    for (int t = 0; t < kRowM; t++)
+#pragma unroll
+      for (int i = 0; i < 8; i++) acc[t][i] = 0.f;
+    for (int kb = 0; kb < K; kb += kChunk) {
+      const int kn = min(kChunk, K - kb);
+      __syncthreads();  // the chunk before (and the sums of the pass before) have been read
+      for (int i = threadIdx.x; i < kn * kRowM; i += kThreads) {
+        const int t = i / kn, k = i % kn;
+        xs[k][t] = t < m ? load_x<XT>(x + (long long)list[e0 + t].x * K + kb + k) : 0.f;
+      }
+      __syncthreads();
+#pragma unroll 2
+      for (int k = 2 * warp + half; k < kn; k += 2 * kWarps) {
+        float v[8];
+        decode8<C, A>(w + (long long)(kb + k) * row_bytes + blk_off, oct, v, tabs);
+        const float4 x0 = *reinterpret_cast<const float4*>(&xs[k][0]), x1 = *reinterpret_cast<const float4*>(&xs[k][4]);
+        const float xv[kRowM] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+#pragma unroll
+        for (int t = 0; t < kRowM; t++)
+#pragma unroll
+          for (int i = 0; i < 8; i++) acc[t][i] = fmaf(xv[t], v[i], acc[t][i]);
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < kRowM; t++) {
+#pragma unroll
+      for (int i = 0; i < 8; i++) acc[t][i] += __shfl_xor_sync(0xffffffffu, acc[t][i], 16);
+      if (half == (t & 1)) {
+        *reinterpret_cast<float4*>(&red[warp][t][8 * oc]) = make_float4(acc[t][0], acc[t][1], acc[t][2], acc[t][3]);
+        *reinterpret_cast<float4*>(&red[warp][t][8 * oc + 4]) = make_float4(acc[t][4], acc[t][5], acc[t][6], acc[t][7]);
+      }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < m * kRowCols; i += kThreads) {
+      const int t = i / kRowCols, c = i % kRowCols;
+      if (blockIdx.x * kRowCols + c >= N) continue;
+      float s = 0.f;
+#pragma unroll
+      for (int v = 0; v < kWarps; v++) s += red[v][t][c];
+      OT* out = static_cast<OT*>(y) + (long long)list[e0 + t].y * N + blockIdx.x * kRowCols + c;
+      if constexpr (std::is_same<OT, __half>::value) *out = __float2half_rn(s);
+      else *out = __float2bfloat16_rn(s);
+    }
+  }
+}
+
+template <int C, int A, typename XT>
+cudaError_t launch_rows(const void* x, void* y, const uint8_t* w, long long row_bytes, int N, int K, cudaStream_t st,
+                        const QvmGather& gq, int n_entries) {
+  cudaLaunchConfig_t cfg = {};
+  const int ctas = (N + kRowCols - 1) / kRowCols * gq.n_experts;
+  // routing may be uneven: where the SMs would not be full anyway, several CTAs share a matrix's entries
+  const int share = std::max(1, std::min((n_entries + kRowM - 1) / kRowM, 4 * 148 / ctas));
+  cfg.gridDim = dim3((N + kRowCols - 1) / kRowCols, gq.n_experts, share);
+  cfg.blockDim = dim3(kThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, qvm_rows_kernel<C, A, XT>, static_cast<const XT*>(x), y, w, row_bytes, N, K, gq,
+                            n_entries);
+}
+
 template <int C, int A, typename XT>
 cudaError_t launch_one(const void* x, long long x_row_stride, void* y, long long y_row_stride, const uint8_t* w,
                        long long row_bytes, int M, int N, int K, cudaStream_t st, QvmGather gq = QvmGather{},
                        long long entries = 1) {
+  // one row an entry and at least as many entries as matrices: some matrix has several rows
+  if (gq.rhs != nullptr && M == 1 && entries >= gq.n_experts && entries <= kRowEntries && gq.n_experts <= 65535)
+    return launch_rows<C, A, XT>(x, y, w, row_bytes, N, K, st, gq, (int)entries);
   const int col_ctas = (N + kCols - 1) / kCols, m_tiles = (M + kMT - 1) / kMT;
   int S = 1;
   while (S < kMaxSplit && (long long)col_ctas * m_tiles * entries * S < 2 * 148 && K / (S * 2) >= 4 * kWarps) S *= 2;

@@ -39,9 +39,17 @@ namespace kq {
 
 namespace {
 
-constexpr int kRwMaxSmem = 227 * 1024 - 1024;
 constexpr int kRwMaxStages = 6;
-constexpr int kRwProducers = 4, kRwHelpers = 4;  // warps
+// Warps of a CTA and its shared memory. Dense: one CTA per SM. Gather (an expert's rows are few blocks, a CTA lives a
+// few microseconds): two, so that one starts while the other works.
+template <bool G>
+struct RowsShape {
+  static constexpr int kWarps = G ? 8 : 16, kProducers = G ? 2 : 4, kHelpers = G ? 2 : 4;
+  static constexpr int kThreads = 32 * (kWarps + kProducers + kHelpers);
+  static constexpr int kCtas = G ? 2 : 1;
+  static constexpr int kMaxSmem = G ? 112 * 1024 : 226 * 1024;
+};
+constexpr int kRwMaxEntries = 1024;  // entries of a gather call: every CTA looks through all of them
 
 // sub-blocks of a superblock, min term, 16-byte blocks
 __host__ __device__ constexpr int rw_nsub(int c) { return c == Q6_K ? 16 : 8; }
@@ -55,11 +63,20 @@ __host__ __device__ constexpr bool rw_sums() { return rw_min(C) || rw_base<C, BF
 // words per (superblock, activation row) of the sums: heads, tails, padding against bank conflicts
 __host__ __device__ constexpr int rw_sum_pitch(int c) { return 2 * rw_nsub(c) + 4; }
 
+// gather_qmm: entry i multiplies activation row lhs[i] by matrix rhs[i]; grid.y counts the matrices, or (by_entry,
+// fewer entries than matrices) the entries, of which the first of every matrix does the work for all.
+struct RowsGather {
+  const uint32_t *lhs, *rhs;
+  int n_entries, n_experts, by_entry;
+  long long x_batch, expert_stride;
+};
+
 struct RowsPlan {
   int R;       // weight rows of a row block
   int rt, wk;  // row tiles of 16, warps to a row tile: rt * wk consumer warps work
   int cs;      // superblocks of a stage; warp column k takes k, k + wk, ...
-  int stages, wpitch, xpitch, stage_bytes, x_off, sum_off, red_off, smem;
+  int half;    // != 0: tile rows 0 .. half - 1 are the block's even rows, the others its odd ones
+  int stages, wpitch, xpitch, stage_bytes, x_off, sum_off, red_off, list_off, smem;
   int n_blocks;
 };
 
@@ -356,24 +373,27 @@ __device__ __forceinline__ void rows_sums(const uint8_t* xrow, float* out, int l
   }
 }
 
-constexpr int kRwWarps = 16;  // consumer warps
 
-template <int C, typename XT, int NT>
-__global__ void __launch_bounds__(32 * (kRwWarps + kRwHelpers + kRwProducers), 1)
-rows_kernel(const GemvArgs a, const RowsPlan pl, int* __restrict__ error_word) {
-  constexpr int NW = kRwWarps, BPB = bpb_of(C);
+template <int C, typename XT, int NT, bool G>
+__global__ void __launch_bounds__(RowsShape<G>::kThreads, RowsShape<G>::kCtas)
+rows_kernel(const GemvArgs a, const RowsPlan pl, const RowsGather ga, int* __restrict__ error_word) {
+  constexpr int NW = RowsShape<G>::kWarps, BPB = bpb_of(C);
+  constexpr int kRwProducers = RowsShape<G>::kProducers, kRwHelpers = RowsShape<G>::kHelpers;
   constexpr bool kBf = std::is_same<XT, __nv_bfloat16>::value;
   constexpr bool kSums = rw_sums<C, kBf>();
   extern __shared__ __align__(128) uint8_t rw_dyn[];
   __shared__ uint64_t full[kRwMaxStages], ready[kRwMaxStages], empty[kRwMaxStages];
-  __shared__ int abort_s;
+  __shared__ int abort_s, count_s;
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int S = pl.stages, M = a.M;
+  const int S = pl.stages;
   const int nsb = a.K >> 8, nst = (nsb + pl.cs - 1) / pl.cs;
+  // Rows of an odd number of two-byte-aligned blocks start alternately on and between multiples of four: a tile takes
+  // rows of one kind, as the lanes' share of a sub-block depends on it.
+  auto row_of = [&](int r) { return pl.half == 0 ? r : (r < pl.half ? 2 * r : 2 * (r - pl.half) + 1); };
   const int live = pl.rt * pl.wk;  // consumer warps with work
   if (threadIdx.x == 0) {
-    abort_s = 0;
+    abort_s = count_s = 0;
     for (int s = 0; s < S; s++) {
       mbar_init(&full[s], 32 * kRwProducers);
       mbar_init(&ready[s], kRwHelpers);
@@ -382,24 +402,43 @@ rows_kernel(const GemvArgs a, const RowsPlan pl, int* __restrict__ error_word) {
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncthreads();
+  // Passes: the dense form walks the row blocks blockIdx.x, + gridDim.x, ... for all M rows; the gather form has one
+  // row block of one matrix and walks its entries, 8 NT at a time (grid.z CTAs share them).
+  int passes = 0, total_m = a.M;
+  const uint8_t* wmat = a.w;
+  int2* list = reinterpret_cast<int2*>(rw_dyn + pl.list_off);  // (row of x, row of y)
+  if constexpr (G) {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the routing may come from the kernel before this one
+    const uint32_t e = ga.by_entry ? ga.rhs[blockIdx.y] : blockIdx.y;
+    if (e >= (uint32_t)ga.n_experts) return;
+    total_m = collect_entries<RowsShape<G>::kThreads>(ga.rhs, ga.lhs, ga.n_entries, ga.x_batch, e, list, &count_s);
+    if (total_m == 0 || (ga.by_entry && list[0].y != (int)blockIdx.y)) return;
+    wmat += (long long)e * ga.expert_stride;
+    passes = ((total_m + 8 * NT - 1) / (8 * NT) - (int)blockIdx.z + (int)gridDim.z - 1) / (int)gridDim.z;
+    if (passes <= 0) return;
+  } else {
+    passes = (pl.n_blocks - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;
+  }
+  auto row_block = [&](int pass) { return ((int)blockIdx.x + (G ? 0 : pass * (int)gridDim.x)) * pl.R; };
+  auto entry0 = [&](int pass) { return 8 * NT * (pass * (int)gridDim.z + (int)blockIdx.z); };  // of the pass (gather)
+  auto rows_of_x = [&](int pass) { return G ? min(8 * NT, total_m - entry0(pass)) : total_m; };
   volatile int* abort_flag = &abort_s;
   auto wait = [&](uint64_t* bar, int parity) { return mbar_wait_err(bar, parity, abort_flag, 0x100, error_word); };
 
   if (warp >= NW + kRwHelpers) {
     // ================= producers =================
     const int pw = warp - NW - kRwHelpers;
-    const int my_blocks = (pl.n_blocks - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;
-    const int total = my_blocks * nst;
-    const uint8_t* wend = a.w + (long long)a.N * a.row_bytes;
-    int blk_w = blockIdx.x, st_w = 0, slot_w = 0, st_x = 0, slot_x = 0;
+    const int total = passes * nst;
+    const uint8_t* wend = wmat + (long long)a.N * a.row_bytes;
+    int pass_w = 0, st_w = 0, slot_w = 0, pass_x = 0, st_x = 0, slot_x = 0;
     // Pieces of sixteen bytes, piece q of a stage: row q / per_row, place q % per_row. A thread takes every 128th:
     // both numbers advance by a constant, no division in the loop.
     const int tid = pw * 32 + lane;
     constexpr int kThreads = 32 * kRwProducers;
     auto copy_w = [&]() {
-      const int row0 = blk_w * pl.R, rows = min(pl.R, a.N - row0), len = min(pl.cs, nsb - st_w * pl.cs) * BPB;
+      const int row0 = row_block(pass_w), rows = min(pl.R, a.N - row0), len = min(pl.cs, nsb - st_w * pl.cs) * BPB;
       const uint32_t dst = smem_u32(rw_dyn + slot_w * pl.stage_bytes);
-      const uint8_t* src = a.w + (long long)row0 * a.row_bytes + (long long)st_w * pl.cs * BPB;
+      const uint8_t* src = wmat + (long long)row0 * a.row_bytes + (long long)st_w * pl.cs * BPB;
       const int rb = (int)a.row_bytes;
       const int per_row = rw_al16(C) ? len >> 4 : (len + 30) >> 4;  // a window holds at most that many
       const int dr = kThreads / per_row, dc = kThreads - dr * per_row;
@@ -427,28 +466,29 @@ rows_kernel(const GemvArgs a, const RowsPlan pl, int* __restrict__ error_word) {
           if (c >= per_row) c -= per_row, r++;
         }
       }
-      if (++st_w == nst) st_w = 0, blk_w += gridDim.x;
+      if (++st_w == nst) st_w = 0, pass_w++;
       if (++slot_w == S) slot_w = 0;
     };
     auto copy_x = [&]() {  // and the arrival of this thread once all its copies of the stage have landed
-      const int per_row = min(pl.cs, nsb - st_x * pl.cs) * 32;
+      const int per_row = min(pl.cs, nsb - st_x * pl.cs) * 32, m = rows_of_x(pass_x);
       const uint32_t dst = smem_u32(rw_dyn + slot_x * pl.stage_bytes + pl.x_off);
       const XT* src = static_cast<const XT*>(a.x) + st_x * pl.cs * 256;
       const int dr = kThreads / per_row, dc = kThreads - dr * per_row;
       int r = tid / per_row, c = tid - r * per_row;
 #pragma unroll 4
-      for (int q = tid; q < M * per_row; q += kThreads) {
-        rw_cp16(dst + r * pl.xpitch + 16 * c, src + ((long long)r * a.x_row_stride + 8 * c));
+      for (int q = tid; q < m * per_row; q += kThreads) {
+        const int row = G ? list[entry0(pass_x) + r].x : r;
+        rw_cp16(dst + r * pl.xpitch + 16 * c, src + ((long long)row * a.x_row_stride + 8 * c));
         r += dr, c += dc;
         if (c >= per_row) c -= per_row, r++;
       }
       asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(smem_u32(&full[slot_x])) : "memory");
-      if (++st_x == nst) st_x = 0;
+      if (++st_x == nst) st_x = 0, pass_x++;
       if (++slot_x == S) slot_x = 0;
     };
     const int first = min(S, total);
     for (int i = 0; i < first; i++) copy_w();
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the activations may come from the kernel before this one
+    if constexpr (!G) asm volatile("griddepcontrol.wait;\n" ::: "memory");  // x may come from the kernel before this one
     for (int i = 0; i < first; i++) copy_x();
     int parity = 0;
     for (int i = first; i < total; i++) {
@@ -461,16 +501,17 @@ rows_kernel(const GemvArgs a, const RowsPlan pl, int* __restrict__ error_word) {
   } else if (warp >= NW) {
     // ================= helpers: the stage's activation sums =================
     if constexpr (kSums) {
-      const int my_blocks = (pl.n_blocks - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;
-      int s = 0, parity = 0, st = 0;
-      for (int i = 0; i < my_blocks * nst; i++) {
+      int s = 0, parity = 0, st = 0, pass = 0;
+      for (int i = 0; i < passes * nst; i++) {
+        const int m = rows_of_x(pass);
         const int here = min(pl.cs, nsb - st * pl.cs);
         if (!wait(&full[s], parity)) break;
         const uint8_t* xs = rw_dyn + (long long)s * pl.stage_bytes + pl.x_off;
         float* sums = reinterpret_cast<float*>(rw_dyn + (long long)s * pl.stage_bytes + pl.sum_off);
         for (int e = warp - NW; e < here * NT; e += kRwHelpers) {
           const int k = e / NT, n = e % NT;
-          rows_sums<C, XT>(xs + min(8 * n + (lane >> 2), M - 1) * pl.xpitch + 512 * k,
+          if (8 * n >= m) continue;
+          rows_sums<C, XT>(xs + min(8 * n + (lane >> 2), m - 1) * pl.xpitch + 512 * k,
                            sums + (k * NT + n) * 8 * rw_sum_pitch(C), lane);
         }
         __syncwarp();
@@ -478,7 +519,7 @@ rows_kernel(const GemvArgs a, const RowsPlan pl, int* __restrict__ error_word) {
           mbar_arrive(&ready[s]);
           mbar_arrive(&empty[s]);
         }
-        if (++st == nst) st = 0;
+        if (++st == nst) st = 0, pass++;
         if (++s == S) s = 0, parity ^= 1;
       }
     }
@@ -490,9 +531,10 @@ rows_kernel(const GemvArgs a, const RowsPlan pl, int* __restrict__ error_word) {
     constexpr int kRedPitch = 8 * NT + 2;
     bool ok = true;
     int s = 0, parity = 0;
-    for (int blk = blockIdx.x; blk < pl.n_blocks; blk += gridDim.x) {
-      const int row0 = blk * pl.R, rows = min(pl.R, a.N - row0);
-      const int l0 = min(16 * tile + g, rows - 1), l1 = min(16 * tile + g + 8, rows - 1);
+    for (int pass = 0; pass < passes; pass++) {
+      const int row0 = row_block(pass), rows = min(pl.R, a.N - row0), m = rows_of_x(pass);
+      const int p0 = row_of(16 * tile + g), p1 = row_of(16 * tile + g + 8);
+      const int l0 = min(p0, rows - 1), l1 = min(p1, rows - 1);  // places past the end read some row, to no effect
       float y[NT][4];
 #pragma unroll
       for (int n = 0; n < NT; n++) y[n][0] = y[n][1] = y[n][2] = y[n][3] = 0.f;
@@ -503,15 +545,23 @@ rows_kernel(const GemvArgs a, const RowsPlan pl, int* __restrict__ error_word) {
         for (int k = ks; k < here; k += pl.wk) {
           const uint8_t *r0 = base + l0 * pl.wpitch + k * BPB, *r1 = base + l1 * pl.wpitch + k * BPB;
           if constexpr (!rw_al16(C)) {  // the bytes of a row start at their offset within a 16-byte word
-            const long long o0 = (long long)(row0 + l0) * a.row_bytes + (long long)st * pl.cs * BPB;
-            const long long o1 = (long long)(row0 + l1) * a.row_bytes + (long long)st * pl.cs * BPB;
+            // (a place past the end keeps its own offset: all lanes agree modulo four)
+            const long long o0 = (long long)(row0 + p0) * a.row_bytes + (long long)st * pl.cs * BPB;
+            const long long o1 = (long long)(row0 + p1) * a.row_bytes + (long long)st * pl.cs * BPB;
             r0 += (int)(o0 & 15), r1 += (int)(o1 & 15);
           }
           const uint8_t* xb[NT];
 #pragma unroll
-          for (int n = 0; n < NT; n++) xb[n] = base + pl.x_off + min(8 * n + g, M - 1) * pl.xpitch + 512 * k;
+          for (int n = 0; n < NT; n++) xb[n] = base + pl.x_off + min(8 * n + g, m - 1) * pl.xpitch + 512 * k;
           const float* sums = reinterpret_cast<const float*>(base + pl.sum_off) + k * NT * 8 * rw_sum_pitch(C);
-          RowsUnit<C, XT, NT>::run(y, r0, r1, xb, sums, g, t);
+          if (!G || NT == 1 || m > 8) {
+            RowsUnit<C, XT, NT>::run(y, r0, r1, xb, sums, g, t);
+          } else {  // (gather) few enough for one column tile
+            const uint8_t* xb1[1] = {xb[0]};
+            float y1[1][4] = {{y[0][0], y[0][1], y[0][2], y[0][3]}};
+            RowsUnit<C, XT, 1>::run(y1, r0, r1, xb1, sums, g, t);
+            y[0][0] = y1[0][0], y[0][1] = y1[0][1], y[0][2] = y1[0][2], y[0][3] = y1[0][3];
+          }
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);
@@ -527,13 +577,14 @@ rows_kernel(const GemvArgs a, const RowsPlan pl, int* __restrict__ error_word) {
       asm volatile("bar.sync 1, %0;\n" ::"r"(live * 32) : "memory");
       if (ok) {
         const int rp = pl.rt * 16;
-        for (int e = threadIdx.x; e < rp * M; e += live * 32) {
-          const int r = e % rp, m = e / rp;
+        for (int e = threadIdx.x; e < rp * m; e += live * 32) {
+          const int place = e % rp, c = e / rp, r = row_of(place);
           if (r < rows) {
             float v = 0.f;
-            for (int k = 0; k < pl.wk; k++) v += red[(long long)(k * rp + r) * kRedPitch + m];
-            if (a.row_scale != nullptr) v *= a.row_scale[m];
-            const long long o = (long long)m * a.y_row_stride + row0 + r;
+            for (int k = 0; k < pl.wk; k++) v += red[(long long)(k * rp + place) * kRedPitch + c];
+            if (a.row_scale != nullptr) v *= a.row_scale[c];
+            const int orow = G ? list[entry0(pass) + c].y : c;
+            const long long o = (long long)orow * a.y_row_stride + row0 + r;
             if (kBf || a.out_bf16) static_cast<__nv_bfloat16*>(a.y)[o] = __float2bfloat16_rn(v);
             else static_cast<__half*>(a.y)[o] = __float2half_rn(v);
           }
@@ -559,58 +610,79 @@ int rows_sm_count() {
 
 // Row blocks as even as the SM count allows, one per SM and pass; a stage as deep as the warps left over by the
 // row tiles can take, shortened until three stages (or all of K) fit shared memory.
-template <int C, bool BF, int NT>
-bool rows_plan(const GemvArgs& a, RowsPlan& p) {
-  constexpr int NW = kRwWarps, BPB = bpb_of(C);
+template <int C, bool BF, int NT, bool G>
+bool rows_plan(const GemvArgs& a, RowsPlan& p, int units) {
+  constexpr int NW = RowsShape<G>::kWarps, BPB = bpb_of(C), kMaxSmem = RowsShape<G>::kMaxSmem;
   const int sms = rows_sm_count();
   if (sms <= 0) return false;
-  const int nsb = a.K >> 8;
-  const int passes = (a.N + sms * 16 * NW - 1) / (sms * 16 * NW);
-  p.R = std::max(8, (a.N + sms * passes - 1) / (sms * passes));
-  p.n_blocks = (a.N + p.R - 1) / p.R;
-  p.rt = (p.R + 15) / 16;
-  p.wk = std::min(NW / p.rt, nsb);
-  for (p.cs = std::min(2 * p.wk, nsb); p.cs >= 1; p.cs--) {
-    p.wk = std::min(p.wk, p.cs);
-    int wb = p.cs * BPB;
-    if (!rw_al16(C)) wb = (wb + 30 + 15) & ~15;
-    // 8-byte reads of four rows, or 4-byte reads of eight, in different banks
-    while (rw_al16(C) ? (wb & 63) != 32 : (wb & 31) != 16) wb += 16;
-    p.wpitch = wb;
-    p.xpitch = p.cs * 512 + (rw_nsub(C) == 8 ? 64 : 32);
-    p.x_off = (p.R * p.wpitch + 127) & ~127;
-    p.sum_off = (p.x_off + a.M * p.xpitch + 15) & ~15;
-    p.stage_bytes = (p.sum_off + (rw_sums<C, BF>() ? p.cs * NT * 8 * rw_sum_pitch(C) * 4 : 0) + 127) & ~127;
-    const int red = p.wk * p.rt * 16 * (8 * NT + 2) * 4;
-    const int nst = (nsb + p.cs - 1) / p.cs * ((p.n_blocks + sms - 1) / sms);
-    p.stages = std::min({kRwMaxStages, nst, (kRwMaxSmem - red) / p.stage_bytes});
-    if (p.stages >= std::min(3, nst)) {
-      p.red_off = p.stages * p.stage_bytes;
-      p.smem = p.red_off + red;
-      return true;
+  const int nsb = a.K >> 8, max_m = G ? 8 * NT : a.M;
+  int r0;
+  if (G) {
+    // whole blocks of 128 rows where they fill the SMs several times over, smaller ones for fewer matrices
+    r0 = 128;
+    while (r0 > 32 && (long long)units * ((a.N + r0 - 1) / r0) < 2 * sms) r0 /= 2;
+  } else {
+    const int passes = (a.N + sms * 16 * NW - 1) / (sms * 16 * NW);
+    r0 = std::max(8, (a.N + sms * passes - 1) / (sms * passes));
+  }
+  const bool alternate = !rw_al16(C) && (a.row_bytes & 3) != 0;
+  if (alternate) r0 = (r0 + 31) & ~31;  // whole tiles of either kind
+  // three stages (or all of K), for the gather form rather with fewer rows; two always fit
+  for (int want = 3; want >= 2; want--) {
+    for (p.R = r0; p.R == r0 || (G && p.R >= 32); p.R /= 2) {
+      p.n_blocks = (a.N + p.R - 1) / p.R;
+      p.rt = (p.R + 15) / 16;
+      p.half = alternate ? p.R / 2 : 0;
+      p.wk = std::min(NW / p.rt, nsb);
+      for (p.cs = std::min(2 * p.wk, nsb); p.cs >= 1; p.cs--) {
+        p.wk = std::min(p.wk, p.cs);
+        int wb = p.cs * BPB;
+        if (!rw_al16(C)) wb = (wb + 30 + 15) & ~15;
+        // 8-byte reads of four rows, or 4-byte reads of eight, in different banks
+        while (rw_al16(C) ? (wb & 63) != 32 : (wb & 31) != 16) wb += 16;
+        p.wpitch = wb;
+        p.xpitch = p.cs * 512 + (rw_nsub(C) == 8 ? 64 : 32);
+        p.x_off = (p.R * p.wpitch + 127) & ~127;
+        p.sum_off = (p.x_off + max_m * p.xpitch + 15) & ~15;
+        p.stage_bytes = (p.sum_off + (rw_sums<C, BF>() ? p.cs * NT * 8 * rw_sum_pitch(C) * 4 : 0) + 127) & ~127;
+        const int red = p.wk * p.rt * 16 * (8 * NT + 2) * 4;
+        const int nst = (nsb + p.cs - 1) / p.cs * (G ? 1 : (p.n_blocks + sms - 1) / sms);
+        p.stages = std::min({kRwMaxStages, nst, (kMaxSmem - red - (G ? 8 * kRwMaxEntries : 0)) / p.stage_bytes});
+        if (p.stages >= std::min(want, nst)) {
+          p.red_off = p.stages * p.stage_bytes;
+          p.list_off = p.red_off + ((red + 15) & ~15);
+          p.smem = p.list_off + (G ? 8 * kRwMaxEntries : 0);
+          return true;
+        }
+      }
     }
   }
   return false;
 }
 
-template <int C, typename XT, int NT>
-cudaError_t launch_rows_nt(const GemvArgs& a, cudaStream_t st) {
+template <int C, typename XT, int NT, bool G>
+cudaError_t launch_rows_nt(const GemvArgs& a, const RowsGather& ga, cudaStream_t st) {
   RowsPlan p;
-  if (!rows_plan<C, std::is_same<XT, __nv_bfloat16>::value, NT>(a, p)) return cudaErrorInvalidConfiguration;
+  const int units = G ? std::min(ga.n_entries, ga.n_experts) : 1;
+  if (!rows_plan<C, std::is_same<XT, __nv_bfloat16>::value, NT, G>(a, p, units)) return cudaErrorInvalidConfiguration;
   static bool attr_set[16] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 16) return cudaErrorInvalidDevice;
   if (!attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(rows_kernel<C, XT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRwMaxSmem);
+    cudaError_t e = cudaFuncSetAttribute(rows_kernel<C, XT, NT, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         RowsShape<G>::kMaxSmem);
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
   int* err = device_error_word();
   if (err == nullptr) return cudaErrorUnknown;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(std::min(p.n_blocks, rows_sm_count()), 1, 1);
-  cfg.blockDim = dim3(32 * (kRwWarps + kRwHelpers + kRwProducers));
+  // routing may be uneven: where the SMs would not be full anyway, several CTAs share a matrix's entries
+  int share = 1;
+  if (G) share = std::max(1, std::min((ga.n_entries + 8 * NT - 1) / (8 * NT), 4 * rows_sm_count() / (p.n_blocks * units)));
+  cfg.gridDim = G ? dim3(p.n_blocks, units, share) : dim3(std::min(p.n_blocks, rows_sm_count()), 1, 1);
+  cfg.blockDim = dim3(RowsShape<G>::kThreads);
   cfg.dynamicSmemBytes = p.smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
@@ -619,13 +691,34 @@ cudaError_t launch_rows_nt(const GemvArgs& a, cudaStream_t st) {
   cfg.attrs = attr;
   static const bool no_pdl = std::getenv("KQ_NO_PDL") != nullptr;  // A/B lever
   cfg.numAttrs = no_pdl ? 0 : 1;
-  return cudaLaunchKernelEx(&cfg, rows_kernel<C, XT, NT>, a, p, err);
+  return cudaLaunchKernelEx(&cfg, rows_kernel<C, XT, NT, G>, a, p, ga, err);
 }
 
 template <int C, typename XT>
-cudaError_t launch_rows_c(const GemvArgs& a, cudaStream_t st) {
-  if (a.M <= 8) return launch_rows_nt<C, XT, 1>(a, st);
-  return launch_rows_nt<C, XT, 2>(a, st);
+cudaError_t launch_rows_c(const GemvArgs& a, const RowsGather* ga, cudaStream_t st) {
+  // gather: with more than six entries a matrix on average, many have more than eight
+  if (ga != nullptr)
+    return ga->n_entries <= 6 * ga->n_experts ? launch_rows_nt<C, XT, 1, true>(a, *ga, st)
+                                              : launch_rows_nt<C, XT, 2, true>(a, *ga, st);
+  if (a.M <= 8) return launch_rows_nt<C, XT, 1, false>(a, RowsGather{}, st);
+  return launch_rows_nt<C, XT, 2, false>(a, RowsGather{}, st);
+}
+
+cudaError_t launch_rows_any(int codec, int x_dtype, const GemvArgs& a, const RowsGather* ga, cudaStream_t st) {
+  if (x_dtype == F16) {
+    switch (codec) {
+      case Q4_K: return launch_rows_c<Q4_K, __half>(a, ga, st);
+      case Q5_K: return launch_rows_c<Q5_K, __half>(a, ga, st);
+      case Q6_K: return launch_rows_c<Q6_K, __half>(a, ga, st);
+    }
+  } else {
+    switch (codec) {
+      case Q4_K: return launch_rows_c<Q4_K, __nv_bfloat16>(a, ga, st);
+      case Q5_K: return launch_rows_c<Q5_K, __nv_bfloat16>(a, ga, st);
+      case Q6_K: return launch_rows_c<Q6_K, __nv_bfloat16>(a, ga, st);
+    }
+  }
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace
@@ -635,26 +728,43 @@ bool gemv_rows_supported(int codec, int x_dtype, const GemvArgs& a) {
   if (!(x_dtype == F16 || x_dtype == BF16) || a.tasks != nullptr || a.bias != nullptr || a.M < 1 || a.M > 16 || a.N < 8 ||
       a.K < 256 || (a.K & 255) != 0 || a.w_align16 == 0 || a.row_bytes != (long long)(a.K >> 8) * bpb_of(codec))
     return false;
-  // q6_k: every row starts on the same phase modulo four
-  if (codec == Q6_K && (a.row_bytes & 3) != 0) return false;
   return (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && (a.x_row_stride & 7) == 0;
 }
 
 cudaError_t launch_gemv_rows(int codec, int x_dtype, const GemvArgs& a, cudaStream_t st) {
-  if (x_dtype == F16) {
-    switch (codec) {
-      case Q4_K: return launch_rows_c<Q4_K, __half>(a, st);
-      case Q5_K: return launch_rows_c<Q5_K, __half>(a, st);
-      case Q6_K: return launch_rows_c<Q6_K, __half>(a, st);
-    }
-  } else {
-    switch (codec) {
-      case Q4_K: return launch_rows_c<Q4_K, __nv_bfloat16>(a, st);
-      case Q5_K: return launch_rows_c<Q5_K, __nv_bfloat16>(a, st);
-      case Q6_K: return launch_rows_c<Q6_K, __nv_bfloat16>(a, st);
-    }
-  }
-  return cudaErrorInvalidValue;
+  return launch_rows_any(codec, x_dtype, a, nullptr, st);
+}
+
+// gather_qmm with one activation row per entry, in one launch: no grouping passes and no scratch.
+bool gather_rows_supported(int codec, int x_dtype, const void* x, int M, int K, const uint8_t* w, long long expert_stride,
+                           long long row_bytes, int N, long long n_entries, int n_experts) {
+  if (M != 1 || n_entries > kRwMaxEntries || n_experts > 65535 || (expert_stride & 15) != 0) return false;
+  GemvArgs a{};
+  a.x = x;
+  a.x_row_stride = K;
+  a.w_align16 = (reinterpret_cast<uintptr_t>(w) & 15) == 0;
+  a.row_bytes = row_bytes;
+  a.N = N;
+  a.K = K;
+  a.M = 1;
+  return gemv_rows_supported(codec, x_dtype, a);
+}
+
+cudaError_t launch_gather_rows(int codec, int x_dtype, const void* x, long long x_batch, int K, const uint8_t* w,
+                               int n_experts, long long expert_stride, long long row_bytes, int N, const uint32_t* lhs,
+                               const uint32_t* rhs, long long n_entries, void* y, cudaStream_t st) {
+  GemvArgs a{};
+  a.x = x;
+  a.x_row_stride = K;
+  a.y = y;
+  a.y_row_stride = N;
+  a.w = w;
+  a.w_align16 = 1;
+  a.row_bytes = row_bytes;
+  a.N = N;
+  a.K = K;
+  RowsGather ga{lhs, rhs, (int)n_entries, n_experts, n_entries < n_experts ? 1 : 0, x_batch, expert_stride};
+  return launch_rows_any(codec, x_dtype, a, &ga, st);
 }
 
 }  // namespace kq

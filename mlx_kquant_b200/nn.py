@@ -147,11 +147,11 @@ class KQuantMultiLinear(_KQuantBase):
         if cached is not None and cached[0] == (B, Hx, dev):
             lhs, rhs = cached[1], cached[2]
         else:
-            rhs = torch.arange(nh, device=dev).reshape(1, nh).expand(B, nh).contiguous()
+            rhs = torch.arange(nh, dtype=torch.int32, device=dev).reshape(1, nh).expand(B, nh).contiguous()
             if Hx == nh:
-                lhs = torch.arange(B * nh, device=dev).reshape(B, nh)
+                lhs = torch.arange(B * nh, dtype=torch.int32, device=dev).reshape(B, nh)
             elif Hx == 1:
-                lhs = torch.arange(B, device=dev).reshape(B, 1).expand(B, nh).contiguous()
+                lhs = torch.arange(B, dtype=torch.int32, device=dev).reshape(B, 1).expand(B, nh).contiguous()
             else:
                 raise ValueError(f"KQuantMultiLinear: head axis {Hx} is neither 1 nor num_heads={nh} "
                                  f"(x.shape={tuple(x.shape)})")

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 # not start on 16-byte boundaries and a matrix whose last byte does not end on one (k = 512 * odd, odd n), more rows
 # than one pass of the SMs holds, both column tiles
 SHAPES = [(2, 8, 512), (3, 333, 512), (8, 2049, 1536), (9, 257, 1024), (16, 40, 4096), (5, 4099, 2560), (12, 3000, 512),
-          (2, 38000, 512)]
+          (2, 38000, 512), (4, 301, 768), (16, 38000, 256)]
 
 
 def _close(y, ref, out_eps):
