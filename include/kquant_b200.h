@@ -103,6 +103,9 @@ KQ_API int kq_quantize_cpu(const void* w, int w_dtype, long long n_weights, long
  *    uses it for the same conversion (several times faster), and a call without it
  *    still works. */
 KQ_API size_t kq_quantized_matmul_workspace_bytes(int x_dtype, long long rows, int K);
+/* The same with room for an fp16 copy of the weights (of at most 128 MiB) where [N, K] products of that many rows
+ * are faster from one; a call that is given only the bytes above works without it. */
+KQ_API size_t kq_quantized_matmul_workspace_bytes_for(const char* kquant_type, int x_dtype, long long rows, int N, int K);
 KQ_API int kq_quantized_matmul(const void* x, int x_dtype, long long rows, int K, long long x_row_stride, const void* w,
                         size_t w_row_bytes, int N, const char* kquant_type, int transpose, void* y,
                         long long y_row_stride, void* workspace, size_t workspace_bytes, void* stream);

@@ -124,6 +124,12 @@ size_t kq_quantized_matmul_workspace_bytes(int x_dtype, long long rows, int K) {
   return kq::gemm_workspace_bytes(x_dtype, rows, K);
 }
 
+size_t kq_quantized_matmul_workspace_bytes_for(const char* kquant_type, int x_dtype, long long rows, int N, int K) {
+  const int ci = find_codec(kquant_type);
+  if (ci < 0 || !dtype_ok(x_dtype) || rows <= 0 || N <= 0 || K <= 0) return 0;
+  return kq::gemm_workspace_bytes_n(ci, x_dtype, rows, N, K);
+}
+
 int kq_quantized_matmul(const void* x, int x_dtype, long long rows, int K, long long x_row_stride, const void* w,
                         size_t w_row_bytes, int N, const char* kquant_type, int transpose, void* y,
                         long long y_row_stride, void* workspace, size_t workspace_bytes, void* stream) {
@@ -173,7 +179,7 @@ int kq_quantized_matmul(const void* x, int x_dtype, long long rows, int K, long 
     if (need > 0 && (reinterpret_cast<uintptr_t>(workspace) & 255) != 0)
       return fail(KQ_ERR_INVALID_ARGUMENT, "[mlx_kquant.quantized_matmul] workspace must be 256-byte aligned.");
     e = kq::launch_gemm(ci, x_dtype, x, x_row_stride, y, y_row_stride, static_cast<const uint8_t*>(w),
-                        (long long)w_row_bytes, (int)rows, N, K, workspace, static_cast<cudaStream_t>(stream));
+                        (long long)w_row_bytes, (int)rows, N, K, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
   } else {
     kq::GemvArgs a{};
     a.x = x;

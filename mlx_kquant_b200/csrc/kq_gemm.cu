@@ -34,6 +34,7 @@
 #include <cooperative_groups.h>
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <type_traits>
@@ -106,6 +107,7 @@ struct GemmArgs {
   const uint8_t* w;
   long long row_bytes;
   int M, N, K;
+  int bn;                  // output columns of a tile: a multiple of 16, at most 128 NB
   const float* row_scale;  // per-row factor applied in the epilogue, or nullptr
   // grouped (mixture-of-experts) mode: CTA row tiles come from a device-built list
   const GemmTile* tiles;       // nullptr = dense
@@ -310,9 +312,11 @@ __device__ __forceinline__ void produce_w_q4k(const Q4kTileLoad& l, int kb, uint
 // each) - the next superblock is then requested one superblock (four K-steps) before its first use.
 __host__ __device__ constexpr int raw_depth(int NB) { return NB == 2 ? 2 : 4; }
 __host__ __device__ constexpr int raw_slot(int NB) { return 128 * NB * 144; }
-template <int C, int A, typename OT, int MT, int NB, bool FASTQ4, bool RAW = false, int KS = 1>
+// HB: the weights are an fp16 matrix already (dequantized before the launch): no producers, the loader brings weight
+// tiles by TMA too.
+template <int C, int A, typename OT, int MT, int NB, bool FASTQ4, bool RAW = false, int KS = 1, bool HB = false>
 __global__ void __launch_bounds__(gemm_threads(MT, NB), 1)
-gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap tmap_x) {
+gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w) {
   constexpr int kProducerThreads = producer_threads(NB), kGemmThreads = gemm_threads(MT, NB);
   constexpr int kMmaWarp = kProducerThreads / 32, kMmaWarps = mma_warps(MT);
   static_assert(!RAW || FASTQ4, "raw ring: q4_k fast producer");
@@ -336,7 +340,7 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap tmap_x) {
   __shared__ __align__(16) uint8_t s_tabs[kIq ? kIqSmemBytes : 16];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * BN;
+  const int n0 = blockIdx.x * a.bn, n_end = min(a.N, n0 + a.bn);
   // Grouped mode: the CTA takes tile blockIdx.y of the device-built list, then every gridDim.y-th after it (the
   // grid is sized on the host for the largest list the call could produce, capped; the list is usually far
   // shorter, and a CTA with no tile leaves before it allocates anything).
@@ -371,7 +375,7 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap tmap_x) {
       const bool again = tile != (int)blockIdx.y;
       for (int s = 0; s < kBStages; s++) {
         if (again) mbar_inval(&b_full[s]), mbar_inval(&b_empty[s]);
-        mbar_init(&b_full[s], kProducerThreads / 32);
+        mbar_init(&b_full[s], HB ? 1 : kProducerThreads / 32);
         mbar_init(&b_empty[s], kMmaWarps);
       }
       for (int s = 0; s < NA; s++) {
@@ -420,12 +424,12 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap tmap_x) {
         for (int d = 0; d < kRawDepth; d++) issue_sb(d);
       }
       Q4kTileLoad cur{};
-      if constexpr (FASTQ4 && !RAW) cur = q4k_tile_load(wrow, kb0);
-      constexpr bool kQ6Pre = (C == Q6_K && A == 8 && NB == 1);  // 8-byte aligned rows, two threads per row
+      if constexpr (FASTQ4 && !RAW && !HB) cur = q4k_tile_load(wrow, kb0);
+      constexpr bool kQ6Pre = (C == Q6_K && A == 8 && NB == 1 && !HB);  // 8-byte aligned rows, two threads per row
       Q6kTileLoad cur6{};
       if constexpr (kQ6Pre) cur6 = q6k_tile_load(wrow, kb0, hh0);
       KQ_TR(long long tr_wait = 0; long long tr_prod = 0; const long long c_loop = clock64();)
-      {
+      if constexpr (!HB) {
       for (int it = 0; it < KB && (ok || RAW); it++) {
         const int kb = kb0 + it;
         const int sti = it / KS, sub = it % KS;  // stage number and 64-deep part of it
@@ -578,12 +582,12 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap tmap_x) {
             const long long orow = sub ? o1 : o0;
             const uint4 q = *reinterpret_cast<const uint4*>(stage + r * kRowBytes + ((chunk ^ (r & (kChunks - 1))) << 4));
             OT* yp = ybase + orow * a.y_row_stride + col;
-            if (col + 8 <= a.N && (reinterpret_cast<uintptr_t>(yp) & 15) == 0) {
+            if (col + 8 <= n_end && (reinterpret_cast<uintptr_t>(yp) & 15) == 0) {
               *reinterpret_cast<uint4*>(yp) = q;
             } else {
               const OT* qe = reinterpret_cast<const OT*>(&q);
               for (int e = 0; e < 8; e++)
-                if (col + e < a.N) yp[e] = qe[e];
+                if (col + e < n_end) yp[e] = qe[e];
             }
           }
         }
@@ -594,7 +598,7 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap tmap_x) {
       // Issuer w takes the row blocks h = w, w + kMmaWarps, ...; the activation tile of (K-step kb, row block h)
       // is tile number kb * mt_live + h of the loader's sequence. Every issuer arrives on every stage barrier
       // (a commit with no MMA of its own completes at once), so the counts do not depend on mt_live.
-      constexpr uint32_t idesc = umma_idesc(0u, BN);
+      const uint32_t idesc = umma_idesc(0u, a.bn);
       const int w = warp - kMmaWarp;
       bool ok = true;
       KQ_TR(long long tr_b = 0; long long tr_a = 0; const long long cm = clock64();)
@@ -637,6 +641,16 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap tmap_x) {
       int t = 0;
       KQ_TR(long long tr_e = 0;)
       for (int sti = 0; sti < KB / KS && ok; sti++) {  // one slot = the KS 64-deep boxes of a stage
+        if constexpr (HB) {  // the weight tile: a box of bn rows
+          const int s = sti % kBStages;
+          if (sti >= kBStages) ok = mbar_wait(&b_empty[s], ((sti / kBStages) & 1) ^ 1, abort_flag, 1);
+          if (!ok) break;
+          if (lane == 0) {
+            mbar_expect_tx(&b_full[s], a.bn * 128);
+            tma_load_2d(b_ring + s * kBStage, &tmap_w, (kb0 + sti) * kBK, n0, &b_full[s]);
+          }
+          __syncwarp();
+        }
         for (int h = 0; h < mt_live && ok; h++, t++) {
           const int slot = t % NA;
           KQ_TR(const long long c0 = clock64();)
@@ -659,6 +673,11 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap tmap_x) {
         const int first = t > NA ? t - NA : 0;
         for (int u = first; u < t; u++)
           if (!mbar_wait(&a_full[u % NA], (u / NA) & 1, abort_flag, 64)) break;
+        if constexpr (HB) {
+          const int n = KB / KS;
+          for (int u = max(0, n - kBStages); u < n; u++)
+            if (!mbar_wait(&b_full[u % kBStages], (u / kBStages) & 1, abort_flag, 64)) break;
+        }
       }
     }
 
@@ -692,7 +711,7 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap tmap_x) {
               const float f[4] = {acc.x, acc.y, acc.z, acc.w};
   #pragma unroll
               for (int i = 0; i < 4; i++) {
-                if (n0 + 4 * c + i < a.N) {
+                if (n0 + 4 * c + i < n_end) {
                   if constexpr (kHalf) yp[i] = __float2half_rn(f[i]);
                   else yp[i] = __float2bfloat16_rn(f[i]);
                 }
@@ -997,13 +1016,13 @@ static EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
-// Tensor map of the fp16 activations [M, K] (row stride in elements): boxes of 64 x 128, 128B swizzle.
-static cudaError_t make_x_map(CUtensorMap* map, const void* x, long long x_row_stride, int M, int K) {
+// Tensor map of an fp16 matrix [M, K] (row stride in elements): boxes of 64 x box_rows, 128B swizzle.
+static cudaError_t make_x_map(CUtensorMap* map, const void* x, long long x_row_stride, int M, int K, int box_rows = 128) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (fn == nullptr) return cudaErrorNotSupported;
   const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)M};
   const cuuint64_t strides[1] = {(cuuint64_t)x_row_stride * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)kBK, 128};
+  const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)box_rows};
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(x), dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -1011,9 +1030,10 @@ static cudaError_t make_x_map(CUtensorMap* map, const void* x, long long x_row_s
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-template <int C, int A, typename OT, int MT, int NB, bool FASTQ4, bool RAW = false, int KS = 1>
-static cudaError_t launch_g(const GemmArgs& a, cudaStream_t st, int grid_y = 0, int ksplit = 1) {
-  auto kern = gemm_kernel<C, A, OT, MT, NB, FASTQ4, RAW, KS>;
+template <int C, int A, typename OT, int MT, int NB, bool FASTQ4, bool RAW = false, int KS = 1, bool HB = false>
+static cudaError_t launch_g(GemmArgs a, cudaStream_t st, int grid_y = 0, int ksplit = 1) {
+  auto kern = gemm_kernel<C, A, OT, MT, NB, FASTQ4, RAW, KS, HB>;
+  if (!HB) a.bn = kBN * NB;
   const size_t dyn = (size_t)(b_stages(NB, RAW, KS) * NB + a_slots(MT, NB, RAW, KS)) * KS * kTileBytes + 1024 +
                      (RAW ? raw_depth(NB) * raw_slot(NB) : 0);
   static bool attr_set[16] = {};
@@ -1027,10 +1047,12 @@ static cudaError_t launch_g(const GemmArgs& a, cudaStream_t st, int grid_y = 0, 
   alignas(64) CUtensorMap map;
   cudaError_t e = make_x_map(&map, a.x, a.x_row_stride, a.M, a.K);
   if (e != cudaSuccess) return e;
+  alignas(64) CUtensorMap map_w = map;  // (not read unless HB)
+  if (HB && (e = make_x_map(&map_w, a.w, a.K, a.N, a.K, a.bn)) != cudaSuccess) return e;
   if (MT * NB > 2) ksplit = 1;  // split K needs the fp32 partial tile in shared memory
-  const dim3 grid((a.N + kBN * NB - 1) / (kBN * NB), grid_y > 0 ? grid_y : (a.M + 128 * MT - 1) / (128 * MT), ksplit);
+  const dim3 grid((a.N + a.bn - 1) / a.bn, grid_y > 0 ? grid_y : (a.M + 128 * MT - 1) / (128 * MT), ksplit);
   if (ksplit == 1) {
-    kern<<<grid, gemm_threads(MT, NB), dyn, st>>>(a, map);
+    kern<<<grid, gemm_threads(MT, NB), dyn, st>>>(a, map, map_w);
     return cudaGetLastError();
   }
   // split K: the ksplit CTAs of one output tile form a cluster
@@ -1046,7 +1068,7 @@ static cudaError_t launch_g(const GemmArgs& a, cudaStream_t st, int grid_y = 0, 
   attr[0].val.clusterDim.z = ksplit;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, a, map);
+  return cudaLaunchKernelEx(&cfg, kern, a, map, map_w);
 }
 
 template <int C, int A, bool FASTQ4>
@@ -1139,10 +1161,61 @@ static cudaError_t launch_codec(bool out_half, const GemmArgs& a, bool aligned, 
   return aligned ? launch_shape<C, NAT, false>(out_half, a, st) : launch_shape<C, 1, false>(out_half, a, st);
 }
 
+// ---- many rows: the weights are dequantized to fp16 once and the tiles of both operands come by TMA
+// rows of the matrix per pass: the fp16 copy stays below kHalfBytes, so that it is still in L2 when it is read
+constexpr long long kHalfBytes = 128ll << 20;
+static int half_chunk(int N, int K) {
+  const long long most = std::max<long long>(256, kHalfBytes / (2ll * K) / 128 * 128);
+  const long long n = (N + most - 1) / most;
+  return (int)std::min<long long>(N, ((N + n - 1) / n + 127) / 128 * 128);
+}
+static size_t half_bytes(int N, int K) { return (2 * (size_t)half_chunk(N, K) * (size_t)K + 255) & ~(size_t)255; }
+// Codecs whose fused producer is decode8<> (all but q4_k and q6_k, and q6_k rows off the 8-byte grid) make a K-step's
+// weights several times slower than the tensor cores use them, whatever the number of rows: the copy wins from the
+// first row on, once the matrix outweighs its extra launch. Measured, fused against copy: q5_k [14336, 4096] x 64 rows
+// 326 / 91 us, q8_0 x 512 444 / 87, iq4_xs x 32 190 / 75, q4_0 [4096, 4096] x 300 129 / 53; q5_k [1000, 1280] x 130
+// 17.7 / 19.5. q6_k, whose producer nearly keeps up: [14336, 4096] x 2048 310 / 267, [4096, 14336] x 512 125 / 182.
+// q4_k never: x 2048 247 / 261.
+static bool use_half(int codec, long long M, int N, int K) {
+  if (codec == Q4_K || (long long)N * K < (4ll << 20)) return false;
+  if (codec == Q6_K && (K & 1023) == 0) return M >= 1024;
+  return true;
+}
+size_t gemm_workspace_bytes_n(int codec, int x_dtype, long long rows, int N, int K) {
+  return gemm_workspace_bytes(x_dtype, rows, K) + (use_half(codec, rows, N, K) ? half_bytes(N, K) : 0);
+}
+
+template <typename OT>
+static cudaError_t launch_half(GemmArgs a, cudaStream_t st) {
+  // Tile shape by the time its waves take. A K-step costs the tensor pipe two cycles per column and 128-row block, the
+  // loads of its (128 mt + bn) x 128 bytes some 2.7 cycles a row out of L2, its handshakes 450; a tile 9000 cycles for
+  // start and epilogue, a further slice of K 3000.
+  const int kb = (a.K + kBK - 1) / kBK;
+  double best = 1e30;
+  int mt = 2, bn = 256, ks = 1;
+  for (int t = 1; t <= 2; t++) {
+    if (t == 2 && a.M <= 128) break;
+    for (int b = 256; b >= 64; b -= 16) {
+      const long long tiles = (long long)((a.N + b - 1) / b) * ((a.M + 128 * t - 1) / (128 * t));
+      for (int z = 1; z <= 8 && kb % z == 0 && (z == 1 || t * (b > 128 ? 2 : 1) <= 2); z *= 2) {
+        const double step = std::max({2.0 * t * b, 2.7 * (128 * t + b), 450.0});
+        const double c = (double)((tiles * z + 147) / 148) * (kb / z * step + 9000.0 + 3000.0 * (z - 1));
+        if (c < best * 0.999) best = c, mt = t, bn = b, ks = z;
+      }
+    }
+  }
+  a.bn = bn;
+  if (mt == 2 && bn > 128) return launch_g<Q4_K, 16, OT, 2, 2, false, false, 1, true>(a, st);
+  if (mt == 2) return launch_g<Q4_K, 16, OT, 2, 1, false, false, 1, true>(a, st, 0, ks);
+  return launch_g<Q4_K, 16, OT, 1, 2, false, false, 1, true>(a, st, 0, ks);
+}
+
 cudaError_t launch_gemm(int codec, int x_dtype, const void* x, long long x_row_stride, void* y, long long y_row_stride,
-                        const uint8_t* w, long long row_bytes, int M, int N, int K, void* workspace, cudaStream_t st) {
+                        const uint8_t* w, long long row_bytes, int M, int N, int K, void* workspace,
+                        size_t workspace_bytes, cudaStream_t st) {
   if (M <= 0 || N <= 0 || K <= 0) return cudaSuccess;
   GemmArgs a;
+  a.bn = kBN;
   a.x = x;
   a.x_row_stride = x_row_stride;
   a.y = y;
@@ -1167,6 +1240,24 @@ cudaError_t launch_gemm(int codec, int x_dtype, const void* x, long long x_row_s
     a.row_scale = rs;
   }
   const bool out_half = x_dtype == F16;
+  const size_t base = gemm_workspace_bytes(x_dtype, M, K);
+  if (use_half(codec, M, N, K) && workspace != nullptr && workspace_bytes >= base + half_bytes(N, K) &&
+      row_bytes == (long long)(K / kCodecs[codec].wpb) * kCodecs[codec].bpb) {
+    uint8_t* wh = static_cast<uint8_t*>(workspace) + base;
+    const int chunk = half_chunk(N, K);
+    for (int n0 = 0; n0 < N; n0 += chunk) {
+      const int n = std::min(chunk, N - n0);
+      cudaError_t e = launch_dequantize(codec, w + (long long)n0 * row_bytes, (long long)n * (K / kCodecs[codec].wpb), F16,
+                                        wh, st);
+      if (e != cudaSuccess) return e;
+      a.w = wh;
+      a.N = n;
+      a.y = static_cast<uint8_t*>(y) + 2ll * n0;
+      e = out_half ? launch_half<__half>(a, st) : launch_half<__nv_bfloat16>(a, st);
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+  }
   const bool aligned = (reinterpret_cast<uintptr_t>(w) & 15) == 0;
   if (codec == Q4_K && aligned) return launch_shape<Q4_K, 16, true>(out_half, a, st);
   // q6_k rows on 8-byte boundaries (K a multiple of 1024): the producer that requests its bytes a K-step ahead

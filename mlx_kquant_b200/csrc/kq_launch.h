@@ -72,7 +72,10 @@ cudaError_t launch_gather_rows(int codec, int x_dtype, const void* x, long long 
 // bf16 / f32 activations need gemm_workspace_bytes() of scratch for their fp16 copy.
 size_t gemm_workspace_bytes(int x_dtype, long long rows, int K);
 cudaError_t launch_gemm(int codec, int x_dtype, const void* x, long long x_row_stride, void* y, long long y_row_stride,
-                        const uint8_t* w, long long row_bytes, int M, int N, int K, void* workspace, cudaStream_t st);
+                        const uint8_t* w, long long row_bytes, int M, int N, int K, void* workspace,
+                        size_t workspace_bytes, cudaStream_t st);
+// With the room for an fp16 copy of (a part of) the weights where the call would use one.
+size_t gemm_workspace_bytes_n(int codec, int x_dtype, long long rows, int N, int K);
 // Grouped (mixture-of-experts) prefill: 256-row tiles of expert-sorted rows, see kq_gather.cu.
 constexpr int kGroupedTileRows = 256;
 constexpr int kSegMapTileRows = 64;  // rows per entry of an expert tile map (the reference kernel's tile height)

@@ -170,7 +170,15 @@ def quantized_matmul(x, w, scales, kquant_type, transpose=True, *, stream=None):
     y = torch.empty((rows, outer), dtype=out_dtype, device=w.device)
     L = _lib.lib()
     ws_bytes = L.kq_quantized_matmul_workspace_bytes(_DT[x.dtype], rows, K)
-    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=w.device) if ws_bytes else None
+    if transpose and rows > 16:  # many rows: perhaps room for an fp16 copy of the weights, if the device has it
+        most = L.kq_quantized_matmul_workspace_bytes_for(kquant_type.encode(), _DT[x.dtype], rows, outer, K)
+        try:
+            ws = torch.empty(most, dtype=torch.uint8, device=w.device) if most else None
+            ws_bytes = most
+        except torch.OutOfMemoryError:
+            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=w.device) if ws_bytes else None
+    else:
+        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=w.device) if ws_bytes else None
     _order_on(stream, w.device, ws, x2, w2, y)
     with torch.cuda.device(w.device):
         check(L.kq_quantized_matmul(x2.data_ptr(), _DT[x.dtype], rows, K, x2.stride(0), w2.data_ptr(),

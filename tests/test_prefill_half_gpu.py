@@ -1,0 +1,37 @@
+"""More than sixteen rows on matrices that are dequantized to fp16 once and multiplied tile by tile (kq_gemm.cu)."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import x_to_torch, y_to_f32
+from oracle.kq_oracle import Oracle
+
+pytestmark = pytest.mark.gpu
+
+# (codec, m, n, k): the smallest matrices of the rule with ragged rows and columns, K not a whole number of K-steps,
+# K split over a cluster, two row blocks, and an fp16 copy made in two parts (128 MiB)
+CASES = [("q5_k", 17, 4099, 1024), ("q8_0", 130, 2051, 2080), ("iq4_xs", 300, 1025, 4096), ("q4_0", 64, 1024, 8192),
+         ("q3_k", 513, 4100, 1280), ("q6_k", 40, 2051, 2304), ("q6_k", 1027, 1056, 4096), ("q2_k", 33, 9000, 8192)]
+
+
+@pytest.mark.parametrize("codec,m,n,k", CASES)
+@pytest.mark.parametrize("dt", ["f16", "bf16", "f32"])
+def test_half_copy_against_float64(codec, m, n, k, dt):
+    import mlx_kquant_b200 as kq
+
+    rng = np.random.default_rng(m * 31 + n + k)
+    some = kq.quantize(torch.from_numpy(rng.standard_normal((64, k)).astype(np.float32) * 0.05), codec)[0].numpy()
+    pick = rng.integers(0, 64, n)
+    x, _ = x_to_torch(rng.standard_normal((m, k)).astype(np.float32), dt)
+    xr = (x.bfloat16() if dt == "f32" else x).double().cpu().numpy()
+    ref = (xr @ Oracle().dequantize(some, codec, "f32").astype(np.float64).T)[:, pick]
+    w = torch.from_numpy(some[pick]).cuda()
+    y = y_to_f32(kq.quantized_matmul(x, w, None, codec)).astype(np.float64)
+    # one rounding of a weight to fp16 is at most 2^-11 of it: over K random terms at most that of the product's root
+    # mean square, six of them for the largest of many outputs; then half a unit of the output type
+    off = np.abs(y - ref) - (2.0 ** -11 if dt == "f16" else 2.0 ** -8) * np.abs(ref)
+    assert off.max() < 6 * 2.0 ** -11 * np.sqrt(np.mean(ref ** 2))
+    # without the room for the copy the same call takes the fused kernel
+    lib = kq._lib.lib()
+    assert lib.kq_quantized_matmul_workspace_bytes_for(codec.encode(), 1, m, n, k) > \
+        lib.kq_quantized_matmul_workspace_bytes(1, m, k)
