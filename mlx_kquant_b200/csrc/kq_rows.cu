@@ -57,7 +57,7 @@ __host__ __device__ constexpr bool rw_min(int c) { return c == Q4_K || c == Q5_K
 __host__ __device__ constexpr bool rw_al16(int c) { return c == Q4_K || c == Q5_K; }
 // what the operand of integer 0 stands for, to be subtracted: the bf16 pattern's 128, and the codec's own offset
 template <int C, bool BF>
-__host__ __device__ constexpr int rw_base() { return (BF ? 128 : 0) + (C == Q6_K ? 32 : 0); }
+__host__ __device__ constexpr int rw_base() { return C == IQ4_XS ? 0 : (BF ? 128 : 0) + (C == Q6_K ? 32 : 0); }
 template <int C, bool BF>
 __host__ __device__ constexpr bool rw_sums() { return rw_min(C) || rw_base<C, BF>() != 0; }
 // words per (superblock, activation row) of the sums: heads, tails, padding against bank conflicts
@@ -92,6 +92,19 @@ __device__ __forceinline__ void rw_mma(float (&c)[4], uint32_t a0, uint32_t a1, 
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+// the same with accumulators of zero (constants: no registers to clear)
+__device__ __forceinline__ void rw_mma0(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                        uint32_t b1, __half) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+__device__ __forceinline__ void rw_mma0(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                        uint32_t b1, __nv_bfloat16) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
 __device__ __forceinline__ void rw_mma_tf32(float (&c)[4], const float (&a)[4], float b0, float b1) {
   asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
@@ -116,7 +129,7 @@ template <int C, typename XT, int NT>
 struct RowsUnit {
   static constexpr bool kBf = std::is_same<XT, __nv_bfloat16>::value;
   static constexpr uint32_t kMagic = kBf ? 0x37373737u : 0u;
-  static constexpr float kUp = 16777216.f;                     // operands are scaled by 2^-24
+  static constexpr float kUp = C == IQ4_XS ? 1.f : 16777216.f;  // operands are scaled by 2^-24
   static constexpr float kSumUp = kBf ? 16777216.f : 1.f;      // and so are the sums of bf16 rows
   static constexpr int kBase = rw_base<C, kBf>();
   static constexpr int kP = rw_sum_pitch(C);
@@ -151,11 +164,15 @@ struct RowsUnit {
     }
   }
   // four weights of either row (one byte each) against b[n] = four activations of column n
+  template <bool FIRST>
   static __device__ __forceinline__ void four(float (&c)[NT][4], uint32_t qa, uint32_t qb, const uint32_t (&b)[NT][2]) {
     const uint32_t a0 = __byte_perm(qa, kMagic, 0x4140), a2 = __byte_perm(qa, kMagic, 0x4342);
     const uint32_t a1 = __byte_perm(qb, kMagic, 0x4140), a3 = __byte_perm(qb, kMagic, 0x4342);
 #pragma unroll
-    for (int n = 0; n < NT; n++) rw_mma(c[n], a0, a1, a2, a3, b[n][0], b[n][1], XT());
+    for (int n = 0; n < NT; n++) {
+      if constexpr (FIRST) rw_mma0(c[n], a0, a1, a2, a3, b[n][0], b[n][1], XT());
+      else rw_mma(c[n], a0, a1, a2, a3, b[n][0], b[n][1], XT());
+    }
   }
   static __device__ __forceinline__ void scale_add(float (&acc)[NT][4], const float (&c)[NT][4], float s0, float s1) {
 #pragma unroll
@@ -200,10 +217,8 @@ struct RowsUnit {
           return q;
         };
         float c[NT][4];
-#pragma unroll
-        for (int n = 0; n < NT; n++) c[n][0] = c[n][1] = c[n][2] = c[n][3] = 0.f;
-        four(c, nib(wa.x, u0.x), nib(wb.x, u1.x), b0);
-        four(c, nib(wa.y, u0.y), nib(wb.y, u1.y), b1);
+        four<true>(c, nib(wa.x, u0.x), nib(wb.x, u1.x), b0);
+        four<false>(c, nib(wa.y, u0.y), nib(wb.y, u1.y), b1);
         scale_add(acc, c, rw_byte(p < 2 ? s0.scl : s0.sch, j & 3), rw_byte(p < 2 ? s1.scl : s1.sch, j & 3));
       }
     }
@@ -297,9 +312,7 @@ struct RowsUnit {
             }
           }
           float c[NT][4];
-#pragma unroll
-          for (int n = 0; n < NT; n++) c[n][0] = c[n][1] = c[n][2] = c[n][3] = 0.f;
-          four(c, q[0], q[1], b);
+          four<true>(c, q[0], q[1], b);
           scale_add(acc, c, rw_byte(sc0[j >> 2], j & 3, 8388736.f), rw_byte(sc1[j >> 2], j & 3, 8388736.f));
         }
       }
@@ -316,11 +329,56 @@ struct RowsUnit {
     sum_term<16>(y, s, sums, g, t, -kSumUp * kBase * d0, -kSumUp * kBase * d1);
   }
 
+  // iq4_xs (src/kquant_cpu_decode.cpp:557-584): a nibble is one of sixteen levels, small integers that both 16-bit
+  // types hold exactly: their two bytes come out of two sixteen-byte tables, four weights a permute. A halfword of
+  // quant bytes holds the selectors of its four nibbles as they lie (bit 3 chooses the half of the table afterwards).
+  struct Pairs {
+    uint32_t low, high;  // the low nibbles of two bytes, the high nibbles, as 16-bit floats
+  };
+  static __device__ __forceinline__ Pairs iq4_pairs(uint32_t half) {
+    constexpr uint32_t L[2][4] = {{0x103080f0u, 0x00806020u, 0xc0408000u, 0x109050a0u}, {0x82a6d0feu, 0x20b00c44u, 0x18c85080u, 0xe2b28a54u}}, H[2][4] = {{0xd4d5d6d7u, 0xc9cdd0d2u, 0x504e4a3cu, 0x57555452u}, {0xc2c2c2c2u, 0xc1c1c2c2u, 0x4241413fu, 0x42424242u}};
+    const uint32_t sel = half & 0x7777u, pick = 0x3210u | ((half >> 1) & 0x4444u);
+    const uint32_t lo = __byte_perm(__byte_perm(L[kBf][0], L[kBf][1], sel), __byte_perm(L[kBf][2], L[kBf][3], sel), pick);
+    const uint32_t hi = __byte_perm(__byte_perm(H[kBf][0], H[kBf][1], sel), __byte_perm(H[kBf][2], H[kBf][3], sel), pick);
+    return {__byte_perm(lo, hi, 0x6240), __byte_perm(lo, hi, 0x7351)};
+  }
+  static __device__ __forceinline__ void run_iq4(float (&y)[NT][4], const uint8_t* r0, const uint8_t* r1,
+                                                 const uint8_t* (&xb)[NT], int t) {
+    float acc[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; n++) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+    const uint2 h0 = *reinterpret_cast<const uint2*>(r0), h1 = *reinterpret_cast<const uint2*>(r1);
+    // 6-bit scales of the even and the odd sub-blocks, a byte each: four bits of scales_l, two of scales_h
+    auto scales = [](const uint2 h, int odd) {
+      const uint32_t u = (h.x >> 16) >> (2 * odd);
+      const uint32_t top = (u & 3u) | ((u & 0x30u) << 4) | ((u & 0x300u) << 8) | ((u & 0x3000u) << 12);
+      return ((h.y >> (4 * odd)) & 0x0f0f0f0fu) | (top << 4);
+    };
+    const uint32_t s0[2] = {scales(h0, 0), scales(h0, 1)}, s1[2] = {scales(h1, 0), scales(h1, 1)};
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const uint32_t wa = rw_lds(r0 + 8 + 16 * j + 4 * t), wb = rw_lds(r1 + 8 + 16 * j + 4 * t);
+      const Pairs a0 = iq4_pairs(wa), a1 = iq4_pairs(wa >> 16), b0 = iq4_pairs(wb), b1 = iq4_pairs(wb >> 16);
+      float c[NT][4];
+#pragma unroll
+      for (int n = 0; n < NT; n++) {
+        const uint2 v0 = *reinterpret_cast<const uint2*>(xb[n] + 64 * j + 8 * t);
+        const uint2 v1 = *reinterpret_cast<const uint2*>(xb[n] + 64 * j + 32 + 8 * t);
+        rw_mma0(c[n], a0.low, b0.low, a1.low, b1.low, v0.x, v0.y, XT());
+        rw_mma(c[n], a0.high, b0.high, a1.high, b1.high, v1.x, v1.y, XT());
+      }
+      scale_add(acc, c, rw_byte(s0[j & 1], j >> 1, 8388640.f), rw_byte(s1[j & 1], j >> 1, 8388640.f));
+    }
+    finish(y, acc, __half2float(__ushort_as_half((unsigned short)h0.x)), __half2float(__ushort_as_half((unsigned short)h1.x)));
+  }
+
   static __device__ __forceinline__ void run(float (&y)[NT][4], const uint8_t* r0, const uint8_t* r1,
                                              const uint8_t* (&xb)[NT], const float* sums, int g, int t) {
     if constexpr (C == Q6_K) {
       if ((smem_u32(r0) & 2) == 0) run_q6<0>(y, r0, r1, xb, sums, g, t);
       else run_q6<1>(y, r0, r1, xb, sums, g, t);
+    } else if constexpr (C == IQ4_XS) {
+      run_iq4(y, r0, r1, xb, t);
     } else {
       run_k4(y, r0, r1, xb, sums, g, t);
     }
@@ -348,9 +406,9 @@ __device__ __forceinline__ void rows_sums(const uint8_t* xrow, float* out, int l
   float c[NS][4];
 #pragma unroll
   for (int j = 0; j < NS; j++) {
-    c[j][0] = c[j][1] = c[j][2] = c[j][3] = 0.f;
+    rw_mma0(c[j], one, one, one, one, b[j * (16 / NS)].x, b[j * (16 / NS)].y, XT());
 #pragma unroll
-    for (int i = 0; i < 16 / NS; i++) rw_mma(c[j], one, one, one, one, b[j * (16 / NS) + i].x, b[j * (16 / NS) + i].y, XT());
+    for (int i = 1; i < 16 / NS; i++) rw_mma(c[j], one, one, one, one, b[j * (16 / NS) + i].x, b[j * (16 / NS) + i].y, XT());
   }
   if (lane < 4) {
 #pragma unroll
@@ -536,14 +594,19 @@ rows_kernel(const GemvArgs a, const RowsPlan pl, const RowsGather ga, int* __res
       const int p0 = row_of(16 * tile + g), p1 = row_of(16 * tile + g + 8);
       const int l0 = min(p0, rows - 1), l1 = min(p1, rows - 1);  // places past the end read some row, to no effect
       float y[NT][4];
+      int xo[NT];  // this lane's activation rows
 #pragma unroll
-      for (int n = 0; n < NT; n++) y[n][0] = y[n][1] = y[n][2] = y[n][3] = 0.f;
+      for (int n = 0; n < NT; n++) {
+        y[n][0] = y[n][1] = y[n][2] = y[n][3] = 0.f;
+        xo[n] = pl.x_off + min(8 * n + g, m - 1) * pl.xpitch;
+      }
+      const int w0 = l0 * pl.wpitch, w1 = l1 * pl.wpitch;
       for (int st = 0; st < nst; st++) {
         if (ok) ok = wait(kSums ? &ready[s] : &full[s], parity);
         const uint8_t* base = rw_dyn + s * pl.stage_bytes;
         const int here = ok ? min(pl.cs, nsb - st * pl.cs) : 0;
         for (int k = ks; k < here; k += pl.wk) {
-          const uint8_t *r0 = base + l0 * pl.wpitch + k * BPB, *r1 = base + l1 * pl.wpitch + k * BPB;
+          const uint8_t *r0 = base + w0 + k * BPB, *r1 = base + w1 + k * BPB;
           if constexpr (!rw_al16(C)) {  // the bytes of a row start at their offset within a 16-byte word
             // (a place past the end keeps its own offset: all lanes agree modulo four)
             const long long o0 = (long long)(row0 + p0) * a.row_bytes + (long long)st * pl.cs * BPB;
@@ -552,7 +615,7 @@ rows_kernel(const GemvArgs a, const RowsPlan pl, const RowsGather ga, int* __res
           }
           const uint8_t* xb[NT];
 #pragma unroll
-          for (int n = 0; n < NT; n++) xb[n] = base + pl.x_off + min(8 * n + g, m - 1) * pl.xpitch + 512 * k;
+          for (int n = 0; n < NT; n++) xb[n] = base + xo[n] + 512 * k;
           const float* sums = reinterpret_cast<const float*>(base + pl.sum_off) + k * NT * 8 * rw_sum_pitch(C);
           if (!G || NT == 1 || m > 8) {
             RowsUnit<C, XT, NT>::run(y, r0, r1, xb, sums, g, t);
@@ -625,7 +688,7 @@ bool rows_plan(const GemvArgs& a, RowsPlan& p, int units) {
     const int passes = (a.N + sms * 16 * NW - 1) / (sms * 16 * NW);
     r0 = std::max(8, (a.N + sms * passes - 1) / (sms * passes));
   }
-  const bool alternate = !rw_al16(C) && (a.row_bytes & 3) != 0;
+  const bool alternate = (a.row_bytes & 3) != 0;
   if (alternate) r0 = (r0 + 31) & ~31;  // whole tiles of either kind
   // three stages (or all of K), for the gather form rather with fewer rows; two always fit
   for (int want = 3; want >= 2; want--) {
@@ -641,7 +704,7 @@ bool rows_plan(const GemvArgs& a, RowsPlan& p, int units) {
         // 8-byte reads of four rows, or 4-byte reads of eight, in different banks
         while (rw_al16(C) ? (wb & 63) != 32 : (wb & 31) != 16) wb += 16;
         p.wpitch = wb;
-        p.xpitch = p.cs * 512 + (rw_nsub(C) == 8 ? 64 : 32);
+        p.xpitch = p.cs * 512 + (rw_al16(C) ? 64 : 32);  // 16- and 8-byte reads of the B operand
         p.x_off = (p.R * p.wpitch + 127) & ~127;
         p.sum_off = (p.x_off + max_m * p.xpitch + 15) & ~15;
         p.stage_bytes = (p.sum_off + (rw_sums<C, BF>() ? p.cs * NT * 8 * rw_sum_pitch(C) * 4 : 0) + 127) & ~127;
@@ -710,12 +773,14 @@ cudaError_t launch_rows_any(int codec, int x_dtype, const GemvArgs& a, const Row
       case Q4_K: return launch_rows_c<Q4_K, __half>(a, ga, st);
       case Q5_K: return launch_rows_c<Q5_K, __half>(a, ga, st);
       case Q6_K: return launch_rows_c<Q6_K, __half>(a, ga, st);
+      case IQ4_XS: return launch_rows_c<IQ4_XS, __half>(a, ga, st);
     }
   } else {
     switch (codec) {
       case Q4_K: return launch_rows_c<Q4_K, __nv_bfloat16>(a, ga, st);
       case Q5_K: return launch_rows_c<Q5_K, __nv_bfloat16>(a, ga, st);
       case Q6_K: return launch_rows_c<Q6_K, __nv_bfloat16>(a, ga, st);
+      case IQ4_XS: return launch_rows_c<IQ4_XS, __nv_bfloat16>(a, ga, st);
     }
   }
   return cudaErrorInvalidValue;
@@ -724,10 +789,13 @@ cudaError_t launch_rows_any(int codec, int x_dtype, const GemvArgs& a, const Row
 }  // namespace
 
 bool gemv_rows_supported(int codec, int x_dtype, const GemvArgs& a) {
-  if (codec != Q4_K && codec != Q5_K && codec != Q6_K) return false;
+  if (codec != Q4_K && codec != Q5_K && codec != Q6_K && codec != IQ4_XS) return false;
   if (!(x_dtype == F16 || x_dtype == BF16) || a.tasks != nullptr || a.bias != nullptr || a.M < 1 || a.M > 16 || a.N < 8 ||
       a.K < 256 || (a.K & 255) != 0 || a.w_align16 == 0 || a.row_bytes != (long long)(a.K >> 8) * bpb_of(codec))
     return false;
+  // iq4_xs: the table lookups (23 instructions for eight weights against 7 of the others) bound it on large matrices:
+  // [1000, 1280] x 2 rows 10.3 -> 3.6 us, but [14336, 4096] 22.7 against 28.9
+  if (codec == IQ4_XS && (long long)a.N * a.K > (4ll << 20)) return false;
   return (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && (a.x_row_stride & 7) == 0;
 }
 
