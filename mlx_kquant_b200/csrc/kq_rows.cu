@@ -5,8 +5,9 @@
 //
 // What bounds it: a tile product is a chain of shared-memory loads, permutes and matrix instructions some 2500 cycles
 // long, with 16 warps on an SM to hide it (without any weight copy [28672, 8192] x 1 row takes 40 of 48 us; without any
-// product 26); HBM is the next bound. Measured [14336, 4096] x 8 bf16 rows: q4_k 17.2 us, q5_k 19.5, q6_k 31 (25.3, 80,
-// 68 on the kernels before it). What it is built around:
+// product 26), half of the issue slots and half of the ALU pipe (byte permutes) busy; HBM is the next bound. Measured
+// [14336, 4096] x 8 bf16 rows: q4_k 17.2 us, q5_k x 16 fp16 rows 22.1; q6_k [4096, 14336] x 8 24.0 (25.3, 80, 97.5 on
+// the kernels before it). What it is built around:
 //   * No value is rounded: a weight is scale x integer (- min), the integer goes into the tensor core as it is and
 //     the scale is applied in float32 to the sum over its 16- or 32-weight sub-block. The bytes become operands
 //     with one byte permute per two weights: for bf16 rows byte q becomes the bf16 number (128 + q) * 2^-24
@@ -75,6 +76,7 @@ struct RowsPlan {
   int R;       // weight rows of a row block
   int rt, wk;  // row tiles of 16, warps to a row tile: rt * wk consumer warps work
   int cs;      // superblocks of a stage; warp column k takes k, k + wk, ...
+  int wlog, xlog;  // log2 of the producer threads on one row of the weights, of x
   int half;    // != 0: tile rows 0 .. half - 1 are the block's even rows, the others its odd ones
   int stages, wpitch, xpitch, stage_bytes, x_off, sum_off, red_off, list_off, smem;
   int n_blocks;
@@ -489,39 +491,40 @@ rows_kernel(const GemvArgs a, const RowsPlan pl, const RowsGather ga, int* __res
     const int total = passes * nst;
     const uint8_t* wend = wmat + (long long)a.N * a.row_bytes;
     int pass_w = 0, st_w = 0, slot_w = 0, pass_x = 0, st_x = 0, slot_x = 0;
-    // Pieces of sixteen bytes, piece q of a stage: row q / per_row, place q % per_row. A thread takes every 128th:
-    // both numbers advance by a constant, no division in the loop.
+    // A row's pieces of sixteen bytes go to neighbouring threads (a power of two of them, 1 << wlog: pl.wlog, pl.xlog),
+    // every thread walks down the rows: two additions a piece (numbering the pieces of a stage and
+    // stepping by the thread count instead: q6_k [4096, 14336] x 8 32 us against 24).
     const int tid = pw * 32 + lane;
     constexpr int kThreads = 32 * kRwProducers;
     auto copy_w = [&]() {
       const int row0 = row_block(pass_w), rows = min(pl.R, a.N - row0), len = min(pl.cs, nsb - st_w * pl.cs) * BPB;
-      const uint32_t dst = smem_u32(rw_dyn + slot_w * pl.stage_bytes);
+      const int step = kThreads >> pl.wlog, r0 = tid >> pl.wlog;
       const uint8_t* src = wmat + (long long)row0 * a.row_bytes + (long long)st_w * pl.cs * BPB;
-      const int rb = (int)a.row_bytes;
-      const int per_row = rw_al16(C) ? len >> 4 : (len + 30) >> 4;  // a window holds at most that many
-      const int dr = kThreads / per_row, dc = kThreads - dr * per_row;
-      int r = tid / per_row, c = tid - r * per_row;
-      if constexpr (rw_al16(C)) {
-        const int n = rows * per_row;
+      const uint32_t dst = smem_u32(rw_dyn + slot_w * pl.stage_bytes);
+      const long long sstep = step * a.row_bytes;
+      const int dstep = step * pl.wpitch;
+      if (rw_al16(C) || (a.row_bytes & 15) == 0) {
+        // every row has the same place within sixteen bytes, and the matrix ends on a whole sixteen
+        const int ph = rw_al16(C) ? 0 : (int)(reinterpret_cast<uintptr_t>(src) & 15);
+        const int per_row = (len + ph + 15) >> 4;
+        for (int c = tid & ((1 << pl.wlog) - 1); c < per_row; c += 1 << pl.wlog) {
+          const uint8_t* p = src - ph + 16 * c + r0 * a.row_bytes;
+          uint32_t d = dst + 16 * c + r0 * pl.wpitch;
 #pragma unroll 4
-        for (int q = tid; q < n; q += kThreads) {
-          rw_cp16(dst + r * pl.wpitch + 16 * c, src + ((long long)r * rb + 16 * c));
-          r += dr, c += dc;
-          if (c >= per_row) c -= per_row, r++;
+          for (int r = r0; r < rows; r += step, p += sstep, d += dstep) rw_cp16(d, p);
         }
       } else {  // the aligned window around the row's bytes; the matrix may end inside it
-        const int n = rows * per_row;
+        const int per_row = (len + 30) >> 4;  // a window holds at most that many
+        for (int c = tid & ((1 << pl.wlog) - 1); c < per_row; c += 1 << pl.wlog) {
+          const uint8_t* p = src + r0 * a.row_bytes;
+          uint32_t d = dst + 16 * c + r0 * pl.wpitch;
 #pragma unroll 4
-        for (int q = tid; q < n; q += kThreads) {
-          const uint8_t* p = src + (long long)r * rb;
-          const int ph = (int)(reinterpret_cast<uintptr_t>(p) & 15);
-          p += 16 * c - ph;
-          if (16 * c < len + ph) {
-            const long long left = wend - p;
-            rw_cp16_upto(dst + r * pl.wpitch + 16 * c, p, left < 16 ? (int)left : 16);
+          for (int r = r0; r < rows; r += step, p += sstep, d += dstep) {
+            const int ph = (int)(reinterpret_cast<uintptr_t>(p) & 15);
+            const uint8_t* q = p - ph + 16 * c;
+            const long long left = wend - q;
+            if (16 * c < len + ph) rw_cp16_upto(d, q, left < 16 ? (int)left : 16);
           }
-          r += dr, c += dc;
-          if (c >= per_row) c -= per_row, r++;
         }
       }
       if (++st_w == nst) st_w = 0, pass_w++;
@@ -529,16 +532,15 @@ rows_kernel(const GemvArgs a, const RowsPlan pl, const RowsGather ga, int* __res
     };
     auto copy_x = [&]() {  // and the arrival of this thread once all its copies of the stage have landed
       const int per_row = min(pl.cs, nsb - st_x * pl.cs) * 32, m = rows_of_x(pass_x);
+      const int step = kThreads >> pl.xlog, r0 = tid >> pl.xlog;
       const uint32_t dst = smem_u32(rw_dyn + slot_x * pl.stage_bytes + pl.x_off);
       const XT* src = static_cast<const XT*>(a.x) + st_x * pl.cs * 256;
-      const int dr = kThreads / per_row, dc = kThreads - dr * per_row;
-      int r = tid / per_row, c = tid - r * per_row;
-#pragma unroll 4
-      for (int q = tid; q < m * per_row; q += kThreads) {
-        const int row = G ? list[entry0(pass_x) + r].x : r;
-        rw_cp16(dst + r * pl.xpitch + 16 * c, src + ((long long)row * a.x_row_stride + 8 * c));
-        r += dr, c += dc;
-        if (c >= per_row) c -= per_row, r++;
+      for (int c = tid & ((1 << pl.xlog) - 1); c < per_row; c += 1 << pl.xlog) {
+#pragma unroll 2
+        for (int r = r0; r < m; r += step) {
+          const int row = G ? list[entry0(pass_x) + r].x : r;
+          rw_cp16(dst + r * pl.xpitch + 16 * c, src + ((long long)row * a.x_row_stride + 8 * c));
+        }
       }
       asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(smem_u32(&full[slot_x])) : "memory");
       if (++st_x == nst) st_x = 0, pass_x++;
@@ -704,6 +706,13 @@ bool rows_plan(const GemvArgs& a, RowsPlan& p, int units) {
         // 8-byte reads of four rows, or 4-byte reads of eight, in different banks
         while (rw_al16(C) ? (wb & 63) != 32 : (wb & 31) != 16) wb += 16;
         p.wpitch = wb;
+        auto log2_of = [&](int pieces) {
+          int l = 0;
+          while ((1 << l) < pieces && (2 << l) <= 32 * RowsShape<G>::kProducers) l++;
+          return l;
+        };
+        p.wlog = log2_of((p.cs * BPB + (rw_al16(C) ? 15 : 30)) >> 4);
+        p.xlog = log2_of(p.cs * 32);
         p.xpitch = p.cs * 512 + (rw_al16(C) ? 64 : 32);  // 16- and 8-byte reads of the B operand
         p.x_off = (p.R * p.wpitch + 127) & ~127;
         p.sum_off = (p.x_off + max_m * p.xpitch + 15) & ~15;
