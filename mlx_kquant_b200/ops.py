@@ -10,6 +10,8 @@ path the benchmark times). All arithmetic happens in the CUDA library behind
 """
 from __future__ import annotations
 
+import contextlib
+
 import torch
 
 from . import _lib
@@ -31,8 +33,14 @@ def codecs() -> list[str]:
     return out
 
 
+_GEOMETRY: dict[str, tuple[int, int, int, bool]] = {}  # of the codecs asked for so far: constants of the registry
+
+
 def codec_geometry(kquant_type: str) -> tuple[int, int, int, bool]:
     """(weights_per_block, bytes_per_block, bits, requires_imatrix) or ValueError."""
+    known = _GEOMETRY.get(kquant_type)
+    if known is not None:
+        return known
     import ctypes as C
 
     L = _lib.lib()
@@ -41,13 +49,25 @@ def codec_geometry(kquant_type: str) -> tuple[int, int, int, bool]:
         raise ValueError(f"[mlx_kquant] Unknown kquant_type: '{kquant_type}'.")
     v = [C.c_int() for _ in range(4)]
     L.kq_codec_info(i, None, *[C.byref(t) for t in v])
-    return v[0].value, v[1].value, v[2].value, bool(v[3].value)
+    return _GEOMETRY.setdefault(kquant_type, (v[0].value, v[1].value, v[2].value, bool(v[3].value)))
 
 
 def _stream_ptr(stream, device) -> int:
     if stream is None:
-        return torch.cuda.current_stream(device).cuda_stream
+        # the handle alone: a torch Stream object for it costs several microseconds of every call
+        index = device.index if device.index is not None else torch.cuda.current_device()
+        return torch._C._cuda_getCurrentRawStream(index)
     return stream.cuda_stream
+
+
+_SAME_DEVICE = contextlib.nullcontext()
+
+
+def _on_device(device):
+    """The context in which to launch on `device`: none where it is the current one."""
+    if device.index is None or device.index == torch.cuda.current_device():
+        return _SAME_DEVICE
+    return torch.cuda.device(device)
 
 
 def _order_on(stream, device, *tensors) -> None:
@@ -85,7 +105,7 @@ def dequantize(w, scales, kquant_type, dtype=None, *, stream=None):
     w_c = w.contiguous()
     out = torch.empty(w.shape[:-1] + (w.shape[-1] // bpb * wpb,), dtype=out_dtype, device=w.device)
     _order_on(stream, w.device, w_c, out)
-    with torch.cuda.device(w.device):
+    with _on_device(w.device):
         check(_lib.lib().kq_dequantize(w_c.data_ptr(), w_c.numel(), kquant_type.encode(), _DT[out_dtype],
                                        out.data_ptr(), _stream_ptr(stream, w.device)))
     return out
@@ -163,13 +183,13 @@ def quantized_matmul(x, w, scales, kquant_type, transpose=True, *, stream=None):
     w2 = w if w.dim() == 2 else w.reshape(-1, w.shape[-2], w.shape[-1])[0]
     w2 = w2.contiguous()
     K = x.shape[-1]
-    x2 = x.reshape(-1, K) if x.dim() != 1 else x.reshape(1, K)
+    x2 = x if x.dim() == 2 else x.reshape(-1, K) if x.dim() != 1 else x.reshape(1, K)
     if x2.stride(-1) != 1 or (x2.stride(0) * x2.element_size()) % 16 != 0 or x2.data_ptr() % 16 != 0:
         x2 = x2.contiguous()
     rows = x2.shape[0]
     y = torch.empty((rows, outer), dtype=out_dtype, device=w.device)
     L = _lib.lib()
-    ws_bytes = L.kq_quantized_matmul_workspace_bytes(_DT[x.dtype], rows, K)
+    ws_bytes = L.kq_quantized_matmul_workspace_bytes(_DT[x.dtype], rows, K) if rows > 1 else 0  # one row needs none
     if transpose and rows > 16:  # many rows: perhaps room for an fp16 copy of the weights, if the device has it
         most = L.kq_quantized_matmul_workspace_bytes_for(kquant_type.encode(), _DT[x.dtype], rows, outer, K)
         try:
@@ -180,12 +200,13 @@ def quantized_matmul(x, w, scales, kquant_type, transpose=True, *, stream=None):
     else:
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=w.device) if ws_bytes else None
     _order_on(stream, w.device, ws, x2, w2, y)
-    with torch.cuda.device(w.device):
+    with _on_device(w.device):
         check(L.kq_quantized_matmul(x2.data_ptr(), _DT[x.dtype], rows, K, x2.stride(0), w2.data_ptr(),
                                     w2.shape[-1], outer, kquant_type.encode(), int(bool(transpose)),
                                     y.data_ptr(), y.stride(0), ws.data_ptr() if ws is not None else None,
                                     ws_bytes, _stream_ptr(stream, w.device)))
-    y = y.reshape(x.shape[:-1] + (outer,))
+    if x2 is not x:
+        y = y.reshape(x.shape[:-1] + (outer,))
     return y.cpu() if on_cpu else y
 
 
@@ -247,7 +268,7 @@ def gather_qmm(x, w, scales, kquant_type, lhs_indices=None, rhs_indices=None, tr
     ws = torch.empty(max(ws_bytes, 256), dtype=torch.uint8, device=dev)
     right_sorted = bool(sorted_indices) and lhs_indices is None
     _order_on(stream, dev, ws, y, x3, w3, lhs32, rhs32)
-    with torch.cuda.device(dev):
+    with _on_device(dev):
         check(L.kq_gather_qmm(x3.data_ptr(), _DT[x.dtype], x3.shape[0], M, K, w3.data_ptr(), E,
                               w3.stride(0) if E > 1 else w3.shape[1] * w3.shape[2], w3.shape[2], outer,
                               kquant_type.encode(), lhs32.data_ptr(), rhs32.data_ptr(), n_entries,
@@ -279,7 +300,7 @@ def expert_tile_map(indices, n_experts, *, stream=None):
     count = torch.zeros(1, dtype=torch.int32, device=dev)
     ws = torch.empty(max(L.kq_expert_tile_map_workspace_bytes(n_experts), 256), dtype=torch.uint8, device=dev)
     _order_on(stream, dev, idx, tile_map, count, ws)
-    with torch.cuda.device(dev):
+    with _on_device(dev):
         check(L.kq_expert_tile_map(idx.data_ptr(), rows, n_experts, tile_map.data_ptr(), count.data_ptr(),
                                    ws.data_ptr(), ws.numel(), _stream_ptr(stream, dev)))
     return tile_map, count
@@ -328,7 +349,7 @@ def gather_qmm_seg(x, w, scales, kquant_type, map, counts, *, stream=None):  # n
     ws = torch.empty(max(L.kq_gather_qmm_seg_workspace_bytes(_DT[x.dtype], rows, K, E, mc.shape[0]), 256),
                      dtype=torch.uint8, device=dev)
     _order_on(stream, dev, xc, wc, mc, cc, ws, y)
-    with torch.cuda.device(dev):
+    with _on_device(dev):
         check(L.kq_gather_qmm_seg(xc.data_ptr(), _DT[x.dtype], rows, K, wc.data_ptr(), E, wc.stride(0), wc.shape[2], N,
                                   kquant_type.encode(), mc.data_ptr(), cc.data_ptr(), mc.shape[0], y.data_ptr(),
                                   ws.data_ptr(), ws.numel(), _stream_ptr(stream, dev)))
@@ -372,7 +393,7 @@ def quantized_matmul_qmv_bias(x, w, scales, bias, kquant_type, *, stream=None):
     bc = bias.to(dev).to(out_dtype).contiguous()
     y = torch.empty(x.shape[:-1] + (N,), dtype=out_dtype, device=dev)
     _order_on(stream, dev, xc, wc, bc, y)
-    with torch.cuda.device(dev):
+    with _on_device(dev):
         check(_lib.lib().kq_quantized_matmul_qmv_bias(xc.data_ptr(), _DT[x.dtype], K, wc.data_ptr(), wc.shape[1], N,
                                                       kquant_type.encode(), bc.data_ptr(), y.data_ptr(),
                                                       _stream_ptr(stream, dev)))
