@@ -130,7 +130,13 @@ __device__ __forceinline__ float ldf16(const uint8_t* p) {
   return __half2float(__ushort_as_half((unsigned short)ld16<A>(p)));
 }
 
-__device__ __forceinline__ float u2f(uint32_t v) { return (float)(int)v; }
+// Small integers to float through the mantissa of 2^23 (exact): one permute or logic instruction and one subtraction
+// where the conversion instruction runs at a quarter of the rate or less. A decode of eight weights had eight of them.
+__device__ __forceinline__ float u2f(uint32_t v) { return __uint_as_float(0x4B000000u | v) - 8388608.f; }  // v < 2^23
+// byte c of w, minus `off`
+__device__ __forceinline__ float b2f(uint32_t w, int c, float off = 0.f) {
+  return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u + c)) - (8388608.f + off);
+}
 
 // Eight 6-bit (scale, min) pairs packed in 12 bytes (q4_k / q5_k),
 // src/kquant_cpu_decode.cpp:155-174. s0..s2 are the three little-endian words.
@@ -161,8 +167,8 @@ __device__ __forceinline__ void decode8(const uint8_t* __restrict__ blk, int j, 
     const uint32_t b = ld32<(A >= 2 ? 2 : 1)>(blk + 6 + 8 * j);
 #pragma unroll
     for (int c = 0; c < 4; c++) {
-      v[c] = d * (float)(int)(int8_t)((a >> (8 * c)) & 0xff);
-      v[c + 4] = d * (float)(int)(int8_t)((b >> (8 * c)) & 0xff);
+      v[c] = d * b2f(a ^ 0x80808080u, c, 128.f);
+      v[c + 4] = d * b2f(b ^ 0x80808080u, c, 128.f);
     }
   } else if constexpr (C == Q4_0 || C == IQ4_NL) {
     // [f16 d][16 B nibbles]: low nibble -> weight i, high nibble -> weight i+16,
@@ -172,14 +178,13 @@ __device__ __forceinline__ void decode8(const uint8_t* __restrict__ blk, int j, 
     const uint8_t* q = blk + 2 + 8 * (j & 1);
     const uint32_t a = ld32<(A >= 2 ? 2 : 1)>(q);
     const uint32_t b = ld32<(A >= 2 ? 2 : 1)>(q + 4);
+    const uint32_t na = (hi ? a >> 4 : a) & 0x0f0f0f0fu, nb = (hi ? b >> 4 : b) & 0x0f0f0f0fu;
 #pragma unroll
     for (int c = 0; c < 8; c++) {
-      const uint32_t byte = ((c < 4 ? a : b) >> (8 * (c & 3))) & 0xff;
-      const uint32_t nib = hi ? (byte >> 4) : (byte & 15u);
       if constexpr (C == Q4_0) {
-        v[c] = d * (float)((int)nib - 8);
+        v[c] = d * b2f(c < 4 ? na : nb, c & 3, 8.f);
       } else {
-        v[c] = d * (float)tabs.iq4nl[nib];
+        v[c] = d * (float)tabs.iq4nl[((c < 4 ? na : nb) >> (8 * (c & 3))) & 15u];
       }
     }
   } else if constexpr (C == Q4_1 || C == Q5_0 || C == Q5_1) {
@@ -197,13 +202,16 @@ __device__ __forceinline__ void decode8(const uint8_t* __restrict__ blk, int j, 
     const uint8_t* q = blk + kQs + 8 * (j & 1);
     const uint32_t a = ld32<(A >= 2 ? 2 : 1)>(q);
     const uint32_t b = ld32<(A >= 2 ? 2 : 1)>(q + 4);
+    uint32_t na = (hi ? a >> 4 : a) & 0x0f0f0f0fu, nb = (hi ? b >> 4 : b) & 0x0f0f0f0fu;
+    if constexpr (C != Q4_1) {  // four bits spread over four bytes by a multiplication
+      const uint32_t u = qh >> (8 * j);
+      na |= (((u & 15u) * 0x00204081u) & 0x01010101u) << 4;
+      nb |= ((((u >> 4) & 15u) * 0x00204081u) & 0x01010101u) << 4;
+    }
 #pragma unroll
     for (int c = 0; c < 8; c++) {
-      const uint32_t byte = ((c < 4 ? a : b) >> (8 * (c & 3))) & 0xff;
-      uint32_t x = hi ? (byte >> 4) : (byte & 15u);
-      if constexpr (C != Q4_1) x |= ((qh >> (8 * j + c)) & 1u) << 4;
-      if constexpr (C == Q5_0) v[c] = d * (float)((int)x - 16);
-      else v[c] = d * (float)x + m;
+      if constexpr (C == Q5_0) v[c] = d * b2f(c < 4 ? na : nb, c & 3, 16.f);
+      else v[c] = d * b2f(c < 4 ? na : nb, c & 3) + m;
     }
   } else if constexpr (C == Q4_K || C == Q5_K) {
     // q4_k: [d][dmin][12 B scales][128 B qs]; q5_k adds qh[32] at +16, qs at +48,
@@ -226,15 +234,13 @@ __device__ __forceinline__ void decode8(const uint8_t* __restrict__ blk, int j, 
       hb = ld32<A>(blk + 20 + i0) >> s;
     }
     const int sh = (s & 1) * 4;
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-      const uint32_t w = c < 4 ? a : b;
-      uint32_t q = (w >> (8 * (c & 3) + sh)) & 15u;
-      if constexpr (C == Q5_K) {
-        q |= (((c < 4 ? ha : hb) >> (8 * (c & 3))) & 1u) << 4;
-      }
-      v[c] = sc * u2f(q) - mn;
+    uint32_t na = (a >> sh) & 0x0f0f0f0fu, nb = (b >> sh) & 0x0f0f0f0fu;
+    if constexpr (C == Q5_K) {
+      na |= (ha & 0x01010101u) << 4;
+      nb |= (hb & 0x01010101u) << 4;
     }
+#pragma unroll
+    for (int c = 0; c < 8; c++) v[c] = sc * b2f(c < 4 ? na : nb, c & 3) - mn;
   } else if constexpr (C == Q6_K) {
     // [ql 128][qh 64][int8 sc 16][f16 d @208], src/kquant_cpu_decode.cpp:238-280
     const float d = ldf16<A>(blk + 208);
@@ -248,14 +254,11 @@ __device__ __forceinline__ void decode8(const uint8_t* __restrict__ blk, int j, 
     const uint32_t ha = ld32<A>(qh), hb = ld32<A>(qh + 4);
     const int is = half * 8 + (l0 >> 4) + 2 * qd;
     const float dsc = d * (float)(int)(int8_t)blk[192 + is];
+    const int nsh = 2 * (qd & 2);
+    const uint32_t qa = ((la >> nsh) & 0x0f0f0f0fu) | (((ha >> (2 * qd)) & 0x03030303u) << 4);
+    const uint32_t qb = ((lb >> nsh) & 0x0f0f0f0fu) | (((hb >> (2 * qd)) & 0x03030303u) << 4);
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-      const uint32_t lw = c < 4 ? la : lb, hw = c < 4 ? ha : hb;
-      const uint32_t lbyte = (lw >> (8 * (c & 3))) & 0xff, hbyte = (hw >> (8 * (c & 3))) & 0xff;
-      const uint32_t lo = (qd & 2) ? (lbyte >> 4) : (lbyte & 15u);
-      const int q = (int)(lo | (((hbyte >> (2 * qd)) & 3u) << 4)) - 32;
-      v[c] = dsc * (float)q;
-    }
+    for (int c = 0; c < 8; c++) v[c] = dsc * b2f(c < 4 ? qa : qb, c & 3, 32.f);
   } else if constexpr (C == Q3_K || C == Q2_K) {
     // q3_k: [hmask 32][qs 64][scales 12][d @108]; q2_k: [scales 16][qs 64][d @80][dmin @82],
     // src/kquant_cpu_decode.cpp:282-377. Output order: half h (128 w), shift si
@@ -274,12 +277,10 @@ __device__ __forceinline__ void decode8(const uint8_t* __restrict__ blk, int j, 
       const uint32_t hi2 = ((uint32_t)s[8 + k] >> (2 * grp)) & 3u;
       const float dl = d * (float)((int)(lo4 | (hi2 << 4)) - 32);
       const uint32_t ma = ld32<A>(blk + e0) >> (h * 4 + si), mb = ld32<A>(blk + e0 + 4) >> (h * 4 + si);
+      const uint32_t qa = (a & 0x03030303u) | ((ma & 0x01010101u) << 2);  // minus 4 where the mask bit is clear
+      const uint32_t qb = (b & 0x03030303u) | ((mb & 0x01010101u) << 2);
 #pragma unroll
-      for (int c = 0; c < 8; c++) {
-        const int q2 = (int)(((c < 4 ? a : b) >> (8 * (c & 3))) & 3u);
-        const int hm = (((c < 4 ? ma : mb) >> (8 * (c & 3))) & 1u) ? 0 : 4;
-        v[c] = dl * (float)(q2 - hm);
-      }
+      for (int c = 0; c < 8; c++) v[c] = dl * b2f(c < 4 ? qa : qb, c & 3, 4.f);
     } else {
       const uint32_t dd = ld32<A>(blk + 80);
       const float d = __half2float(__ushort_as_half((unsigned short)(dd & 0xffff)));
@@ -287,9 +288,7 @@ __device__ __forceinline__ void decode8(const uint8_t* __restrict__ blk, int j, 
       const uint32_t scb = blk[is];
       const float dl = d * u2f(scb & 15u), ml = dmin * u2f(scb >> 4);
 #pragma unroll
-      for (int c = 0; c < 8; c++) {
-        v[c] = dl * u2f(((c < 4 ? a : b) >> (8 * (c & 3))) & 3u) - ml;
-      }
+      for (int c = 0; c < 8; c++) v[c] = dl * b2f((c < 4 ? a : b) & 0x03030303u, c & 3) - ml;
     }
   } else if constexpr (C == IQ4_XS) {
     // [d][u16 scales_h][4 B scales_l][128 B qs], src/kquant_cpu_decode.cpp:441-465

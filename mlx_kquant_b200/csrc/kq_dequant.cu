@@ -143,10 +143,37 @@ dequant_kernel(const uint8_t* __restrict__ w, T* __restrict__ out, long long n_b
       float v[8];
 #pragma unroll
       for (int c = 0; c < 4; c++) {
-        v[c] = sm.x * u2f((n0 >> (8 * c)) & 0xffu) - sm.y;
-        v[c + 4] = sm.x * u2f((n1 >> (8 * c)) & 0xffu) - sm.y;
+        v[c] = sm.x * b2f(n0, c) - sm.y;
+        v[c + 4] = sm.x * b2f(n1, c) - sm.y;
       }
       Pack8<T>::store(out_t + (size_t)o * 8, v, out_vec != 0);
+    }
+    return;
+  }
+  if constexpr (C == Q6_K && A >= 2) {
+    // Weights l, l + 32, l + 64, l + 96 of a half share bytes: a thread makes eight of each from one read of them
+    // (two-byte loads: 14 for 32 weights instead of 40), 256 such units a tile. Same products as decode8<>, exact in
+    // fp32 in any order. [14336, 4096] -> bf16: 43.9 us with decode8 per eight weights.
+    for (int o = threadIdx.x; o < nb * 8; o += kDqThreads) {
+      const uint8_t* bp = tile_s + (o >> 3) * BPB;
+      const int half = (o >> 2) & 1, l0 = (o & 3) * 8;
+      const uint8_t *ql = bp + 64 * half + l0, *qh = bp + 128 + 32 * half + l0;
+      const uint32_t l[2][2] = {{ld32<2>(ql), ld32<2>(ql + 4)}, {ld32<2>(ql + 32), ld32<2>(ql + 36)}};
+      const uint32_t h[2] = {ld32<2>(qh), ld32<2>(qh + 4)};
+      const float d = ldf16<2>(bp + 208);
+      const uint8_t* sc = bp + 192 + 8 * half + (l0 >> 4);
+#pragma unroll
+      for (int qd = 0; qd < 4; qd++) {
+        const float dsc = d * (float)(int)(int8_t)sc[2 * qd];
+        float v[8];
+#pragma unroll
+        for (int p = 0; p < 2; p++) {
+          const uint32_t q = ((l[qd & 1][p] >> (2 * (qd & 2))) & 0x0f0f0f0fu) | (((h[p] >> (2 * qd)) & 0x03030303u) << 4);
+#pragma unroll
+          for (int c = 0; c < 4; c++) v[4 * p + c] = dsc * b2f(q, c, 32.f);
+        }
+        Pack8<T>::store(out_t + (size_t)(o >> 3) * 256 + 128 * half + 32 * qd + l0, v, out_vec != 0);
+      }
     }
     return;
   }
