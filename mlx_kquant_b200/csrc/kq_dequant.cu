@@ -2,22 +2,33 @@
 // reference's CPU decoders (src/kquant_dequantize.cpp:59-91 ->
 // src/kquant_cpu_decode.cpp:1136-1207).
 //
-// HBM-bound streaming kernel. One CTA handles a tile of kTileW consecutive
-// weights: the tile's wire bytes (tile_blocks * bytes_per_block, not a multiple
-// of 16 for most codecs) are brought into shared memory with 16-byte loads that
-// start at the 16-byte boundary below the tile, so global reads are fully
-// coalesced whatever the block size; every thread then decodes eight
-// consecutive weights at a time from shared memory and writes them with one or
-// two 16-byte stores, consecutive threads writing consecutive chunks.
+// HBM-bound streaming kernel. A tile is kTileW consecutive weights: its wire bytes
+// (tile_blocks * bytes_per_block, not a multiple of 16 for most codecs) are brought
+// into shared memory by one bulk copy that starts at the 16-byte boundary below the
+// tile, so global reads are contiguous whatever the block size; every thread then
+// decodes eight consecutive weights at a time from shared memory and writes them with
+// one or two 16-byte stores, consecutive threads writing consecutive chunks. For
+// 16-bit outputs as many CTAs as fit the SMs walk the tiles through two buffers each,
+// so that a tile's bytes are under way while the one before is decoded (a CTA per tile
+// that loads, waits and decodes spends a third of its life on the load: [14336, 4096]
+// -> fp16, q6_k 45 -> 31 us = 5.3 TB/s, q4_k 35 -> 29).
 // Algorithmic bytes per weight: bytes_per_block / weights_per_block read plus
 // sizeof(out type) written.
+#include <algorithm>
+
 #include "kq_common.cuh"
 #include "kq_launch.h"
+#include "kq_imma_q4k.cuh"
+#include "kq_tcgen05.cuh"
 
 namespace kq {
 
 constexpr int kDqThreads = 256;
-constexpr int kTileW = 8192;  // weights per CTA tile
+constexpr int kTileW = 8192;  // weights per tile
+// Two buffers and as many CTAs as fit for 16-bit outputs; float32 outputs, bound by their stores, are faster with a
+// CTA per tile in launch order (q4_k [14336, 4096] 53 us against 65; fp16 35 against 29).
+template <typename T>
+constexpr int dq_bufs() { return sizeof(T) == 4 ? 1 : 2; }
 
 template <typename T>
 struct Pack8;
@@ -25,8 +36,8 @@ template <>
 struct Pack8<float> {
   static __device__ __forceinline__ void store(float* o, const float (&v)[8], bool vec) {
     if (vec) {
-      reinterpret_cast<float4*>(o)[0] = make_float4(v[0], v[1], v[2], v[3]);
-      reinterpret_cast<float4*>(o)[1] = make_float4(v[4], v[5], v[6], v[7]);
+      __stcs(reinterpret_cast<float4*>(o), make_float4(v[0], v[1], v[2], v[3]));
+      __stcs(reinterpret_cast<float4*>(o) + 1, make_float4(v[4], v[5], v[6], v[7]));
     } else {
 #pragma unroll
       for (int i = 0; i < 8; i++) o[i] = v[i];
@@ -67,121 +78,157 @@ struct Pack8<__nv_bfloat16> {
 // the address phase modulo 16.
 template <int C, int A, typename T>
 __global__ void __launch_bounds__(kDqThreads)
-dequant_kernel(const uint8_t* __restrict__ w, T* __restrict__ out, long long n_blocks, int out_vec) {
+dequant_kernel(const uint8_t* __restrict__ w, T* __restrict__ out, long long n_blocks, int out_vec, int* error_word) {
   constexpr int WPB = wpb_of(C), BPB = bpb_of(C);
   constexpr int TB = kTileW / WPB;            // blocks per tile
   constexpr int OPB = WPB / 8;                // octets per block
   constexpr int kStage = TB * BPB + 32;       // tile bytes + phase + round-up
+  constexpr int kBuf = (kStage + 15) & ~15, kBufs = dq_bufs<T>();
   extern __shared__ __align__(16) uint8_t smem[];
-  uint8_t* stage = smem;
+  __shared__ uint64_t full[2];
+  __shared__ int abort_s;
   IqTables tabs = global_iq_tables();
-  if constexpr (C == IQ4_NL || C == IQ4_XS || C == IQ2_XXS) {
-    tabs = stage_iq_tables(smem + ((kStage + 15) & ~15), threadIdx.x, kDqThreads);
-  }
+  if constexpr (C == IQ4_NL || C == IQ4_XS || C == IQ2_XXS)
+    tabs = stage_iq_tables(smem + kBufs * kBuf, threadIdx.x, kDqThreads);
 
-  const long long tile = blockIdx.x;
-  const long long b0 = tile * TB;
-  const int nb = (int)min((long long)TB, n_blocks - b0);
-  if (nb <= 0) return;
-  const uint8_t* src = w + b0 * BPB;
-  const int bytes = nb * BPB;
+  const long long tiles = (n_blocks + TB - 1) / TB;
   const uint8_t* w_end = w + n_blocks * BPB;
-
-  int phase;
-  if constexpr (A >= 2) {
-    // 16-byte loads from the boundary at or below src; a chunk that would run
-    // past the end of the wire buffer is copied byte by byte instead.
-    phase = (int)(reinterpret_cast<uintptr_t>(src) & 15);
-    const uint8_t* a0 = src - phase;
-    const int nchunks = (phase + bytes + 15) >> 4;
-    for (int c = threadIdx.x; c < nchunks; c += kDqThreads) {
-      const uint8_t* g = a0 + 16 * c;
-      if (g + 16 <= w_end) {
-        reinterpret_cast<uint4*>(stage)[c] = *reinterpret_cast<const uint4*>(g);
-      } else {
-        for (int i = 0; i < 16; i++)
-          if (g + i < w_end) stage[16 * c + i] = g[i];
-      }
+  // one bulk copy from the 16-byte boundary at or below the tile; the bytes past the last whole sixteen of the
+  // wire buffer (its last tile only) are stored one by one, before the arrival
+  auto fetch = [&](long long tile, int buf) {
+    const long long b0 = tile * TB;
+    const uint8_t* src = w + b0 * BPB;
+    const uint8_t* end = w + min(b0 + TB, n_blocks) * BPB;
+    const uint8_t* a0 = reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(src) & ~(uintptr_t)15);
+    uint32_t n = (uint32_t)((end - a0 + 15) & ~(long long)15);
+    if (a0 + n > w_end) {
+      n -= 16;
+      for (const uint8_t* q = a0 + n; q < end; q++) smem[buf * kBuf + (q - a0)] = *q;
     }
-  } else {
-    phase = 0;
-    for (int i = threadIdx.x; i < bytes; i += kDqThreads) stage[i] = src[i];
+    st_mbar_expect_tx(&full[buf], n);
+    if (n > 0) st_bulk_g2s(smem + buf * kBuf, a0, n, &full[buf]);
+  };
+  constexpr bool kBulk = A >= 2 && kBufs > 1;
+  if constexpr (kBulk) {
+    if (threadIdx.x == 0) {
+      abort_s = 0;
+      st_mbar_init(&full[0], 1);
+      st_mbar_init(&full[1], 1);
+      asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+      for (int i = 0; i < kBufs; i++)
+        if (blockIdx.x + (long long)i * gridDim.x < tiles) fetch(blockIdx.x + (long long)i * gridDim.x, i);
+    }
   }
   __syncthreads();
+  int it = 0;
+  for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x, it++) {
+    const long long b0 = tile * TB;
+    const int nb = (int)min((long long)TB, n_blocks - b0);
+    const int buf = it % kBufs;
+    uint8_t* stage = smem + buf * kBuf;
+    int phase;
+    if constexpr (A >= 2) {
+      phase = (int)(reinterpret_cast<uintptr_t>(w + b0 * BPB) & 15);
+      if constexpr (kBufs == 1) {
+      // one tile a CTA: sixteen-byte loads by all threads (a bulk copy here: q3_k -> float32 56 us against 49); a chunk
+      // that would run past the end of the wire buffer is copied byte by byte
+      const uint8_t* a0 = w + b0 * BPB - phase;
+      const int nchunks = (phase + nb * BPB + 15) >> 4;
+      for (int c = threadIdx.x; c < nchunks; c += kDqThreads) {
+        const uint8_t* g = a0 + 16 * c;
+        if (g + 16 <= w_end) {
+          reinterpret_cast<uint4*>(stage)[c] = *reinterpret_cast<const uint4*>(g);
+        } else {
+          for (int i = 0; i < 16; i++)
+            if (g + i < w_end) stage[16 * c + i] = g[i];
+        }
+      }
+      __syncthreads();
+    } else if (!mbar_wait_err(&full[buf], (it / kBufs) & 1, &abort_s, 0x200, error_word)) return;
+    } else {
+      phase = 0;
+      const uint8_t* src = w + b0 * BPB;
+      for (int i = threadIdx.x; i < nb * BPB; i += kDqThreads) stage[i] = src[i];
+      __syncthreads();
+    }
 
-  const uint8_t* tile_s = stage + phase;
-  T* out_t = out + b0 * WPB;
-  const int n_oct = nb * OPB;
-  if constexpr ((C == Q4_K || C == Q5_K) && A >= 4) {
-    // The 6-bit scale / min pair of a sub-block serves 32 weights: unpack each pair once per tile
-    // (one per thread: TB * 8 = 256 of them) instead of once per eight weights. Same arithmetic as
-    // decode8<>: sc = d * scale, mn = dmin * min in fp32, v = sc * q - mn (sc * q is exact).
-    float2* scmn = reinterpret_cast<float2*>(smem + ((kStage + 15) & ~15));
-    for (int i = threadIdx.x; i < nb * 8; i += kDqThreads) {
-      const uint8_t* blk = tile_s + (i >> 3) * BPB;
-      const uint32_t h = ld32<A>(blk);
-      const float d = __half2float(__ushort_as_half((unsigned short)(h & 0xffff)));
-      const float dmin = __half2float(__ushort_as_half((unsigned short)(h >> 16)));
-      uint32_t rsc, rmn;
-      k4_scale_min(ld32<A>(blk + 4), ld32<A>(blk + 8), ld32<A>(blk + 12), i & 7, rsc, rmn);
-      scmn[i] = make_float2(d * u2f(rsc), dmin * u2f(rmn));
-    }
-    __syncthreads();
-    for (int o = threadIdx.x; o < n_oct; o += kDqThreads) {
-      const int blk = o / OPB, j = o % OPB;
-      const int sb = j >> 2, i0 = (j & 3) * 8;
-      const float2 sm = scmn[blk * 8 + sb];
-      const uint8_t* bp = tile_s + blk * BPB;
-      const uint8_t* qs = bp + (C == Q4_K ? 16 : 48) + (sb >> 1) * 32 + i0;
-      const int sh = (sb & 1) * 4;
-      // four nibbles per word in the low halves of its bytes, then one conversion per byte
-      uint32_t n0 = (ld32<A>(qs) >> sh) & 0x0f0f0f0fu, n1 = (ld32<A>(qs + 4) >> sh) & 0x0f0f0f0fu;
-      if constexpr (C == Q5_K) {
-        n0 |= ((ld32<A>(bp + 16 + i0) >> sb) & 0x01010101u) << 4;
-        n1 |= ((ld32<A>(bp + 20 + i0) >> sb) & 0x01010101u) << 4;
+    const uint8_t* tile_s = stage + phase;
+    T* out_t = out + b0 * WPB;
+    const int n_oct = nb * OPB;
+    if constexpr ((C == Q4_K || C == Q5_K) && A >= 4) {
+      // The 6-bit scale / min pair of a sub-block serves 32 weights: unpack each pair once per tile
+      // (one per thread: TB * 8 = 256 of them) instead of once per eight weights. Same arithmetic as
+      // decode8<>: sc = d * scale, mn = dmin * min in fp32, v = sc * q - mn (sc * q is exact).
+      float2* scmn = reinterpret_cast<float2*>(smem + kBufs * kBuf);
+      for (int i = threadIdx.x; i < nb * 8; i += kDqThreads) {
+        const uint8_t* blk = tile_s + (i >> 3) * BPB;
+        const uint32_t h = ld32<A>(blk);
+        const float d = __half2float(__ushort_as_half((unsigned short)(h & 0xffff)));
+        const float dmin = __half2float(__ushort_as_half((unsigned short)(h >> 16)));
+        uint32_t rsc, rmn;
+        k4_scale_min(ld32<A>(blk + 4), ld32<A>(blk + 8), ld32<A>(blk + 12), i & 7, rsc, rmn);
+        scmn[i] = make_float2(d * u2f(rsc), dmin * u2f(rmn));
       }
-      float v[8];
-#pragma unroll
-      for (int c = 0; c < 4; c++) {
-        v[c] = sm.x * b2f(n0, c) - sm.y;
-        v[c + 4] = sm.x * b2f(n1, c) - sm.y;
-      }
-      Pack8<T>::store(out_t + (size_t)o * 8, v, out_vec != 0);
-    }
-    return;
-  }
-  if constexpr (C == Q6_K && A >= 2) {
-    // Weights l, l + 32, l + 64, l + 96 of a half share bytes: a thread makes eight of each from one read of them
-    // (two-byte loads: 14 for 32 weights instead of 40), 256 such units a tile. Same products as decode8<>, exact in
-    // fp32 in any order. [14336, 4096] -> bf16: 43.9 us with decode8 per eight weights.
-    for (int o = threadIdx.x; o < nb * 8; o += kDqThreads) {
-      const uint8_t* bp = tile_s + (o >> 3) * BPB;
-      const int half = (o >> 2) & 1, l0 = (o & 3) * 8;
-      const uint8_t *ql = bp + 64 * half + l0, *qh = bp + 128 + 32 * half + l0;
-      const uint32_t l[2][2] = {{ld32<2>(ql), ld32<2>(ql + 4)}, {ld32<2>(ql + 32), ld32<2>(ql + 36)}};
-      const uint32_t h[2] = {ld32<2>(qh), ld32<2>(qh + 4)};
-      const float d = ldf16<2>(bp + 208);
-      const uint8_t* sc = bp + 192 + 8 * half + (l0 >> 4);
-#pragma unroll
-      for (int qd = 0; qd < 4; qd++) {
-        const float dsc = d * (float)(int)(int8_t)sc[2 * qd];
+      __syncthreads();
+      for (int o = threadIdx.x; o < n_oct; o += kDqThreads) {
+        const int blk = o / OPB, j = o % OPB;
+        const int sb = j >> 2, i0 = (j & 3) * 8;
+        const float2 sm = scmn[blk * 8 + sb];
+        const uint8_t* bp = tile_s + blk * BPB;
+        const uint8_t* qs = bp + (C == Q4_K ? 16 : 48) + (sb >> 1) * 32 + i0;
+        const int sh = (sb & 1) * 4;
+        // four nibbles per word in the low halves of its bytes, then one conversion per byte
+        uint32_t n0 = (ld32<A>(qs) >> sh) & 0x0f0f0f0fu, n1 = (ld32<A>(qs + 4) >> sh) & 0x0f0f0f0fu;
+        if constexpr (C == Q5_K) {
+          n0 |= ((ld32<A>(bp + 16 + i0) >> sb) & 0x01010101u) << 4;
+          n1 |= ((ld32<A>(bp + 20 + i0) >> sb) & 0x01010101u) << 4;
+        }
         float v[8];
 #pragma unroll
-        for (int p = 0; p < 2; p++) {
-          const uint32_t q = ((l[qd & 1][p] >> (2 * (qd & 2))) & 0x0f0f0f0fu) | (((h[p] >> (2 * qd)) & 0x03030303u) << 4);
-#pragma unroll
-          for (int c = 0; c < 4; c++) v[4 * p + c] = dsc * b2f(q, c, 32.f);
+        for (int c = 0; c < 4; c++) {
+          v[c] = sm.x * b2f(n0, c) - sm.y;
+          v[c + 4] = sm.x * b2f(n1, c) - sm.y;
         }
-        Pack8<T>::store(out_t + (size_t)(o >> 3) * 256 + 128 * half + 32 * qd + l0, v, out_vec != 0);
+        Pack8<T>::store(out_t + (size_t)o * 8, v, out_vec != 0);
+      }
+    } else if constexpr (C == Q6_K && A >= 2 && sizeof(T) == 2) {
+      // Weights l, l + 32, l + 64, l + 96 of a half share bytes: a thread makes eight of each from one read of them
+      // (two-byte loads: 14 for 32 weights instead of 40), 256 such units a tile. Same products as decode8<>, exact in
+      // fp32 in any order. 16-bit outputs only: their 64-byte runs cost nothing, those of float32 a third.
+      for (int o = threadIdx.x; o < nb * 8; o += kDqThreads) {
+        const uint8_t* bp = tile_s + (o >> 3) * BPB;
+        const int half = (o >> 2) & 1, l0 = (o & 3) * 8;
+        const uint8_t *ql = bp + 64 * half + l0, *qh = bp + 128 + 32 * half + l0;
+        const uint32_t l[2][2] = {{ld32<2>(ql), ld32<2>(ql + 4)}, {ld32<2>(ql + 32), ld32<2>(ql + 36)}};
+        const uint32_t h[2] = {ld32<2>(qh), ld32<2>(qh + 4)};
+        const float d = ldf16<2>(bp + 208);
+        const uint8_t* sc = bp + 192 + 8 * half + (l0 >> 4);
+#pragma unroll
+        for (int qd = 0; qd < 4; qd++) {
+          const float dsc = d * (float)(int)(int8_t)sc[2 * qd];
+          float v[8];
+#pragma unroll
+          for (int p = 0; p < 2; p++) {
+            const uint32_t q = ((l[qd & 1][p] >> (2 * (qd & 2))) & 0x0f0f0f0fu) | (((h[p] >> (2 * qd)) & 0x03030303u) << 4);
+#pragma unroll
+            for (int c = 0; c < 4; c++) v[4 * p + c] = dsc * b2f(q, c, 32.f);
+          }
+          Pack8<T>::store(out_t + (size_t)(o >> 3) * 256 + 128 * half + 32 * qd + l0, v, out_vec != 0);
+        }
+      }
+    } else {
+      for (int o = threadIdx.x; o < n_oct; o += kDqThreads) {
+        const int blk = o / OPB, j = o % OPB;
+        float v[8];
+        decode8<C, A>(tile_s + blk * BPB, j, v, tabs);
+        Pack8<T>::store(out_t + (size_t)o * 8, v, out_vec != 0);
       }
     }
-    return;
-  }
-  for (int o = threadIdx.x; o < n_oct; o += kDqThreads) {
-    const int blk = o / OPB, j = o % OPB;
-    float v[8];
-    decode8<C, A>(tile_s + blk * BPB, j, v, tabs);
-    Pack8<T>::store(out_t + (size_t)o * 8, v, out_vec != 0);
+    __syncthreads();  // the buffer has been read
+    if constexpr (kBulk) {
+      if (threadIdx.x == 0 && tile + (long long)kBufs * gridDim.x < tiles)
+        fetch(tile + (long long)kBufs * gridDim.x, buf);
+    }
   }
 }
 
@@ -191,9 +238,23 @@ static cudaError_t launch_one(const uint8_t* w, void* out, long long n_blocks, c
   const long long tiles = (n_blocks + TB - 1) / TB;
   if (tiles == 0) return cudaSuccess;
   static_assert(kIqSmemBytes >= (kTileW / 256) * 8 * 8, "the k-quant scale table shares the IQ table area");
-  const int smem = ((TB * BPB + 32 + 15) & ~15) + kIqSmemBytes;
+  const int smem = dq_bufs<T>() * ((TB * BPB + 32 + 15) & ~15) + kIqSmemBytes;
   const int out_vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-  dequant_kernel<C, A, T><<<(unsigned)tiles, kDqThreads, smem, st>>>(w, static_cast<T*>(out), n_blocks, out_vec);
+  static int resident[16] = {};  // CTAs that fit the device at once
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 16) return cudaErrorInvalidDevice;
+  if (resident[dev] == 0) {
+    int per_sm = 0, sms = 0;
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dequant_kernel<C, A, T>, kDqThreads, smem);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    resident[dev] = std::max(1, per_sm * sms);
+  }
+  int* err = device_error_word();
+  if (err == nullptr) return cudaErrorUnknown;
+  dequant_kernel<C, A, T><<<(unsigned)(dq_bufs<T>() == 1 ? tiles : std::min<long long>(tiles, resident[dev])), kDqThreads, smem, st>>>(
+      w, static_cast<T*>(out), n_blocks, out_vec, err);
   return cudaGetLastError();
 }
 

@@ -878,6 +878,49 @@ __device__ __forceinline__ uint4 cvt_scale8(const uint4& q, float s1, float s2) 
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
 constexpr int kCvtChunks = 8;
+// A CTA per row, for calls with fewer rows than the SMs hold warps: a row's chunks are then read by 256 threads at once
+// instead of one after the other by 32 (61 rows of 8192 bf16: the call 110.9 -> 106.9 us); with 2300 rows
+// it is 3 us slower. Dense rows only.
+template <typename XT>
+__global__ void __launch_bounds__(256)
+convert_rows_kernel(const XT* __restrict__ x, long long x_row_stride, int K, __half* __restrict__ xh,
+                    float* __restrict__ row_scale) {
+  __shared__ float s_max[8];
+  const XT* xr = x + blockIdx.x * x_row_stride;
+  __half* o = xh + blockIdx.x * (long long)K;
+  const int nch = K >> 3;
+  uint4 keep[kCvtChunks];  // further chunks are read again
+  float mx = 0.f;
+#pragma unroll
+  for (int j = 0; j < kCvtChunks; j++) {
+    const int c = threadIdx.x + 256 * j;
+    if (c < nch) {
+      keep[j] = cvt_load8_bf16<XT>(xr + 8 * c);
+      mx = cvt_finite_absmax(mx, keep[j]);  // infinities propagate on their own, the factor comes from the finite values
+    }
+  }
+  for (int c = threadIdx.x + 256 * kCvtChunks; c < nch; c += 256) mx = cvt_finite_absmax(mx, cvt_load8_bf16<XT>(xr + 8 * c));
+  for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+  if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  mx = s_max[0];
+#pragma unroll
+  for (int i = 1; i < 8; i++) mx = fmaxf(mx, s_max[i]);
+  // normalised as in convert_x_kernel; 2^-e in two exact halves, since it can overflow float32
+  int e = 0;
+  if (mx > 0.f) e = ilogbf(mx) - 14;
+  const int eh = (-e) / 2;
+  const float down1 = ldexpf(1.f, eh), down2 = ldexpf(1.f, -e - eh);
+  if (threadIdx.x == 0) row_scale[blockIdx.x] = ldexpf(1.f, e);
+#pragma unroll
+  for (int j = 0; j < kCvtChunks; j++) {
+    const int c = threadIdx.x + 256 * j;
+    if (c < nch) *reinterpret_cast<uint4*>(o + 8 * c) = cvt_scale8(keep[j], down1, down2);
+  }
+  for (int c = threadIdx.x + 256 * kCvtChunks; c < nch; c += 256)
+    *reinterpret_cast<uint4*>(o + 8 * c) = cvt_scale8(cvt_load8_bf16<XT>(xr + 8 * c), down1, down2);
+}
+
 template <typename XT, bool GLU>
 __global__ void __launch_bounds__(256, 3)
 convert_x_kernel(const XT* __restrict__ x, long long x_row_stride, int K, __half* __restrict__ xh,
@@ -956,6 +999,10 @@ static void launch_convert_t(const void* x, long long x_row_stride, int K, long 
     if constexpr (sizeof(XT) == 2)
       convert_x_kernel<XT, true><<<gv, 256, 0, st>>>(xp, x_row_stride, K, o, row_scale, order, lhs, lhs_div, M, yrow,
                                                      n_valid, rows);
+  } else if (vec && !std::is_same<XT, __half>::value && order == nullptr && lhs == nullptr &&
+             n_valid == nullptr && rows <= 148 * 4) {
+    if constexpr (!std::is_same<XT, __half>::value)
+      convert_rows_kernel<XT><<<(unsigned)rows, 256, 0, st>>>(xp, x_row_stride, K, o, row_scale);
   } else if (vec) {
     convert_x_kernel<XT, false><<<gv, 256, 0, st>>>(xp, x_row_stride, K, o, row_scale, order, lhs, lhs_div, M, yrow,
                                                     n_valid, rows);
@@ -1174,11 +1221,12 @@ static size_t half_bytes(int N, int K) { return (2 * (size_t)half_chunk(N, K) * 
 // weights several times slower than the tensor cores use them, whatever the number of rows: the copy wins from the
 // first row on, once the matrix outweighs its extra launch. Measured, fused against copy: q5_k [14336, 4096] x 64 rows
 // 326 / 91 us, q8_0 x 512 444 / 87, iq4_xs x 32 190 / 75, q4_0 [4096, 4096] x 300 129 / 53; q5_k [1000, 1280] x 130
-// 17.7 / 19.5. q6_k, whose producer nearly keeps up: [14336, 4096] x 2048 310 / 267, [4096, 14336] x 512 125 / 182.
-// q4_k never: x 2048 247 / 261.
+// 17.7 / 19.5. q6_k, whose producer nearly keeps up, from 257 rows on (a second row block for the fused kernel): [14336, 4096] x 256
+// 75.7 / 76.0, x 512 143 / 85, x 8192 1119 / 930; [4096, 14336] x 256 68 / 116, x 384 116 / 106. q4_k never: x 2048
+// 247 / 261.
 static bool use_half(int codec, long long M, int N, int K) {
   if (codec == Q4_K || (long long)N * K < (4ll << 20)) return false;
-  if (codec == Q6_K && (K & 1023) == 0) return M >= 1024;
+  if (codec == Q6_K && (K & 1023) == 0) return M > 256;
   return true;
 }
 size_t gemm_workspace_bytes_n(int codec, int x_dtype, long long rows, int N, int K) {
