@@ -921,8 +921,10 @@ convert_rows_kernel(const XT* __restrict__ x, long long x_row_stride, int K, __h
     *reinterpret_cast<uint4*>(o + 8 * c) = cvt_scale8(cvt_load8_bf16<XT>(xr + 8 * c), down1, down2);
 }
 
-template <typename XT, bool GLU>
-__global__ void __launch_bounds__(256, 3)
+// CH: chunks of a lane that stay in registers. Rows of at most 1024 values need four, which lets twice the warps reside:
+// a row is a chain of loads, a reduction and stores, and only other rows hide it.
+template <typename XT, bool GLU, int CH>
+__global__ void __launch_bounds__(256, CH == 4 ? 6 : 3)
 convert_x_kernel(const XT* __restrict__ x, long long x_row_stride, int K, __half* __restrict__ xh,
                  float* __restrict__ row_scale, const int* __restrict__ order, const uint32_t* __restrict__ lhs,
                  int lhs_div, int M, int* __restrict__ yrow, const int* __restrict__ n_valid, long long rows) {
@@ -950,26 +952,26 @@ convert_x_kernel(const XT* __restrict__ x, long long x_row_stride, int K, __half
       for (int c = lane; c < nch; c += 32) *reinterpret_cast<uint4*>(o + 8 * c) = cvt_fetch8<XT, GLU>(xr, K, c);
       if (lane == 0) row_scale[row] = 1.f;
     } else {
-      uint4 keep[kCvtChunks];  // the row's values as bf16 pairs (they are bf16 values: nothing is lost)
+      uint4 keep[CH];  // the row's values as bf16 pairs (they are bf16 values: nothing is lost)
       __nv_bfloat162 m2 = __floats2bfloat162_rn(0.f, 0.f);
   #pragma unroll
-      for (int j = 0; j < kCvtChunks; j++) {
+      for (int j = 0; j < CH; j++) {
         const int c = lane + 32 * j;
         if (c < nch) {
           keep[j] = cvt_fetch8<XT, GLU>(xr, K, c);
           m2 = cvt_absmax(m2, keep[j]);
         }
       }
-      for (int c = lane + 32 * kCvtChunks; c < nch; c += 32) m2 = cvt_absmax(m2, cvt_fetch8<XT, GLU>(xr, K, c));
+      for (int c = lane + 32 * CH; c < nch; c += 32) m2 = cvt_absmax(m2, cvt_fetch8<XT, GLU>(xr, K, c));
       float mx = fmaxf(__low2float(m2), __high2float(m2));
       for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
       if (!(mx < INFINITY)) {
         // a row with infinities: they propagate on their own, the factor comes from the finite values
         mx = 0.f;
   #pragma unroll
-        for (int j = 0; j < kCvtChunks; j++)
+        for (int j = 0; j < CH; j++)
           if (lane + 32 * j < nch) mx = cvt_finite_absmax(mx, keep[j]);
-        for (int c = lane + 32 * kCvtChunks; c < nch; c += 32) mx = cvt_finite_absmax(mx, cvt_fetch8<XT, GLU>(xr, K, c));
+        for (int c = lane + 32 * CH; c < nch; c += 32) mx = cvt_finite_absmax(mx, cvt_fetch8<XT, GLU>(xr, K, c));
         for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
       }
       // Every row is normalised (see the scalar kernel); 2^-e in two exact halves, since it can overflow float32.
@@ -979,11 +981,11 @@ convert_x_kernel(const XT* __restrict__ x, long long x_row_stride, int K, __half
       const float down1 = ldexpf(1.f, eh), down2 = ldexpf(1.f, -e - eh);
       if (lane == 0) row_scale[row] = ldexpf(1.f, e);
   #pragma unroll
-      for (int j = 0; j < kCvtChunks; j++) {
+      for (int j = 0; j < CH; j++) {
         const int c = lane + 32 * j;
         if (c < nch) *reinterpret_cast<uint4*>(o + 8 * c) = cvt_scale8(keep[j], down1, down2);
       }
-      for (int c = lane + 32 * kCvtChunks; c < nch; c += 32)
+      for (int c = lane + 32 * CH; c < nch; c += 32)
         *reinterpret_cast<uint4*>(o + 8 * c) = cvt_scale8(cvt_fetch8<XT, GLU>(xr, K, c), down1, down2);
     }
   }
@@ -997,15 +999,15 @@ static void launch_convert_t(const void* x, long long x_row_stride, int K, long 
   const unsigned gv = (unsigned)std::min<long long>((rows + 7) / 8, 148 * 64);  // strided beyond; a lower cap left a thin second pass
   if (glu) {
     if constexpr (sizeof(XT) == 2)
-      convert_x_kernel<XT, true><<<gv, 256, 0, st>>>(xp, x_row_stride, K, o, row_scale, order, lhs, lhs_div, M, yrow,
-                                                     n_valid, rows);
+      (K <= 1024 ? convert_x_kernel<XT, true, 4> : convert_x_kernel<XT, true, kCvtChunks>)<<<gv, 256, 0, st>>>(
+          xp, x_row_stride, K, o, row_scale, order, lhs, lhs_div, M, yrow, n_valid, rows);
   } else if (vec && !std::is_same<XT, __half>::value && order == nullptr && lhs == nullptr &&
              n_valid == nullptr && rows <= 148 * 4) {
     if constexpr (!std::is_same<XT, __half>::value)
       convert_rows_kernel<XT><<<(unsigned)rows, 256, 0, st>>>(xp, x_row_stride, K, o, row_scale);
   } else if (vec) {
-    convert_x_kernel<XT, false><<<gv, 256, 0, st>>>(xp, x_row_stride, K, o, row_scale, order, lhs, lhs_div, M, yrow,
-                                                    n_valid, rows);
+    (K <= 1024 ? convert_x_kernel<XT, false, 4> : convert_x_kernel<XT, false, kCvtChunks>)<<<gv, 256, 0, st>>>(
+        xp, x_row_stride, K, o, row_scale, order, lhs, lhs_div, M, yrow, n_valid, rows);
   } else {
     convert_x_scalar_kernel<XT><<<(unsigned)rows, 256, 0, st>>>(xp, x_row_stride, K, o, row_scale, order, lhs, M, yrow,
                                                                 n_valid);

@@ -94,17 +94,30 @@ __global__ void __launch_bounds__(256) combine_kernel(const T* __restrict__ d, c
   const long long t = blockIdx.x;
   for (int c = threadIdx.x * 8; c < H; c += blockDim.x * 8) {
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int j = 0; j < k; j++) {
-      const float w = p[t * k + j];
-      if (w == 0.f) continue;
-      if (idx != nullptr && idx[t * k + j] >= n_experts) continue;
-      const uint4 v = *reinterpret_cast<const uint4*>(d + (t * k + j) * (long long)H + c);
-      const uint32_t vw[4] = {v.x, v.y, v.z, v.w};
+    // four rows are requested before the first is used; a row whose weight is zero or whose expert is out of range is
+    // not read (one row after the other, each behind the look at its weight: 4096 x 8 rows of 2048 33 us)
+    for (int j0 = 0; j0 < k; j0 += 4) {
+      float w[4];
+      uint4 v[4];
+      bool on[4];
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const float2 f = pair_to_float<T>(vw[q]);
-        acc[2 * q] = fmaf(w, f.x, acc[2 * q]);
-        acc[2 * q + 1] = fmaf(w, f.y, acc[2 * q + 1]);
+      for (int u = 0; u < 4; u++) {
+        w[u] = j0 + u < k ? p[t * k + j0 + u] : 0.f;
+        on[u] = w[u] != 0.f && (idx == nullptr || idx[t * k + j0 + u] < n_experts);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (on[u]) v[u] = *reinterpret_cast<const uint4*>(d + (t * k + j0 + u) * (long long)H + c);
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        if (!on[u]) continue;
+        const uint32_t vw[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const float2 f = pair_to_float<T>(vw[q]);
+          acc[2 * q] = fmaf(w[u], f.x, acc[2 * q]);
+          acc[2 * q + 1] = fmaf(w[u], f.y, acc[2 * q + 1]);
+        }
       }
     }
     store8<OT>(y + t * (long long)H + c, acc);

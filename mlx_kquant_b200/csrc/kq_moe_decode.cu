@@ -554,7 +554,10 @@ __device__ __forceinline__ float md_logit(const void* p, int dtype, long long i)
   return __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]);
 }
 
-// One warp per token; lane l holds experts l, l + 32, ... (E <= 1024: at most 32 per lane).
+// One warp per token; lane l holds experts l, l + 32, ... (E <= 32 NI: at most NI per lane). With arrays of 32 whatever
+// E, the arg-max rounds over 128 experts spent seven of eight comparisons on places that hold none (4096 tokens, top 8:
+// 21 us).
+template <int NI>
 __global__ void __launch_bounds__(256) router_topk_kernel(const RouterArgs a) {
   // the kernel that consumes the indices may start its prologue now; it reads them again after this grid is done
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
@@ -562,11 +565,11 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const RouterArgs a) {
   const int token = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (token >= a.T) return;
   const long long row = (long long)token * (a.E + a.shared);
-  float p[32], rk[32];
+  float p[NI], rk[NI];
   float gsum = 1.f;
   if (a.scoring == 1) {   // sqrt(softplus(x)), softplus in its overflow-free form
 #pragma unroll
-    for (int i = 0; i < 32; i++) {
+    for (int i = 0; i < NI; i++) {
       const int e = lane + 32 * i;
       float v = -INFINITY;
       if (e < a.E) {
@@ -578,7 +581,7 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const RouterArgs a) {
   } else {
     float m = -INFINITY;
 #pragma unroll
-    for (int i = 0; i < 32; i++) {
+    for (int i = 0; i < NI; i++) {
       const int e = lane + 32 * i;
       p[i] = e < a.E ? md_logit(a.logits, a.dtype, row + e) : -INFINITY;
       m = fmaxf(m, p[i]);
@@ -587,7 +590,7 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const RouterArgs a) {
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     float s = 0.f;
 #pragma unroll
-    for (int i = 0; i < 32; i++) {
+    for (int i = 0; i < NI; i++) {
       const int e = lane + 32 * i;
       const float v = e < a.E ? expf(p[i] - m) : 0.f;
       p[i] = e < a.E ? v : -INFINITY;
@@ -598,7 +601,7 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const RouterArgs a) {
     gsum = s;
   }
 #pragma unroll
-  for (int i = 0; i < 32; i++) {
+  for (int i = 0; i < NI; i++) {
     const int e = lane + 32 * i;
     rk[i] = (a.bias != nullptr && e < a.E) ? p[i] + a.bias[e] : p[i];
   }
@@ -609,7 +612,7 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const RouterArgs a) {
     float bv = -INFINITY;
     uint32_t bi = 0xffffffffu;
 #pragma unroll
-    for (int i = 0; i < 32; i++) {   // ascending expert index within the lane: '>' keeps the lowest on ties
+    for (int i = 0; i < NI; i++) {   // ascending expert index within the lane: '>' keeps the lowest on ties
       if (rk[i] > bv) {
         bv = rk[i];
         bi = (uint32_t)(lane + 32 * i);
@@ -627,7 +630,7 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const RouterArgs a) {
     // the emitted score is the unbiased one; its owner lane removes the expert from the ranking
     float pv = 0.f;
 #pragma unroll
-    for (int i = 0; i < 32; i++) {
+    for (int i = 0; i < NI; i++) {
       if ((uint32_t)(lane + 32 * i) == bi) {
         pv = p[i];
         rk[i] = -INFINITY;
@@ -863,7 +866,9 @@ cudaError_t launch_router_topk(const void* logits, int dtype, int T, int E, int 
                                cudaStream_t st) {
   if (T <= 0) return cudaSuccess;
   RouterArgs a{logits, dtype, T, E, top_k, norm, shared, scoring, pes, bias, scale, indices, scores};
-  router_topk_kernel<<<(T + 7) / 8, 256, 0, st>>>(a);
+  const int warps = T <= 4 * 148 ? 2 : 8;  // few tokens: spread over the SMs
+  auto kern = E <= 128 ? router_topk_kernel<4> : E <= 256 ? router_topk_kernel<8> : router_topk_kernel<32>;
+  kern<<<(T + warps - 1) / warps, 32 * warps, 0, st>>>(a);
   return cudaGetLastError();
 }
 
