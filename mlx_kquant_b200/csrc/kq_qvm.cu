@@ -130,7 +130,7 @@ qvm_kernel(const XT* __restrict__ x, long long x_row_stride, void* __restrict__ 
 // and multiplies up to eight of them per pass over the weights, so a weight is decoded once for eight rows where the
 // kernel above decodes it for each. A warp's halves take two rows of W at a time, a lane eight columns; the partial
 // sums meet by one shuffle and in shared memory. Bound by the decode arithmetic and the latency of its byte loads;
-// 64 heads [128, 512] q6_k, eight rows each: 39.7 -> 6 us a launch.
+// 64 heads [128, 512] q6_k, eight rows each: 39.6 -> 9.7 us a launch.
 constexpr int kRowCols = 128, kRowM = 8;
 constexpr int kRowEntries = 512;  // every CTA looks through all entries
 template <int C, int A, typename XT>
@@ -152,7 +152,7 @@ qvm_rows_kernel(const XT* __restrict__ x, void* __restrict__ y, const uint8_t* _
   __syncthreads();
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   const uint32_t e = blockIdx.y;
-  const int count = collect_entries<kThreads>(gq.rhs, gq.lhs, n_entries, gq.x_batch, e, list, &count_s);
+  const int count = collect_entries<kThreads>(gq.rhs, gq.lhs, n_entries, gq.x_batch, e, list, &count_s, gridDim.z > 1);
   if (count == 0) return;
   w += (long long)e * gq.expert_stride;
 
@@ -176,7 +176,7 @@ qvm_rows_kernel(const XT* __restrict__ x, void* __restrict__ y, const uint8_t* _
         xs[k][t] = t < m ? load_x<XT>(x + (long long)list[e0 + t].x * K + kb + k) : 0.f;
       }
       __syncthreads();
-#pragma unroll 2
+#pragma unroll 4
       for (int k = 2 * warp + half; k < kn; k += 2 * kWarps) {
         float v[8];
         decode8<C, A>(w + (long long)(kb + k) * row_bytes + blk_off, oct, v, tabs);
@@ -216,8 +216,8 @@ cudaError_t launch_rows(const void* x, void* y, const uint8_t* w, long long row_
                         const QvmGather& gq, int n_entries) {
   cudaLaunchConfig_t cfg = {};
   const int ctas = (N + kRowCols - 1) / kRowCols * gq.n_experts;
-  // routing may be uneven: where the SMs would not be full anyway, several CTAs share a matrix's entries
-  const int share = std::max(1, std::min((n_entries + kRowM - 1) / kRowM, 4 * 148 / ctas));
+  // routing may be uneven: while the CTAs are hardly more than reside at once, several share a matrix's entries
+  const int share = std::max(1, std::min((n_entries + kRowM - 1) / kRowM, 3 * 148 / ctas));
   cfg.gridDim = dim3((N + kRowCols - 1) / kRowCols, gq.n_experts, share);
   cfg.blockDim = dim3(kThreads);
   cfg.stream = st;

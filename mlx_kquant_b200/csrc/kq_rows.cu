@@ -471,7 +471,8 @@ rows_kernel(const GemvArgs a, const RowsPlan pl, const RowsGather ga, int* __res
     asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the routing may come from the kernel before this one
     const uint32_t e = ga.by_entry ? ga.rhs[blockIdx.y] : blockIdx.y;
     if (e >= (uint32_t)ga.n_experts) return;
-    total_m = collect_entries<RowsShape<G>::kThreads>(ga.rhs, ga.lhs, ga.n_entries, ga.x_batch, e, list, &count_s);
+    total_m = collect_entries<RowsShape<G>::kThreads>(ga.rhs, ga.lhs, ga.n_entries, ga.x_batch, e, list, &count_s,
+                                                      ga.by_entry || gridDim.z > 1);
     if (total_m == 0 || (ga.by_entry && list[0].y != (int)blockIdx.y)) return;
     wmat += (long long)e * ga.expert_stride;
     passes = ((total_m + 8 * NT - 1) / (8 * NT) - (int)blockIdx.z + (int)gridDim.z - 1) / (int)gridDim.z;
@@ -750,9 +751,9 @@ cudaError_t launch_rows_nt(const GemvArgs& a, const RowsGather& ga, cudaStream_t
   int* err = device_error_word();
   if (err == nullptr) return cudaErrorUnknown;
   cudaLaunchConfig_t cfg = {};
-  // routing may be uneven: where the SMs would not be full anyway, several CTAs share a matrix's entries
+  // routing may be uneven: while all CTAs are resident at once, several share a matrix's entries
   int share = 1;
-  if (G) share = std::max(1, std::min((ga.n_entries + 8 * NT - 1) / (8 * NT), 4 * rows_sm_count() / (p.n_blocks * units)));
+  if (G) share = std::max(1, std::min((ga.n_entries + 8 * NT - 1) / (8 * NT), RowsShape<G>::kCtas * rows_sm_count() / (p.n_blocks * units)));
   cfg.gridDim = G ? dim3(p.n_blocks, units, share) : dim3(std::min(p.n_blocks, rows_sm_count()), 1, 1);
   cfg.blockDim = dim3(RowsShape<G>::kThreads);
   cfg.dynamicSmemBytes = p.smem;
