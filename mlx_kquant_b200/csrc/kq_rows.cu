@@ -817,6 +817,9 @@ cudaError_t launch_gemv_rows(int codec, int x_dtype, const GemvArgs& a, cudaStre
 bool gather_rows_supported(int codec, int x_dtype, const void* x, int M, int K, const uint8_t* w, long long expert_stride,
                            long long row_bytes, int N, long long n_entries, int n_experts) {
   if (M != 1 || n_entries > kRwMaxEntries || n_experts > 65535 || (expert_stride & 15) != 0) return false;
+  // q4_k has a grouped kernel of its own that spreads a busy expert's rows over more CTAs: 512 rows over 128 experts
+  // [1536, 2048] evenly at random 126 us there and 105 here, but 118 and 152 with a fifth of the rows in one expert
+  if (codec == Q4_K && (long long)N * K > (1 << 20) && n_entries > 2ll * n_experts) return false;
   GemvArgs a{};
   a.x = x;
   a.x_row_stride = K;
