@@ -213,7 +213,11 @@ qvm_rows_kernel(const XT* __restrict__ x, void* __restrict__ y, const uint8_t* _
 
 template <int C, int A, typename XT>
 cudaError_t launch_rows(const void* x, void* y, const uint8_t* w, long long row_bytes, int N, int K, cudaStream_t st,
-                        const QvmGather& gq, int n_entries) {
+                        QvmGather gq, int n_entries) {
+  // the kernel counts its entries from 0: a slice of a longer call starts at its own indices and outputs
+  gq.lhs += gq.entry0;
+  gq.rhs += gq.entry0;
+  y = static_cast<uint16_t*>(y) + gq.entry0 * N;  // both output types have two bytes
   cudaLaunchConfig_t cfg = {};
   const int ctas = (N + kRowCols - 1) / kRowCols * gq.n_experts;
   // routing may be uneven: while the CTAs are hardly more than reside at once, several share a matrix's entries

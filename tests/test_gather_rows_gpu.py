@@ -64,3 +64,21 @@ def test_entries_out_of_range_stay_unwritten(transpose):
     keep = torch.ones(entries, dtype=torch.bool, device="cuda")
     keep[3] = keep[5] = False
     assert torch.equal(y[keep], good[keep]) and (y[~keep] == 7.0).all()
+
+
+def test_last_slice_of_a_long_call():
+    """[K, N] weights take at most 65535 entries a launch: the entries of the second one are its own."""
+    import mlx_kquant_b200 as kq
+
+    rng = np.random.default_rng(11)
+    E, k, n, tail = 4, 32, 32, 9   # the second slice fits the shared decode: at least E entries, at most 512
+    wire = kq.quantize(torch.from_numpy(rng.standard_normal((E * k, n)).astype(np.float32)), "q8_0")[0]
+    dense = Oracle().dequantize(wire.numpy(), "q8_0", "f32").astype(np.float64).reshape(E, k, n)
+    entries = 65535 + tail
+    x = torch.from_numpy(rng.standard_normal((64, 1, k))).half()
+    lhs, rhs = rng.integers(0, 64, entries), rng.integers(0, E, entries)
+    y = kq.gather_qmm(x.cuda(), wire.reshape(E, k, -1).cuda(), None, "q8_0", lhs_indices=torch.from_numpy(lhs).cuda(),
+                      rhs_indices=torch.from_numpy(rhs).cuda(), transpose=False)[:, 0].double().cpu().numpy()
+    ref = np.einsum("ek,ekn->en", x[:, 0].double().numpy()[lhs], dense[rhs])
+    # half a unit of fp16, and float32 sums of 32 terms
+    assert (np.abs(y - ref) <= 2.0 ** -11 * np.abs(ref) + 2.0 ** -18 * np.sqrt(np.mean(ref ** 2))).all()
