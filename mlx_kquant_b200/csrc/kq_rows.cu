@@ -433,6 +433,29 @@ __device__ __forceinline__ void rows_sums(const uint8_t* xrow, float* out, int l
   }
 }
 
+// One output by itself: decoded weights times activations in float32, as the generic kernel has it. For outputs that
+// the split into integers, offsets and sub-block sums leaves without a finite value although they may have one, or an
+// infinity: an infinite activation meets the offset's sum (inf - inf), and a sum of integers can overflow before its
+// scale is applied. Rare, so one thread an output, without care for speed.
+template <int C, typename XT>
+__device__ __noinline__ float rows_plain(const uint8_t* w, const XT* x, int nsb) {
+  constexpr int A = rw_al16(C) ? 16 : (C == IQ4_XS ? 8 : 2);
+  const IqTables tabs = global_iq_tables();
+  float sum = 0.f;
+#pragma unroll 1
+  for (int o = 0; o < 32 * nsb; o++) {
+    float v[8];
+    decode8<C, A>(w + (long long)(o >> 5) * bpb_of(C), o & 31, v, tabs);
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      float xv;
+      if constexpr (std::is_same<XT, __half>::value) xv = __half2float(x[8 * o + i]);
+      else xv = __bfloat162float(x[8 * o + i]);
+      sum = fmaf(xv, v[i], sum);
+    }
+  }
+  return sum;
+}
 
 template <int C, typename XT, int NT, bool G>
 __global__ void __launch_bounds__(RowsShape<G>::kThreads, RowsShape<G>::kCtas)
@@ -648,8 +671,12 @@ rows_kernel(const GemvArgs a, const RowsPlan pl, const RowsGather ga, int* __res
           if (r < rows) {
             float v = 0.f;
             for (int k = 0; k < pl.wk; k++) v += red[(long long)(k * rp + place) * kRedPitch + c];
+            const int2 entry = G ? list[entry0(pass) + c] : make_int2(c, c);  // (row of x, row of y)
+            if (!(fabsf(v) < INFINITY))
+              v = rows_plain<C, XT>(wmat + (row0 + r) * a.row_bytes,
+                                    static_cast<const XT*>(a.x) + entry.x * a.x_row_stride, nsb);
             if (a.row_scale != nullptr) v *= a.row_scale[c];
-            const int orow = G ? list[entry0(pass) + c].y : c;
+            const int orow = entry.y;
             const long long o = (long long)orow * a.y_row_stride + row0 + r;
             if (kBf || a.out_bf16) static_cast<__nv_bfloat16*>(a.y)[o] = __float2bfloat16_rn(v);
             else static_cast<__half*>(a.y)[o] = __float2half_rn(v);

@@ -57,3 +57,51 @@ def test_rows_largest_finite_bf16():
         ref = x.double().numpy() @ Oracle().dequantize(w.numpy(), codec, "f32").astype(np.float64).T
         y = kq.quantized_matmul(x.cuda(), w.cuda(), None, codec).double().cpu().numpy()
         _close(y, ref, 2.0 ** -8)
+
+
+def _gathered(x, w, codec):
+    """The same product as a gather of one row per entry from a stack of one matrix."""
+    import mlx_kquant_b200 as kq
+
+    at = torch.arange(x.shape[0], dtype=torch.int32, device="cuda")
+    return kq.gather_qmm(x[:, None], w[None], None, codec, lhs_indices=at, rhs_indices=torch.zeros_like(at))[:, 0]
+
+
+@pytest.mark.parametrize("codec", ["q4_k", "q5_k", "q6_k", "iq4_xs"])
+@pytest.mark.parametrize("dt", ["f16", "bf16", "f32"])
+@pytest.mark.parametrize("m,k", [(5, 1024), (12, 768)])
+@pytest.mark.parametrize("gather", [False, True])
+def test_rows_not_finite(codec, dt, m, k, gather):
+    """Infinite activations give signed infinities (NaN where the weight is zero), NaN gives NaN, and the rows beside
+    them are as ever."""
+    import mlx_kquant_b200 as kq
+
+    if gather and dt == "f32":
+        pytest.skip("another kernel's range")
+    rng = np.random.default_rng(m * 7 + k)
+    wire = kq.quantize(torch.from_numpy(rng.standard_normal((40, k)).astype(np.float32) * 0.05), codec)[0]
+    x_f32 = rng.standard_normal((m, k)).astype(np.float32)
+    x_f32[0, 37], x_f32[1, k - 1], x_f32[2, 300] = np.inf, -np.inf, np.nan
+    x, _ = x_to_torch(x_f32, dt)
+    xr = (x.bfloat16() if dt == "f32" else x).double().cpu().numpy()
+    with np.errstate(invalid="ignore"):
+        ref = xr @ Oracle().dequantize(wire.numpy(), codec, "f32").astype(np.float64).T
+    y = _gathered(x, wire.cuda(), codec) if gather else kq.quantized_matmul(x, wire.cuda(), None, codec)
+    y = y_to_f32(y).astype(np.float64)
+    np.testing.assert_array_equal(y[:3], ref[:3])
+    for r in range(3, m):
+        _close(y[r], ref[r], 2.0 ** -11 if dt == "f16" else 2.0 ** -8)
+
+
+@pytest.mark.parametrize("codec", ["q4_k", "q5_k", "q6_k", "iq4_xs"])
+@pytest.mark.parametrize("gather", [False, True])
+def test_rows_of_one_sign_near_the_largest_bf16(codec, gather):
+    """Sums of offset integers overflow long before the products of weights and activations do."""
+    import mlx_kquant_b200 as kq
+
+    rng = np.random.default_rng(6)
+    w = kq.quantize(torch.from_numpy(rng.standard_normal((64, 512)).astype(np.float32) * 1e-3), codec)[0]
+    x = (torch.from_numpy(rng.standard_normal((4, 512))).abs().clamp(max=3) * 1e38).bfloat16()
+    ref = x.double().numpy() @ Oracle().dequantize(w.numpy(), codec, "f32").astype(np.float64).T
+    y = _gathered(x.cuda(), w.cuda(), codec) if gather else kq.quantized_matmul(x.cuda(), w.cuda(), None, codec)
+    _close(y.double().cpu().numpy(), ref, 2.0 ** -8)
