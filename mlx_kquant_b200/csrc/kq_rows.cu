@@ -10,11 +10,12 @@
 // the kernels before it). What it is built around:
 //   * No value is rounded: a weight is scale x integer (- min), the integer goes into the tensor core as it is and
 //     the scale is applied in float32 to the sum over its 16- or 32-weight sub-block. The bytes become operands
-//     with one byte permute per two weights: for bf16 rows byte q becomes the bf16 number (128 + q) * 2^-24
-//     (0x3700 | q), for fp16 rows the subnormal q * 2^-24 (the power of two keeps the sums of the largest finite bf16
-//     rows finite); what the constant offset adds (and the min term of the codecs that have one) is coefficient_j *
-//     (sum of the activations of sub-block j), a product of its own with tf32 instructions over the float32 sums
-//     split in two parts. The sums of a stage are made once per CTA by a helper warp.
+//     with one byte permute per two weights: for bf16 rows byte q becomes the bf16 number 128 + q (0x4300 | q), for
+//     fp16 rows the subnormal q * 2^-24; what the constant offset adds (and the min term of the codecs that have one)
+//     is coefficient_j * (sum of the activations of sub-block j), a product of its own with tf32 instructions over the
+//     float32 sums split in two parts. The sums of a stage are made once per CTA by helper warps. No operand is scaled
+//     down, so that products with the smallest normal bf16 activations stay normal float32 numbers (with 128 + q scaled
+//     by 2^-24, rows of 1e-36 came out with tens of times their size); sums that overflow are caught by rows_plain.
 //   * One CTA per SM owns N / SM count consecutive weight rows (rows are independent, so tiles need not be whole) and
 //     walks K in stages of WK superblocks: four producer warps bring the stage's bytes of every row, and the
 //     activations of that K range, into shared memory with 16-byte asynchronous copies, three or more stages in
@@ -130,9 +131,9 @@ __device__ __forceinline__ uint32_t rw_lds(const uint8_t* p) { return *reinterpr
 template <int C, typename XT, int NT>
 struct RowsUnit {
   static constexpr bool kBf = std::is_same<XT, __nv_bfloat16>::value;
-  static constexpr uint32_t kMagic = kBf ? 0x37373737u : 0u;
-  static constexpr float kUp = C == IQ4_XS ? 1.f : 16777216.f;  // operands are scaled by 2^-24
-  static constexpr float kSumUp = kBf ? 16777216.f : 1.f;      // and so are the sums of bf16 rows
+  static constexpr uint32_t kMagic = kBf ? 0x43434343u : 0u;
+  static constexpr float kUp = C == IQ4_XS || kBf ? 1.f : 16777216.f;  // fp16 operands are scaled by 2^-24
+  static constexpr float kSumUp = kBf ? 1.f / 8192.f : 1.f;  // the sums of bf16 rows by 2^13: tails of small ones stay normal
   static constexpr int kBase = rw_base<C, kBf>();
   static constexpr int kP = rw_sum_pitch(C);
 
@@ -392,7 +393,7 @@ struct RowsUnit {
 template <int C, typename XT>
 __device__ __forceinline__ void rows_sums(const uint8_t* xrow, float* out, int lane) {
   constexpr int NS = rw_nsub(C), P = rw_sum_pitch(C);
-  constexpr uint32_t one = std::is_same<XT, __half>::value ? 0x3C003C00u : 0x33803380u;
+  constexpr uint32_t one = std::is_same<XT, __half>::value ? 0x3C003C00u : 0x46004600u;
   const int t = lane & 3;
   uint2 b[16];  // all loads before the first store: the compiler cannot tell that they do not overlap
 #pragma unroll

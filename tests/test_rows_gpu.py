@@ -59,6 +59,20 @@ def test_rows_largest_finite_bf16():
         _close(y, ref, 2.0 ** -8)
 
 
+@pytest.mark.parametrize("codec", ["q4_k", "q5_k", "q6_k", "iq4_xs"])
+@pytest.mark.parametrize("m", [3, 13])
+def test_rows_of_small_bf16(codec, m):
+    """Rows of 5e-35 (2^-114), whose products with the weights are normal float32 numbers still."""
+    import mlx_kquant_b200 as kq
+
+    rng = np.random.default_rng(7)
+    w = kq.quantize(torch.from_numpy(rng.standard_normal((64, 512)).astype(np.float32) * 0.5), codec)[0]
+    x = (torch.from_numpy(rng.standard_normal((m, 512))) * 2.0 ** -114).bfloat16()
+    ref = x.double().numpy() @ Oracle().dequantize(w.numpy(), codec, "f32").astype(np.float64).T
+    y = kq.quantized_matmul(x.cuda(), w.cuda(), None, codec).double().cpu().numpy()
+    _close(y * 2.0 ** 114, ref * 2.0 ** 114, 2.0 ** -8)
+
+
 def _gathered(x, w, codec):
     """The same product as a gather of one row per entry from a stack of one matrix."""
     import mlx_kquant_b200 as kq
