@@ -1291,8 +1291,9 @@ cudaError_t launch_gemm(int codec, int x_dtype, const void* x, long long x_row_s
   }
   const bool out_half = x_dtype == F16;
   const size_t base = gemm_workspace_bytes(x_dtype, M, K);
-  if (use_half(codec, M, N, K) && workspace != nullptr && workspace_bytes >= base + half_bytes(N, K) &&
-      row_bytes == (long long)(K / kCodecs[codec].wpb) * kCodecs[codec].bpb) {
+  // fp16 rows need no workspace: one that cannot hold the copy, for its size or its alignment, is left alone
+  if (use_half(codec, M, N, K) && workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255) == 0 &&
+      workspace_bytes >= base + half_bytes(N, K) && row_bytes == (long long)(K / kCodecs[codec].wpb) * kCodecs[codec].bpb) {
     uint8_t* wh = static_cast<uint8_t*>(workspace) + base;
     const int chunk = half_chunk(N, K);
     for (int n0 = 0; n0 < N; n0 += chunk) {

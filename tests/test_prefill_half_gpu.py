@@ -31,7 +31,27 @@ def test_half_copy_against_float64(codec, m, n, k, dt):
     # mean square, six of them for the largest of many outputs; then half a unit of the output type
     off = np.abs(y - ref) - (2.0 ** -11 if dt == "f16" else 2.0 ** -8) * np.abs(ref)
     assert off.max() < 6 * 2.0 ** -11 * np.sqrt(np.mean(ref ** 2))
-    # without the room for the copy the same call takes the fused kernel
+
+
+def test_unaligned_workspace_of_fp16_rows():
+    """fp16 rows need no workspace: a large one off the 256-byte grid is no error, the call does without the copy."""
+    import mlx_kquant_b200 as kq
+
     lib = kq._lib.lib()
-    assert lib.kq_quantized_matmul_workspace_bytes_for(codec.encode(), 1, m, n, k) > \
-        lib.kq_quantized_matmul_workspace_bytes(1, m, k)
+    m, n, k = 24, 1024, 4096
+    rng = np.random.default_rng(3)
+    wire = kq.quantize(torch.from_numpy(rng.standard_normal((n, k)).astype(np.float32) * 0.05), "q8_0")[0]
+    x = torch.from_numpy(rng.standard_normal((m, k))).half().cuda()
+    want = kq.quantized_matmul(x, wire.cuda(), None, "q8_0")
+    room = lib.kq_quantized_matmul_workspace_bytes_for(b"q8_0", kq.ops._DT[torch.float16], m, n, k)
+    assert room > 0
+    ws = torch.empty(room + 256, dtype=torch.uint8, device="cuda")
+    y, w = torch.empty_like(want), wire.cuda()
+    for shift in (0, 8):
+        y.zero_()
+        kq._lib.check(lib.kq_quantized_matmul(
+            x.data_ptr(), kq.ops._DT[torch.float16], m, k, k, w.data_ptr(), w.shape[1], n, b"q8_0", 1, y.data_ptr(), n,
+            ws.data_ptr() + shift, room, torch.cuda.current_stream().cuda_stream))
+        # both kernels multiply the same fp16 weights; sums in another order, one rounding to fp16
+        ref = want.double()
+        assert ((y.double() - ref).abs() <= 2.0 ** -10 * ref.abs() + 1e-5 * ref.square().mean().sqrt()).all()
