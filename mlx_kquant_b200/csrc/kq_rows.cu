@@ -20,7 +20,9 @@
 //     walks K in stages of WK superblocks: four producer warps bring the stage's bytes of every row, and the
 //     activations of that K range, into shared memory with 16-byte asynchronous copies, three or more stages in
 //     flight (one bulk copy per row instead was four times slower: a bulk copy costs the SM some 80 cycles); the consumer warps are RT row tiles x WK superblocks, so that a stage is one tile product per warp.
-//   * The weight copies of the first stages are issued before griddepcontrol.wait.
+//   * Nothing is read before griddepcontrol.wait: the weights may have been written by the kernel before. Copies of the
+//     first stages ahead of the wait were 0.1-0.6 us a launch faster (q4_k bf16 x 8 rows [4096, 4096] 7.1 against 7.3 us,
+//     [14336, 4096] 16.8 against 17.4); fetching them into L2 ahead of it instead was slower than waiting (18.8).
 // Blocks that are not whole numbers of 16 bytes (q6_k) are copied as the 16-byte aligned window around a row's
 // bytes; a block then starts on an even byte, and where that is not a multiple of four the words are taken from the
 // next aligned position, with the sub-block's weights handed to the lanes in another order (the sum over a
@@ -572,8 +574,9 @@ rows_kernel(const GemvArgs a, const RowsPlan pl, const RowsGather ga, int* __res
       if (++slot_x == S) slot_x = 0;
     };
     const int first = min(S, total);
+    // x and, for all that is known here, the weights may come from the kernel before this one
+    if constexpr (!G) asm volatile("griddepcontrol.wait;\n" ::: "memory");
     for (int i = 0; i < first; i++) copy_w();
-    if constexpr (!G) asm volatile("griddepcontrol.wait;\n" ::: "memory");  // x may come from the kernel before this one
     for (int i = 0; i < first; i++) copy_x();
     int parity = 0;
     for (int i = first; i < total; i++) {

@@ -119,3 +119,21 @@ def test_rows_of_one_sign_near_the_largest_bf16(codec, gather):
     ref = x.double().numpy() @ Oracle().dequantize(w.numpy(), codec, "f32").astype(np.float64).T
     y = _gathered(x.cuda(), w.cuda(), codec) if gather else kq.quantized_matmul(x.cuda(), w.cuda(), None, codec)
     _close(y.double().cpu().numpy(), ref, 2.0 ** -8)
+
+
+@pytest.mark.parametrize("codec,m", [("q4_k", 8), ("q6_k", 2), ("q5_k", 16)])
+def test_weights_written_just_before(codec, m):
+    """The weights may come from the kernel before: nothing of them is read ahead of its end."""
+    import mlx_kquant_b200 as kq
+
+    n, k = 4096, 1024
+    rows = torch.randn(2, 256, k, generator=torch.Generator().manual_seed(2)) * 0.05
+    pair = [kq.quantize(r, codec)[0].repeat(n // 256, 1).cuda() for r in rows]
+    x = torch.randn(m, k, dtype=torch.bfloat16, device="cuda")
+    want = [kq.quantized_matmul(x, w, None, codec) for w in pair]
+    buf, got = torch.empty_like(pair[0]), []
+    for i in range(64):
+        buf.copy_(pair[i % 2])
+        got.append(kq.quantized_matmul(x, buf, None, codec))
+    for i, y in enumerate(got):
+        assert torch.equal(y, want[i % 2])
