@@ -447,10 +447,11 @@ __device__ __forceinline__ IqTables stage_iq_tables(uint8_t* smem, int tid, int 
 }
 
 // The entries i of a gather call that multiply by matrix e, with an activation row in range, as (row of x, i), in the
-// order of i if `ordered` (CTAs that share them must agree on it), else in any; all threads of the CTA take part, `count` (shared) starts at 0. n at most 4 * TH.
+// order of i (CTAs that share them must agree on it), in any if there are at most `unordered` of them; all threads of the
+// CTA take part, `count` (shared) starts at 0. n at most 4 * TH.
 template <int TH>
 __device__ __forceinline__ int collect_entries(const uint32_t* __restrict__ rhs, const uint32_t* __restrict__ lhs, int n,
-                                               long long x_batch, uint32_t e, int2* list, int* count, bool ordered) {
+                                               long long x_batch, uint32_t e, int2* list, int* count, int unordered) {
   for (int i = threadIdx.x; i < n; i += TH) {
     if (rhs[i] != e) continue;
     const uint32_t l = lhs[i];
@@ -458,7 +459,7 @@ __device__ __forceinline__ int collect_entries(const uint32_t* __restrict__ rhs,
   }
   __syncthreads();
   const int c = *count;
-  if (!ordered) return c;
+  if (c <= unordered) return c;
   int2 mine[4];
   int rank[4];
 #pragma unroll

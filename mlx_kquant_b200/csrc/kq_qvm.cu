@@ -152,7 +152,7 @@ qvm_rows_kernel(const XT* __restrict__ x, void* __restrict__ y, const uint8_t* _
   __syncthreads();
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   const uint32_t e = blockIdx.y;
-  const int count = collect_entries<kThreads>(gq.rhs, gq.lhs, n_entries, gq.x_batch, e, list, &count_s, gridDim.z > 1);
+  const int count = collect_entries<kThreads>(gq.rhs, gq.lhs, n_entries, gq.x_batch, e, list, &count_s, gridDim.z > 1 ? 0 : n_entries);
   if (count == 0) return;
   w += (long long)e * gq.expert_stride;
 

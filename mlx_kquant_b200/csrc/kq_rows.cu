@@ -68,11 +68,13 @@ __host__ __device__ constexpr bool rw_sums() { return rw_min(C) || rw_base<C, BF
 __host__ __device__ constexpr int rw_sum_pitch(int c) { return 2 * rw_nsub(c) + 4; }
 
 // gather_qmm: entry i multiplies activation row lhs[i] by matrix rhs[i]; grid.y counts the matrices, or (by_entry,
-// fewer entries than matrices) the entries, of which the first of every matrix does the work for all.
+// fewer entries than matrices) the entries, of which the first of every matrix does the work for all. Routing may be
+// uneven: a CTA makes at most `deep` passes over its matrix, and CTAs of y >= units take what is left (rows_left_over).
 struct RowsGather {
   const uint32_t *lhs, *rhs;
   int n_entries, n_experts, by_entry;
   long long x_batch, expert_stride;
+  int units, deep;
 };
 
 struct RowsPlan {
@@ -460,6 +462,40 @@ __device__ __noinline__ float rows_plain(const uint8_t* w, const XT* x, int nsb)
   return sum;
 }
 
+// The matrix and the first pass of left-over group j: the matrices' passes (of `rows` entries) beyond the first `base`,
+// ga.deep of them a group, numbered by matrix. counts: n_experts words of shared memory; all threads of the CTA take
+// part. x: the matrix, or n_experts where there is no such group.
+template <int TH>
+__device__ __forceinline__ int2 rows_left_over(const RowsGather& ga, int rows, int base, int j, int* counts, int2* found) {
+  for (int e = threadIdx.x; e < ga.n_experts; e += TH) counts[e] = 0;
+  if (threadIdx.x == 0) *found = make_int2(ga.n_experts, 0);
+  __syncthreads();
+  for (int i = threadIdx.x; i < ga.n_entries; i += TH) {
+    const uint32_t e = ga.rhs[i];
+    if (e < (uint32_t)ga.n_experts && (long long)ga.lhs[i] < ga.x_batch) atomicAdd(&counts[e], 1);
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    for (int e0 = 0; e0 < ga.n_experts; e0 += 32) {
+      const int e = e0 + (int)threadIdx.x;
+      const int over = e < ga.n_experts ? max(0, (counts[e] + rows - 1) / rows - base) : 0;
+      const int groups = (over + ga.deep - 1) / ga.deep;
+      int upto = groups;  // of this matrix and those before it among the 32
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, o);
+        if ((int)threadIdx.x >= o) upto += v;
+      }
+      if (j < upto && j >= upto - groups) *found = make_int2(e, base + (j - upto + groups) * ga.deep);
+      const int all = __shfl_sync(0xffffffffu, upto, 31);
+      if (j < all) break;
+      j -= all;
+    }
+  }
+  __syncthreads();
+  return *found;
+}
+
 template <int C, typename XT, int NT, bool G>
 __global__ void __launch_bounds__(RowsShape<G>::kThreads, RowsShape<G>::kCtas)
 rows_kernel(const GemvArgs a, const RowsPlan pl, const RowsGather ga, int* __restrict__ error_word) {
@@ -489,26 +525,45 @@ rows_kernel(const GemvArgs a, const RowsPlan pl, const RowsGather ga, int* __res
   }
   __syncthreads();
   // Passes: the dense form walks the row blocks blockIdx.x, + gridDim.x, ... for all M rows; the gather form has one
-  // row block of one matrix and walks its entries, 8 NT at a time (grid.z CTAs share them).
-  int passes = 0, total_m = a.M;
+  // row block of one matrix and walks its entries, 8 NT at a time (grid.z CTAs share them; where there are CTAs for what
+  // is left over, at most ga.deep of them).
+  int passes = 0;
+  __shared__ int2 walk_s;  // first pass over the matrix's entries and step (kept here, and count_s, to spare registers)
   const uint8_t* wmat = a.w;
   int2* list = reinterpret_cast<int2*>(rw_dyn + pl.list_off);  // (row of x, row of y)
   if constexpr (G) {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the routing may come from the kernel before this one
-    const uint32_t e = ga.by_entry ? ga.rhs[blockIdx.y] : blockIdx.y;
+    constexpr int TH = RowsShape<G>::kThreads;
+    __shared__ int2 found_s;
+    const int share = (int)gridDim.z, base = ga.deep * share;
+    const bool more = (int)gridDim.y > ga.units, left_over = (int)blockIdx.y >= ga.units;
+    uint32_t e;
+    int pass0 = (int)blockIdx.z, pass_step = share;
+    if (left_over) {
+      const int2 f = rows_left_over<TH>(ga, 8 * NT, base, ((int)blockIdx.y - ga.units) * share + (int)blockIdx.z,
+                                        reinterpret_cast<int*>(rw_dyn), &found_s);
+      e = (uint32_t)f.x;
+      pass0 = f.y;
+      pass_step = 1;
+    } else {
+      e = ga.by_entry ? ga.rhs[blockIdx.y] : blockIdx.y;
+    }
     if (e >= (uint32_t)ga.n_experts) return;
-    total_m = collect_entries<RowsShape<G>::kThreads>(ga.rhs, ga.lhs, ga.n_entries, ga.x_batch, e, list, &count_s,
-                                                      ga.by_entry || gridDim.z > 1);
-    if (total_m == 0 || (ga.by_entry && list[0].y != (int)blockIdx.y)) return;
+    if (threadIdx.x == 0) walk_s = make_int2(pass0, pass_step);
+    const bool shared = ga.by_entry || share > 1 || left_over;
+    const int total_m = collect_entries<TH>(ga.rhs, ga.lhs, ga.n_entries, ga.x_batch, e, list, &count_s,
+                                            shared ? 0 : (more ? 8 * NT * base : ga.n_entries));
+    if (total_m == 0 || (ga.by_entry && !left_over && list[0].y != (int)blockIdx.y)) return;
     wmat += (long long)e * ga.expert_stride;
-    passes = ((total_m + 8 * NT - 1) / (8 * NT) - (int)blockIdx.z + (int)gridDim.z - 1) / (int)gridDim.z;
+    passes = ((total_m + 8 * NT - 1) / (8 * NT) - pass0 + pass_step - 1) / pass_step;
+    if (more) passes = min(passes, ga.deep);
     if (passes <= 0) return;
   } else {
     passes = (pl.n_blocks - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;
   }
   auto row_block = [&](int pass) { return ((int)blockIdx.x + (G ? 0 : pass * (int)gridDim.x)) * pl.R; };
-  auto entry0 = [&](int pass) { return 8 * NT * (pass * (int)gridDim.z + (int)blockIdx.z); };  // of the pass (gather)
-  auto rows_of_x = [&](int pass) { return G ? min(8 * NT, total_m - entry0(pass)) : total_m; };
+  auto entry0 = [&](int pass) { return 8 * NT * (walk_s.x + pass * walk_s.y); };  // of the pass (gather)
+  auto rows_of_x = [&](int pass) { return G ? min(8 * NT, count_s - entry0(pass)) : a.M; };
   volatile int* abort_flag = &abort_s;
   auto wait = [&](uint64_t* bar, int parity) { return mbar_wait_err(bar, parity, abort_flag, 0x100, error_word); };
 
@@ -785,7 +840,19 @@ cudaError_t launch_rows_nt(const GemvArgs& a, const RowsGather& ga, cudaStream_t
   // routing may be uneven: while all CTAs are resident at once, several share a matrix's entries
   int share = 1;
   if (G) share = std::max(1, std::min((ga.n_entries + 8 * NT - 1) / (8 * NT), RowsShape<G>::kCtas * rows_sm_count() / (p.n_blocks * units)));
-  cfg.gridDim = G ? dim3(p.n_blocks, units, share) : dim3(std::min(p.n_blocks, rows_sm_count()), 1, 1);
+  // ... and what is more than `deep` passes a CTA goes to CTAs of its own: a matrix of c entries leaves at most
+  // (c - 1) / (8 NT deep) - share + 1 groups. Where there are none such a CTA costs some 1.5 us, a pass over few superblocks
+  // 3-4 us: two passes there, one where K is long. Before, a busy matrix's passes ran one after the other. 128 matrices
+  // of iq4_xs [768, 2048], 512 entries, a fifth of them in one: 221 -> 83 us (the general path 102), evenly at random
+  // 85 -> 72; q4_k [512, 512] 1024 entries 83 -> 35, evenly 20.3 -> 20.4.
+  RowsGather gl = ga;
+  gl.units = units;
+  gl.deep = a.K >= 1536 ? 1 : 2;
+  int more = 0;
+  if (G && 4ll * ga.n_experts <= p.red_off) more = std::max(0, (ga.n_entries - 1) / (8 * NT * gl.deep) - share + 1);
+  more = (more + share - 1) / share;
+  if (units + more > 65535) more = 0;
+  cfg.gridDim = G ? dim3(p.n_blocks, units + more, share) : dim3(std::min(p.n_blocks, rows_sm_count()), 1, 1);
   cfg.blockDim = dim3(RowsShape<G>::kThreads);
   cfg.dynamicSmemBytes = p.smem;
   cfg.stream = st;
@@ -795,7 +862,7 @@ cudaError_t launch_rows_nt(const GemvArgs& a, const RowsGather& ga, cudaStream_t
   cfg.attrs = attr;
   static const bool no_pdl = std::getenv("KQ_NO_PDL") != nullptr;  // A/B lever
   cfg.numAttrs = no_pdl ? 0 : 1;
-  return cudaLaunchKernelEx(&cfg, rows_kernel<C, XT, NT, G>, a, p, ga, err);
+  return cudaLaunchKernelEx(&cfg, rows_kernel<C, XT, NT, G>, a, p, gl, err);
 }
 
 template <int C, typename XT>
@@ -848,9 +915,10 @@ cudaError_t launch_gemv_rows(int codec, int x_dtype, const GemvArgs& a, cudaStre
 bool gather_rows_supported(int codec, int x_dtype, const void* x, int M, int K, const uint8_t* w, long long expert_stride,
                            long long row_bytes, int N, long long n_entries, int n_experts) {
   if (M != 1 || n_entries > kRwMaxEntries || n_experts > 65535 || (expert_stride & 15) != 0) return false;
-  // q4_k has a grouped kernel of its own that spreads a busy expert's rows over more CTAs: 512 rows over 128 experts
-  // [1536, 2048] evenly at random 126 us there and 105 here, but 118 and 152 with a fifth of the rows in one expert
-  if (codec == Q4_K && (long long)N * K > (1 << 20) && n_entries > 2ll * n_experts) return false;
+  // q4_k has a grouped kernel of its own for matrices of this size, as fast from eight entries a matrix on unless K is
+  // long: 1024 entries of 128 matrices [2048, 768] 96 us there and 91 here evenly at random, 100 and 108 with a fifth of
+  // them in one matrix; 512 entries 88 and 66, 85 and 71; 1024 of [768, 2048] 84 and 70, 84 and 77.
+  if (codec == Q4_K && (long long)N * K > (1 << 20) && K < 1536 && n_entries >= 8ll * n_experts) return false;
   GemvArgs a{};
   a.x = x;
   a.x_row_stride = K;
