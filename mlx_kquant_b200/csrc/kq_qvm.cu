@@ -11,6 +11,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "kq_common.cuh"
@@ -211,6 +212,27 @@ qvm_rows_kernel(const XT* __restrict__ x, void* __restrict__ y, const uint8_t* _
   }
 }
 
+// routing may be uneven: while the CTAs are hardly more than reside at once, several share a matrix's entries
+int row_share(int N, int n_experts, long long entries) {
+  const long long ctas = (long long)((N + kRowCols - 1) / kRowCols) * n_experts;
+  return (int)std::max(1ll, std::min((entries + kRowM - 1) / kRowM, 3 * 148 / ctas));
+}
+
+// One row an entry, at least as many entries as matrices: the shared decode against the kernel above with K split S
+// ways. Both take time by the rows of K a CTA walks (a third of it there, of 128 columns and eight entries; of 256
+// columns and one entry here) and by the CTAs beyond those that reside at once. Within 1-2 % of the faster one on average
+// over 780 calls of q4_k, q6_k, iq4_xs and q8_0, 1 to 128 matrices and 1 to 128 entries each. 64 heads [128, 512] q6_k,
+// one entry each 11.9 -> 8.2 us, eight 39.6 -> 9.2; but one matrix [4096, 4096] with one entry 34 us above, 90 here, and
+// eight [2048, 1024] with one each 24 and 57.
+bool rows_pay(int N, int K, int S, int n_experts, long long entries) {
+  const double share = row_share(N, n_experts, entries);
+  const double ctas = (double)((N + kRowCols - 1) / kRowCols) * n_experts * share;
+  const double above = (double)((N + kCols - 1) / kCols) * entries * S;
+  const double rows = (double)((entries + n_experts - 1) / n_experts);
+  const double passes = std::max(1.0, std::ceil(std::ceil(rows / kRowM) / share));
+  return 0.35 * passes * S * std::max(1.0, ctas / (3 * 148)) < std::max(1.0, above / (2 * 148));
+}
+
 template <int C, int A, typename XT>
 cudaError_t launch_rows(const void* x, void* y, const uint8_t* w, long long row_bytes, int N, int K, cudaStream_t st,
                         QvmGather gq, int n_entries) {
@@ -219,9 +241,7 @@ cudaError_t launch_rows(const void* x, void* y, const uint8_t* w, long long row_
   gq.rhs += gq.entry0;
   y = static_cast<uint16_t*>(y) + gq.entry0 * N;  // both output types have two bytes
   cudaLaunchConfig_t cfg = {};
-  const int ctas = (N + kRowCols - 1) / kRowCols * gq.n_experts;
-  // routing may be uneven: while the CTAs are hardly more than reside at once, several share a matrix's entries
-  const int share = std::max(1, std::min((n_entries + kRowM - 1) / kRowM, 3 * 148 / ctas));
+  const int share = row_share(N, gq.n_experts, n_entries);
   cfg.gridDim = dim3((N + kRowCols - 1) / kRowCols, gq.n_experts, share);
   cfg.blockDim = dim3(kThreads);
   cfg.stream = st;
@@ -238,12 +258,12 @@ template <int C, int A, typename XT>
 cudaError_t launch_one(const void* x, long long x_row_stride, void* y, long long y_row_stride, const uint8_t* w,
                        long long row_bytes, int M, int N, int K, cudaStream_t st, QvmGather gq = QvmGather{},
                        long long entries = 1) {
-  // one row an entry and at least as many entries as matrices: some matrix has several rows
-  if (gq.rhs != nullptr && M == 1 && entries >= gq.n_experts && entries <= kRowEntries && gq.n_experts <= 65535)
-    return launch_rows<C, A, XT>(x, y, w, row_bytes, N, K, st, gq, (int)entries);
   const int col_ctas = (N + kCols - 1) / kCols, m_tiles = (M + kMT - 1) / kMT;
   int S = 1;
   while (S < kMaxSplit && (long long)col_ctas * m_tiles * entries * S < 2 * 148 && K / (S * 2) >= 4 * kWarps) S *= 2;
+  if (gq.rhs != nullptr && M == 1 && entries >= gq.n_experts && entries <= kRowEntries && gq.n_experts <= 65535 &&
+      rows_pay(N, K, S, gq.n_experts, entries))
+    return launch_rows<C, A, XT>(x, y, w, row_bytes, N, K, st, gq, (int)entries);
   gq.m_tiles = m_tiles;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(col_ctas, S, (unsigned)(m_tiles * entries));

@@ -14,7 +14,9 @@ pytestmark = pytest.mark.gpu
 CASES = [(40, 136, 512, 7, "any"), (16, 72, 256, 200, "one"), (5, 1000, 768, 33, "any"), (64, 128, 512, 512, "even"),
          (8, 40, 1280, 513, "any"), (3, 264, 2048, 1024, "any"), (3, 264, 256, 1025, "one"),
          # a busy matrix's passes in groups of one and of two, among more matrices than 32 and than entries
-         (70, 136, 1536, 300, "one"), (2000, 24, 512, 900, "one"), (33, 200, 512, 1024, "one")]
+         (70, 136, 1536, 300, "one"), (2000, 24, 512, 900, "one"), (33, 200, 512, 1024, "one"),
+         # [K, N]: one entry a matrix on either side of the rule, few matrices with few and with many entries
+         (64, 128, 512, 64, "even"), (1, 512, 512, 3, "even"), (2, 512, 256, 300, "even"), (5, 136, 1280, 5, "even")]
 
 
 @pytest.mark.parametrize("codec", ["q4_k", "q5_k", "q6_k", "iq4_xs", "q8_0"])
