@@ -193,14 +193,16 @@ int kq_quantized_matmul(const void* x, int x_dtype, long long rows, int K, long 
     a.K = K;
     a.M = (int)rows;
     // 2-16 rows the row kernel (kq_rows.cu) does not take as they are - f32 rows, and bf16 rows of q4_k matrices of
-    // a form it does not cover - with scratch at hand: exact fp16 copy of the rows (per-row power-of-two factor),
-    // then the fp16 kernel writing bf16(sum * factor), several times faster than the kernels that take such rows
-    // directly. Without scratch those still serve.
+    // a form it does not cover - with scratch at hand: fp16 copy of the rows (per-row power-of-two factor, exact but for
+    // values below 2^-32 of the row's largest), then the fp16 kernel writing bf16(sum * factor), several times faster than
+    // the kernels that take such rows directly. Without scratch those still serve. iq4_xs rows of whole sixteen bytes have
+    // a table kernel that takes f32 rows: [512, 512] x 2 3.5 us, 5.9 with the copy's launch; [4096, 1024] x 8 6.5 and 7.1.
     const size_t need = kq::gemm_workspace_bytes(x_dtype, rows, K);
     int eff_dtype = x_dtype;
     const bool direct = rows >= 2 && kq::gemv_rows_supported(ci, x_dtype, a);
     const bool q4k = ci == kq::Q4_K && a.w_align16 && (w_row_bytes & 15) == 0;
-    if (x_dtype != KQ_F16 && rows >= 2 && !direct && (q4k || kq::gemv_rows_supported(ci, KQ_F16, a)) &&
+    const bool tables = ci == kq::IQ4_XS && (w_row_bytes & 15) == 0;
+    if (x_dtype != KQ_F16 && rows >= 2 && !direct && !tables && (q4k || kq::gemv_rows_supported(ci, KQ_F16, a)) &&
         workspace != nullptr && workspace_bytes >= need && need > 0 &&
         (reinterpret_cast<uintptr_t>(workspace) & 255) == 0) {
       float* rs = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) +
