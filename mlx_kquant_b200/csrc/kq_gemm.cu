@@ -1211,7 +1211,8 @@ static cudaError_t launch_codec(bool out_half, const GemmArgs& a, bool aligned, 
 }
 
 // ---- many rows: the weights are dequantized to fp16 once and the tiles of both operands come by TMA
-// rows of the matrix per pass: the fp16 copy stays below kHalfBytes, so that it is still in L2 when it is read
+// rows of the matrix per pass: the fp16 copy stays below kHalfBytes (or 256 rows), so that most of it is still in
+// the 126 MB L2 when it is read
 constexpr long long kHalfBytes = 128ll << 20;
 static int half_chunk(int N, int K) {
   const long long most = std::max<long long>(256, kHalfBytes / (2ll * K) / 128 * 128);
@@ -1235,11 +1236,43 @@ size_t gemm_workspace_bytes_n(int codec, int x_dtype, long long rows, int N, int
   return gemm_workspace_bytes(x_dtype, rows, K) + (use_half(codec, rows, N, K) ? half_bytes(N, K) : 0);
 }
 
+// CTAs of the copy path's kernels that reside at once in clusters of z = 1, 2, 4, 8 (148, 148, 132 and 120 on a B200:
+// clusters of more than two leave SMs of the smaller GPCs idle).
+static int half_resident(int z) {
+  static int known[16][9] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return 148;
+  if (known[dev][z] == 0) {
+    auto kern = gemm_kernel<Q4_K, 16, __half, 1, 2, false, false, 1, true>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, 1, z);
+    cfg.blockDim = dim3(gemm_threads(1, 2));
+    cfg.dynamicSmemBytes = (size_t)(b_stages(2, false, 1) * 2 + a_slots(1, 2, false, 1)) * kTileBytes + 1024;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = z;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
+      (void)cudaGetLastError();
+      n = 120 / z;
+    }
+    known[dev][z] = n * z;
+  }
+  return known[dev][z];
+}
+
 template <typename OT>
 static cudaError_t launch_half(GemmArgs a, cudaStream_t st) {
   // Tile shape by the time its waves take. A K-step costs the tensor pipe two cycles per column and 128-row block, the
-  // loads of its (128 mt + bn) x 128 bytes some 2.7 cycles a row out of L2, its handshakes 450; a tile 9000 cycles for
-  // start and epilogue, a further slice of K 3000.
+  // loads of its (128 mt + bn) x 128 bytes two cycles a row out of L2, its handshakes 700; a tile 9000 cycles for start
+  // and epilogue, a further slice of K 1000. Constants from a sweep of tile shapes over twenty sizes, where the shape
+  // taken is within 6 % of the best one (2.7, 450, 9000, 3000, and 148 CTAs at once whatever the cluster: up to 43 % off -
+  // x 64 [4096, 4096] took 148 CTAs in clusters of four, two waves, 36.6 us against 23).
   const int kb = (a.K + kBK - 1) / kBK;
   double best = 1e30;
   int mt = 2, bn = 256, ks = 1;
@@ -1248,8 +1281,9 @@ static cudaError_t launch_half(GemmArgs a, cudaStream_t st) {
     for (int b = 256; b >= 64; b -= 16) {
       const long long tiles = (long long)((a.N + b - 1) / b) * ((a.M + 128 * t - 1) / (128 * t));
       for (int z = 1; z <= 8 && kb % z == 0 && (z == 1 || t * (b > 128 ? 2 : 1) <= 2); z *= 2) {
-        const double step = std::max({2.0 * t * b, 2.7 * (128 * t + b), 450.0});
-        const double c = (double)((tiles * z + 147) / 148) * (kb / z * step + 9000.0 + 3000.0 * (z - 1));
+        const int cap = half_resident(z);
+        const double step = std::max({2.0 * t * b, 2.0 * (128 * t + b), 700.0});
+        const double c = (double)((tiles * z + cap - 1) / cap) * (kb / z * step + 9000.0 + 1000.0 * (z - 1));
         if (c < best * 0.999) best = c, mt = t, bn = b, ks = z;
       }
     }
