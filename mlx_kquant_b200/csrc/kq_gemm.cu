@@ -1222,15 +1222,26 @@ static int half_chunk(int N, int K) {
 static size_t half_bytes(int N, int K) { return (2 * (size_t)half_chunk(N, K) * (size_t)K + 255) & ~(size_t)255; }
 // Codecs whose fused producer is decode8<> (all but q4_k and q6_k, and q6_k rows off the 8-byte grid) make a K-step's
 // weights several times slower than the tensor cores use them, whatever the number of rows: the copy wins from the
-// first row on, once the matrix outweighs its extra launch. Measured, fused against copy: q5_k [14336, 4096] x 64 rows
-// 326 / 91 us, q8_0 x 512 444 / 87, iq4_xs x 32 190 / 75, q4_0 [4096, 4096] x 300 129 / 53; q5_k [1000, 1280] x 130
-// 17.7 / 19.5. q6_k, whose producer nearly keeps up, from 257 rows on (a second row block for the fused kernel): [14336, 4096] x 256
-// 75.7 / 76.0, x 512 143 / 85, x 8192 1119 / 930; [4096, 14336] x 256 68 / 116, x 384 116 / 106. q4_k never: x 2048
-// 247 / 261.
+// first row on, once the matrix outweighs its extra launch. Measured, fused against copy: q5_k [4096, 1024] x 17 rows
+// 18.4 / 14.0 us, [4096, 4096] x 64 88.5 / 28.8, q8_0 [1024, 4096] x 17 35.3 / 16.3, [4096, 4096] x 512 124 / 41, iq4_xs x 17
+// 55 / 27.5, q4_0 x 300 128 / 38; q5_k [1000, 1280] x 130 17.7 / 19.5. q6_k, whose producer nearly keeps up, from 257 rows
+// on (a second row block for the fused kernel): [2048, 2048] x 257 20.3 / 19.2, [14336, 4096] x 256 76 / 75, x 512 143 / 85;
+// [4096, 14336] x 256 68 / 79, x 384 117 / 106. q4_k stays fused: [14336, 4096] x 512 65 / 92, x 2048 270 / 266, though the
+// copy would gain on smaller matrices with more than 256 rows ([4096, 4096] x 300 60 / 40).
+// With up to 256 rows and short K the lighter decoders keep up: q2_k [4096, 1024] x 128 13.7 / 16.6 us (x 300 22.0 / 19.7),
+// iq4_xs 14.9 / 17.5, q4_0 17.4 / 17.4 there but [16384, 512] 17.8 / 19.8; q5_k and the others gain at every K.
+static int half_min_k(int codec) {
+  switch (codec) {
+    case Q2_K: return 2560;
+    case IQ4_XS: case IQ2_XXS: case IQ3_XXS: case IQ2_XS: case IQ2_S: case IQ1_S: case IQ1_M: return 1536;
+    case Q4_0: case IQ4_NL: case MXFP4: return 1024;
+  }
+  return 0;
+}
 static bool use_half(int codec, long long M, int N, int K) {
   if (codec == Q4_K || (long long)N * K < (4ll << 20)) return false;
   if (codec == Q6_K && (K & 1023) == 0) return M > 256;
-  return true;
+  return M > 256 || K >= half_min_k(codec);
 }
 size_t gemm_workspace_bytes_n(int codec, int x_dtype, long long rows, int N, int K) {
   return gemm_workspace_bytes(x_dtype, rows, K) + (use_half(codec, rows, N, K) ? half_bytes(N, K) : 0);

@@ -11,7 +11,9 @@ pytestmark = pytest.mark.gpu
 # (codec, m, n, k): the smallest matrices of the rule with ragged rows and columns, K not a whole number of K-steps,
 # K split over a cluster, two row blocks, and an fp16 copy made in two parts (128 MiB)
 CASES = [("q5_k", 17, 4099, 1024), ("q8_0", 130, 2051, 2080), ("iq4_xs", 300, 1025, 4096), ("q4_0", 64, 1024, 8192),
-         ("q3_k", 513, 4100, 1280), ("q6_k", 40, 2051, 2304), ("q6_k", 1027, 1056, 4096), ("q2_k", 33, 9000, 8192)]
+         ("q3_k", 513, 4100, 1280), ("q6_k", 40, 2051, 2304), ("q6_k", 1027, 1056, 4096), ("q2_k", 33, 9000, 8192),
+         # either side of the shortest K with few rows, and of 256 rows
+         ("iq4_xs", 256, 4104, 1024), ("iq4_xs", 257, 4104, 1024), ("q4_0", 100, 8200, 512), ("q4_0", 40, 4100, 1024)]
 
 
 @pytest.mark.parametrize("codec,m,n,k", CASES)
