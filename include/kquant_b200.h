@@ -99,12 +99,19 @@ KQ_API int kq_quantize_cpu(const void* w, int w_dtype, long long n_weights, long
  *    device memory, 256-byte aligned (0 bytes, and NULL allowed, for fp16
  *    activations or a single row). Calls with more than 16 rows run on the tensor
  *    cores in fp16; bf16 / f32 activations are converted there first, exactly, with
- *    a per-row power-of-two factor. With 2-16 rows the workspace is optional: q4_k
- *    uses it for the same conversion (several times faster), and a call without it
- *    still works. */
+ *    a per-row power-of-two factor. With 2-16 rows the workspace is optional: f32
+ *    rows use it for the same conversion (q4_k, q5_k, q6_k, and iq4_xs matrices of at
+ *    most 4 M weights whose rows are not whole numbers of 16 bytes: up to several times
+ *    faster; values below 2^-32 of their row's largest lose bits), and so do bf16 rows
+ *    of q4_k matrices with fewer than eight rows; a call without it still works.
+ *  - w: written before the launch that comes ahead of this call in the stream. With one
+ *    row, and for some codecs up to sixteen, the kernels start to read weights while
+ *    that launch may still be running (programmatic dependent launch). After a kernel
+ *    that writes weights, another launch has to come first. */
 KQ_API size_t kq_quantized_matmul_workspace_bytes(int x_dtype, long long rows, int K);
-/* The same with room for an fp16 copy of the weights (of at most 128 MiB) where [N, K] products of that many rows
- * are faster from one; a call that is given only the bytes above works without it. */
+/* The same with room for an fp16 copy of (a part of) the weights, of at most 128 MiB or 256 rows, where [N, K] products
+ * of that many rows are faster from one: more than 16 rows on matrices of 4 M weights and more of every codec but q4_k
+ * (q6_k with K a multiple of 1024: more than 256 rows). A call that is given only the bytes above works without it. */
 KQ_API size_t kq_quantized_matmul_workspace_bytes_for(const char* kquant_type, int x_dtype, long long rows, int N, int K);
 KQ_API int kq_quantized_matmul(const void* x, int x_dtype, long long rows, int K, long long x_row_stride, const void* w,
                         size_t w_row_bytes, int N, const char* kquant_type, int transpose, void* y,

@@ -82,6 +82,12 @@ def _order_on(stream, device, *tensors) -> None:
             t.record_stream(stream)
 
 
+def _output(shape, dtype, device, w, w_used):
+    """The output of a product. Decode kernels may read weights before the launch ahead of them has ended; where that
+    would be the copy that made the weights contiguous, the output is cleared in between."""
+    return (torch.empty if w_used.data_ptr() == w.data_ptr() else torch.zeros)(shape, dtype=dtype, device=device)
+
+
 def _require_cuda(w: torch.Tensor, op: str) -> None:
     if not w.is_cuda:
         raise RuntimeError(f"[mlx_kquant.{op}] w must live on a CUDA device; there is no CPU path.")
@@ -187,7 +193,7 @@ def quantized_matmul(x, w, scales, kquant_type, transpose=True, *, stream=None):
     if x2.stride(-1) != 1 or (x2.stride(0) * x2.element_size()) % 16 != 0 or x2.data_ptr() % 16 != 0:
         x2 = x2.contiguous()
     rows = x2.shape[0]
-    y = torch.empty((rows, outer), dtype=out_dtype, device=w.device)
+    y = _output((rows, outer), out_dtype, w.device, w, w2)
     L = _lib.lib()
     ws_bytes = L.kq_quantized_matmul_workspace_bytes(_DT[x.dtype], rows, K) if rows > 1 else 0  # one row needs none
     if transpose and rows > 16:  # many rows: perhaps room for an fp16 copy of the weights, if the device has it
@@ -391,7 +397,7 @@ def quantized_matmul_qmv_bias(x, w, scales, bias, kquant_type, *, stream=None):
     xc = x.reshape(1, K).contiguous()
     wc = w.contiguous()
     bc = bias.to(dev).to(out_dtype).contiguous()
-    y = torch.empty(x.shape[:-1] + (N,), dtype=out_dtype, device=dev)
+    y = _output(x.shape[:-1] + (N,), out_dtype, dev, w, wc)
     _order_on(stream, dev, xc, wc, bc, y)
     with _on_device(dev):
         check(_lib.lib().kq_quantized_matmul_qmv_bias(xc.data_ptr(), _DT[x.dtype], K, wc.data_ptr(), wc.shape[1], N,

@@ -137,3 +137,18 @@ def test_weights_written_just_before(codec, m):
         got.append(kq.quantized_matmul(x, buf, None, codec))
     for i, y in enumerate(got):
         assert torch.equal(y, want[i % 2])
+
+
+def test_strided_weights_of_one_row():
+    """A copy made for the call is written before the one-row kernel, which reads ahead, can see it."""
+    import mlx_kquant_b200 as kq
+
+    n, k = 2048, 4096
+    rows = torch.randn(2, 64, k, generator=torch.Generator().manual_seed(4)) * 0.05
+    pair = [kq.quantize(r, "q4_k")[0].repeat(n // 64, 1).cuda() for r in rows]
+    wide = torch.stack(pair, 1)   # [n, 2, bytes]: either matrix with the other between its rows
+    x = torch.randn(1, k, dtype=torch.float16, device="cuda")
+    want = [kq.quantized_matmul(x, w, None, "q4_k") for w in pair]
+    got = [kq.quantized_matmul(x, wide[:, i % 2], None, "q4_k") for i in range(64)]
+    for i, y in enumerate(got):
+        assert torch.equal(y, want[i % 2])
