@@ -1,4 +1,4 @@
-// q4_k decode product (one to four activation rows) on the integer tensor pipe.
+// q4_k decode product (one activation row, or two of float32) on the integer tensor pipe.
 //
 // Same arithmetic as the integer dot-product kernel of kq_gemv.cu, with mma.sync.m16n8k32 (u8 x s8 ->
 // s32) doing the products: the activations of every 256-weight superblock are quantized to 16-bit
@@ -352,15 +352,16 @@ cudaError_t launch_imma(const GemvArgs& a, cudaStream_t st) {
 template <typename XT>
 cudaError_t launch_imma_rows(const GemvArgs& a, cudaStream_t st) {
   if (a.M == 1) return launch_imma<XT, 1>(a, st);
-  if (a.M == 2) return launch_imma<XT, 2>(a, st);
+  if constexpr (std::is_same<XT, float>::value)
+    if (a.M == 2) return launch_imma<XT, 2>(a, st);
   return cudaErrorInvalidValue;
 }
 
 }  // namespace
 
 bool gemv_imma_supported(int codec, int x_dtype, const GemvArgs& a) {
-  (void)x_dtype;
-  return codec == Q4_K && a.tasks == nullptr && a.M >= 1 && a.M <= 2 && a.w_align16 != 0 && (a.K & 255) == 0 &&
+  // two rows: float32 without scratch only, 16-bit rows have the row kernel (kq_rows.cu)
+  return codec == Q4_K && a.tasks == nullptr && (a.M == 1 || (a.M == 2 && x_dtype == F32)) && a.w_align16 != 0 && (a.K & 255) == 0 &&
          a.K <= kImMaxK && (a.row_bytes & 15) == 0 && (a.x_row_stride & 7) == 0 &&
          (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && a.out_bf16 == 0;
 }

@@ -1,7 +1,8 @@
 """The integer tensor-pipe q4_k decode kernel (lever KQ_GEMV_IMMA) against the fp64 product of the
 dequantized weights, and against the run with the lever off.
 
-The lever is read once per process, so each setting runs in a child process."""
+Two rows reach it as float32 through the C ABI without a workspace (16-bit rows, and float32 rows with one, run on the
+row kernel either way). The lever is read once per process, so each setting runs in a child process."""
 import os
 import subprocess
 import sys
@@ -17,8 +18,8 @@ import mlx_kquant_b200 as kq
 from mlx_kquant_b200.synth import random_wire
 out = sys.argv[1]
 res = {}
-cases = [(128, 256, 1, 'f16'), (1000, 2048, 1, 'f16'), (4096, 4096, 2, 'f16'), (515, 14336, 1, 'bf16'),
-         (4100, 4096, 1, 'f32'), (9600, 1024, 1, 'f16'), (33, 16384, 2, 'bf16'), (20000, 512, 2, 'f16')]
+cases = [(128, 256, 1, 'f16'), (1000, 2048, 1, 'f16'), (4096, 4096, 2, 'f32'), (515, 14336, 1, 'bf16'),
+         (4100, 4096, 1, 'f32'), (9600, 1024, 1, 'f16'), (33, 16384, 2, 'f32'), (20000, 512, 2, 'f32')]
 DT = {'f16': torch.float16, 'bf16': torch.bfloat16, 'f32': torch.float32}
 for (N, K, M, dt) in cases:
     W = random_wire('q4_k', N, K, seed=11)
@@ -26,7 +27,13 @@ for (N, K, M, dt) in cases:
     if (N, dt) == (1000, 'f16'):
         x[0, 300:333] = 0          # a whole sub-block of zeros and an outlier
         x[0, 7] = 900.0
-    y = kq.quantized_matmul(x, W, None, 'q4_k')
+    if M == 1:
+        y = kq.quantized_matmul(x, W, None, 'q4_k')
+    else:
+        y = torch.empty(M, N, dtype=torch.bfloat16, device='cuda')
+        kq._lib.check(kq._lib.lib().kq_quantized_matmul(
+            x.data_ptr(), kq.ops._DT[x.dtype], M, K, K, W.data_ptr(), W.shape[1], N, b'q4_k', 1, y.data_ptr(), N, None, 0,
+            torch.cuda.current_stream().cuda_stream))
     xr = x.to(torch.bfloat16).double() if dt == 'f32' else x.double()
     ref = xr @ kq.dequantize(W, None, 'q4_k', dtype=torch.float32).double().T
     res[f'y_{N}_{K}_{M}_{dt}'] = y.float().cpu().numpy()
