@@ -1,5 +1,6 @@
 """The integer dot-product decode kernels (one to four activation rows; task lists of gather_qmm) against the
-CPU oracle, on shapes chosen to reach their corners: every codec with every activation dtype, random wire
+CPU oracle (several rows of q4_k, q5_k and q6_k go through the same cases on the row kernel; those two codecs reach the
+integer kernels with float32 rows and no workspace, by a case of their own), on shapes chosen to reach their corners: every codec with every activation dtype, random wire
 bytes (all scale / sign bit patterns), a ragged N, a K long enough for the weight ring to wrap, the large
 iq2_xxs case that takes the lattice kernel, and expert task lists with more rows than one four-row slice.
 Tolerance as in test_matmul_gpu.py: 2e-3 relative Frobenius and peak-normalised max error (after the one
@@ -39,6 +40,19 @@ def test_random_wire_bytes_all_dtypes(oracle, codec, dt, M):
     out = "f16" if dt == "f16" else "bf16"
     assert tuple(y.shape) == (M, N)
     assert_close(y_to_f32(y), ref64(oracle, store, dt, wire, codec), out, TOL)
+
+
+@pytest.mark.parametrize("codec", ["q5_k", "q6_k"])
+@pytest.mark.parametrize("M", [2, 3, 4])
+def test_float32_rows_without_workspace(oracle, codec, M):
+    N, K = 100, 2048
+    wire = synthetic_wire(codec, N, K, seed=45 + M)
+    x, store = x_to_torch(np.random.default_rng(46).normal(0, 1, (M, K)).astype(np.float32), "f32")
+    w, y = torch.from_numpy(wire).cuda(), torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    kq._lib.check(kq._lib.lib().kq_quantized_matmul(
+        x.data_ptr(), kq.ops._DT[x.dtype], M, K, K, w.data_ptr(), w.shape[1], N, codec.encode(), 1, y.data_ptr(), N, None, 0,
+        torch.cuda.current_stream().cuda_stream))
+    assert_close(y_to_f32(y), ref64(oracle, store, "f32", wire, codec), "bf16", TOL)
 
 
 @pytest.mark.parametrize("codec", ["q4_k", "q6_k", "q3_k", "q8_0", "iq4_xs"])

@@ -35,6 +35,31 @@ def test_half_copy_against_float64(codec, m, n, k, dt):
     assert off.max() < 6 * 2.0 ** -11 * np.sqrt(np.mean(ref ** 2))
 
 
+@pytest.mark.parametrize("codec,m,n,k", [("q5_k", 17, 4099, 1024), ("q8_0", 130, 2051, 2080), ("q6_k", 300, 1056, 4096),
+                                         ("q3_k", 64, 4100, 1280), ("iq4_xs", 40, 1025, 4096)])
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
+def test_without_room_for_the_copy(codec, m, n, k, dt):
+    """A call with the smaller workspace (none for fp16 rows) takes the fused kernel, to the same bound."""
+    import mlx_kquant_b200 as kq
+
+    lib = kq._lib.lib()
+    rng = np.random.default_rng(m + n)
+    some = kq.quantize(torch.from_numpy(rng.standard_normal((64, k)).astype(np.float32) * 0.05), codec)[0].numpy()
+    pick = rng.integers(0, 64, n)
+    x, _ = x_to_torch(rng.standard_normal((m, k)).astype(np.float32), dt)
+    code = kq.ops._DT[x.dtype]
+    need = lib.kq_quantized_matmul_workspace_bytes(code, m, k)
+    assert lib.kq_quantized_matmul_workspace_bytes_for(codec.encode(), code, m, n, k) > need
+    ref = (x.double().cpu().numpy() @ Oracle().dequantize(some, codec, "f32").astype(np.float64).T)[:, pick]
+    w, y = torch.from_numpy(some[pick]).cuda(), torch.empty(m, n, dtype=x.dtype, device="cuda")
+    ws = torch.empty(need, dtype=torch.uint8, device="cuda") if need else None
+    kq._lib.check(lib.kq_quantized_matmul(
+        x.data_ptr(), code, m, k, k, w.data_ptr(), w.shape[1], n, codec.encode(), 1, y.data_ptr(), n,
+        ws.data_ptr() if need else None, need, torch.cuda.current_stream().cuda_stream))
+    off = np.abs(y_to_f32(y).astype(np.float64) - ref) - (2.0 ** -11 if dt == "f16" else 2.0 ** -8) * np.abs(ref)
+    assert off.max() < 6 * 2.0 ** -11 * np.sqrt(np.mean(ref ** 2))
+
+
 def test_unaligned_workspace_of_fp16_rows():
     """fp16 rows need no workspace: a large one off the 256-byte grid is no error, the call does without the copy."""
     import mlx_kquant_b200 as kq
