@@ -130,21 +130,23 @@ dequant_kernel(const uint8_t* __restrict__ w, T* __restrict__ out, long long n_b
     if constexpr (A >= 2) {
       phase = (int)(reinterpret_cast<uintptr_t>(w + b0 * BPB) & 15);
       if constexpr (kBufs == 1) {
-      // one tile a CTA: sixteen-byte loads by all threads (a bulk copy here: q3_k -> float32 56 us against 49); a chunk
-      // that would run past the end of the wire buffer is copied byte by byte
-      const uint8_t* a0 = w + b0 * BPB - phase;
-      const int nchunks = (phase + nb * BPB + 15) >> 4;
-      for (int c = threadIdx.x; c < nchunks; c += kDqThreads) {
-        const uint8_t* g = a0 + 16 * c;
-        if (g + 16 <= w_end) {
-          reinterpret_cast<uint4*>(stage)[c] = *reinterpret_cast<const uint4*>(g);
-        } else {
-          for (int i = 0; i < 16; i++)
-            if (g + i < w_end) stage[16 * c + i] = g[i];
+        // one tile a CTA: sixteen-byte loads by all threads (a bulk copy here: q3_k -> float32 56 us against 49); a chunk
+        // that would run past the end of the wire buffer is copied byte by byte
+        const uint8_t* a0 = w + b0 * BPB - phase;
+        const int nchunks = (phase + nb * BPB + 15) >> 4;
+        for (int c = threadIdx.x; c < nchunks; c += kDqThreads) {
+          const uint8_t* g = a0 + 16 * c;
+          if (g + 16 <= w_end) {
+            reinterpret_cast<uint4*>(stage)[c] = *reinterpret_cast<const uint4*>(g);
+          } else {
+            for (int i = 0; i < 16; i++)
+              if (g + i < w_end) stage[16 * c + i] = g[i];
+          }
         }
+        __syncthreads();
+      } else {
+        if (!mbar_wait_err(&full[buf], (it / kBufs) & 1, &abort_s, 0x200, error_word)) return;
       }
-      __syncthreads();
-    } else if (!mbar_wait_err(&full[buf], (it / kBufs) & 1, &abort_s, 0x200, error_word)) return;
     } else {
       phase = 0;
       const uint8_t* src = w + b0 * BPB;

@@ -1533,7 +1533,7 @@ cudaError_t launch_gemv(int codec, int x_dtype, const GemvArgs& a, cudaStream_t 
   if (groups <= 0) return cudaSuccess;
   if (groups > 65535) return cudaErrorInvalidConfiguration;
   // Two to sixteen dense rows of q4_k, q5_k, q6_k: the integers themselves on mma.sync. Measured against the kernels
-  // below, [14336, 4096] x 8 rows: q4_k bf16 25.3 -> 17.2 us, q5_k 80 -> 19.5; q6_k [4096, 14336] 97.5 -> 24; q4_k [4096, 4096] 14.6 -> 7.3.
+  // below, [14336, 4096] x 8 rows: q4_k bf16 25.3 -> 17.4 us, q5_k 80 -> 19.5; q6_k [4096, 14336] 97.5 -> 24; q4_k [4096, 4096] 14.6 -> 7.3.
   // One row stays below (q4_k [14336, 4096] 10.8 us against 16.0): there the matrix instruction has seven idle columns.
   // Against two to four rows' own kernels: q4_k fp16 x 2 [4096, 4096] 6.8 us, 6.5 on the integer kernel below, [14336,
   // 4096] 15.5 against 12.5; its 16-bit activations cost precision that these rows now have, so they stay here. Nine to

@@ -6,7 +6,7 @@
 // What bounds it: a tile product is a chain of shared-memory loads, permutes and matrix instructions some 2500 cycles
 // long, with 16 warps on an SM to hide it (without any weight copy [28672, 8192] x 1 row takes 40 of 48 us; without any
 // product 26), half of the issue slots and half of the ALU pipe (byte permutes) busy; HBM is the next bound. Measured
-// [14336, 4096] x 8 bf16 rows: q4_k 17.2 us, q5_k x 16 fp16 rows 22.1; q6_k [4096, 14336] x 8 24.0 (25.3, 80, 97.5 on
+// [14336, 4096] x 8 bf16 rows: q4_k 17.4 us, q5_k x 16 fp16 rows 22.1; q6_k [4096, 14336] x 8 24.0 (25.3, 80, 97.5 on
 // the kernels before it). What it is built around:
 //   * No value is rounded: a weight is scale x integer (- min), the integer goes into the tensor core as it is and
 //     the scale is applied in float32 to the sum over its 16- or 32-weight sub-block. The bytes become operands
@@ -343,7 +343,12 @@ struct RowsUnit {
     uint32_t low, high;  // the low nibbles of two bytes, the high nibbles, as 16-bit floats
   };
   static __device__ __forceinline__ Pairs iq4_pairs(uint32_t half) {
-    constexpr uint32_t L[2][4] = {{0x103080f0u, 0x00806020u, 0xc0408000u, 0x109050a0u}, {0x82a6d0feu, 0x20b00c44u, 0x18c85080u, 0xe2b28a54u}}, H[2][4] = {{0xd4d5d6d7u, 0xc9cdd0d2u, 0x504e4a3cu, 0x57555452u}, {0xc2c2c2c2u, 0xc1c1c2c2u, 0x4241413fu, 0x42424242u}};
+    // bytes of the sixteen levels (-127, -104, -83, -65, -49, -35, -22, -10, 1, 13, 25, 38, 53, 69, 89, 113), level 0 in the
+    // lowest byte: L the low, H the high ones of their fp16 numbers (first row) and of their bf16 numbers
+    constexpr uint32_t L[2][4] = {{0x103080f0u, 0x00806020u, 0xc0408000u, 0x109050a0u},
+                                  {0x82a6d0feu, 0x20b00c44u, 0x18c85080u, 0xe2b28a54u}};
+    constexpr uint32_t H[2][4] = {{0xd4d5d6d7u, 0xc9cdd0d2u, 0x504e4a3cu, 0x57555452u},
+                                  {0xc2c2c2c2u, 0xc1c1c2c2u, 0x4241413fu, 0x42424242u}};
     const uint32_t sel = half & 0x7777u, pick = 0x3210u | ((half >> 1) & 0x4444u);
     const uint32_t lo = __byte_perm(__byte_perm(L[kBf][0], L[kBf][1], sel), __byte_perm(L[kBf][2], L[kBf][3], sel), pick);
     const uint32_t hi = __byte_perm(__byte_perm(H[kBf][0], H[kBf][1], sel), __byte_perm(H[kBf][2], H[kBf][3], sel), pick);
