@@ -193,7 +193,8 @@ def quantized_matmul(x, w, scales, kquant_type, transpose=True, *, stream=None):
     if x2.stride(-1) != 1 or (x2.stride(0) * x2.element_size()) % 16 != 0 or x2.data_ptr() % 16 != 0:
         x2 = x2.contiguous()
     rows = x2.shape[0]
-    y = _output((rows, outer), out_dtype, w.device, w, w2)
+    y = torch.empty((rows, outer), dtype=out_dtype, device=w.device) if w2 is w else \
+        _output((rows, outer), out_dtype, w.device, w, w2)
     L = _lib.lib()
     ws_bytes = L.kq_quantized_matmul_workspace_bytes(_DT[x.dtype], rows, K) if rows > 1 else 0  # one row needs none
     if transpose and rows > 16:  # many rows: perhaps room for an fp16 copy of the weights, if the device has it
