@@ -1285,6 +1285,7 @@ static cudaError_t launch_half(GemmArgs a, cudaStream_t st) {
   // taken is within 6 % of the best one (2.7, 450, 9000, 3000, and 148 CTAs at once whatever the cluster: up to 43 % off -
   // x 64 [4096, 4096] took 148 CTAs in clusters of four, two waves, 36.6 us against 23).
   const int kb = (a.K + kBK - 1) / kBK;
+  const int cap[9] = {0, half_resident(1), half_resident(2), 0, half_resident(4), 0, 0, 0, half_resident(8)};
   double best = 1e30;
   int mt = 2, bn = 256, ks = 1;
   for (int t = 1; t <= 2; t++) {
@@ -1292,9 +1293,8 @@ static cudaError_t launch_half(GemmArgs a, cudaStream_t st) {
     for (int b = 256; b >= 64; b -= 16) {
       const long long tiles = (long long)((a.N + b - 1) / b) * ((a.M + 128 * t - 1) / (128 * t));
       for (int z = 1; z <= 8 && kb % z == 0 && (z == 1 || t * (b > 128 ? 2 : 1) <= 2); z *= 2) {
-        const int cap = half_resident(z);
         const double step = std::max({2.0 * t * b, 2.0 * (128 * t + b), 700.0});
-        const double c = (double)((tiles * z + cap - 1) / cap) * (kb / z * step + 9000.0 + 1000.0 * (z - 1));
+        const double c = (double)((tiles * z + cap[z] - 1) / cap[z]) * (kb / z * step + 9000.0 + 1000.0 * (z - 1));
         if (c < best * 0.999) best = c, mt = t, bn = b, ks = z;
       }
     }
