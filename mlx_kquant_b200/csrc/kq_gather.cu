@@ -33,6 +33,14 @@ static bool use_grouped(long long n_entries, int M, int n_experts, int K) {
   return K > 0 && (K % 8) == 0 && rows >= 512 && rows >= 16LL * n_experts && rows < (1LL << 31);
 }
 
+// Rows of a tile: what an expert has on average and half as much again, so that few experts need a second tile; the tile
+// kernel keeps two accumulators, and its epilogues out of the way, up to 128.
+static int grouped_tile_rows(long long rows, int n_experts) {
+  const long long avg = rows / (n_experts > 0 ? n_experts : 1);
+  const int t = avg <= 40 ? 64 : (avg <= 85 ? 128 : kGroupedTileRows);
+  return rows / t + n_experts <= 65535 ? t : kGroupedTileRows;
+}
+
 GatherLayout gather_layout(long long n_entries, int M, int n_experts, int K) {
   GatherLayout L;
   const long long rows = n_entries * (long long)M;
@@ -42,7 +50,8 @@ GatherLayout gather_layout(long long n_entries, int M, int n_experts, int K) {
   if (mt < 1) mt = 1;
   L.max_tasks = mt;
   L.grouped = use_grouped(n_entries, M, n_experts, K);
-  L.max_tiles = rows / kGroupedTileRows + n_experts;
+  L.tile_rows = grouped_tile_rows(rows, n_experts);
+  L.max_tiles = rows / L.tile_rows + n_experts;
   size_t off = 0;
   L.counts = off;    off = align_up(off + sizeof(int) * (size_t)n_experts, 256);
   L.cursor = off;    off = align_up(off + sizeof(int) * (size_t)n_experts, 256);
@@ -170,23 +179,28 @@ __global__ void gather_tasks_kernel(const uint8_t* w, long long expert_stride, i
   }
 }
 
-// grid.x = expert: the expert's c*M sorted rows cut into tiles of kGroupedTileRows
+// Tile j of nt tiles that an expert's rows are cut into: even parts, whole sixteens but for the last (266 rows as 144 and
+// 122 rather than 256 and 10: a tile's weights are dequantized whatever its rows).
 struct GatherTile {
   int expert, row_start, rows, pad;
 };
-__global__ void gather_tiles_kernel(int M, const int* __restrict__ offsets, const int* __restrict__ tile_base,
+__device__ __forceinline__ GatherTile even_tile(int expert, long long start, long long rows, int nt, int j) {
+  const long long per = ((rows + nt - 1) / nt + 15) / 16 * 16;
+  const long long from = j * per;  // < rows: per <= tile_rows, and nt - 1 full tiles would not hold all rows
+  GatherTile t;
+  t.expert = expert;
+  t.row_start = (int)(start + from);
+  t.rows = (int)min(per, rows - from);
+  t.pad = 0;
+  return t;
+}
+// grid.x = expert: the expert's c*M sorted rows cut into tiles of at most tile_rows
+__global__ void gather_tiles_kernel(int M, int tile_rows, const int* __restrict__ offsets, const int* __restrict__ tile_base,
                                     GatherTile* tiles) {
   const int e = blockIdx.x;
   const long long start = (long long)offsets[e] * M, rows = (long long)(offsets[e + 1] - offsets[e]) * M;
-  const int nt = (int)((rows + kGroupedTileRows - 1) / kGroupedTileRows);
-  for (int j = threadIdx.x; j < nt; j += blockDim.x) {
-    GatherTile t;
-    t.expert = e;
-    t.row_start = (int)(start + (long long)j * kGroupedTileRows);
-    t.rows = (int)min((long long)kGroupedTileRows, rows - (long long)j * kGroupedTileRows);
-    t.pad = 0;
-    tiles[tile_base[e] + j] = t;
-  }
+  const int nt = (int)((rows + tile_rows - 1) / tile_rows);
+  for (int j = threadIdx.x; j < nt; j += blockDim.x) tiles[tile_base[e] + j] = even_tile(e, start, rows, nt, j);
 }
 
 // ---------------------------------------------------------------- tile map + segment product
@@ -239,12 +253,12 @@ cudaError_t launch_tile_map(const uint32_t* indices, long long rows, int n_exper
 
 // gather_qmm_seg (src/kquant_ops.cpp:466-548): the caller's map becomes the tile kernel's list. Maps built by
 // expert_tile_map or by the host recipe (mlx_kquant/nn.py:33-47) give every expert ONE run of consecutive rows cut in
-// 64-row pieces; such a run is re-cut into tiles of kGroupedTileRows rows, so that a weight tile is dequantized once
-// per 256 rows instead of once per 64. A map whose pieces of an expert do not add up to one run is taken piece by
+// 64-row pieces; such a run is re-cut into tiles of up to tile_rows rows, so that a weight tile is dequantized once for
+// them instead of once per 64. A map whose pieces of an expert do not add up to one run is taken piece by
 // piece (pieces longer than a tile are split). One CTA; seg = 3 n_experts ints of scratch.
 __global__ void __launch_bounds__(1024)
 seg_tiles_kernel(const uint32_t* __restrict__ map, const uint32_t* __restrict__ count, int cap, int n_experts,
-                 long long rows_total, int* seg, GatherTile* tiles, int max_tiles, int* n_tiles) {
+                 long long rows_total, int* seg, GatherTile* tiles, int max_tiles, int tile_rows, int* n_tiles) {
   __shared__ int s_scan[1024];
   __shared__ int irregular, carry, appended;
   int* seg_start = seg;
@@ -273,7 +287,7 @@ seg_tiles_kernel(const uint32_t* __restrict__ map, const uint32_t* __restrict__ 
     for (int base = 0; base < n_experts; base += 1024) {
       const int e = base + threadIdx.x;
       const int len = e < n_experts ? seg_len[e] : 0;
-      const int nt = (len + kGroupedTileRows - 1) / kGroupedTileRows;
+      const int nt = (len + tile_rows - 1) / tile_rows;
       s_scan[threadIdx.x] = nt;
       __syncthreads();
       for (int d = 1; d < 1024; d <<= 1) {
@@ -285,12 +299,7 @@ seg_tiles_kernel(const uint32_t* __restrict__ map, const uint32_t* __restrict__ 
       const int first = carry + s_scan[threadIdx.x] - nt;
       for (int j = 0; j < nt; j++) {
         if (first + j >= max_tiles) break;
-        GatherTile t;
-        t.expert = e;
-        t.row_start = seg_start[e] + j * kGroupedTileRows;
-        t.rows = min(kGroupedTileRows, len - j * kGroupedTileRows);
-        t.pad = 0;
-        tiles[first + j] = t;
+        tiles[first + j] = even_tile(e, seg_start[e], len, nt, j);
       }
       __syncthreads();
       if (threadIdx.x == 1023) carry += s_scan[1023];
@@ -301,13 +310,13 @@ seg_tiles_kernel(const uint32_t* __restrict__ map, const uint32_t* __restrict__ 
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
       const uint32_t e = map[3 * t], r0 = map[3 * t + 1], nr = map[3 * t + 2];
       if (nr == 0 || e >= (uint32_t)n_experts || (long long)r0 + nr > rows_total) continue;
-      for (uint32_t off = 0; off < nr; off += kGroupedTileRows) {
+      for (uint32_t off = 0; off < nr; off += tile_rows) {
         const int slot = atomicAdd(&appended, 1);
         if (slot >= max_tiles) break;
         GatherTile g;
         g.expert = (int)e;
         g.row_start = (int)(r0 + off);
-        g.rows = (int)min((uint32_t)kGroupedTileRows, nr - off);
+        g.rows = (int)min((uint32_t)tile_rows, nr - off);
         g.pad = 0;
         tiles[slot] = g;
       }
@@ -317,11 +326,17 @@ seg_tiles_kernel(const uint32_t* __restrict__ map, const uint32_t* __restrict__ 
   }
 }
 
-static long long seg_max_tiles(long long rows, long long cap) { return cap + rows / kGroupedTileRows + 1; }
+static int seg_tile_rows(long long rows, long long cap, int n_experts) {
+  const int t = grouped_tile_rows(rows, n_experts);
+  return cap + rows / t + 1 <= 65535 ? t : kGroupedTileRows;
+}
+static long long seg_max_tiles(long long rows, long long cap, int n_experts) {
+  return cap + rows / seg_tile_rows(rows, cap, n_experts) + 1;
+}
 
 size_t gather_seg_workspace_bytes(int x_dtype, long long rows, int K, int n_experts, long long cap) {
   size_t b = ((size_t)(3 * n_experts + 1) * 4 + 255) & ~(size_t)255;                        // seg + n_tiles
-  b += ((size_t)seg_max_tiles(rows, cap) * sizeof(GatherTile) + 255) & ~(size_t)255;        // tiles
+  b += ((size_t)seg_max_tiles(rows, cap, n_experts) * sizeof(GatherTile) + 255) & ~(size_t)255;        // tiles
   if (x_dtype != F16) {
     b += ((size_t)rows * (size_t)K * 2 + 255) & ~(size_t)255;                               // fp16 copy of x
     b += ((size_t)rows * 4 + 255) & ~(size_t)255;                                           // row factors
@@ -339,10 +354,11 @@ cudaError_t launch_gather_seg(int codec, int x_dtype, const void* x, long long r
   int* n_tiles = seg + 3 * n_experts;
   size_t off = ((size_t)(3 * n_experts + 1) * 4 + 255) & ~(size_t)255;
   GatherTile* tiles = reinterpret_cast<GatherTile*>(ws + off);
-  const long long max_tiles = seg_max_tiles(rows, cap);
+  const long long max_tiles = seg_max_tiles(rows, cap, n_experts);
   if (max_tiles > 65535) return cudaErrorInvalidConfiguration;
   off += ((size_t)max_tiles * sizeof(GatherTile) + 255) & ~(size_t)255;
-  seg_tiles_kernel<<<1, 1024, 0, st>>>(map, count, (int)cap, n_experts, rows, seg, tiles, (int)max_tiles, n_tiles);
+  seg_tiles_kernel<<<1, 1024, 0, st>>>(map, count, (int)cap, n_experts, rows, seg, tiles, (int)max_tiles,
+                                       seg_tile_rows(rows, cap, n_experts), n_tiles);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
   const void* xh = x;
@@ -356,7 +372,7 @@ cudaError_t launch_gather_seg(int codec, int x_dtype, const void* x, long long r
     rs = rsw;
   }
   return launch_gemm_tiles(codec, x_dtype == F16, xh, rows, K, w, expert_stride, row_bytes, N, y, rs, nullptr, tiles,
-                           n_tiles, (int)max_tiles, st);
+                           n_tiles, (int)max_tiles, n_experts, seg_tile_rows(rows, cap, n_experts), st);
 }
 
 cudaError_t launch_gather(int codec, int x_dtype, const void* x, long long x_batch, int M, int K, const uint8_t* w,
@@ -382,19 +398,19 @@ cudaError_t launch_gather(int codec, int x_dtype, const void* x, long long x_bat
   const int th = 256;
   const unsigned nb = (unsigned)((n_entries + th - 1) / th);
   gather_hist_kernel<<<nb, th, 0, st>>>(rhs, lhs, x_batch, n_entries, n_experts, counts);
-  gather_scan_kernel<<<1, 1024, 0, st>>>(counts, n_experts, M, L.grouped ? kGroupedTileRows : 16, offsets, task_base,
+  gather_scan_kernel<<<1, 1024, 0, st>>>(counts, n_experts, M, L.grouped ? L.tile_rows : 16, offsets, task_base,
                                          n_tasks);
   gather_scatter_kernel<<<nb, th, 0, st>>>(rhs, lhs, x_batch, n_entries, n_experts, offsets, cursor, order);
 
   if (L.grouped) {
     GatherTile* tiles = reinterpret_cast<GatherTile*>(ws + L.tiles);
-    gather_tiles_kernel<<<n_experts, 64, 0, st>>>(M, offsets, task_base, tiles);
+    gather_tiles_kernel<<<n_experts, 64, 0, st>>>(M, L.tile_rows, offsets, task_base, tiles);
     if ((err = cudaGetLastError()) != cudaSuccess) return err;
     if (L.max_tiles > 65535) return cudaErrorInvalidConfiguration;
     return launch_gemm_grouped(codec, x_dtype, x, M, K, w, expert_stride, row_bytes, N, lhs, order,
                                n_entries * (long long)M, y, reinterpret_cast<__half*>(ws + L.xh),
                                reinterpret_cast<float*>(ws + L.row_scale), reinterpret_cast<int*>(ws + L.yrow), tiles,
-                               n_tasks, (int)L.max_tiles, offsets + n_experts, st);
+                               n_tasks, (int)L.max_tiles, n_experts, L.tile_rows, offsets + n_experts, st);
   }
 
   GemvTask* tasks = reinterpret_cast<GemvTask*>(ws + L.tasks);
@@ -453,11 +469,13 @@ namespace {
 struct MoeBlockLayout {
   size_t counts, cursor, offsets, tile_base, n_tiles, order, tiles, yrow, scale1, scale2, xh, gu, hh, total;
   long long max_tiles;
+  int tile_rows;
 };
 MoeBlockLayout moe_block_layout(long long T, int k, int E, int H, int F) {
   MoeBlockLayout L;
   const size_t rows = (size_t)(T * k);
-  L.max_tiles = (long long)rows / kGroupedTileRows + E;
+  L.tile_rows = grouped_tile_rows((long long)rows, E);
+  L.max_tiles = (long long)rows / L.tile_rows + E;
   size_t off = 0;
   L.counts = off;    off = align_up(off + 4 * (size_t)E, 256);
   L.cursor = off;    off = align_up(off + 4 * (size_t)E, 256);
@@ -518,9 +536,9 @@ cudaError_t launch_moe_block(int codec, int x_dtype, const void* x, long long x_
   const int th = 256;
   const unsigned nb = (unsigned)((n + th - 1) / th);
   gather_hist_kernel<<<nb, th, 0, st>>>(idx, nullptr, 0, n, n_experts, counts);
-  gather_scan_kernel<<<1, 1024, 0, st>>>(counts, n_experts, 1, kGroupedTileRows, offsets, tile_base, n_tiles);
+  gather_scan_kernel<<<1, 1024, 0, st>>>(counts, n_experts, 1, L.tile_rows, offsets, tile_base, n_tiles);
   gather_scatter_kernel<<<nb, th, 0, st>>>(idx, nullptr, 0, n, n_experts, offsets, cursor, order);
-  gather_tiles_kernel<<<n_experts, 64, 0, st>>>(1, offsets, tile_base, tiles);
+  gather_tiles_kernel<<<n_experts, 64, 0, st>>>(1, L.tile_rows, offsets, tile_base, tiles);
   if ((err = cudaGetLastError()) != cudaSuccess) return err;
   const int* n_valid = offsets + n_experts;  // entries whose expert is in range: the sorted rows that exist
   const bool half = x_dtype == F16;
@@ -529,13 +547,13 @@ cudaError_t launch_moe_block(int codec, int x_dtype, const void* x, long long x_
                             st)) != cudaSuccess)
     return err;
   if ((err = launch_gemm_tiles(codec, half, xh, n, H, wgu, stride_gu, rb_h, 2 * F, gu, half ? nullptr : scale1, nullptr,
-                               tiles, n_tiles, (int)L.max_tiles, st)) != cudaSuccess)
+                               tiles, n_tiles, (int)L.max_tiles, n_experts, L.tile_rows, st)) != cudaSuccess)
     return err;
   if ((err = launch_convert(x_dtype, gu, 2LL * F, F, n, nullptr, nullptr, 1, 1, hh, scale2, nullptr, n_valid, true, st)) !=
       cudaSuccess)
     return err;
   if ((err = launch_gemm_tiles(codec, half, hh, n, F, wd, stride_d, rb_f, H, d, half ? nullptr : scale2, yrow, tiles,
-                               n_tiles, (int)L.max_tiles, st)) != cudaSuccess)
+                               n_tiles, (int)L.max_tiles, n_experts, L.tile_rows, st)) != cudaSuccess)
     return err;
   if (scatter != nullptr)
     return launch_moe_combine_scatter(x_dtype, d, scores, idx, (uint32_t)n_experts, T, k, H, scatter->tokens_per_rank,

@@ -76,8 +76,8 @@ cudaError_t launch_gemm(int codec, int x_dtype, const void* x, long long x_row_s
                         size_t workspace_bytes, cudaStream_t st);
 // With the room for an fp16 copy of (a part of) the weights where the call would use one.
 size_t gemm_workspace_bytes_n(int codec, int x_dtype, long long rows, int N, int K);
-// Grouped (mixture-of-experts) prefill: 256-row tiles of expert-sorted rows, see kq_gather.cu.
-constexpr int kGroupedTileRows = 256;
+// Grouped (mixture-of-experts) prefill: tiles of expert-sorted rows, see kq_gather.cu.
+constexpr int kGroupedTileRows = 256;  // most rows of a tile
 constexpr int kSegMapTileRows = 64;  // rows per entry of an expert tile map (the reference kernel's tile height)
 // expert_tile_map / gather_qmm_seg (kq_gather.cu)
 size_t tile_map_workspace_bytes(int n_experts);
@@ -91,11 +91,35 @@ cudaError_t launch_gemm_grouped(int codec, int x_dtype, const void* x, int M, in
                                 long long expert_stride, long long row_bytes, int N, const uint32_t* lhs,
                                 const int* order, long long rows_total, void* y, __half* xh, float* row_scale,
                                 int* yrow, const void* tiles, const int* n_tiles_dev, int max_tiles,
-                                const int* n_valid_dev, cudaStream_t st);
+                                int n_experts, int tile_rows, const int* n_valid_dev, cudaStream_t st);
 cudaError_t launch_gemm_tiles(int codec, bool out_half, const void* xh, long long rows_total, int K, const uint8_t* w,
                               long long expert_stride, long long row_bytes, int N, void* y, const float* row_scale,
-                              const int* yrow, const void* tiles, const int* n_tiles_dev, int max_tiles,
-                              cudaStream_t st);
+                              const int* yrow, const void* tiles, const int* n_tiles_dev, int max_tiles, int n_experts,
+                              int tile_rows, cudaStream_t st);
+// The tile kernel with the weights on the M side (kq_tile.cu). x: fp16 rows [M, K]; w: wire bytes of a codec that
+// tile_supported() takes, or (half_weights) an fp16 matrix [N, K]; tiles: grouped mode, at most max_tiles row tiles.
+struct GemmTile {
+  int expert, row_start, rows, pad;
+};
+struct TileArgs {
+  const void* x;
+  long long x_row_stride;
+  const uint8_t* w;
+  long long row_bytes, expert_stride;
+  int n_experts;
+  void* y;
+  long long y_row_stride;
+  const float* row_scale;
+  const int* yrow;
+  int M, N, K;
+  const GemmTile* tiles;
+  const int* n_tiles_dev;
+  int max_tiles, tile_rows;  // tile_rows: most rows of a tile, a multiple of 16, at most 256
+};
+bool tile_supported(int codec, const uint8_t* w, long long row_bytes, int N, int K, long long expert_stride);
+// estimated cycles of a dense call (half_weights: without the dequantization)
+double tile_cycles(int codec, bool half_weights, int M, int N, int K);
+cudaError_t launch_tile(int codec, bool half_weights, bool out_half, const TileArgs& t, cudaStream_t st);
 // Flags raised by kernels that gave up on a bounded wait (0 = none); synchronises the device.
 cudaError_t read_device_error(int* out, bool clear);
 int* device_error_word();  // device address of that flag word on the current device (nullptr on failure)
@@ -173,6 +197,7 @@ struct GatherLayout {
   bool grouped;
   size_t xh, row_scale, yrow, tiles;
   long long max_tiles;
+  int tile_rows;  // most rows of a tile
 };
 // K > 0 lets the layout include the grouped regime's buffers when that regime would be chosen;
 // K == 0 is the decode-only layout (the skinny kernel over task lists).
