@@ -372,7 +372,7 @@ cudaError_t launch_gather_seg(int codec, int x_dtype, const void* x, long long r
     rs = rsw;
   }
   return launch_gemm_tiles(codec, x_dtype == F16, xh, rows, K, w, expert_stride, row_bytes, N, y, rs, nullptr, tiles,
-                           n_tiles, (int)max_tiles, n_experts, seg_tile_rows(rows, cap, n_experts), st);
+                           n_tiles, (int)max_tiles, n_experts, seg_tile_rows(rows, cap, n_experts), x_dtype != F16, st);
 }
 
 cudaError_t launch_gather(int codec, int x_dtype, const void* x, long long x_batch, int M, int K, const uint8_t* w,
@@ -547,13 +547,13 @@ cudaError_t launch_moe_block(int codec, int x_dtype, const void* x, long long x_
                             st)) != cudaSuccess)
     return err;
   if ((err = launch_gemm_tiles(codec, half, xh, n, H, wgu, stride_gu, rb_h, 2 * F, gu, half ? nullptr : scale1, nullptr,
-                               tiles, n_tiles, (int)L.max_tiles, n_experts, L.tile_rows, st)) != cudaSuccess)
+                               tiles, n_tiles, (int)L.max_tiles, n_experts, L.tile_rows, true, st)) != cudaSuccess)
     return err;
   if ((err = launch_convert(x_dtype, gu, 2LL * F, F, n, nullptr, nullptr, 1, 1, hh, scale2, nullptr, n_valid, true, st)) !=
       cudaSuccess)
     return err;
   if ((err = launch_gemm_tiles(codec, half, hh, n, F, wd, stride_d, rb_f, H, d, half ? nullptr : scale2, yrow, tiles,
-                               n_tiles, (int)L.max_tiles, n_experts, L.tile_rows, st)) != cudaSuccess)
+                               n_tiles, (int)L.max_tiles, n_experts, L.tile_rows, true, st)) != cudaSuccess)
     return err;
   if (scatter != nullptr)
     return launch_moe_combine_scatter(x_dtype, d, scores, idx, (uint32_t)n_experts, T, k, H, scatter->tokens_per_rank,

@@ -457,6 +457,7 @@ __global__ void __launch_bounds__(256)
 convert_x_scalar_kernel(const XT* __restrict__ x, long long x_row_stride, int K, __half* __restrict__ xh,
                  float* __restrict__ row_scale, const int* __restrict__ order, const uint32_t* __restrict__ lhs, int M,
                  int* __restrict__ yrow, const int* __restrict__ n_valid) {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");  // the tile kernel fetches weights meanwhile
   const long long row = blockIdx.x;
   long long src_row = row;
   // gather mode: entries whose expert index is out of range were never placed in `order`; its tail is unset
@@ -589,6 +590,7 @@ template <typename XT>
 __global__ void __launch_bounds__(256)
 convert_rows_kernel(const XT* __restrict__ x, long long x_row_stride, int K, __half* __restrict__ xh,
                     float* __restrict__ row_scale) {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   __shared__ float s_max[8];
   const XT* xr = x + blockIdx.x * x_row_stride;
   __half* o = xh + blockIdx.x * (long long)K;
@@ -633,6 +635,7 @@ convert_x_kernel(const XT* __restrict__ x, long long x_row_stride, int K, __half
                  float* __restrict__ row_scale, const int* __restrict__ order, const uint32_t* __restrict__ lhs,
                  int lhs_div, int M, int* __restrict__ yrow, const int* __restrict__ n_valid, long long rows) {
   static_assert(!GLU || sizeof(XT) == 2, "the fused activation takes fp16 / bf16 gate | up rows");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   const int lane = threadIdx.x & 31;
   // rows that exist: all, or the first *n_valid * M in gather mode (see the scalar kernel). The grid is capped on
   // the host and the warps stride over the rows, so a list sized for many more rows than it holds costs nothing.
@@ -923,6 +926,7 @@ cudaError_t launch_gemm(int codec, int x_dtype, const void* x, long long x_row_s
   t.M = M;
   t.N = N;
   t.K = K;
+  t.after_prepass = x_dtype != F16;
   // fp16 rows need no workspace: one that cannot hold the copy, for its size or its alignment, is left alone
   const bool room = use_half(codec, M, N, K) && workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255) == 0 &&
                     workspace_bytes >= base + half_bytes(N, K) &&
@@ -938,6 +942,7 @@ cudaError_t launch_gemm(int codec, int x_dtype, const void* x, long long x_row_s
     const int chunk = half_chunk(N, K);
     t.w = wh;
     t.row_bytes = 2ll * K;
+    t.after_prepass = 1;
     for (int n0 = 0; n0 < N; n0 += chunk) {
       t.N = std::min(chunk, N - n0);
       cudaError_t e = launch_dequantize(codec, w + (long long)n0 * row_bytes, (long long)t.N * (K / kCodecs[codec].wpb), F16,
@@ -994,7 +999,7 @@ cudaError_t launch_gemm_grouped(int codec, int x_dtype, const void* x, int M, in
   if (e != cudaSuccess) return e;
   return launch_gemm_tiles(codec, x_dtype == F16, xh, rows_total, K, w, expert_stride, row_bytes, N, y,
                            x_dtype == F16 ? nullptr : row_scale, yrow, tiles, n_tiles_dev, max_tiles, n_experts, tile_rows,
-                           st);
+                           true, st);
 }
 
 // The tile kernels over a device-built list of (expert, row_start, rows <= tile_rows) tiles: fp16 activations xh
@@ -1002,12 +1007,13 @@ cudaError_t launch_gemm_grouped(int codec, int x_dtype, const void* x, int M, in
 cudaError_t launch_gemm_tiles(int codec, bool out_half, const void* xh, long long rows_total, int K, const uint8_t* w,
                               long long expert_stride, long long row_bytes, int N, void* y, const float* row_scale,
                               const int* yrow, const void* tiles, const int* n_tiles_dev, int max_tiles, int n_experts,
-                              int tile_rows, cudaStream_t st) {
+                              int tile_rows, bool after_prepass, cudaStream_t st) {
   if (rows_total <= 0 || N <= 0 || K <= 0 || max_tiles <= 0) return cudaSuccess;
   if (max_tiles > 65535) return cudaErrorInvalidConfiguration;
   if (tile_supported(codec, w, row_bytes, N, K, expert_stride)) {
     TileArgs t{xh,   K,         w,    row_bytes, expert_stride,  n_experts, y, N, row_scale, yrow, (int)rows_total,
-               N,    K,         static_cast<const GemmTile*>(tiles), n_tiles_dev, max_tiles, tile_rows};
+               N,    K,         static_cast<const GemmTile*>(tiles), n_tiles_dev, max_tiles, tile_rows,
+               after_prepass};
     return launch_tile(codec, false, out_half, t, st);
   }
   // The list may hold up to max_tiles tiles but usually holds far fewer (an expert-parallel rank sizes it for all

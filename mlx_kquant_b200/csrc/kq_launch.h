@@ -95,7 +95,7 @@ cudaError_t launch_gemm_grouped(int codec, int x_dtype, const void* x, int M, in
 cudaError_t launch_gemm_tiles(int codec, bool out_half, const void* xh, long long rows_total, int K, const uint8_t* w,
                               long long expert_stride, long long row_bytes, int N, void* y, const float* row_scale,
                               const int* yrow, const void* tiles, const int* n_tiles_dev, int max_tiles, int n_experts,
-                              int tile_rows, cudaStream_t st);
+                              int tile_rows, bool after_prepass, cudaStream_t st);
 // The tile kernel with the weights on the M side (kq_tile.cu). x: fp16 rows [M, K]; w: wire bytes of a codec that
 // tile_supported() takes, or (half_weights) an fp16 matrix [N, K]; tiles: grouped mode, at most max_tiles row tiles.
 struct GemmTile {
@@ -115,6 +115,8 @@ struct TileArgs {
   const GemmTile* tiles;
   const int* n_tiles_dev;
   int max_tiles, tile_rows;  // tile_rows: most rows of a tile, a multiple of 16, at most 256
+  int after_prepass;  // the launch before on this stream makes x and row_scale (launch_convert) or the fp16 weights: the
+                      // kernel starts beside it and waits for what it writes
 };
 bool tile_supported(int codec, const uint8_t* w, long long row_bytes, int N, int K, long long expert_stride);
 // estimated cycles of a dense call (half_weights: without the dequantization)

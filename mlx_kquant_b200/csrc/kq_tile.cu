@@ -67,6 +67,7 @@ struct TilePlan {
   int stages, raw_stages, n_acc, acc_cols, tmem_cols;
   int lg;                     // wire rows are whole multiples of 16 bytes in groups of 1 << lg (q4_k: 0)
   int row_bytes;
+  int after_prepass;          // the launch before is the pre-pass of this call: its results are waited for here
   int stage_bytes, raw_off, stg_off, stg_tokens;
   int* error_word;
 };
@@ -417,6 +418,7 @@ tile_kernel(const TilePlan a, const __grid_constant__ CUtensorMap map_x, const _
     bool ok = true;
     int done = 0;
     Tile next = tile_at(first);
+    if (a.after_prepass) asm volatile("griddepcontrol.wait;\n" ::: "memory");  // row_scale, yrow
     for (int t = first; t < total && ok; t += stride, done++) {
       const Tile tl = next;
       if (t + stride < total) next = tile_at(t + stride);  // (fetched a tile ahead: grouped tiles come from memory)
@@ -563,6 +565,7 @@ tile_kernel(const TilePlan a, const __grid_constant__ CUtensorMap map_x, const _
     int s = 0, it = 0;
     uint32_t ph = 1;
     const uint32_t bytes = KS * CG * (x_tile + (kFused ? 0 : kWTileBytes));
+    if (a.after_prepass) asm volatile("griddepcontrol.wait;\n" ::: "memory");  // fp16 rows, or fp16 weights
     Tile next = tile_at(first);
     for (int t = first; t < total && ok; t += stride) {
       const Tile tl = next;
@@ -816,13 +819,18 @@ cudaError_t launch_tile_t(TileCall c, int tn, cudaStream_t st) {
   cfg.blockDim = dim3(tile_threads(SRC));
   cfg.dynamicSmemBytes = dyn;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CG;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = c.ks;
-  cfg.attrs = attr;
-  cfg.numAttrs = CG * c.ks > 1 ? 1 : 0;
+  // Everything before the pre-pass has ended when this kernel may start (the pre-pass itself is launched plainly), so the
+  // weights, tile lists and so on are read at once; only what the pre-pass writes is waited for.
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = CG;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = c.ks;
+  const int skip = c.p.after_prepass ? 0 : 1;
+  cfg.attrs = attr + skip;
+  cfg.numAttrs = (CG * c.ks > 1 ? 2 : 1) - skip;
   return cudaLaunchKernelEx(&cfg, kern, c.p, map_x, map_w);
 }
 
@@ -963,6 +971,7 @@ cudaError_t launch_tile(int codec, bool half_weights, bool out_half, const TileA
   c.p.tblk = t.max_tiles;
   c.p.lg = half_weights ? 0 : row_group(t.row_bytes);
   c.p.row_bytes = (int)t.row_bytes;
+  c.p.after_prepass = t.after_prepass;
   c.x = t.x;
   c.x_row_stride = t.x_row_stride;
   c.x_rows = t.M;
