@@ -226,6 +226,21 @@ __device__ __forceinline__ void expect_tx(uint32_t e, uint64_t* bar, uint32_t by
       "r"(bytes), "r"(e)
       : "memory");
 }
+// 16 lanes x 16 columns of tensor memory: thread t holds lanes t / 4 (r[0], r[1], r[4], r[5]) and 8 + t / 4, columns
+// 2 (t % 4) and the one after it of the first eight (r[0] .. r[3]) and of the second
+__device__ __forceinline__ void tmem_ld_16x16(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+// four 8 x 8 matrices of 16-bit values, transposed: thread i gives the address of row i % 8 of matrix i / 8
+__device__ __forceinline__ void store_trans(uint32_t addr, const uint32_t (&v)[4]) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};\n" ::"r"(addr), "r"(v[0]), "r"(v[1]),
+               "r"(v[2]), "r"(v[3])
+               : "memory");
+}
+
 // ------------------------------------------------------------------ producers: half a superblock of a row
 // A producer thread makes 128 weights of its row at a time, 64 TMEM columns in two pieces of 32 registers: what a
 // piece of work costs besides the weights (waits, arrivals, the block's header) was half of the instructions with 64.
@@ -439,9 +454,9 @@ tile_kernel(const TilePlan a, const __grid_constant__ CUtensorMap map_x, const _
       if (!ok) break;
       tc_fence_after();
       const uint32_t acc = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(as * a.acc_cols);
-      // weight row of this thread's TMEM lane: classes of rows modulo 1 << lg one after the other
-      const int at = 32 * warp + lane, n_row = ((at & ((128 >> a.lg) - 1)) << a.lg) | (at >> (7 - a.lg));
       if (gridDim.z > 1) {
+        // weight row of this thread's TMEM lane: classes of rows modulo 1 << lg one after the other
+        const int at = 32 * warp + lane, n_row = ((at & ((128 >> a.lg) - 1)) << a.lg) | (at >> (7 - a.lg));
         float* part = reinterpret_cast<float*>(ring);  // [token][128] (the rings are idle: every MMA has completed)
         for (int c0 = 0; c0 < tl.cols; c0 += 16) {
           uint32_t v[16];
@@ -453,32 +468,47 @@ tile_kernel(const TilePlan a, const __grid_constant__ CUtensorMap map_x, const _
         break;
       }
       for (int cb = 0; cb < tl.cols; cb += a.stg_tokens) {
-        // A thread owns a weight row, i.e. a column of y: it writes two bytes per token, a warp 64 neighbouring ones.
+        // Rows of the accumulator are columns of y: the fragments are stored transposed, [token][128], the sixteen 16-byte
+        // pieces of a row XOR-swizzled by the token. The next columns are on their way while these are rounded. (A thread
+        // per weight row with a two-byte store per token took 27 cycles a column, 7000 a tile; now 8.)
         const int ce = min(tl.cols, cb + a.stg_tokens);
-        uint8_t* stg = ring + a.stg_off + 2 * n_row;
-        for (int c0 = cb; c0 < ce; c0 += 32) {
-          uint32_t va[16], vb[16];
-          const bool two = c0 + 16 < ce;
-          tmem_ld16(acc + c0, va);
-          if (two) tmem_ld16(acc + c0 + 16, vb);
-          tmem_ld_wait();
-          auto put = [&](const uint32_t (&v)[16], int c) {
+        const int tok = lane & 7, piece = 4 * warp + (lane >> 3);
+        const uint32_t stg = smem_u32(ring) + a.stg_off + tok * 256 + ((piece ^ tok) << 4);
+        uint32_t r0[2][8], r1[2][8];
+        auto fetch = [&](uint32_t (&r)[2][8], int c) {
+          tmem_ld_16x16(acc + c, r[0]);
+          tmem_ld_16x16(acc + (16u << 16) + c, r[1]);
+        };
+        auto put = [&](const uint32_t (&r)[2][8], int c) {
 #pragma unroll
-            for (int i = 0; i < 16; i += 4) {
-              const float4 s4 = *reinterpret_cast<const float4*>(&s_scale[c + i]);
-              const float f[4] = {__uint_as_float(v[i]) * s4.x, __uint_as_float(v[i + 1]) * s4.y,
-                                  __uint_as_float(v[i + 2]) * s4.z, __uint_as_float(v[i + 3]) * s4.w};
+          for (int j = 0; j < 2; j++) {
+            const float2 f = *reinterpret_cast<const float2*>(&s_scale[c + 8 * j + 2 * (lane & 3)]);
+            uint32_t v[4];
 #pragma unroll
-              for (int j = 0; j < 4; j++) {
-                OT o;
-                if constexpr (kHalfOut) o = __float2half_rn(f[j]);
-                else o = __float2bfloat16_rn(f[j]);
-                *reinterpret_cast<OT*>(stg + (c + i + j - cb) * 256) = o;
+            for (int h = 0; h < 4; h++) {
+              const float lo = __uint_as_float(r[h >> 1][4 * j + 2 * (h & 1)]) * f.x;
+              const float hi = __uint_as_float(r[h >> 1][4 * j + 2 * (h & 1) + 1]) * f.y;
+              if constexpr (kHalfOut) {
+                const __half2 o = __floats2half2_rn(lo, hi);
+                v[h] = *reinterpret_cast<const uint32_t*>(&o);
+              } else {
+                const __nv_bfloat162 o = __floats2bfloat162_rn(lo, hi);
+                v[h] = *reinterpret_cast<const uint32_t*>(&o);
               }
             }
-          };
-          put(va, c0);
-          if (two) put(vb, c0 + 16);
+            store_trans(stg + (c + 8 * j - cb) * 256, v);
+          }
+        };
+        fetch(r0, cb);
+        for (int c0 = cb; c0 < ce; c0 += 32) {
+          tmem_ld_wait();
+          if (c0 + 16 < ce) fetch(r1, c0 + 16);
+          put(r0, c0);
+          if (c0 + 16 < ce) {
+            tmem_ld_wait();
+            if (c0 + 32 < ce) fetch(r0, c0 + 32);
+            put(r1, c0 + 16);
+          }
         }
         if (ce == tl.cols) {  // the accumulator has been read
           tc_fence_before();
@@ -503,7 +533,19 @@ tile_kernel(const TilePlan a, const __grid_constant__ CUtensorMap map_x, const _
           const long long o0 = __shfl_sync(0xffffffffu, mine0, i), o1 = __shfl_sync(0xffffffffu, mine1, i);
           const int r = 2 * warp + sub + 8 * i;
           if (r >= live) continue;
-          const uint4 q = *reinterpret_cast<const uint4*>(ring + a.stg_off + r * 256 + 16 * chunk);
+          const uint8_t* row = ring + a.stg_off + r * 256;
+          uint4 q;
+          if (SRC != kSrcQ6K || a.lg == 0) {
+            q = *reinterpret_cast<const uint4*>(row + ((chunk ^ (r & 7)) << 4));
+          } else {  // rows of one class lie together: eight neighbouring rows are in as many places
+            uint32_t* qw = &q.x;
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+              const int n = 8 * chunk + e, at = (n >> a.lg) | ((n & ((1 << a.lg) - 1)) << (7 - a.lg));
+              const uint32_t v = *reinterpret_cast<const unsigned short*>(row + (((at >> 3) ^ (r & 7)) << 4) + 2 * (at & 7));
+              qw[e >> 1] = (e & 1) ? qw[e >> 1] | (v << 16) : v;
+            }
+          }
           OT* yp = static_cast<OT*>(a.y) + (sub ? o1 : o0) * a.y_row_stride + col;
           if (col + 8 <= n_end && (reinterpret_cast<uintptr_t>(yp) & 15) == 0) {
             *reinterpret_cast<uint4*>(yp) = q;
