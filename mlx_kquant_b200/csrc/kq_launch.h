@@ -57,6 +57,11 @@ cudaError_t launch_gemv(int codec, int x_dtype, const GemvArgs& a, cudaStream_t 
 bool gemv_dp4a_supported(int codec, int x_dtype, const GemvArgs& a);
 cudaError_t launch_gemv_dp4a(int codec, int x_dtype, const GemvArgs& a, cudaStream_t st);
 
+// One dense row of q4_k, q5_k, q6_k whose rows are whole sixteens: products on the integer dot-product pipe, wire bytes by
+// TMA (kq_gemv_one.cu).
+bool gemv_one_supported(int codec, const GemvArgs& a);
+cudaError_t launch_gemv_one(int codec, int x_dtype, const GemvArgs& a, cudaStream_t st);
+
 // 1 to 16 dense rows of fp16 / bf16 on mma.sync over the integers themselves (kq_rows.cu).
 bool gemv_rows_supported(int codec, int x_dtype, const GemvArgs& a);
 cudaError_t launch_gemv_rows(int codec, int x_dtype, const GemvArgs& a, cudaStream_t st);

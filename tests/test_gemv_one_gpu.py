@@ -1,0 +1,73 @@
+"""One dense row: the TMA kernel of q4_k, q5_k, q6_k (kq_gemv_one.cu), and the integer dot-product kernels with rows that are
+not whole sixteens (kq_gemv_dp4a.cuh)."""
+import numpy as np
+import pytest
+import torch
+
+import mlx_kquant_b200 as kq
+from gpu_util import x_to_torch, y_to_f32
+from oracle.kq_oracle import Oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def product(codec, m, n, k, dt, seed):
+    rng = np.random.default_rng(seed)
+    rows = torch.from_numpy(rng.standard_normal((48, k)).astype(np.float32) * 0.05)
+    some = kq.quantize(rows, codec, torch.ones(k) if codec == "iq2_xxs" else None)[0].numpy()
+    pick = rng.integers(0, 48, n)
+    x, _ = x_to_torch(rng.standard_normal((m, k)).astype(np.float32), dt)
+    xr = (x.bfloat16() if dt == "f32" else x).double().cpu().numpy()
+    ref = (xr @ Oracle().dequantize(some, codec, "f32").astype(np.float64).T)[:, pick]
+    return x, torch.from_numpy(some[pick]).cuda(), ref
+
+
+def check(y, ref, dt):
+    # An activation as an integer is off by at most 2^-16 of the largest of its 32 (below 3 here), evenly spread: 2.6e-5 root
+    # mean square. The quants of q4_k and q5_k have a mean of half their range, twice the weights they stand for. Six of that
+    # for the largest of many outputs: 3.2e-4 < 2^-11 of the outputs' root mean square; then half a unit of the output type.
+    off = np.abs(y_to_f32(y).astype(np.float64) - ref) - (2.0 ** -11 if dt == "f16" else 2.0 ** -8) * np.abs(ref)
+    assert off.max() < 2.0 ** -11 * np.sqrt(np.mean(ref ** 2))
+
+
+# one block and several a CTA, rows that leave the last one short, fewer rows than SMs; superblocks fewer and more than warps
+# x slots, and the longest row; q6_k's K are multiples of 2048 here (whole sixteens)
+@pytest.mark.parametrize("codec,n,k", [("q4_k", 12300, 2048), ("q4_k", 33, 8192), ("q4_k", 1537, 16384), ("q4_k", 20001, 4096),
+                                       ("q5_k", 1024, 2048), ("q5_k", 5001, 768), ("q5_k", 90, 8448), ("q5_k", 14336, 256),
+                                       ("q6_k", 1025, 2048), ("q6_k", 4800, 4096), ("q6_k", 77, 14336), ("q6_k", 9999, 2048)])
+@pytest.mark.parametrize("dt", ["f16", "bf16", "f32"])
+def test_one_row(codec, n, k, dt):
+    x, w, ref = product(codec, 1, n, k, dt, n + k)
+    check(kq.quantized_matmul(x, w, None, codec), ref, dt)
+
+
+@pytest.mark.parametrize("codec", ["q4_k", "q5_k", "q6_k"])
+def test_not_finite(codec):
+    """An infinity or a NaN among the activations reaches every output; the largest bf16 numbers stay finite."""
+    x, w, ref = product(codec, 1, 1500, 8192, "bf16", 9)
+    for bad in (float("inf"), float("-inf"), float("nan")):
+        xb = x.clone()
+        xb[0, 4100] = bad
+        assert not torch.isfinite(kq.quantized_matmul(xb, w, None, codec)).any()
+    big = torch.zeros_like(x)
+    big[0, 7] = 1e38
+    assert torch.isfinite(kq.quantized_matmul(big, w, None, codec)).all()
+
+
+# rows of 2, 4 and 8 bytes past a sixteen: one to four of them, odd numbers of rows (a last block of one parity alone)
+@pytest.mark.parametrize("codec,m,n,k", [("q6_k", 1, 1001, 2304), ("q6_k", 1, 63, 5120), ("q3_k", 1, 1000, 1280), ("q3_k", 2, 31, 768),
+                                         ("q3_k", 4, 515, 1536), ("q2_k", 1, 400, 1536), ("q2_k", 3, 97, 256), ("iq4_xs", 1, 333, 2304),
+                                         ("iq2_xxs", 1, 20000, 2816), ("q6_k", 3, 129, 1280), ("q3_k", 1, 4100, 256)])
+@pytest.mark.parametrize("dt", ["f16", "f32"])
+def test_ragged_rows(codec, m, n, k, dt):
+    x, w, ref = product(codec, m, n, k, dt, n + k)
+    check(kq.quantized_matmul(x, w, None, codec), ref, dt)
+
+
+def test_ragged_rows_end_at_the_matrix():
+    """The last row's window runs past the matrix, which here is followed by nothing of its own: poisoned bytes do not matter."""
+    x, w, ref = product("q6_k", 1, 65, 1280, "f16", 4)
+    pad = torch.full((w.numel() + 4096,), 0xff, dtype=torch.uint8, device="cuda")
+    inside = pad[:w.numel()].view(w.shape)
+    inside.copy_(w)
+    check(kq.quantized_matmul(x, inside, None, "q6_k"), ref, "f16")
