@@ -1161,15 +1161,17 @@ cudaError_t launch_gemv(int codec, int x_dtype, const GemvArgs& a, cudaStream_t 
   const int groups = a.tasks ? a.n_tasks : (a.M + 15) / 16;
   if (groups <= 0) return cudaSuccess;
   if (groups > 65535) return cudaErrorInvalidConfiguration;
-  // Two to sixteen dense rows of q4_k, q5_k, q6_k: the integers themselves on mma.sync. Measured against the kernels
-  // below, [14336, 4096] x 8 rows: q4_k bf16 25.3 -> 17.4 us, q5_k 80 -> 19.5; q6_k [4096, 14336] 97.5 -> 24; q4_k [4096, 4096] 14.6 -> 7.3.
-  // One row stays below (q4_k [14336, 4096] 10.8 us against 16.0): there the matrix instruction has seven idle columns.
-  // Against two to four rows' own kernels: q4_k fp16 x 2 [4096, 4096] 6.8 us, 6.5 on the integer kernel below, [14336,
-  // 4096] 15.5 against 12.5; its 16-bit activations cost precision that these rows now have, so they stay here. Nine to
-  // sixteen fp16 rows of q4_k with K >= 8192 >= 2 N were up to 27 % faster on the fp16 kernel ([4096, 14336] x 16 24.4
-  // against 28.7), which loses infinities and activations below 1e-5.
-  // iq4_xs with long K in fp16 keeps its table kernel ([512, 8192] x 2 6.9 us against 7.4, [256, 14336] x 16 16.4 / 18.4).
+  // Two to sixteen dense rows of q4_k, q5_k, q6_k: the integers themselves on mma.sync, in kq_few.cu or kq_rows.cu. Against
+  // the kernels below, [14336, 4096] x 8 rows: q4_k bf16 25.3 -> 14.1 us, q5_k 80 -> 15.4; q4_k [4096, 4096] 14.6 -> 7.1.
+  // q4_k fp16 x 2 [14336, 4096] takes 13.1 us, on the integer kernel below 12.5: its 16-bit activations cost precision
+  // that these rows have, so they stay here. Nine to sixteen fp16 rows of q4_k with K >= 8192 >= 2 N were up to 27 % faster
+  // on the fp16 kernel ([4096, 14336] x 16 24.4 against 28.7), which loses infinities and activations below 1e-5.
+  // iq4_xs in fp16 with K too long for kq_few.cu keeps its table kernel ([256, 14336] x 16 16.4 us against 18.4).
   const bool iq4_long = codec == IQ4_XS && x_dtype == F16 && a.out_bf16 == 0 && a.K >= 8192 && (a.row_bytes & 15) == 0;
+  if (gemv_few_supported(codec, x_dtype, a)) {
+    const cudaError_t e = launch_gemv_few(codec, x_dtype, a, st);
+    if (e != cudaErrorNotSupported) return e;
+  }
   if (a.M >= 2 && !iq4_long && gemv_rows_supported(codec, x_dtype, a)) return launch_gemv_rows(codec, x_dtype, a, st);
   // K split (= cluster size). Measured on B200: what matters is (a) at least two
   // CTAs per SM, whatever it costs, and (b) beyond that, slices of at least four

@@ -65,6 +65,10 @@ cudaError_t launch_gemv_one(int codec, int x_dtype, const GemvArgs& a, cudaStrea
 // 1 to 16 dense rows of fp16 / bf16 on mma.sync over the integers themselves (kq_rows.cu).
 bool gemv_rows_supported(int codec, int x_dtype, const GemvArgs& a);
 cudaError_t launch_gemv_rows(int codec, int x_dtype, const GemvArgs& a, cudaStream_t st);
+// 2 to 16 dense rows of the same types on larger matrices (kq_few.cu); cudaErrorNotSupported, with nothing launched, where
+// the activations do not fit into shared memory.
+bool gemv_few_supported(int codec, int x_dtype, const GemvArgs& a);
+cudaError_t launch_gemv_few(int codec, int x_dtype, const GemvArgs& a, cudaStream_t st);
 
 // gather_qmm with one row per entry on the same kernel, up to 1024 entries.
 bool gather_rows_supported(int codec, int x_dtype, const void* x, int M, int K, const uint8_t* w, long long expert_stride,
