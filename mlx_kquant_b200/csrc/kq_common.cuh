@@ -452,10 +452,18 @@ __device__ __forceinline__ IqTables stage_iq_tables(uint8_t* smem, int tid, int 
 template <int TH>
 __device__ __forceinline__ int collect_entries(const uint32_t* __restrict__ rhs, const uint32_t* __restrict__ lhs, int n,
                                                long long x_batch, uint32_t e, int2* list, int* count, int unordered) {
-  for (int i = threadIdx.x; i < n; i += TH) {
-    if (rhs[i] != e) continue;
-    const uint32_t l = lhs[i];
-    if ((long long)l < x_batch) list[atomicAdd(count, 1)] = make_int2((int)l, i);
+  // both indices of up to four entries a thread in flight at once: one latency, not one for each
+  for (int i = threadIdx.x; i < n; i += 4 * TH) {
+    uint32_t r[4], l[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int at = i + q * TH;
+      r[q] = at < n ? rhs[at] : ~e;
+      l[q] = at < n ? lhs[at] : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if (r[q] == e && (long long)l[q] < x_batch) list[atomicAdd(count, 1)] = make_int2((int)l[q], i + q * TH);
   }
   __syncthreads();
   const int c = *count;

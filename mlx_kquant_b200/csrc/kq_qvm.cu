@@ -129,39 +129,72 @@ qvm_kernel(const XT* __restrict__ x, long long x_row_stride, void* __restrict__ 
 // The gather form for calls whose entries share matrices (absorbed attention: every sequence multiplies by the head's
 // matrix): a CTA owns one matrix and 128 output columns, collects the matrix's entries from the index arrays by itself
 // and multiplies up to eight of them per pass over the weights, so a weight is decoded once for eight rows where the
-// kernel above decodes it for each. A warp's halves take two rows of W at a time, a lane eight columns; the partial
-// sums meet by one shuffle and in shared memory. Bound by the decode arithmetic and the latency of its byte loads;
-// 64 heads [128, 512] q6_k, eight rows each: 39.6 -> 9.7 us a launch.
+// kernel above decodes it for each. Up to 256 rows of the weights are copied to shared memory as the aligned windows
+// around their bytes while the entries are looked for and the activations come (decoded from global memory, they were
+// waited for once more each four rows, and one byte at a time where a row is no whole sixteens). A warp's halves take two
+// rows of W at a time, a lane eight columns; the partial sums meet by one shuffle and in shared memory. Bound by the
+// decode arithmetic (a third of the issue slots) and the chain index - activation - product; 64 heads [128, 512] q6_k,
+// eight rows each: 9.1 -> 7.05 us a launch (the kernel above 39.6), q8_0 7.9 -> 6.5, 8 heads [512, 2048] q6_k 20.7 -> 18.4.
 constexpr int kRowCols = 128, kRowM = 8;
 constexpr int kRowEntries = 512;  // every CTA looks through all entries
+constexpr int kRowChunk = 256;    // rows of W in shared memory at once
+constexpr int kRowXPitch = 12;    // floats of a row of x in shared memory, by columns: stores of 32 k in eight banks
+// bytes of a row's blocks in shared memory: 128 columns' and the aligned window around them
+__host__ __device__ constexpr int row_pitch(int c) { return (std::max(1, kRowCols / wpb_of(c)) * bpb_of(c) + 30) / 16 * 16; }
+constexpr int kRowFixed = kRowChunk * kRowXPitch * 4 + kWarps * kRowM * kRowCols * 4 + kRowEntries * 8;
 template <int C, int A, typename XT>
 __global__ void __launch_bounds__(kThreads, 2)
 qvm_rows_kernel(const XT* __restrict__ x, void* __restrict__ y, const uint8_t* __restrict__ w, long long row_bytes,
                 int N, int K, QvmGather gq, int n_entries) {
   using OT = typename std::conditional<std::is_same<XT, __half>::value, __half, __nv_bfloat16>::type;
-  constexpr int BPB = bpb_of(C), kChunk = 256;
+  constexpr int BPB = bpb_of(C), kPitch = row_pitch(C);
   constexpr bool kIq = (C == IQ4_NL || C == IQ4_XS || C == IQ2_XXS);
-  __shared__ __align__(16) float xs[kChunk][kRowM];          // activations of a K chunk
-  __shared__ float red[kWarps][kRowM][kRowCols];
+  extern __shared__ __align__(16) uint8_t qr_dyn[];
+  float (*xs)[kRowXPitch] = reinterpret_cast<float (*)[kRowXPitch]>(qr_dyn);  // activations of a K chunk
+  float (*red)[kRowM][kRowCols] = reinterpret_cast<float (*)[kRowM][kRowCols]>(qr_dyn + kRowChunk * kRowXPitch * 4);
+  int2* list = reinterpret_cast<int2*>(qr_dyn + kRowFixed - kRowEntries * 8);  // (row of x, row of y)
+  uint8_t* ws = qr_dyn + kRowFixed;
   __shared__ __align__(16) uint8_t s_tabs[kIq ? kIqSmemBytes : 16];
-  __shared__ int2 list[kRowEntries];                         // (row of x, row of y)
   __shared__ int count_s;
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   IqTables tabs = global_iq_tables();
   if constexpr (kIq) tabs = stage_iq_tables(s_tabs, threadIdx.x, kThreads);
   if (threadIdx.x == 0) count_s = 0;
   __syncthreads();
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
   const uint32_t e = blockIdx.y;
-  const int count = collect_entries<kThreads>(gq.rhs, gq.lhs, n_entries, gq.x_batch, e, list, &count_s, gridDim.z > 1 ? 0 : n_entries);
-  if (count == 0) return;
   w += (long long)e * gq.expert_stride;
+  const int first = (int)block_of<C>(blockIdx.x * kRowCols);  // block of the CTA's first column
+  const int len = min(std::max(1, kRowCols / wpb_of(C)), N / wpb_of(C) - first) * BPB;
+  const uint8_t* wcols = w + (long long)first * BPB;
+  const uint32_t place = (uint32_t)reinterpret_cast<uintptr_t>(wcols);
+  auto stage = [&](int kb, int kn) {
+    const uint8_t* wend = w + (long long)K * row_bytes;
+    constexpr int P = kPitch / 16;
+    for (int i = threadIdx.x; i < kn * P; i += kThreads) {
+      const int r = i / P, c = i - r * P;
+      const uint8_t* p = wcols + (long long)(kb + r) * row_bytes;
+      const int ph = (int)(reinterpret_cast<uintptr_t>(p) & 15);
+      const uint8_t* q = p - ph + 16 * c;
+      const long long left = wend - q;
+      const int bytes = left < 16 ? (int)left : 16;
+      if (16 * c < len + ph)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(ws + 16 * i)), "l"(q), "r"(bytes) : "memory");
+    }
+  };
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  stage(0, min(kRowChunk, K));  // on their way while the entries are looked for
+  const int count = collect_entries<kThreads>(gq.rhs, gq.lhs, n_entries, gq.x_batch, e, list, &count_s, gridDim.z > 1 ? 0 : n_entries);
+  if (count == 0) {
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    return;
+  }
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4, oc = lane & 15;
   const int c0 = blockIdx.x * kRowCols + 8 * oc;
   const bool live = c0 < N;  // N is a whole number of blocks: eight columns exist or none
-  const long long blk_off = live ? block_of<C>(c0) * BPB : 0;
+  const int blk_off = live ? ((int)block_of<C>(c0) - first) * BPB : 0;
   const int oct = octet_of<C>(live ? c0 : 0);
+  int staged = 0;  // the chunk in shared memory
   for (int e0 = kRowM * blockIdx.z; e0 < count; e0 += kRowM * gridDim.z) {  // grid.z CTAs share the entries
     const int m = min(kRowM, count - e0);
     float acc[kRowM][8];
@@ -169,18 +202,22 @@ qvm_rows_kernel(const XT* __restrict__ x, void* __restrict__ y, const uint8_t* _
     for (int t = 0; t < kRowM; t++)
 #pragma unroll
       for (int i = 0; i < 8; i++) acc[t][i] = 0.f;
-    for (int kb = 0; kb < K; kb += kChunk) {
-      const int kn = min(kChunk, K - kb);
+    for (int kb = 0; kb < K; kb += kRowChunk) {
+      const int kn = min(kRowChunk, K - kb);
       __syncthreads();  // the chunk before (and the sums of the pass before) have been read
-      for (int i = threadIdx.x; i < kn * kRowM; i += kThreads) {
-        const int t = i / kn, k = i % kn;
-        xs[k][t] = t < m ? load_x<XT>(x + (long long)list[e0 + t].x * K + kb + k) : 0.f;
-      }
+      if (kb != staged) stage(kb, kn);
+      staged = kb;
+      static_assert(kRowM == kWarps, "a row of x to a warp");
+      const XT* xr = x + (long long)list[e0 + min(warp, m - 1)].x * K + kb;
+#pragma unroll 4
+      for (int k = lane; k < kn; k += 32) xs[k][warp] = warp < m ? load_x<XT>(xr + k) : 0.f;
+      asm volatile("cp.async.wait_all;\n" ::: "memory");
       __syncthreads();
 #pragma unroll 4
       for (int k = 2 * warp + half; k < kn; k += 2 * kWarps) {
         float v[8];
-        decode8<C, A>(w + (long long)(kb + k) * row_bytes + blk_off, oct, v, tabs);
+        const int ph = (place + (uint32_t)(kb + k) * (uint32_t)row_bytes) & 15;
+        decode8<C, A>(ws + k * kPitch + ph + blk_off, oct, v, tabs);
         const float4 x0 = *reinterpret_cast<const float4*>(&xs[k][0]), x1 = *reinterpret_cast<const float4*>(&xs[k][4]);
         const float xv[kRowM] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
 #pragma unroll
@@ -222,7 +259,7 @@ int row_share(int N, int n_experts, long long entries) {
 // ways. Both take time by the rows of K a CTA walks (a third of it there, of 128 columns and eight entries; of 256
 // columns and one entry here) and by the CTAs beyond those that reside at once. Within 1-2 % of the faster one on average
 // over 780 calls of q4_k, q6_k, iq4_xs and q8_0, 1 to 128 matrices and 1 to 128 entries each. 64 heads [128, 512] q6_k,
-// one entry each 11.9 -> 8.2 us, eight 39.6 -> 9.2; but one matrix [4096, 4096] with one entry 34 us above, 90 here, and
+// one entry each 11.9 -> 6.3 us, eight 39.6 -> 7.1; but one matrix [4096, 4096] with one entry 34 us above, 90 here, and
 // eight [2048, 1024] with one each 24 and 57.
 bool rows_pay(int N, int K, int S, int n_experts, long long entries) {
   const double share = row_share(N, n_experts, entries);
@@ -244,6 +281,17 @@ cudaError_t launch_rows(const void* x, void* y, const uint8_t* w, long long row_
   const int share = row_share(N, gq.n_experts, n_entries);
   cfg.gridDim = dim3((N + kRowCols - 1) / kRowCols, gq.n_experts, share);
   cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kRowFixed + std::min(kRowChunk, K) * row_pitch(C);
+  static bool attr_set[16] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 16) return cudaErrorInvalidDevice;
+  if (!attr_set[dev]) {
+    const cudaError_t err = cudaFuncSetAttribute(qvm_rows_kernel<C, A, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 kRowFixed + kRowChunk * row_pitch(C));
+    if (err != cudaSuccess) return err;
+    attr_set[dev] = true;
+  }
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -285,7 +333,8 @@ template <int C, int NAT>
 cudaError_t launch_codec(int x_dtype, const void* x, long long x_row_stride, void* y, long long y_row_stride,
                          const uint8_t* w, long long row_bytes, int M, int N, int K, cudaStream_t st,
                          QvmGather gq = QvmGather{}, long long entries = 1) {
-  const bool aligned = (reinterpret_cast<uintptr_t>(w) & 15) == 0 && (row_bytes & 15) == 0 && (gq.expert_stride & 15) == 0;
+  // what decode8 loads at once, of every block
+  const bool aligned = ((reinterpret_cast<uintptr_t>(w) | row_bytes | gq.expert_stride) & (NAT - 1)) == 0;
 #define KQ_QVM(XT)                                                                                                    \
   return aligned ? launch_one<C, NAT, XT>(x, x_row_stride, y, y_row_stride, w, row_bytes, M, N, K, st, gq, entries)  \
                  : launch_one<C, 1, XT>(x, x_row_stride, y, y_row_stride, w, row_bytes, M, N, K, st, gq, entries)

@@ -65,6 +65,7 @@ struct RowsGather {
   int n_entries, n_experts, by_entry;
   long long x_batch, expert_stride;
   int units, deep;
+  int early;  // the weights of a CTA's first stages are fetched while it looks for its entries
 };
 
 struct RowsPlan {
@@ -146,6 +147,49 @@ rows_kernel(const GemvArgs a, const RowsPlan pl, const RowsGather ga, int* __res
   __shared__ int2 walk_s;  // first pass over the matrix's entries and step (kept here, and count_s, to spare registers)
   const uint8_t* wmat = a.w;
   int2* list = reinterpret_cast<int2*>(rw_dyn + pl.list_off);  // (row of x, row of y)
+  auto row_block = [&](int pass) { return ((int)blockIdx.x + (G ? 0 : pass * (int)gridDim.x)) * pl.R; };
+  // A row's pieces of sixteen bytes go to neighbouring threads (a power of two of them, 1 << wlog: pl.wlog, pl.xlog),
+  // every thread walks down the rows: two additions a piece (numbering the pieces of a stage and
+  // stepping by the thread count instead: q6_k [4096, 14336] x 8 32 us against 24).
+  const int tid = (warp - NW - kRwHelpers) * 32 + lane;  // of the producers
+  constexpr int kThreads = 32 * kRwProducers;
+  int pass_w = 0, st_w = 0, slot_w = 0;
+  auto copy_w = [&]() {
+    const int row0 = row_block(pass_w), rows = min(pl.R, a.N - row0), len = min(pl.cs, nsb - st_w * pl.cs) * BPB;
+    const int step = kThreads >> pl.wlog, r0 = tid >> pl.wlog;
+    const uint8_t* wend = wmat + (long long)a.N * a.row_bytes;
+    const uint8_t* src = wmat + (long long)row0 * a.row_bytes + (long long)st_w * pl.cs * BPB;
+    const uint32_t dst = smem_u32(rw_dyn + slot_w * pl.stage_bytes);
+    const long long sstep = step * a.row_bytes;
+    const int dstep = step * pl.wpitch;
+    if (rw_al16(C) || (a.row_bytes & 15) == 0) {
+      // every row has the same place within sixteen bytes, and the matrix ends on a whole sixteen
+      const int ph = rw_al16(C) ? 0 : (int)(reinterpret_cast<uintptr_t>(src) & 15);
+      const int per_row = (len + ph + 15) >> 4;
+      for (int c = tid & ((1 << pl.wlog) - 1); c < per_row; c += 1 << pl.wlog) {
+        const uint8_t* p = src - ph + 16 * c + r0 * a.row_bytes;
+        uint32_t d = dst + 16 * c + r0 * pl.wpitch;
+#pragma unroll 4
+        for (int r = r0; r < rows; r += step, p += sstep, d += dstep) rw_cp16(d, p);
+      }
+    } else {  // the aligned window around the row's bytes; the matrix may end inside it
+      const int per_row = (len + 30) >> 4;  // a window holds at most that many
+      for (int c = tid & ((1 << pl.wlog) - 1); c < per_row; c += 1 << pl.wlog) {
+        const uint8_t* p = src + r0 * a.row_bytes;
+        uint32_t d = dst + 16 * c + r0 * pl.wpitch;
+#pragma unroll 4
+        for (int r = r0; r < rows; r += step, p += sstep, d += dstep) {
+          const int ph = (int)(reinterpret_cast<uintptr_t>(p) & 15);
+          const uint8_t* q = p - ph + 16 * c;
+          const long long left = wend - q;
+          if (16 * c < len + ph) rw_cp16_upto(d, q, left < 16 ? (int)left : 16);
+        }
+      }
+    }
+    if (++st_w == nst) st_w = 0, pass_w++;
+    if (++slot_w == S) slot_w = 0;
+  };
+  int early = 0;  // stages whose weights are on their way already
   if constexpr (G) {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the routing may come from the kernel before this one
     constexpr int TH = RowsShape<G>::kThreads;
@@ -164,19 +208,29 @@ rows_kernel(const GemvArgs a, const RowsPlan pl, const RowsGather ga, int* __res
       e = ga.by_entry ? ga.rhs[blockIdx.y] : blockIdx.y;
     }
     if (e >= (uint32_t)ga.n_experts) return;
+    wmat += (long long)e * ga.expert_stride;
+    if (ga.early && !left_over) {
+      early = min(S, nst);
+      if (warp >= NW + kRwHelpers)
+        for (int i = 0; i < early; i++) copy_w();
+    }
     if (threadIdx.x == 0) walk_s = make_int2(pass0, pass_step);
     const bool shared = ga.by_entry || share > 1 || left_over;
     const int total_m = collect_entries<TH>(ga.rhs, ga.lhs, ga.n_entries, ga.x_batch, e, list, &count_s,
                                             shared ? 0 : (more ? 8 * NT * base : ga.n_entries));
-    if (total_m == 0 || (ga.by_entry && !left_over && list[0].y != (int)blockIdx.y)) return;
-    wmat += (long long)e * ga.expert_stride;
+    if (total_m == 0 || (ga.by_entry && !left_over && list[0].y != (int)blockIdx.y)) {
+      asm volatile("cp.async.wait_all;\n" ::: "memory");
+      return;
+    }
     passes = ((total_m + 8 * NT - 1) / (8 * NT) - pass0 + pass_step - 1) / pass_step;
     if (more) passes = min(passes, ga.deep);
-    if (passes <= 0) return;
+    if (passes <= 0) {
+      asm volatile("cp.async.wait_all;\n" ::: "memory");
+      return;
+    }
   } else {
     passes = (pl.n_blocks - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;
   }
-  auto row_block = [&](int pass) { return ((int)blockIdx.x + (G ? 0 : pass * (int)gridDim.x)) * pl.R; };
   auto entry0 = [&](int pass) { return 8 * NT * (walk_s.x + pass * walk_s.y); };  // of the pass (gather)
   auto rows_of_x = [&](int pass) { return G ? min(8 * NT, count_s - entry0(pass)) : a.M; };
   volatile int* abort_flag = &abort_s;
@@ -184,49 +238,8 @@ rows_kernel(const GemvArgs a, const RowsPlan pl, const RowsGather ga, int* __res
 
   if (warp >= NW + kRwHelpers) {
     // ================= producers =================
-    const int pw = warp - NW - kRwHelpers;
     const int total = passes * nst;
-    const uint8_t* wend = wmat + (long long)a.N * a.row_bytes;
-    int pass_w = 0, st_w = 0, slot_w = 0, pass_x = 0, st_x = 0, slot_x = 0;
-    // A row's pieces of sixteen bytes go to neighbouring threads (a power of two of them, 1 << wlog: pl.wlog, pl.xlog),
-    // every thread walks down the rows: two additions a piece (numbering the pieces of a stage and
-    // stepping by the thread count instead: q6_k [4096, 14336] x 8 32 us against 24).
-    const int tid = pw * 32 + lane;
-    constexpr int kThreads = 32 * kRwProducers;
-    auto copy_w = [&]() {
-      const int row0 = row_block(pass_w), rows = min(pl.R, a.N - row0), len = min(pl.cs, nsb - st_w * pl.cs) * BPB;
-      const int step = kThreads >> pl.wlog, r0 = tid >> pl.wlog;
-      const uint8_t* src = wmat + (long long)row0 * a.row_bytes + (long long)st_w * pl.cs * BPB;
-      const uint32_t dst = smem_u32(rw_dyn + slot_w * pl.stage_bytes);
-      const long long sstep = step * a.row_bytes;
-      const int dstep = step * pl.wpitch;
-      if (rw_al16(C) || (a.row_bytes & 15) == 0) {
-        // every row has the same place within sixteen bytes, and the matrix ends on a whole sixteen
-        const int ph = rw_al16(C) ? 0 : (int)(reinterpret_cast<uintptr_t>(src) & 15);
-        const int per_row = (len + ph + 15) >> 4;
-        for (int c = tid & ((1 << pl.wlog) - 1); c < per_row; c += 1 << pl.wlog) {
-          const uint8_t* p = src - ph + 16 * c + r0 * a.row_bytes;
-          uint32_t d = dst + 16 * c + r0 * pl.wpitch;
-#pragma unroll 4
-          for (int r = r0; r < rows; r += step, p += sstep, d += dstep) rw_cp16(d, p);
-        }
-      } else {  // the aligned window around the row's bytes; the matrix may end inside it
-        const int per_row = (len + 30) >> 4;  // a window holds at most that many
-        for (int c = tid & ((1 << pl.wlog) - 1); c < per_row; c += 1 << pl.wlog) {
-          const uint8_t* p = src + r0 * a.row_bytes;
-          uint32_t d = dst + 16 * c + r0 * pl.wpitch;
-#pragma unroll 4
-          for (int r = r0; r < rows; r += step, p += sstep, d += dstep) {
-            const int ph = (int)(reinterpret_cast<uintptr_t>(p) & 15);
-            const uint8_t* q = p - ph + 16 * c;
-            const long long left = wend - q;
-            if (16 * c < len + ph) rw_cp16_upto(d, q, left < 16 ? (int)left : 16);
-          }
-        }
-      }
-      if (++st_w == nst) st_w = 0, pass_w++;
-      if (++slot_w == S) slot_w = 0;
-    };
+    int pass_x = 0, st_x = 0, slot_x = 0;
     auto copy_x = [&]() {  // and the arrival of this thread once all its copies of the stage have landed
       const int per_row = min(pl.cs, nsb - st_x * pl.cs) * 32, m = rows_of_x(pass_x);
       const int step = kThreads >> pl.xlog, r0 = tid >> pl.xlog;
@@ -246,7 +259,7 @@ rows_kernel(const GemvArgs a, const RowsPlan pl, const RowsGather ga, int* __res
     const int first = min(S, total);
     // x and, for all that is known here, the weights may come from the kernel before this one
     if constexpr (!G) asm volatile("griddepcontrol.wait;\n" ::: "memory");
-    for (int i = 0; i < first; i++) copy_w();
+    for (int i = early; i < first; i++) copy_w();
     for (int i = 0; i < first; i++) copy_x();
     int parity = 0;
     for (int i = first; i < total; i++) {
@@ -462,6 +475,9 @@ cudaError_t launch_rows_nt(const GemvArgs& a, const RowsGather& ga, cudaStream_t
   // 85 -> 72; q4_k [512, 512] 1024 entries 83 -> 35, evenly 20.3 -> 20.4.
   RowsGather gl = ga;
   gl.units = units;
+  // 64 matrices [128, 512] of q6_k, eight entries each 7.6 -> 7.2 us, q4_k 5.9 -> 5.4 (with fewer entries a matrix some have
+  // none, whose weights would be fetched for nothing)
+  gl.early = !ga.by_entry && ga.n_entries >= 4 * ga.n_experts ? 1 : 0;
   gl.deep = a.K >= 1536 ? 1 : 2;
   int more = 0;
   if (G && 4ll * ga.n_experts <= p.red_off) more = std::max(0, (ga.n_entries - 1) / (8 * NT * gl.deep) - share + 1);
