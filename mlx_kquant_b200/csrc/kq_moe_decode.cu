@@ -17,6 +17,7 @@
 // are in memory then; after the wait the indices are read again and a CTA whose expert changed copies again
 // (its first copy has landed by then). The activations are only read after the wait.
 // Arithmetic and shared-memory layout of the products: kq_imma_q4k.cuh / kq_gemv_stream.cu.
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -28,6 +29,7 @@
 #include "kq_common.cuh"
 #include "kq_imma_q4k.cuh"
 #include "kq_launch.h"
+#include "kq_rows_unit.cuh"
 
 namespace kq {
 
@@ -92,7 +94,6 @@ struct GluArgs {
   void* y;                  // [T * R, F]
   int act;
   float limit;
-  int tiles_per_cta;        // grouped kernel only: consecutive 16-feature tiles a CTA walks
 };
 
 // shared memory: gate tile | up tile (4 groups each) | planes 2 K | XS K / 32 | SX K / 256 (padded) | red 8 x 32 | mbar
@@ -309,231 +310,240 @@ __global__ void __launch_bounds__(kMdThreads, 2) moe_mix_kernel(const MixArgs a,
 
 // ---------------------------------------------------------------------------------- grouped by expert
 // From a few dozen routed entries on, entries that share an expert share its weight stream: the entries are
-// grouped by expert on the device (kq_gather.cu) and cut into tasks of at most kTaskEntries entries. A CTA brings
-// its rows of the task's expert into shared memory once and multiplies them by the task's activation rows four
-// at a time (the B operand has room for four rows' byte planes).
-constexpr int kTaskEntries = 16;
-struct Task4 {
+// grouped by expert on the device (kq_gather.cu) and cut into tasks of 8 NT entries. The products are those of the dense
+// kernel for few rows (kq_few.cu): integers as matrix operands, sixteen warps with a ring of TMA boxes each.
+// All tasks' 16-row tiles stand in one row, CTA c of one per SM takes an even part of it, and within a task the units
+// (tile, superblock) are shared evenly by the warps. Tiles that a warp has whole leave from its registers, the others meet
+// in shared memory. The gate and the up rows of the same features are a unit together, so that the activation function is
+// applied to float32 sums. Boxes of the next task are on their way while a task's activations are staged.
+// Measured on B200, 512 entries of 128 experts, K 2048, F 768 (226 MB and 113 MB of weights): gate | up 109 -> 74 us, down
+// 51 -> 43 (before: tasks of sixteen entries, four at a time as byte planes in int8 operands, a CTA for 64 features, whose
+// ten microseconds of serial latencies two CTAs an SM did not hide).
+template <int NT>
+struct Tasks {
   int expert, m;
-  int ent[kTaskEntries];   // entry indices; slots past m repeat the last one
+  int ent[8 * NT];   // entry indices; slots past m repeat the last one
 };
 
-__global__ void moe_tasks4_kernel(const int* __restrict__ offsets, const int* __restrict__ task_base,
-                                  const int* __restrict__ order, Task4* tasks) {
+template <int NT>
+__global__ void moe_tasks_kernel(const int* __restrict__ offsets, const int* __restrict__ task_base,
+                                 const int* __restrict__ order, Tasks<NT>* tasks) {
+  constexpr int kN = 8 * NT;
   const int e = blockIdx.x;
   const int o0 = offsets[e], c = offsets[e + 1] - o0;
-  const int nt = (c + kTaskEntries - 1) / kTaskEntries, tb = task_base[e];
+  const int nt = (c + kN - 1) / kN, tb = task_base[e];
   for (int k = threadIdx.x; k < nt; k += blockDim.x) {
-    Task4 t;
+    Tasks<NT> t;
     t.expert = e;
-    t.m = min(kTaskEntries, c - kTaskEntries * k);
+    t.m = min(kN, c - kN * k);
 #pragma unroll
-    for (int j = 0; j < kTaskEntries; j++) t.ent[j] = order[o0 + kTaskEntries * k + min(j, t.m - 1)];
+    for (int j = 0; j < kN; j++) t.ent[j] = order[o0 + kN * k + min(j, t.m - 1)];
     tasks[tb + k] = t;
   }
 }
 
-__device__ __forceinline__ float md_pick4(const float (&v)[4], int t) {
-  return t == 0 ? v[0] : (t == 1 ? v[1] : (t == 2 ? v[2] : v[3]));
-}
-
-// shared memory: gate tile | up tile | planes 4 x 2 K | XS 4 x K / 32 | SX 4 x padded K / 256 | red 8 x 32 x 4 | mbar
-// Feature tiles per CTA of the grouped gate | up kernel: a CTA keeps its task's quantized activations and walks
-// kGluTiles consecutive 16-feature tiles through a two-deep ring of weight buffers, the copy of tile i + 2 issued
-// as soon as tile i has been used. (One tile per CTA left the CTA's ~10 us of serial latencies - task load, copy
-// issue, activation fetch and quantization, first weight bytes, reduction - in front of every 36 KB of weights.)
-constexpr int kGluTiles = 4;
-inline int glu4_smem_bytes(int K, int row_bytes) {
-  return 16 * md_group_stride(row_bytes) + 8 * K + (K / 32) * 16 + (((K / 256) + 3) & ~3) * 16 + kMdWarps * 32 * 16 + 32;
-}
-
-template <typename XT>
-__global__ void __launch_bounds__(kMdThreads, 2)
-moe_glu_tasks_kernel(const GluArgs a, const Task4* __restrict__ tasks, const int* __restrict__ n_tasks,
-                     int* __restrict__ error_word) {
-  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
-  if ((int)blockIdx.y >= *n_tasks) return;
-  extern __shared__ __align__(128) uint8_t md_dyn[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const int K = a.K, nchunks = K >> 8, ncp = (nchunks + 3) & ~3, RB = a.row_bytes;
-  const int gb = 4 * RB, GS = gb + ((32 - (gb & 127)) & 127);
-  uint8_t* wbuf = md_dyn;                       // two buffers of (gate tile | up tile), 4 groups each
-  uint8_t* planes = wbuf + 16 * GS;
-  float* XS = reinterpret_cast<float*>(planes + 8 * K);
-  float* SX = XS + 4 * (K / 32);
-  float* red = SX + 4 * ncp;
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(red + kMdWarps * 32 * 4);   // [2]
-  const Task4 tk = tasks[blockIdx.y];
-  const int all_tiles = (a.F + 15) >> 4;
-  const int tile0 = blockIdx.x * a.tiles_per_cta, ntile = min(a.tiles_per_cta, all_tiles - tile0);
-  const int npass = (tk.m + 3) >> 2, total = npass * ntile;   // weight copies: tiles of a pass, pass after pass
-  // Warp 0 issues a tile's eight bulk copies (four-row groups of the gate and of the up rows), one per lane: a
-  // single thread issuing all eight kept the other warps waiting at the tile's barrier for its issue time.
-  auto issue = [&](int seq) {
-    const int f0 = (tile0 + seq % ntile) * 16, rows = min(16, a.F - f0);
-    uint8_t* wb = wbuf + (seq & 1) * 8 * GS;
-    if (lane == 0) st_mbar_expect_tx(&mbar[seq & 1], (uint32_t)(2 * rows * RB));
-    __syncwarp();
-    if (lane < 8) {
-      const int grp = lane & 3, r = 4 * grp;
-      if (r < rows) {
-        const uint8_t* src = (lane < 4 ? a.wg + (long long)tk.expert * a.stride_g : a.wu + (long long)tk.expert * a.stride_u) +
-                             (long long)(f0 + r) * RB;
-        st_bulk_g2s(wb + (lane < 4 ? 0 : 4 * GS) + grp * GS, src, (uint32_t)(min(4, rows - r) * RB), &mbar[seq & 1]);
-      }
-    }
-  };
-  if (warp == 0) {
-    if (lane == 0) {
-      st_mbar_init(&mbar[0], 1);
-      st_mbar_init(&mbar[1], 1);
-      asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    }
-    __syncwarp();
-    issue(0);
-    if (total > 1) issue(1);
-  }
-  const uint8_t* bcol = planes + min(g >> 1, 3) * 2 * K + (g & 1) * K + 8 * t;
-  const int rA = 4 * (g & 3) + (g >> 2);
-  const int rrow[4] = {rA, rA + 2, 16 + rA, 16 + rA + 2};
-  int seq = 0;
-  for (int m0 = 0; m0 < tk.m; m0 += 4) {   // four activation rows per pass over the CTA's tiles
-    for (int sb = warp; sb < nchunks; sb += kMdWarps) {
-      uint4 raw[4];   // the four loads in flight together
-#pragma unroll
-      for (int m = 0; m < 4; m++) {
-        const XT* x = static_cast<const XT*>(a.x) + (long long)(tk.ent[min(m0 + m, kTaskEntries - 1)] / a.R) * K;
-        raw[m] = st_ld_cg16(x + sb * 256 + lane * 8);
-      }
-#pragma unroll
-      for (int m = 0; m < 4; m++)
-        st_quantize<XT>(raw[m], sb, lane, K, planes + m * 2 * K, XS + m * (K / 32), SX + m * ncp);
-    }
-    __syncthreads();  // first pass: the barriers are initialised
-    for (int ti = 0; ti < ntile; ti++, seq++) {
-      const int f0 = (tile0 + ti) * 16, rows = min(16, a.F - f0);
-      const uint8_t* wb = wbuf + (seq & 1) * 8 * GS;
-      if (!md_wait(&mbar[seq & 1], (uint32_t)((seq >> 1) & 1), error_word)) return;
-      const int lrA = min(rA, rows - 1), lrB = min(rA + 2, rows - 1);
-      const uint8_t* base[4] = {wb + (lrA >> 2) * GS + (lrA & 3) * RB, wb + (lrB >> 2) * GS + (lrB & 3) * RB,
-                                wb + (4 + (lrA >> 2)) * GS + (lrA & 3) * RB, wb + (4 + (lrB >> 2)) * GS + (lrB & 3) * RB};
-      float ydot[4] = {0.f, 0.f, 0.f, 0.f}, ymin[4][4] = {};
-      for (int sb = warp; sb < nchunks; sb += kMdWarps) {
-        const uint8_t* const blk[4] = {base[0] + sb * 144, base[1] + sb * 144, base[2] + sb * 144, base[3] + sb * 144};
-        st_unit_mx<2, 4>(blk, bcol + sb * 256, XS + sb * 8, K / 32, SX + sb, ncp, t, ydot, ymin);
-      }
-#pragma unroll
-      for (int r = 0; r < 4; r++) {
-#pragma unroll
-        for (int m = 0; m < 4; m++) {
-          ymin[r][m] += __shfl_xor_sync(0xffffffffu, ymin[r][m], 1);
-          ymin[r][m] += __shfl_xor_sync(0xffffffffu, ymin[r][m], 2);
-        }
-        red[(warp * 32 + rrow[r]) * 4 + t] = ydot[r] - md_pick4(ymin[r], t);   // activation row m0 + t of this lane
-      }
-      __syncthreads();   // every warp has read this tile's weights and left its partial sums
-      if (warp == 0 && seq + 2 < total) issue(seq + 2);   // the buffer is free: the copy after next goes in
-      if (threadIdx.x < 64) {
-        const int r = threadIdx.x & 15, m = threadIdx.x >> 4;
-        if (r < rows && m0 + m < tk.m) {
-          float gs = 0.f, us = 0.f;
-#pragma unroll
-          for (int w = 0; w < kMdWarps; w++) {
-            gs += red[(w * 32 + r) * 4 + m];
-            us += red[(w * 32 + 16 + r) * 4 + m];
-          }
-          md_store(static_cast<XT*>(a.y) + (long long)tk.ent[m0 + m] * a.F + f0 + r, md_act(gs, us, a.act, a.limit));
-        }
-      }
-      __syncthreads();   // red (and, after the last tile, the planes) are free again
-    }
-  }
-}
-
-struct RowsArgs {
-  const void* x;            // [entries, K]: row of entry b = x + b * K
-  const uint8_t* w;
-  long long stride_w;
-  int row_bytes, K, N;
-  void* y;                  // [entries, N]
+struct TaskArgs {
+  const void* x;            // entry b's row is b / R
+  int K, F, R;              // F: rows of a matrix (of gate and of up each)
+  const uint8_t *wg, *wu;   // wu: nullptr in the form of one matrix
+  long long stride_g, stride_u;
+  int row_bytes;
+  void* y;                  // [entries, F]
+  int act;
+  float limit;
+  int D;                    // slots of a warp
+  int x_pitch, x_off, sum_off, red_off;
 };
 
-// 128 rows per CTA, one 16-row tile per warp (for short rows: few superblocks, nothing to split over the warps)
-// shared memory: 32 groups | planes 4 x 2 K | XS 4 x K / 32 | SX 4 x padded K / 256 | mbar
-inline int rows4_smem_bytes(int K, int row_bytes) {
-  return 32 * md_group_stride(row_bytes) + 8 * K + (K / 32) * 16 + (((K / 256) + 3) & ~3) * 16 + 16;
+constexpr int kTkWarps = 16, kTkThreads = 32 * kTkWarps, kTkMaxSlots = 4, kTkSlot = 16 * 144;
+constexpr int kTkSmem = 226 * 1024 - 512;
+
+__device__ __forceinline__ void tk_load(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+      : "memory");
 }
 
-template <typename XT>
-__global__ void __launch_bounds__(kMdThreads, 3)
-moe_rows_tasks_kernel(const RowsArgs a, const Task4* __restrict__ tasks, const int* __restrict__ n_tasks,
-                      int* __restrict__ error_word) {
+template <typename XT, int NT, bool GLU>
+__global__ void __launch_bounds__(kTkThreads, 1)
+moe_tasks_product_kernel(const TaskArgs a, const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_u,
+                         const Tasks<NT>* __restrict__ tasks, const int* __restrict__ n_tasks, int* __restrict__ error_word) {
+  constexpr int H = GLU ? 2 : 1;                       // matrices
+  constexpr int kRedPitch = 8 * NT + (NT == 1 ? 2 : 0);
+  constexpr int kSumWords = NT * 8 * rw_sum_pitch(Q4_K);
+  extern __shared__ __align__(128) uint8_t tk_dyn[];
+  __shared__ uint64_t full[kTkWarps][kTkMaxSlots];
+  __shared__ int abort_s, ent_s[8 * NT];
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
-  if ((int)blockIdx.y >= *n_tasks) return;
-  extern __shared__ __align__(128) uint8_t md_dyn[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const int K = a.K, nchunks = K >> 8, ncp = (nchunks + 3) & ~3, RB = a.row_bytes;
-  const int gb = 4 * RB, GS = gb + ((32 - (gb & 127)) & 127);
-  uint8_t* wbuf = md_dyn;
-  uint8_t* planes = wbuf + 32 * GS;
-  float* XS = reinterpret_cast<float*>(planes + 8 * K);
-  float* SX = XS + 4 * (K / 32);
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(SX + 4 * ncp);
-  const Task4 tk = tasks[blockIdx.y];
-  const int n0 = blockIdx.x * 128, rows = min(128, a.N - n0);
-  if (warp == 0) {
-    if (lane == 0) {
-      st_mbar_init(mbar, 1);
-      asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-      st_mbar_expect_tx(mbar, (uint32_t)(rows * RB));
-    }
-    __syncwarp();
-    const int r = 4 * lane;   // one group of four rows per lane
-    if (r < rows)
-      st_bulk_g2s(wbuf + lane * GS, a.w + (long long)tk.expert * a.stride_w + (long long)(n0 + r) * RB,
-                  (uint32_t)(min(4, rows - r) * RB), mbar);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int nsb = a.K >> 8, D = a.D, nt = (a.F + 15) >> 4;
+  if (threadIdx.x == 0) abort_s = 0;
+  if (lane == 0) {
+    for (int d = 0; d < D; d++) mbar_init(&full[warp][d], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  const int rowsT = rows - 16 * warp;   // rows of this warp's tile (<= 0: the warp only helps quantizing)
-  const uint8_t* bcol = planes + min(g >> 1, 3) * 2 * K + (g & 1) * K + 8 * t;
-  const int rA = 4 * (g & 3) + (g >> 2);
-  const int hi = max(min(rowsT, 16) - 1, 0);
-  const int lrA = 16 * warp + min(rA, hi), lrB = 16 * warp + min(rA + 2, hi);
-  const uint8_t* pA = wbuf + (lrA >> 2) * GS + (lrA & 3) * RB;
-  const uint8_t* pB = wbuf + (lrB >> 2) * GS + (lrB & 3) * RB;
-  for (int m0 = 0; m0 < tk.m; m0 += 4) {
-    for (int u = warp; u < 4 * nchunks; u += kMdWarps) {
-      const int m = u / nchunks, sb = u - m * nchunks;
-      const XT* x = static_cast<const XT*>(a.x) + (long long)tk.ent[min(m0 + m, kTaskEntries - 1)] * K;
-      st_quantize<XT>(st_ld_cg16(x + sb * 256 + lane * 8), sb, lane, K, planes + m * 2 * K, XS + m * (K / 32),
-                      SX + m * ncp);
+  __syncthreads();
+  volatile int* abort_flag = &abort_s;
+  uint8_t* const ring = tk_dyn + warp * D * kTkSlot;
+  uint8_t* const xs = tk_dyn + a.x_off;
+  float* const sums = reinterpret_cast<float*>(tk_dyn + a.sum_off);
+  float* const red = reinterpret_cast<float*>(tk_dyn + a.red_off);  // [warp][first tile, last][matrix][16][kRedPitch]
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  const long long total = (long long)*n_tasks * nt;
+  const int t0 = (int)(total * blockIdx.x / gridDim.x), t1 = (int)(total * (blockIdx.x + 1) / gridDim.x);  // this CTA's tiles
+  auto end_of = [&](int from) { return min(t1, (from / nt + 1) * nt); };  // of the tiles of a task
+
+  // boxes: the next one of this warp's share
+  int is_from = t0, is_d = 0, is_row = 0, is_sb = 0, is_half = 0, is_left = 0, is_expert = 0;
+  auto open = [&]() {  // the share in the tasks from is_from on
+    while (is_left == 0 && is_from < t1) {
+      const int end = end_of(is_from), all = (end - is_from) * nsb, u0 = (warp * all) >> 4, u1 = ((warp + 1) * all) >> 4;
+      if (u1 > u0) {
+        const int tile = u0 / nsb, task = is_from / nt;
+        is_row = 16 * (is_from - task * nt + tile);
+        is_sb = u0 - tile * nsb;
+        is_left = u1 - u0;
+        is_expert = tasks[task].expert;
+      }
+      is_from = end;
+    }
+  };
+  auto issue = [&]() {
+    if (is_left == 0) return;
+    if (lane == 0) {
+      mbar_expect_tx(&full[warp][is_d], kTkSlot);
+      tk_load(smem_u32(ring + is_d * kTkSlot), GLU && is_half ? &map_u : &map_g, 144 * is_sb, is_row, is_expert, &full[warp][is_d]);
+    }
+    if (++is_d == D) is_d = 0;
+    if (GLU && is_half == 0) {
+      is_half = 1;
+      return;
+    }
+    is_half = 0;
+    if (++is_sb == nsb) is_sb = 0, is_row += 16;
+    if (--is_left == 0) open();
+  };
+
+  int d = 0;
+  uint32_t par = 0;
+  bool ok = true, begun = false;
+  for (int from = t0, end; from < t1; from = end) {
+    end = end_of(from);
+    const int task = from / nt, tile0 = from - task * nt, expert = tasks[task].expert, m = tasks[task].m;
+    const int all = (end - from) * nsb;
+    auto cut = [&](int w) { return (w * all) >> 4; };  // the first unit of warp w
+    __syncthreads();  // the activations and the partial sums of the task before have been read
+    if (threadIdx.x < 8 * NT) ent_s[threadIdx.x] = tasks[task].ent[threadIdx.x];
+    for (int i = warp; i < m; i += kTkWarps) {
+      const XT* src = static_cast<const XT*>(a.x) + (long long)(tasks[task].ent[i] / a.R) * a.K;
+      const uint32_t dst = smem_u32(xs + i * a.x_pitch);
+      for (int c = lane; c < 32 * nsb; c += 32) rw_cp16(dst + 16 * c, src + 8 * c);
+    }
+    if (!begun) {
+      begun = true;
+      open();
+      for (int i = 0; i < D; i++) issue();
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    for (int e = warp; e < nsb * NT; e += kTkWarps) {
+      const int k = e / NT, n = e % NT;
+      if (8 * n < m)
+        rows_sums<Q4_K, XT>(xs + min(8 * n + g, m - 1) * a.x_pitch + 512 * k, sums + (k * NT + n) * 8 * rw_sum_pitch(Q4_K), lane);
     }
     __syncthreads();
-    if (m0 == 0 && !md_wait(mbar, 0, error_word)) return;
-    if (rowsT > 0) {
-      float ydot[2] = {0.f, 0.f}, ymin[2][4] = {};
-      for (int sb = 0; sb < nchunks; sb++) {
-        const uint8_t* const blk[2] = {pA + sb * 144, pB + sb * 144};
-        st_unit_mx<1, 4>(blk, bcol + sb * 256, XS + sb * 8, K / 32, SX + sb, ncp, t, ydot, ymin);
+
+    auto finish = [&](int row, int c, float vg, float vu) {  // row of the matrix, activation row of the task
+      if (row >= a.F || c >= m) return;
+      const int entry = ent_s[c];
+      if (!(fabsf(vg) < INFINITY) || (GLU && !(fabsf(vu) < INFINITY))) {
+        const XT* xr = static_cast<const XT*>(a.x) + (long long)(entry / a.R) * a.K;
+        vg = rows_plain<Q4_K, XT>(a.wg + (long long)expert * a.stride_g + (long long)row * a.row_bytes, xr, nsb);
+        if (GLU) vu = rows_plain<Q4_K, XT>(a.wu + (long long)expert * a.stride_u + (long long)row * a.row_bytes, xr, nsb);
       }
+      md_store(static_cast<XT*>(a.y) + (long long)entry * a.F + row, GLU ? md_act(vg, vu, a.act, a.limit) : vg);
+    };
+
+    const int u0 = cut(warp), u1 = cut(warp + 1);
+    float y[H][NT][4];
 #pragma unroll
-      for (int r = 0; r < 2; r++) {
+    for (int h = 0; h < H; h++)
 #pragma unroll
-        for (int m = 0; m < 4; m++) {
-          ymin[r][m] += __shfl_xor_sync(0xffffffffu, ymin[r][m], 1);
-          ymin[r][m] += __shfl_xor_sync(0xffffffffu, ymin[r][m], 2);
+      for (int n = 0; n < NT; n++) y[h][n][0] = y[h][n][1] = y[h][n][2] = y[h][n][3] = 0.f;
+    int tile = u0 / nsb, sb = u0 - tile * nsb, second = 0;
+    bool whole = sb == 0;
+    for (int u = u0; u < u1; u++) {
+      const uint8_t* xb[NT];
+#pragma unroll
+      for (int n = 0; n < NT; n++) xb[n] = xs + min(8 * n + g, m - 1) * a.x_pitch + 512 * sb;
+#pragma unroll
+      for (int h = 0; h < H; h++) {
+        if (ok) ok = mbar_wait_err(&full[warp][d], par, abort_flag, 0x500, error_word);
+        if (ok) {
+          const uint8_t* r0 = ring + d * kTkSlot + g * 144;
+          if (NT == 1 || m > 8) {
+            RowsUnit<Q4_K, XT, NT>::run(y[h], r0, r0 + 8 * 144, xb, sums + sb * kSumWords, g, t);
+          } else {
+            const uint8_t* xb1[1] = {xb[0]};
+            float y1[1][4] = {{y[h][0][0], y[h][0][1], y[h][0][2], y[h][0][3]}};
+            RowsUnit<Q4_K, XT, 1>::run(y1, r0, r0 + 8 * 144, xb1, sums + sb * kSumWords, g, t);
+            y[h][0][0] = y1[0][0], y[h][0][1] = y1[0][1], y[h][0][2] = y1[0][2], y[h][0][3] = y1[0][3];
+          }
+        }
+        __syncwarp();  // the slot has been read
+        issue();
+        if (++d == D) d = 0, par ^= 1;
+      }
+      if (++sb < nsb && u + 1 < u1) continue;
+      if (whole && sb == nsb) {
+        if (ok) {
+          const int row = 16 * (tile0 + tile) + g;
+#pragma unroll
+          for (int n = 0; n < NT; n++)
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+              finish(row + (i >> 1) * 8, 8 * n + 2 * t + (i & 1), y[0][n][i], y[H - 1][n][i]);
+        }
+      } else {
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+          float* mine = red + (((2 * warp + second) * H + h) * 16 + g) * kRedPitch + 2 * t;
+#pragma unroll
+          for (int n = 0; n < NT; n++) {
+            *reinterpret_cast<float2*>(mine + 8 * n) = make_float2(y[h][n][0], y[h][n][1]);
+            *reinterpret_cast<float2*>(mine + 8 * kRedPitch + 8 * n) = make_float2(y[h][n][2], y[h][n][3]);
+          }
         }
       }
-      if (m0 + t < tk.m) {
-        XT* out = static_cast<XT*>(a.y) + (long long)tk.ent[m0 + t] * a.N + n0 + 16 * warp;
-        if (rA < rowsT) md_store(out + rA, ydot[0] - md_pick4(ymin[0], t));
-        if (rA + 2 < rowsT) md_store(out + rA + 2, ydot[1] - md_pick4(ymin[1], t));
+      sb = 0, tile++, second = 1, whole = true;
+#pragma unroll
+      for (int h = 0; h < H; h++)
+#pragma unroll
+        for (int n = 0; n < NT; n++) y[h][n][0] = y[h][n][1] = y[h][n][2] = y[h][n][3] = 0.f;
+    }
+    __syncthreads();
+    // tiles that a cut between two warps goes through, the parts in order
+    if (abort_s == 0) {
+      for (int i = threadIdx.x; i < (kTkWarps - 1) * 16 * m; i += kTkThreads) {
+        const int w = 1 + i / (16 * m), at = i - (w - 1) * 16 * m, place = at & 15, c = at >> 4;
+        const int tl = cut(w) / nsb, u = tl * nsb;
+        if (cut(w) == u || cut(w - 1) > u) continue;  // no tile is cut here, or it was cut before
+        float v[2] = {0.f, 0.f};
+        for (int q = w - 1; q < kTkWarps && cut(q) < u + nsb; q++) {
+          if (cut(q + 1) <= u || cut(q + 1) == cut(q)) continue;
+          const float* part = red + ((2 * q + (cut(q) / nsb == tl ? 0 : 1)) * H * 16 + place) * kRedPitch + c;
+          v[0] += part[0];
+          if (GLU) v[1] += part[16 * kRedPitch];
+        }
+        finish(16 * (tile0 + tl) + place, c, v[0], v[1]);
       }
     }
-    __syncthreads();   // the planes are free for the next pass
+  }
+  if (abort_s != 0) {  // given up: what is in flight lands long before this
+    const unsigned long long since = globaltimer_ns();
+    while (globaltimer_ns() - since < 1000000ull) {
+    }
   }
 }
 
@@ -704,9 +714,9 @@ static MoeWs moe_ws_layout(long long n_entries, int n_experts, long long d_bytes
   L.task_base = 3 * e1;
   L.n_tasks = 4 * e1;
   L.order = up(4 * e1 + 4);
-  L.max_tasks = n_entries / kTaskEntries + n_experts + 1;
+  L.max_tasks = n_entries / 16 + n_experts + 1;
   L.tasks = up(L.order + (size_t)n_entries * 4);
-  L.d = up(L.tasks + (size_t)L.max_tasks * sizeof(Task4));
+  L.d = up(L.tasks + (size_t)L.max_tasks * sizeof(Tasks<2>));
   L.total = up(L.d + (size_t)d_bytes);
   return L;
 }
@@ -715,30 +725,99 @@ size_t moe_grouped_workspace_bytes(long long n_entries, int n_experts, long long
   return moe_ws_layout(n_entries, n_experts, d_bytes).total;
 }
 
+// Tasks of eight entries where experts have few, of sixteen where a good part of them has more than eight. (Those of eight
+// fit into the room of the others: 40 (n / 8 + E) <= 72 (n / 16 + E).) Both products of a call see the same sizes here.
+static bool moe_small_tasks(long long n_entries, int n_experts) { return n_entries <= 5ll * n_experts; }
+
 static cudaError_t moe_build_tasks(const uint32_t* idx, long long n_entries, int n_experts, uint8_t* ws, const MoeWs& L,
                                    cudaStream_t st) {
   int* offsets = reinterpret_cast<int*>(ws + L.offsets);
   int* task_base = reinterpret_cast<int*>(ws + L.task_base);
   int* order = reinterpret_cast<int*>(ws + L.order);
-  cudaError_t e = launch_group_by_expert(idx, n_entries, n_experts, kTaskEntries, reinterpret_cast<int*>(ws + L.counts),
+  const bool small = moe_small_tasks(n_entries, n_experts);
+  cudaError_t e = launch_group_by_expert(idx, n_entries, n_experts, small ? 8 : 16, reinterpret_cast<int*>(ws + L.counts),
                                          reinterpret_cast<int*>(ws + L.cursor), offsets, task_base,
                                          reinterpret_cast<int*>(ws + L.n_tasks), order, st);
   if (e != cudaSuccess) return e;
-  moe_tasks4_kernel<<<n_experts, 64, 0, st>>>(offsets, task_base, order, reinterpret_cast<Task4*>(ws + L.tasks));
+  if (small)
+    moe_tasks_kernel<1><<<n_experts, 64, 0, st>>>(offsets, task_base, order, reinterpret_cast<Tasks<1>*>(ws + L.tasks));
+  else
+    moe_tasks_kernel<2><<<n_experts, 64, 0, st>>>(offsets, task_base, order, reinterpret_cast<Tasks<2>*>(ws + L.tasks));
   return cudaGetLastError();
 }
 
-template <typename KernelT, typename ArgsT>
-static cudaError_t md_launch_tasks(KernelT kern, dim3 grid, int smem, const ArgsT& a, const Task4* tasks,
-                                   const int* n_tasks, cudaStream_t st) {
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static EncodeTiledFn md_encode_fn() {
+  static EncodeTiledFn fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      p = nullptr;
+    return reinterpret_cast<EncodeTiledFn>(p);
+  }();
+  return fn;
+}
+// all experts' rows of one matrix
+static cudaError_t md_map(CUtensorMap* map, const uint8_t* w, long long row_bytes, int F, int n_experts, long long stride) {
+  EncodeTiledFn enc = md_encode_fn();
+  if (enc == nullptr) return cudaErrorNotSupported;
+  const cuuint64_t dims[3] = {(cuuint64_t)row_bytes, (cuuint64_t)F, (cuuint64_t)n_experts};
+  const cuuint64_t strides[2] = {(cuuint64_t)row_bytes, (cuuint64_t)stride};
+  const cuuint32_t box[3] = {144u, 16u, 1u}, estr[3] = {1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<uint8_t*>(w), dims, strides, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+// shared memory: rings | activations | their sums | partial sums; false where a slot of a matrix and one more do not fit
+template <int NT, bool GLU>
+static bool md_plan(TaskArgs& a, int& smem) {
+  const int nsb = a.K >> 8;
+  a.x_pitch = 2 * a.K + 64;
+  const int x = 8 * NT * a.x_pitch, sum = nsb * NT * 8 * rw_sum_pitch(Q4_K) * 4;
+  const int red = kTkWarps * 2 * (GLU ? 2 : 1) * 16 * (8 * NT + (NT == 1 ? 2 : 0)) * 4;
+  a.D = std::min(kTkMaxSlots, (kTkSmem - x - sum - red) / (kTkWarps * kTkSlot));
+  if (kTkSmem - x - sum - red < 0 || a.D < 2) return false;
+  a.x_off = a.D * kTkWarps * kTkSlot;
+  a.sum_off = a.x_off + x;
+  a.red_off = a.sum_off + sum;
+  smem = a.red_off + red;
+  return true;
+}
+
+template <typename XT, int NT, bool GLU>
+static cudaError_t md_launch_product(TaskArgs a, int n_experts, const void* tasks, const int* n_tasks, cudaStream_t st) {
+  int smem = 0;
+  if (!md_plan<NT, GLU>(a, smem)) return cudaErrorInvalidConfiguration;  // (not reached: moe_grouped_supported)
   int* err = device_error_word();
   if (err == nullptr) return cudaErrorUnknown;
+  static bool done[16] = {};
+  cudaError_t e = md_set_smem(moe_tasks_product_kernel<XT, NT, GLU>, kTkSmem, done);
+  if (e != cudaSuccess) return e;
+  alignas(64) CUtensorMap mg{}, mu{};
+  if ((e = md_map(&mg, a.wg, a.row_bytes, a.F, n_experts, a.stride_g)) != cudaSuccess) return e;
+  if (GLU && (e = md_map(&mu, a.wu, a.row_bytes, a.F, n_experts, a.stride_u)) != cudaSuccess) return e;
+  int dev = 0, sms = 0;
+  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(kMdThreads);
+  cfg.gridDim = dim3(sms);
+  cfg.blockDim = dim3(kTkThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  return cudaLaunchKernelEx(&cfg, kern, a, tasks, n_tasks, err);
+  return cudaLaunchKernelEx(&cfg, moe_tasks_product_kernel<XT, NT, GLU>, a, mg, mu, static_cast<const Tasks<NT>*>(tasks), n_tasks, err);
+}
+template <bool GLU>
+static cudaError_t md_launch_products(int x_dtype, const TaskArgs& a, long long n_entries, int n_experts, const void* tasks,
+                                      const int* n_tasks, cudaStream_t st) {
+  if (moe_small_tasks(n_entries, n_experts))
+    return x_dtype == F16 ? md_launch_product<__half, 1, GLU>(a, n_experts, tasks, n_tasks, st)
+                          : md_launch_product<__nv_bfloat16, 1, GLU>(a, n_experts, tasks, n_tasks, st);
+  return x_dtype == F16 ? md_launch_product<__half, 2, GLU>(a, n_experts, tasks, n_tasks, st)
+                        : md_launch_product<__nv_bfloat16, 2, GLU>(a, n_experts, tasks, n_tasks, st);
 }
 
 // the grouping alone (for a caller whose own grouped kernel does not apply but whose workspace is handed on)
@@ -749,8 +828,8 @@ cudaError_t launch_moe_grouping_only(const uint32_t* idx, long long n_entries, i
 }
 
 bool moe_grouped_supported(int K, long long row_bytes, bool rows_kernel) {
-  const int smem = rows_kernel ? rows4_smem_bytes(K, (int)row_bytes) : glu4_smem_bytes(K, (int)row_bytes);
-  return smem <= 110 * 1024;   // two CTAs per SM
+  (void)row_bytes;
+  return K <= (rows_kernel ? 1280 : 2304);
 }
 
 cudaError_t launch_moe_glu_grouped(int x_dtype, const void* x, int K, const uint8_t* wg, long long stride_g,
@@ -763,24 +842,11 @@ cudaError_t launch_moe_glu_grouped(int x_dtype, const void* x, int K, const uint
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   cudaError_t e = moe_build_tasks(idx, n_entries, n_experts, ws, L, st);
   if (e != cudaSuccess) return e;
-  static const int tiles_env = [] {
-    const char* e = std::getenv("KQ_MOE_GLU_TILES");   // A/B lever
-    const int v = e ? std::atoi(e) : 0;
-    return v >= 1 && v <= 64 ? v : kGluTiles;
-  }();
-  GluArgs a{x, wg, wu, stride_g, stride_u, (int)row_bytes, K, F, R, (int)n_entries, n_experts, idx, y, act, limit,
-            tiles_env};
-  const int smem = glu4_smem_bytes(K, (int)row_bytes);
-  const dim3 grid(((F + 15) / 16 + tiles_env - 1) / tiles_env, (unsigned)L.max_tasks, 1);
-  const Task4* tasks = reinterpret_cast<const Task4*>(ws + L.tasks);
-  const int* nt = reinterpret_cast<const int*>(ws + L.n_tasks);
-  static bool done_h[16] = {}, done_b[16] = {};
-  if (x_dtype == F16) {
-    if ((e = md_set_smem(moe_glu_tasks_kernel<__half>, kMdMaxSmem, done_h)) != cudaSuccess) return e;
-    return md_launch_tasks(moe_glu_tasks_kernel<__half>, grid, smem, a, tasks, nt, st);
-  }
-  if ((e = md_set_smem(moe_glu_tasks_kernel<__nv_bfloat16>, kMdMaxSmem, done_b)) != cudaSuccess) return e;
-  return md_launch_tasks(moe_glu_tasks_kernel<__nv_bfloat16>, grid, smem, a, tasks, nt, st);
+  TaskArgs a{};
+  a.x = x, a.K = K, a.F = F, a.R = R;
+  a.wg = wg, a.wu = wu, a.stride_g = stride_g, a.stride_u = stride_u, a.row_bytes = (int)row_bytes;
+  a.y = y, a.act = act, a.limit = limit;
+  return md_launch_products<true>(x_dtype, a, n_entries, n_experts, ws + L.tasks, reinterpret_cast<const int*>(ws + L.n_tasks), st);
 }
 
 // d[b] = x[b] . W[idx[b]]^T for every entry b (entries grouped by expert), then y[t] = sum_s scores[t, s] d[t S + s]
@@ -798,19 +864,11 @@ cudaError_t launch_moe_mix_grouped(int x_dtype, const void* x, int K, const uint
   if (!reuse_grouping && (e = moe_build_tasks(idx, n_entries, n_experts, ws, L, st)) != cudaSuccess) return e;
   // entries of experts out of range get no task: their d rows must not carry old bytes into the weighted sum
   if ((e = cudaMemsetAsync(ws + L.d, 0, (size_t)n_entries * N * 2, st)) != cudaSuccess) return e;
-  RowsArgs a{x, w, stride_w, (int)row_bytes, K, N, ws + L.d};
-  const int smem = rows4_smem_bytes(K, (int)row_bytes);
-  const dim3 grid((N + 127) / 128, (unsigned)L.max_tasks, 1);
-  const Task4* tasks = reinterpret_cast<const Task4*>(ws + L.tasks);
-  const int* nt = reinterpret_cast<const int*>(ws + L.n_tasks);
-  static bool done_h[16] = {}, done_b[16] = {};
-  if (x_dtype == F16) {
-    if ((e = md_set_smem(moe_rows_tasks_kernel<__half>, kMdMaxSmem, done_h)) != cudaSuccess) return e;
-    e = md_launch_tasks(moe_rows_tasks_kernel<__half>, grid, smem, a, tasks, nt, st);
-  } else {
-    if ((e = md_set_smem(moe_rows_tasks_kernel<__nv_bfloat16>, kMdMaxSmem, done_b)) != cudaSuccess) return e;
-    e = md_launch_tasks(moe_rows_tasks_kernel<__nv_bfloat16>, grid, smem, a, tasks, nt, st);
-  }
+  TaskArgs a{};
+  a.x = x, a.K = K, a.F = N, a.R = 1;
+  a.wg = w, a.stride_g = stride_w, a.row_bytes = (int)row_bytes;
+  a.y = ws + L.d;
+  e = md_launch_products<false>(x_dtype, a, n_entries, n_experts, ws + L.tasks, reinterpret_cast<const int*>(ws + L.n_tasks), st);
   if (e != cudaSuccess) return e;
   return launch_moe_combine(x_dtype, ws + L.d, scores, T, S, N, y, false, st);
 }
