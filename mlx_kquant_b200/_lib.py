@@ -107,6 +107,28 @@ def lib() -> C.CDLL:
     return _lib
 
 
+_front = None
+
+
+def torch_front():
+    """The native front of quantized_matmul (csrc/kq_torch.cpp), or None where it was not built."""
+    global _front
+    if _front is None:
+        path = HERE / "_kq_torch.so"
+        if not path.exists():
+            return None
+        import importlib.util
+
+        spec = importlib.util.spec_from_file_location("_kq_torch", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        handle = lib()
+        module.init(*[C.cast(getattr(handle, name), C.c_void_p).value for name in
+                      ("kq_codec_find", "kq_codec_info", "kq_quantized_matmul_workspace_bytes", "kq_quantized_matmul")])
+        _front = module
+    return _front
+
+
 def check(rc: int) -> None:
     """Map a KQ_ERR_* code to the exception the reference's binding raises."""
     if rc == 0:
