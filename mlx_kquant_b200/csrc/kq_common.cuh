@@ -450,7 +450,7 @@ __device__ __forceinline__ IqTables stage_iq_tables(uint8_t* smem, int tid, int 
 // order of i (CTAs that share them must agree on it), in any if there are at most `unordered` of them; all threads of the
 // CTA take part, `count` (shared) starts at 0. n at most 4 * TH.
 template <int TH>
-__device__ __forceinline__ int collect_entries(const uint32_t* __restrict__ rhs, const uint32_t* __restrict__ lhs, int n,
+__device__ __forceinline__ int collect_entries(const uint32_t* rhs, const uint32_t* lhs, int n,
                                                long long x_batch, uint32_t e, int2* list, int* count, int unordered) {
   // both indices of up to four entries a thread in flight at once: one latency, not one for each
   for (int i = threadIdx.x; i < n; i += 4 * TH) {

@@ -219,9 +219,9 @@ cudaError_t launch_gather(int codec, int x_dtype, const void* x, long long x_bat
                           const uint32_t* rhs, long long n_entries, void* y, void* workspace, bool allow_grouped,
                           cudaStream_t st);
 
-// memset + histogram + scan + scatter of kq_gather.cu for other callers: see the definition.
+// the grouping of kq_gather.cu for other callers: see launch_group there.
 cudaError_t launch_group_by_expert(const uint32_t* rhs, long long n, int n_experts, int unit, int* counts, int* cursor,
-                                   int* offsets, int* unit_base, int* n_units, int* order, cudaStream_t st);
+                                   int* offsets, int* unit_base, int* n_units, int* order, int* tasks, cudaStream_t st);
 
 // The body of kq_gather_qmm; allow_grouped = false pins the decode regime (fixed-size scratch);
 // builtin_scratch = true words a too-small workspace as the limit of the library's fixed array.

@@ -325,23 +325,6 @@ struct Tasks {
   int ent[8 * NT];   // entry indices; slots past m repeat the last one
 };
 
-template <int NT>
-__global__ void moe_tasks_kernel(const int* __restrict__ offsets, const int* __restrict__ task_base,
-                                 const int* __restrict__ order, Tasks<NT>* tasks) {
-  constexpr int kN = 8 * NT;
-  const int e = blockIdx.x;
-  const int o0 = offsets[e], c = offsets[e + 1] - o0;
-  const int nt = (c + kN - 1) / kN, tb = task_base[e];
-  for (int k = threadIdx.x; k < nt; k += blockDim.x) {
-    Tasks<NT> t;
-    t.expert = e;
-    t.m = min(kN, c - kN * k);
-#pragma unroll
-    for (int j = 0; j < kN; j++) t.ent[j] = order[o0 + kN * k + min(j, t.m - 1)];
-    tasks[tb + k] = t;
-  }
-}
-
 struct TaskArgs {
   const void* x;            // entry b's row is b / R
   int K, F, R;              // F: rows of a matrix (of gate and of up each)
@@ -368,7 +351,8 @@ __device__ __forceinline__ void tk_load(uint32_t dst, const CUtensorMap* map, in
 template <typename XT, int NT, bool GLU>
 __global__ void __launch_bounds__(kTkThreads, 1)
 moe_tasks_product_kernel(const TaskArgs a, const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_u,
-                         const Tasks<NT>* __restrict__ tasks, const int* __restrict__ n_tasks, int* __restrict__ error_word) {
+                         const Tasks<NT>* tasks, const int* n_tasks, int* __restrict__ error_word) {
+  // (tasks, n_tasks: not __restrict__, whose loads may be moved ahead of griddepcontrol.wait)
   constexpr int H = GLU ? 2 : 1;                       // matrices
   constexpr int kRedPitch = 8 * NT + (NT == 1 ? 2 : 0);
   constexpr int kSumWords = NT * 8 * rw_sum_pitch(Q4_K);
@@ -731,19 +715,11 @@ static bool moe_small_tasks(long long n_entries, int n_experts) { return n_entri
 
 static cudaError_t moe_build_tasks(const uint32_t* idx, long long n_entries, int n_experts, uint8_t* ws, const MoeWs& L,
                                    cudaStream_t st) {
-  int* offsets = reinterpret_cast<int*>(ws + L.offsets);
-  int* task_base = reinterpret_cast<int*>(ws + L.task_base);
-  int* order = reinterpret_cast<int*>(ws + L.order);
-  const bool small = moe_small_tasks(n_entries, n_experts);
-  cudaError_t e = launch_group_by_expert(idx, n_entries, n_experts, small ? 8 : 16, reinterpret_cast<int*>(ws + L.counts),
-                                         reinterpret_cast<int*>(ws + L.cursor), offsets, task_base,
-                                         reinterpret_cast<int*>(ws + L.n_tasks), order, st);
-  if (e != cudaSuccess) return e;
-  if (small)
-    moe_tasks_kernel<1><<<n_experts, 64, 0, st>>>(offsets, task_base, order, reinterpret_cast<Tasks<1>*>(ws + L.tasks));
-  else
-    moe_tasks_kernel<2><<<n_experts, 64, 0, st>>>(offsets, task_base, order, reinterpret_cast<Tasks<2>*>(ws + L.tasks));
-  return cudaGetLastError();
+  return launch_group_by_expert(idx, n_entries, n_experts, moe_small_tasks(n_entries, n_experts) ? 8 : 16,
+                                reinterpret_cast<int*>(ws + L.counts), reinterpret_cast<int*>(ws + L.cursor),
+                                reinterpret_cast<int*>(ws + L.offsets), reinterpret_cast<int*>(ws + L.task_base),
+                                reinterpret_cast<int*>(ws + L.n_tasks), reinterpret_cast<int*>(ws + L.order),
+                                reinterpret_cast<int*>(ws + L.tasks), st);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -808,6 +784,11 @@ static cudaError_t md_launch_product(TaskArgs a, int n_experts, const void* task
   cfg.blockDim = dim3(kTkThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, moe_tasks_product_kernel<XT, NT, GLU>, a, mg, mu, static_cast<const Tasks<NT>*>(tasks), n_tasks, err);
 }
 template <bool GLU>

@@ -17,17 +17,17 @@ def stack(E, n, k, seed):
     return np.stack([mint_wire("q4_k", np.random.default_rng(seed + e).normal(0, 0.02, (n, k)).astype(np.float32)) for e in range(E)])
 
 
-def glu(x, wg, wu, ids, dt):
+def glu(x, wg, wu, ids, dt, ws=None):
     T, K = x.shape
     E, F, R = wg.shape[0], wg.shape[1], ids.shape[1]
     L = _lib.lib()
     y = torch.full((T, R, F), 3.0, dtype=x.dtype, device="cuda")
-    ws = torch.empty(L.kq_moe_decode_workspace_bytes(T * R, E, 0), dtype=torch.uint8, device="cuda")
-    idx = torch.from_numpy(ids.astype(np.int32)).cuda()
+    if ws is None:
+        ws = torch.empty(L.kq_moe_decode_workspace_bytes(T * R, E, 0), dtype=torch.uint8, device="cuda")
+    idx = ids if isinstance(ids, torch.Tensor) else torch.from_numpy(ids.astype(np.int32)).cuda()
     _lib.check(L.kq_moe_glu_gather(x.data_ptr(), _lib.KQ_F16 if dt == "f16" else _lib.KQ_BF16, T, K, wg.data_ptr(), wg.stride(0),
                                    wu.data_ptr(), wu.stride(0), wg.shape[2], F, E, b"q4_k", idx.data_ptr(), R, b"silu", 0.0,
                                    y.data_ptr(), ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream))
-    torch.cuda.synchronize()
     return y
 
 
@@ -85,3 +85,23 @@ def test_not_finite():
     xb = torch.zeros_like(x)
     xb[3, 5] = 1e18
     assert torch.isfinite(glu(xb, wg, wu, ids, "bf16")).all()
+
+
+def test_replayed_with_other_routing():
+    """The products start beside the grouping in a captured graph, and take the task list only once it is there."""
+    E, F, K, T, R = 40, 64, 512, 50, 4
+    wg, wu = torch.from_numpy(stack(E, F, K, 1)).cuda(), torch.from_numpy(stack(E, F, K, 500)).cuda()
+    x = torch.randn(T, K, generator=torch.Generator().manual_seed(1)).bfloat16().cuda()
+    ws = torch.zeros(_lib.lib().kq_moe_decode_workspace_bytes(T * R, E, 0), dtype=torch.uint8, device="cuda")
+    idx = torch.zeros((T, R), dtype=torch.int32, device="cuda")
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        y = glu(x, wg, wu, idx, "bf16", ws)
+    for seed in range(3):
+        ids = torch.from_numpy(routing(E, T, R, 0.3 * seed, seed).astype(np.int32)).cuda()
+        want = glu(x, wg, wu, ids, "bf16")
+        torch.cuda.synchronize()
+        idx.copy_(ids)
+        ws.zero_()
+        g.replay()
+        assert torch.equal(y, want)

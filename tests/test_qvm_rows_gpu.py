@@ -4,7 +4,7 @@ import pytest
 import torch
 
 import mlx_kquant_b200 as kq
-from gpu_util import x_to_torch, y_to_f32
+from gpu_util import mint_wire, x_to_torch, y_to_f32
 from oracle.kq_oracle import Oracle
 
 pytestmark = pytest.mark.gpu
@@ -19,7 +19,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("dt", ["f16", "bf16"])
 def test_shared_matrices(codec, experts, k, n, entries, off, dt):
     rng = np.random.default_rng(k + n)
-    wire = kq.quantize(torch.from_numpy(rng.standard_normal((experts * k, n)).astype(np.float32) * 0.05), codec, None)[0]
+    wire = torch.from_numpy(mint_wire(codec, rng.standard_normal((experts * k, n)).astype(np.float32) * 0.05))
     wire = wire.reshape(experts, k, -1)
     room = torch.zeros(wire.numel() + 16, dtype=torch.uint8, device="cuda")
     w = room[off:off + wire.numel()].view(wire.shape)
