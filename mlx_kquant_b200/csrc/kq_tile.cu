@@ -295,7 +295,8 @@ struct Q4kHalf {
 
 // q6_k (src/kquant_cpu_decode.cpp:238-280): a half is four quarters of 32 weights; the low nibbles of its 64 ql bytes are
 // quarters 0 and 1, the high ones 2 and 3, bits 2 j of its 32 qh bytes belong to quarter j. A weight is
-// (q - 32) * fp16(d * scale). The block starts `phase` bytes (even, the same for all rows) into a 16-byte aligned window.
+// (q - 32) * (d * scale), the scale in two fp16 parts, so that the product is rounded once but for the last bit of a small
+// correction, as dequantization to fp16 is (a scale in one part: errors a third larger; 4-8 % faster). The block starts `phase` bytes (even, the same for all rows) into a 16-byte aligned window.
 template <int UNIT>
 struct Q6kHalf {
   uint32_t ql[16], qh[8], sc[2];
@@ -330,21 +331,30 @@ struct Q6kHalf {
     }
   }
   __device__ __forceinline__ void header(int) {}
+  // v = hi + lo; a scale that overflows stays an infinity
+  static __device__ __forceinline__ void two(float v, __half2& hi, __half2& lo) {
+    hi = __float2half2_rn(v);
+    const float rest = v - __low2float(hi);
+    lo = __float2half2_rn(fabsf(rest) < 65504.f ? rest : 0.f);
+  }
   template <int P>
   __device__ __forceinline__ void make(uint32_t (&o)[32]) const {
     const __half2 k1056 = __float2half2_rn(1056.f);
 #pragma unroll
     for (int hh = 0; hh < 2; hh++) {
-      const __half2 sA = __float2half2_rn(d * (float)(int)(int8_t)((sc[P] >> (16 * hh)) & 0xffu));
-      const __half2 sB = __float2half2_rn(d * (float)(int)(int8_t)((sc[P] >> (16 * hh + 8)) & 0xffu));
+      __half2 sA, sB, tA, tB;
+      two(d * (float)(int)(int8_t)((sc[P] >> (16 * hh)) & 0xffu), sA, tA);
+      two(d * (float)(int)(int8_t)((sc[P] >> (16 * hh + 8)) & 0xffu), sB, tB);
 #pragma unroll
       for (int i = 0; i < 8; i++) {
         const uint32_t hb = P == 0 ? (hh == 0 ? qh[i] << 4 : qh[i] << 2) : (hh == 0 ? qh[i] : qh[i] >> 2);
         const uint32_t l = ql[8 * hh + i];
         const uint32_t q4 = ((P ? l >> 4 : l) & 0x0f0f0f0fu) | (hb & 0x30303030u);
-        const __half2 s = i < 4 ? sA : sB;
-        o[16 * hh + 2 * i] = as_u32(__hmul2(__hsub2(as_h2(__byte_perm(q4, 0x64646464u, 0x4140)), k1056), s));
-        o[16 * hh + 2 * i + 1] = as_u32(__hmul2(__hsub2(as_h2(__byte_perm(q4, 0x64646464u, 0x4342)), k1056), s));
+        const __half2 s = i < 4 ? sA : sB, t = i < 4 ? tA : tB;
+        const __half2 q0 = __hsub2(as_h2(__byte_perm(q4, 0x64646464u, 0x4140)), k1056);
+        const __half2 q1 = __hsub2(as_h2(__byte_perm(q4, 0x64646464u, 0x4342)), k1056);
+        o[16 * hh + 2 * i] = as_u32(__hfma2(q0, s, __hmul2(q0, t)));
+        o[16 * hh + 2 * i + 1] = as_u32(__hfma2(q1, s, __hmul2(q1, t)));
       }
     }
   }

@@ -91,3 +91,18 @@ def test_grouped(codec, k, counts):
     full = x[:, 0].double().cpu().numpy() @ Oracle().dequantize(some, codec, "f32").astype(np.float64).T   # [100, 64]
     ref = np.stack([full[a, pick[b]] for a, b in zip(lhs, rhs)])
     check(y.reshape(rhs.size, n), ref, "bf16")
+
+
+@pytest.mark.parametrize("rows", [64, 600])
+def test_q6k_weights_are_rounded_once(rows):
+    """One-hot activations show the producers' weights: those of dequantize to fp16, but for the last bit of a few where the
+    scale's second part (2^-11 of the first, itself in fp16) decides a tie."""
+    g = torch.Generator().manual_seed(6)
+    w = kq.quantize(torch.randn(512, 2048, generator=g) * 0.05, "q6_k", None)[0].cuda()
+    k = torch.randperm(2048, generator=g)[:rows].cuda()
+    x = torch.zeros(rows, 2048, dtype=torch.float16, device="cuda")
+    x[torch.arange(rows, device="cuda"), k] = 1
+    y = kq.quantized_matmul(x, w, None, "q6_k")
+    ref = kq.dequantize(w, None, "q6_k", torch.float16)[:, k].T
+    off = (y.view(torch.int16).int() - ref.contiguous().view(torch.int16).int()).abs()
+    assert int(off.max()) <= 1 and float((off > 0).float().mean()) < 0.02
