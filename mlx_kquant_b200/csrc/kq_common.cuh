@@ -449,22 +449,22 @@ __device__ __forceinline__ IqTables stage_iq_tables(uint8_t* smem, int tid, int 
 // The entries i of a gather call that multiply by matrix e, with an activation row in range, as (row of x, i), in the
 // order of i (CTAs that share them must agree on it), in any if there are at most `unordered` of them; all threads of the
 // CTA take part, `count` (shared) starts at 0. n at most 4 * TH.
-template <int TH>
-__device__ __forceinline__ int collect_entries(const uint32_t* rhs, const uint32_t* lhs, int n,
-                                               long long x_batch, uint32_t e, int2* list, int* count, int unordered) {
-  // both indices of up to four entries a thread in flight at once: one latency, not one for each
-  for (int i = threadIdx.x; i < n; i += 4 * TH) {
-    uint32_t r[4], l[4];
+// `meanwhile` runs in all threads while the indices are on their way.
+template <int TH, typename F>
+__device__ __forceinline__ int collect_entries(const uint32_t* rhs, const uint32_t* lhs, int n, long long x_batch, uint32_t e,
+                                               int2* list, int* count, int unordered, F&& meanwhile) {
+  // both indices of a thread's entries in flight at once: one latency, not one for each
+  uint32_t r[4], l[4];
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int at = i + q * TH;
-      r[q] = at < n ? rhs[at] : ~e;
-      l[q] = at < n ? lhs[at] : 0;
-    }
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-      if (r[q] == e && (long long)l[q] < x_batch) list[atomicAdd(count, 1)] = make_int2((int)l[q], i + q * TH);
+  for (int q = 0; q < 4; q++) {
+    const int at = threadIdx.x + q * TH;
+    r[q] = at < n ? rhs[at] : ~e;
+    l[q] = at < n ? lhs[at] : 0;
   }
+  meanwhile();
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+    if (r[q] == e && (long long)l[q] < x_batch) list[atomicAdd(count, 1)] = make_int2((int)l[q], (int)threadIdx.x + q * TH);
   __syncthreads();
   const int c = *count;
   if (c <= unordered) return c;

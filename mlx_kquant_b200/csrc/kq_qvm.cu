@@ -182,8 +182,8 @@ qvm_rows_kernel(const XT* __restrict__ x, void* __restrict__ y, const uint8_t* _
     }
   };
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
-  stage(0, min(kRowChunk, K));  // on their way while the entries are looked for
-  const int count = collect_entries<kThreads>(gq.rhs, gq.lhs, n_entries, gq.x_batch, e, list, &count_s, gridDim.z > 1 ? 0 : n_entries);
+  const int count = collect_entries<kThreads>(gq.rhs, gq.lhs, n_entries, gq.x_batch, e, list, &count_s,
+                                              gridDim.z > 1 ? 0 : n_entries, [&]() { stage(0, min(kRowChunk, K)); });
   if (count == 0) {
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     return;
