@@ -843,15 +843,15 @@ cudaError_t launch_moe_mix_grouped(int x_dtype, const void* x, int K, const uint
   cudaError_t e = cudaSuccess;
   // reuse_grouping: the workspace still holds the task list that launch_moe_glu_grouped built from these indices
   if (!reuse_grouping && (e = moe_build_tasks(idx, n_entries, n_experts, ws, L, st)) != cudaSuccess) return e;
-  // entries of experts out of range get no task: their d rows must not carry old bytes into the weighted sum
-  if ((e = cudaMemsetAsync(ws + L.d, 0, (size_t)n_entries * N * 2, st)) != cudaSuccess) return e;
   TaskArgs a{};
   a.x = x, a.K = K, a.F = N, a.R = 1;
   a.wg = w, a.stride_g = stride_w, a.row_bytes = (int)row_bytes;
   a.y = ws + L.d;
   e = md_launch_products<false>(x_dtype, a, n_entries, n_experts, ws + L.tasks, reinterpret_cast<const int*>(ws + L.n_tasks), st);
   if (e != cudaSuccess) return e;
-  return launch_moe_combine(x_dtype, ws + L.d, scores, T, S, N, y, false, st);
+  // entries of experts out of range get no task: the weighted sum does not read their d rows (with rows of zeros instead, the
+  // memset between the two products kept them apart)
+  return launch_moe_combine(x_dtype, ws + L.d, scores, T, S, N, y, false, st, idx, (uint32_t)n_experts);
 }
 
 bool moe_decode_supported(int codec, int x_dtype, int K, long long row_bytes, const void* x, const void* w0,
