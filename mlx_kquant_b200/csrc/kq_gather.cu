@@ -203,6 +203,26 @@ __global__ void gather_tiles_kernel(int M, int tile_rows, const int* __restrict_
   for (int j = threadIdx.x; j < nt; j += blockDim.x) tiles[tile_base[e] + j] = even_tile(e, start, rows, nt, j);
 }
 
+// Tasks take an expert's entries in the order of the entries, not in the one the counters happened to give: a task's products
+// are cut where the SMs' shares end, so that which entries share a task decides the order of their sums. The place of an
+// entry is the number of its expert's entries before it, counted where an expert has more than one task (0.3 us of the 275 us
+// of two blocks of 64 tokens; in the counters' order 298 of 300 calls gave other bits than the first).
+__device__ __forceinline__ void put_task(int* task, int unit, int expert, int rows, int rank, int entry) {
+  const int k = rank / unit, j = rank - k * unit, m = min(unit, rows - k * unit);
+  task += (long long)k * (unit + 2);
+  if (j == 0) task[0] = expert, task[1] = m;
+  task[2 + j] = entry;
+  if (j == m - 1)  // the last one repeated
+    for (int i = m; i < unit; i++) task[2 + i] = entry;
+}
+template <typename F>
+__device__ __forceinline__ int rank_in(const int* list, int n, int entry, F&& load) {
+  int rank = 0;
+#pragma unroll 8
+  for (int i = 0; i < n; i++) rank += load(list + i) < entry ? 1 : 0;
+  return rank;
+}
+
 // The grouping in one launch, up to kGroupMax entries: histogram, scans, order and tile list by a cluster of CTAs (one for a
 // few entries) that keeps its counters in shared memory and the entries' experts and places in registers. A counter's old
 // value is its entry's place among this CTA's, so the indices are read once; the CTAs' counts meet over distributed shared
@@ -216,6 +236,7 @@ group_kernel(const uint32_t* __restrict__ rhs, const uint32_t* __restrict__ lhs,
   __shared__ int count[kGroupExperts], first[kGroupExperts];           // this CTA's entries; where they go
   __shared__ int start[kGroupExperts + 1], units[kGroupExperts + 1];   // of all CTAs' entries, exclusive sums
   __shared__ int sum_c[32], sum_u[32];
+  __shared__ int listed[2 * kGroupThreads];                            // the order, of one CTA's entries
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = gridDim.x, r = blockIdx.x;
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   auto meet = [&]() {
@@ -266,7 +287,10 @@ group_kernel(const uint32_t* __restrict__ rhs, const uint32_t* __restrict__ lhs,
   meet();  // ... and every CTA has read the others' counts
 #pragma unroll
   for (int q = 0; q < kGroupEach; q++)
-    if (order != nullptr && e[q] < (uint32_t)n_experts) order[first[e[q]] + place[q]] = b0 + tid + q * kGroupThreads;
+    if (order != nullptr && e[q] < (uint32_t)n_experts) {
+      order[first[e[q]] + place[q]] = b0 + tid + q * kGroupThreads;
+      if (C == 1) listed[first[e[q]] + place[q]] = tid + q * kGroupThreads;
+    }
   if (r == 0 && tid <= n_experts && tid < kGroupThreads) offsets[tid] = start[tid], unit_base[tid] = units[tid];
   if (r == 0 && tid == 0) {
     offsets[n_experts] = start[n_experts], unit_base[n_experts] = units[n_experts];
@@ -280,23 +304,25 @@ group_kernel(const uint32_t* __restrict__ rhs, const uint32_t* __restrict__ lhs,
     }
   if (tasks != nullptr) {
     meet();  // the order is complete
-    for (int x = r * 32 + warp; x < n_experts; x += 32 * C) {
-      const int rows = start[x + 1] - start[x], words = (units[x + 1] - units[x]) * (unit + 2);
-      for (int i = lane; i < words; i += 32) {
-        const int k = i / (unit + 2), j = i - k * (unit + 2), m = min(unit, rows - k * unit);
-        const int v = j == 0 ? x : j == 1 ? m : __ldcg(order + start[x] + k * unit + min(j - 2, m - 1));
-        tasks[units[x] * (unit + 2) + i] = v;
+#pragma unroll
+    for (int q = 0; q < kGroupEach; q++)
+      if (e[q] < (uint32_t)n_experts) {
+        const int x = (int)e[q], from = start[x], rows = start[x + 1] - from, i = b0 + tid + q * kGroupThreads;
+        const int rank = rows <= unit ? first[x] + place[q] - from
+                                      : (C == 1 ? rank_in(listed + from, rows, i, [](const int* p) { return *p; })
+                                                : rank_in(order + from, rows, i, [](const int* p) { return __ldcg(p); }));
+        put_task(tasks + (long long)units[x] * (unit + 2), unit, x, rows, rank, i);
       }
-    }
   }
 }
 
 __global__ void group_tasks_kernel(int unit, const int* __restrict__ offsets, const int* __restrict__ unit_base,
                                    const int* __restrict__ order, int* tasks) {
   const int x = blockIdx.x, from = offsets[x], rows = offsets[x + 1] - from;
-  for (int i = threadIdx.x; i < (unit_base[x + 1] - unit_base[x]) * (unit + 2); i += blockDim.x) {
-    const int k = i / (unit + 2), j = i - k * (unit + 2), m = min(unit, rows - k * unit);
-    tasks[unit_base[x] * (unit + 2) + i] = j == 0 ? x : j == 1 ? m : order[from + k * unit + min(j - 2, m - 1)];
+  for (int at = threadIdx.x; at < rows; at += blockDim.x) {
+    const int i = order[from + at];
+    const int rank = rows <= unit ? at : rank_in(order + from, rows, i, [](const int* p) { return *p; });
+    put_task(tasks + (long long)unit_base[x] * (unit + 2), unit, x, rows, rank, i);
   }
 }
 
