@@ -19,6 +19,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 // The GGUF IQ lookup tables (generated by gen_tables.py) as per-translation-unit
 // __device__ arrays: kq_tab_iq4nl[16], kq_tab_iq2xxs_grid[256], kq_tab_ksigns[128], kq_tab_mxfp4[16],
 // kq_tab_iq3xxs_grid[256], kq_tab_iq3s_grid[512], kq_tab_iq2xs_grid[512], kq_tab_iq2s_grid[1024],
@@ -444,6 +446,30 @@ __device__ __forceinline__ IqTables stage_iq_tables(uint8_t* smem, int tid, int 
   t.grid = sg;
   t.ksigns = sk;
   return t;
+}
+
+// One output by itself: decoded weights times activations in float32 (float32 rows rounded to bf16 first), as the generic
+// kernel has it. For outputs that a split into integers, offsets, sums and scales leaves without a finite value although they
+// may have one, or an infinity: an infinite activation meets an offset's sum (inf - inf) or integers of zero, and a sum can
+// overflow before its scale is applied. Rare, so one thread an output, without care for speed.
+template <int C, int A, typename XT>
+__device__ __forceinline__ float plain_dot(const uint8_t* w, const XT* x, int K) {
+  const IqTables tabs = global_iq_tables();
+  float sum = 0.f;
+#pragma unroll 1
+  for (int k = 0; k < K; k += 8) {
+    float v[8];
+    decode8<C, A>(w + block_of<C>(k) * bpb_of(C), octet_of<C>(k), v, tabs);
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      float xv;
+      if constexpr (std::is_same<XT, __half>::value) xv = __half2float(x[k + i]);
+      else if constexpr (std::is_same<XT, float>::value) xv = __bfloat162float(__float2bfloat16_rn(x[k + i]));
+      else xv = __bfloat162float(x[k + i]);
+      sum = fmaf(xv, v[i], sum);
+    }
+  }
+  return sum;
 }
 
 // The entries i of a gather call that multiply by matrix e, with an activation row in range, as (row of x, i), in the

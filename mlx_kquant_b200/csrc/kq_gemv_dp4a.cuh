@@ -392,9 +392,41 @@ __host__ __device__ static inline int x_bytes(int K) { return 2 * K + (K / 32) *
 template <int C>
 int dyn_smem(int K, int D, int MT) { return kWarps * D * slot_bytes<C>() + MT * x_bytes(K); }
 
+// The scale of a 32-group whose largest magnitude has these bits, and its inverse, which stays finite: for the smallest groups
+// the scale is 2^-112 / 32767, half the smallest normal number. A group with an infinity or a NaN, which order above all numbers
+// as bits, becomes zeros with that as the scale: zero times it makes every output NaN, and dp_again makes them again.
+struct XUnit {
+  float inv, scale;
+};
+__device__ __forceinline__ XUnit x_unit(uint32_t top) {
+  const float amax = fmaxf(__uint_as_float(top), 0x1p-112f);
+  XUnit u;
+  u.inv = 32767.f * __frcp_rn(amax);
+  u.scale = amax * (1.f / 32767.f);
+  if (top >= 0x7f800000u) u.inv = 0.f, u.scale = __uint_as_float(top);
+  return u;
+}
+
+// All outputs of a CTA again, from decoded weights (an output of it has no finite value).
+template <int C, typename XT, typename OT>
+__device__ __noinline__ void dp_again(const GemvArgs& a, int row0, int rstep, int rows, int mt) {
+  const GemvTask* tk = a.tasks != nullptr ? a.tasks + blockIdx.y : nullptr;
+  const int t0 = tk != nullptr ? mt * (int)blockIdx.z : 0, m = min(tk != nullptr ? tk->m - t0 : a.M, mt);
+  for (int i = threadIdx.x; i < m * rows; i += kThreads) {
+    const int t = i / rows, n = row0 + (i - t * rows) * rstep;
+    if (n >= a.N) continue;
+    const long long xrow = tk != nullptr ? tk->xrow[t0 + t] : t, yrow = tk != nullptr ? tk->yrow[t0 + t] : t;
+    float sum = plain_dot<C, 1>((tk != nullptr ? tk->w : a.w) + (long long)n * a.row_bytes, static_cast<const XT*>(a.x) + xrow * a.x_row_stride, a.K);
+    if (a.bias != nullptr) sum += (float)static_cast<const OT*>(a.bias)[n];
+    OT* out = static_cast<OT*>(a.y) + yrow * a.y_row_stride + n;
+    if constexpr (std::is_same<OT, __half>::value) *out = __float2half_rn(sum);
+    else *out = __float2bfloat16_rn(sum);
+  }
+}
+
 // KP: parts of K in a warp. ROWA: rows are whole multiples of 16 bytes.
 template <int C, typename XT, int MT, int KP, bool ROWA>
-__global__ void __launch_bounds__(kThreads, MT == 1 ? 3 : 2) gemv_dp4a_kernel(const GemvArgs a, const int D) {
+__global__ void __launch_bounds__(kThreads, MT == 1 ? 3 : 2) gemv_dp4a_kernel(const __grid_constant__ GemvArgs a, const int D) {
   using OT = typename std::conditional<std::is_same<XT, __half>::value, __half, __nv_bfloat16>::type;
   using G = Geom<C>;
   constexpr int kSlot = slot_bytes<C>(), kStride = 16 * G::kP;
@@ -515,21 +547,22 @@ __global__ void __launch_bounds__(kThreads, MT == 1 ? 3 : 2) gemv_dp4a_kernel(co
           v[2 * i + 1] = f.y;
         }
       }
-      float amax = 0.f, sum = 0.f;
+      // the largest magnitude as bits: infinities and NaNs order above all numbers and survive (fmaxf drops a NaN)
+      uint32_t top = 0u;
+      float sum = 0.f;
 #pragma unroll
       for (int i = 0; i < 8; i++) {
-        amax = fmaxf(amax, fabsf(v[i]));
+        top = max(top, __float_as_uint(v[i]) & 0x7fffffffu);
         sum += v[i];
       }
-      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+      top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));
+      top = max(top, __shfl_xor_sync(0xffffffffu, top, 2));
       sum += __shfl_xor_sync(0xffffffffu, sum, 1);  // 16-group
-      const bool finite = amax > 0.f && amax < INFINITY;
-      const float inv = finite ? 32767.f * __frcp_rn(amax) : 0.f;
+      const XUnit unit = x_unit(top);
       int xi[8], isum = 0;
 #pragma unroll
       for (int i = 0; i < 8; i++) {
-        xi[i] = __float2int_rn(v[i] * inv);
+        xi[i] = __float2int_rn(v[i] * unit.inv);
         isum += xi[i];
       }
       isum += __shfl_xor_sync(0xffffffffu, isum, 1);
@@ -568,8 +601,7 @@ __global__ void __launch_bounds__(kThreads, MT == 1 ? 3 : 2) gemv_dp4a_kernel(co
         XI16[c >> 1] = isum;
         XS16[c >> 1] = sum;
       }
-      // a group holding inf / nan keeps them: the scale carries the non-finite value into the sum
-      if ((c & 3) == 0) SG[c >> 2] = finite ? amax * (1.f / 32767.f) : (amax > 0.f ? amax : 0.f);
+      if ((c & 3) == 0) SG[c >> 2] = unit.scale;
     }
   }
   __syncthreads();
@@ -607,6 +639,7 @@ __global__ void __launch_bounds__(kThreads, MT == 1 ? 3 : 2) gemv_dp4a_kernel(co
 #pragma unroll
   for (int t = 0; t < MT; t++) red[warp][t][lane] = y[t];
   __syncthreads();
+  bool bad = false;
   for (int idx = threadIdx.x; idx < MT * kRows; idx += kThreads) {
     const int t = idx / kRows, r = idx % kRows, n = row0 + r * rstep;
     if (t < m && n < a.N) {
@@ -619,12 +652,14 @@ __global__ void __launch_bounds__(kThreads, MT == 1 ? 3 : 2) gemv_dp4a_kernel(co
 #pragma unroll
       for (int u = 1; u < MT; u++)
         if (t == u) yrow = yr[u];
+      bad |= !(fabsf(sum) < INFINITY);
       OT* out = static_cast<OT*>(a.y) + (long long)yrow * a.y_row_stride + n;
       if (a.bias != nullptr) sum += (float)static_cast<const OT*>(a.bias)[n];
       if constexpr (std::is_same<OT, __half>::value) *out = __float2half_rn(sum);
       else *out = __float2bfloat16_rn(sum);
     }
   }
+  if (__syncthreads_or(bad)) dp_again<C, XT, OT>(a, row0, rstep, kRows, MT);
 }
 
 // Parts of K in a warp: two, i.e. sixteen rows a CTA, where thirty-two rows leave SMs with one CTA or none.

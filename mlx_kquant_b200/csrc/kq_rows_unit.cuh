@@ -382,28 +382,10 @@ __device__ __forceinline__ void rows_sums(const uint8_t* xrow, float* out, int l
   }
 }
 
-// One output by itself: decoded weights times activations in float32, as the generic kernel has it. For outputs that
-// the split into integers, offsets and sub-block sums leaves without a finite value although they may have one, or an
-// infinity: an infinite activation meets the offset's sum (inf - inf), and a sum of integers can overflow before its
-// scale is applied. Rare, so one thread an output, without care for speed.
+// plain_dot (kq_common.cuh) with what is known of the alignment of these codecs' rows here
 template <int C, typename XT>
 __device__ __noinline__ float rows_plain(const uint8_t* w, const XT* x, int nsb) {
-  constexpr int A = rw_al16(C) ? 16 : (C == IQ4_XS ? 8 : 2);
-  const IqTables tabs = global_iq_tables();
-  float sum = 0.f;
-#pragma unroll 1
-  for (int o = 0; o < 32 * nsb; o++) {
-    float v[8];
-    decode8<C, A>(w + (long long)(o >> 5) * bpb_of(C), o & 31, v, tabs);
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      float xv;
-      if constexpr (std::is_same<XT, __half>::value) xv = __half2float(x[8 * o + i]);
-      else xv = __bfloat162float(x[8 * o + i]);
-      sum = fmaf(xv, v[i], sum);
-    }
-  }
-  return sum;
+  return plain_dot<C, rw_al16(C) ? 16 : (C == IQ4_XS ? 8 : 2)>(w, x, 256 * nsb);
 }
 
 }  // namespace
