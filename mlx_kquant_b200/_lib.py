@@ -8,6 +8,7 @@ CUDA kernels.
 from __future__ import annotations
 
 import ctypes as C
+import warnings
 from pathlib import Path
 
 HERE = Path(__file__).resolve().parent
@@ -107,26 +108,40 @@ def lib() -> C.CDLL:
     return _lib
 
 
-_front = None
+_front = None  # the module, or False where there is none that can be used
 
 
 def torch_front():
-    """The native front of quantized_matmul (csrc/kq_torch.cpp), or None where it was not built."""
+    """The native front of quantized_matmul (csrc/kq_torch.cpp), or None where it was not built, or not for this torch: the
+    library itself does not know torch, and every product works without the front, through ctypes."""
     global _front
     if _front is None:
-        path = HERE / "_kq_torch.so"
-        if not path.exists():
-            return None
-        import importlib.util
+        _front = _load_front(HERE / "_kq_torch.so") or False
+    return _front or None
 
-        spec = importlib.util.spec_from_file_location("_kq_torch", path)
+
+def _load_front(path):
+    if not path.exists():
+        return None
+    import importlib.util
+
+    import torch
+
+    spec = importlib.util.spec_from_file_location("_kq_torch", path)
+    try:
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
-        handle = lib()
-        module.init(*[C.cast(getattr(handle, name), C.c_void_p).value for name in
-                      ("kq_codec_find", "kq_codec_info", "kq_quantized_matmul_workspace_bytes", "kq_quantized_matmul")])
-        _front = module
-    return _front
+        built_for = getattr(module, "torch_version", "of another version")
+        if built_for != torch.__version__:
+            raise ImportError(f"built for torch {built_for}, this is {torch.__version__}")
+    except (ImportError, OSError) as e:
+        warnings.warn(f"mlx_kquant_b200: {path.name} is not used ({e}); build it again with make -C {HERE / 'csrc'}. "
+                      "Products of a few rows take some microseconds more of host time without it.", RuntimeWarning, stacklevel=4)
+        return None
+    handle = lib()
+    module.init(*[C.cast(getattr(handle, name), C.c_void_p).value for name in
+                  ("kq_codec_find", "kq_codec_info", "kq_quantized_matmul_workspace_bytes", "kq_quantized_matmul")])
+    return module
 
 
 def check(rc: int) -> None:

@@ -98,4 +98,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_kq_torch", nullptr, -1, methods, 
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__kq_torch() { return PyModule_Create(&module); }
+// torch_version: of the torch that this was compiled against, whose classes it takes apart; _lib.py uses it with no other
+PyMODINIT_FUNC PyInit__kq_torch() {
+  PyObject* m = PyModule_Create(&module);
+  if (m != nullptr && PyModule_AddStringConstant(m, "torch_version", KQ_TORCH_VERSION) != 0) Py_CLEAR(m);
+  return m;
+}

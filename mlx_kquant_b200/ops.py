@@ -166,12 +166,15 @@ def _expanded_inner(w, kquant_type, op):
     return w.shape[-1] // bpb * wpb
 
 
-def _front_qmm(x, w, kquant_type, transpose):
-    """The first call: the native front takes this name, or a stand-in where there is none."""
+def _first_qmm(x, w, kquant_type, transpose):
+    """The first call of _front_qmm: the native front takes its place, or a stand-in where there is none."""
     global _front_qmm
     front = _lib.torch_front()
     _front_qmm = front.qmm if front is not None else lambda *args: None
     return _front_qmm(x, w, kquant_type, transpose)
+
+
+_front_qmm = _first_qmm
 
 
 def quantized_matmul(x, w, scales, kquant_type, transpose=True, *, stream=None):
