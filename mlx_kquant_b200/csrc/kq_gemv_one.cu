@@ -29,6 +29,8 @@ namespace {
 
 constexpr int kOneWarps = 12, kOneThreads = 32 * kOneWarps, kOneSlots = 4, kOneBlocks = 16;
 constexpr int kOneMaxK = 16384, kOneSmem = 222 * 1024;
+// the least maximum that a scale is made for: 32767 / amax stays finite
+constexpr float kOneLeast = 0x1p-112f;
 // bytes of a box row: the superblock, for q6_k the aligned window around it
 __host__ __device__ constexpr int one_pitch(int c) { return c == Q4_K ? 144 : (c == Q5_K ? 176 : 240); }
 // XH [K] | XL [K] | scale per 32 [K / 32] | integer sums per 16 [K / 16] | float sums per 32 [K / 32]
@@ -168,7 +170,7 @@ gemv_one_kernel(const GemvArgs a, const OnePlan pl, const __grid_constant__ CUte
   constexpr int kPitch = one_pitch(C), kBlk = bpb_of(C);
   extern __shared__ __align__(128) uint8_t one_dyn[];
   __shared__ uint64_t full[kOneWarps][kOneSlots];
-  __shared__ int abort_s, huge_s;
+  __shared__ int abort_s;
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int K = a.K, nsb = K >> 8, D = pl.D;
@@ -178,7 +180,7 @@ gemv_one_kernel(const GemvArgs a, const OnePlan pl, const __grid_constant__ CUte
     for (int d = 0; d < D; d++) mbar_init(&full[warp][d], 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  if (threadIdx.x == 0) abort_s = huge_s = 0;
+  if (threadIdx.x == 0) abort_s = 0;
   __syncwarp();
   uint8_t* ring = one_dyn + warp * D * pl.slot;
   float(*red)[kOneWarps][32] = reinterpret_cast<float(*)[kOneWarps][32]>(one_dyn + pl.red_off);  // [block]
@@ -249,9 +251,8 @@ gemv_one_kernel(const GemvArgs a, const OnePlan pl, const __grid_constant__ CUte
       top = max(top, __shfl_xor_sync(0xffffffffu, top, 2));
       sum += __shfl_xor_sync(0xffffffffu, sum, 1);
       sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-      const float amax = __uint_as_float(top);
       const bool finite = top > 0 && top < 0x7f800000u;
-      if (top >= 0x5f000000u) huge_s = 1;  // 2^63
+      const float amax = finite ? fmaxf(__uint_as_float(top), kOneLeast) : __uint_as_float(top);
       const float inv = finite ? 32767.f * __frcp_rn(amax) : 0.f;
       int xi[8], isum = 0;
       uint32_t h[2], l[2];
@@ -272,19 +273,13 @@ gemv_one_kernel(const GemvArgs a, const OnePlan pl, const __grid_constant__ CUte
       if ((c & 1) == 0) XI[c >> 1] = isum;
       if ((c & 3) == 0) {
         XS[c >> 2] = sum;
-        // a group holding inf / nan keeps them: the scale carries the non-finite value into the sum
+        // a group holding inf / nan: its integers are zeros, and zero times the scale makes every output a NaN, which is
+        // computed again below
         SG[c >> 2] = finite ? amax * (1.f / 32767.f) : amax;
       }
     }
   }
   __syncthreads();
-  // Sub-block scales and sums come before the superblock's scale, which is small: activations beyond 2^63 are taken by 2^-64,
-  // the outputs by 2^64.
-  const bool huge = huge_s != 0;
-  if (huge) {
-    for (int i = threadIdx.x; i < K / 32; i += kOneThreads) SG[i] *= 0x1p-64f, XS[i] *= 0x1p-64f;
-    __syncthreads();
-  }
 
   volatile int* abort_flag = &abort_s;
   float y = 0.f;
@@ -325,7 +320,9 @@ gemv_one_kernel(const GemvArgs a, const OnePlan pl, const __grid_constant__ CUte
     float sum = 0.f;
 #pragma unroll
     for (int w = 0; w < kOneWarps; w++) sum += red[b][w][r];
-    if (huge) sum *= 0x1p64f;
+    // Infinities and NaN among the activations; and the sums of 32 activations and the sub-blocks' scales come before the
+    // superblock's scale, which is small, and can overflow for the largest of them.
+    if (!(fabsf(sum) < INFINITY)) sum = plain_dot<C, C == Q6_K ? 2 : 16>(a.w + (long long)n * a.row_bytes, xrow, K);
     OT* out = static_cast<OT*>(a.y) + n;
     if constexpr (std::is_same<OT, __half>::value) *out = __float2half_rn(sum);
     else *out = __float2bfloat16_rn(sum);

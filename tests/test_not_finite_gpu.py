@@ -87,6 +87,14 @@ def test_dot_product_kernels(codec, m, n, k, dt):
     check(codec, m, n, k, dt)
 
 
+# kq_gemv_one.cu
+@pytest.mark.parametrize("codec,n,k", [("q4_k", 70, 8192), ("q4_k", 6200, 4096), ("q5_k", 1030, 2048), ("q5_k", 40, 8448),
+                                       ("q6_k", 1030, 2048), ("q6_k", 90, 14336)])
+@pytest.mark.parametrize("dt", ["f16", "bf16", "f32"])
+def test_one_row(codec, n, k, dt):
+    check(codec, 1, n, k, dt)
+
+
 @pytest.mark.parametrize("codec", ["q2_k", "q3_k", "q8_0", "q4_0"])
 def test_task_lists(codec):
     """gather_qmm of a few rows an expert: the same kernels over task lists."""
