@@ -314,6 +314,12 @@ gemv_one_kernel(const GemvArgs a, const OnePlan pl, const __grid_constant__ CUte
   }
   red[blk][warp][lane] = y;
   __syncthreads();
+  if (abort_s != 0) {  // given up: no outputs; what is in flight lands long before this
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 1000000ull) {
+    }
+    return;
+  }
   for (int i = threadIdx.x; i < blocks * pl.R; i += kOneThreads) {
     const int b = i / pl.R, r = i - b * pl.R, n = row0 + i;
     if (n >= a.N) continue;
