@@ -461,8 +461,9 @@ cudaError_t launch_few_x(int codec, const GemvArgs& a, cudaStream_t st) {
 
 bool gemv_few_supported(int codec, int x_dtype, const GemvArgs& a) {
   if (codec != Q4_K && codec != Q5_K && codec != Q6_K && codec != IQ4_XS) return false;
+  // (half of a longer row would not fit into shared memory, and few_plan counts bytes in int)
   if (!(x_dtype == F16 || x_dtype == BF16) || a.tasks != nullptr || a.bias != nullptr || a.M < 1 || a.M > 16 || a.N < 8 ||
-      a.K < 256 || (a.K & 255) != 0 || a.w_align16 == 0 || a.row_bytes != (long long)(a.K >> 8) * bpb_of(codec))
+      a.K < 256 || a.K > (1 << 18) || (a.K & 255) != 0 || a.w_align16 == 0 || a.row_bytes != (long long)(a.K >> 8) * bpb_of(codec))
     return false;
   if ((reinterpret_cast<uintptr_t>(a.x) & 15) != 0 || (a.x_row_stride & 7) != 0) return false;
   const long long size = (long long)a.N * a.K;

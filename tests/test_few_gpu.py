@@ -55,3 +55,21 @@ def test_not_finite(codec):
     big = torch.zeros_like(x)
     big[0, 7] = 1e38
     assert torch.isfinite(kq.quantized_matmul(big, w, None, codec)).all()
+
+
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
+def test_rows_too_long_to_count_in_int(dt):
+    """Sixteen rows of 2^26 are 2^31 bytes: more than any shared memory, and the table kernel has them."""
+    k, n, m = 1 << 26, 8, 16
+    g = torch.Generator().manual_seed(1)
+    pool = kq.quantize(torch.randn(256, 256, generator=g) * k ** -0.5, "iq4_xs", None)[0].cuda()
+    w = pool[torch.randint(0, 256, (n, k // 256), generator=g).cuda()].reshape(n, -1)
+    x = torch.randn(m, k, device="cuda", dtype=torch.float16 if dt == "f16" else torch.bfloat16)
+    y = kq.quantized_matmul(x, w, None, "iq4_xs").double()
+    ref = torch.zeros(m, n, dtype=torch.float64, device="cuda")
+    step = 1 << 22
+    for k0 in range(0, k, step):
+        d = kq.dequantize(w[:, k0 // 256 * 136:(k0 + step) // 256 * 136].contiguous(), None, "iq4_xs", torch.float32)
+        ref += x[:, k0:k0 + step].double() @ d.double().T
+    # half a unit of the output, and float32 sums of 2^26 terms in eight or more parts: 2^-24 sqrt(2^26) of their size at most
+    assert float((y - ref).norm() / ref.norm()) < (2.0 ** -11 if dt == "f16" else 2.0 ** -8) + 2.0 ** -11
