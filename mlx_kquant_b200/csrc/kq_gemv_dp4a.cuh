@@ -9,7 +9,7 @@
 // and the inner sums run on dp4a once the activations are integers too: each 32-group of x is
 // quantized once per CTA to 16 bits with the group's own scale (xi = rint(x * 32767 / max|x|),
 // |error| <= 2^-16 of the group maximum - far below the fp16 / bf16 rounding the activations
-// already carry) and stored as two int8 planes (xi = 256 xh + xl). A few logic ops unpack FOUR
+// already carry; ragged rows: x_unit) and stored as two int8 planes (xi = 256 xh + xl). A few logic ops unpack FOUR
 // weights into one register, one dp4a per plane multiplies them; integer sums are exact, scales are
 // applied in fp32 per 16- or 32-weight sub-group. "- off" costs nothing: off * sum_k xi is taken
 // from the per-16 integer sums of x.
@@ -392,17 +392,29 @@ __host__ __device__ static inline int x_bytes(int K) { return 2 * K + (K / 32) *
 template <int C>
 int dyn_smem(int K, int D, int MT) { return kWarps * D * slot_bytes<C>() + MT * x_bytes(K); }
 
-// The scale of a 32-group whose largest magnitude has these bits, and its inverse, which stays finite: for the smallest groups
-// the scale is 2^-112 / 32767, half the smallest normal number. A group with an infinity or a NaN, which order above all numbers
-// as bits, becomes zeros with that as the scale: zero times it makes every output NaN, and dp_again makes them again.
+// The scale of a 32-group whose largest magnitude has these bits, and its inverse, which stays finite (for the smallest groups
+// the scale is half the smallest normal number). POW2: a power of two, the largest becomes 2^14 to 2^15 - 1, and what has no
+// bits below the unit stays exact: bf16 down to 2^-7 of the largest, fp16 down to 2^-4. For rows that are no whole sixteens,
+// whose activations the kernel before (kq_gemv.cu) took unrounded: errors beyond the output's rounding, q6_k [5120, 5120] x 1
+// bf16, 0.18e-5 of the outputs' size there, 1.9e-5 with 32767 / largest, 0.24e-5 so; fp16 20e-5 there (weights in fp16), 2.1e-5,
+// 1.1e-5. The others keep 32767 / largest, which is up to twice as fine where one activation dwarfs the rest of its 32.
+// A group with an infinity or a NaN, which order above all numbers as bits, becomes zeros with that as the scale: zero times it
+// makes every output NaN, and dp_again makes them again.
 struct XUnit {
   float inv, scale;
 };
+template <bool POW2>
 __device__ __forceinline__ XUnit x_unit(uint32_t top) {
-  const float amax = fmaxf(__uint_as_float(top), 0x1p-112f);
   XUnit u;
-  u.inv = 32767.f * __frcp_rn(amax);
-  u.scale = amax * (1.f / 32767.f);
+  if constexpr (POW2) {
+    const uint32_t e = max(top & 0x7f800000u, 14u << 23);  // exponent of the largest, -113 at least
+    u.inv = __uint_as_float((268u << 23) - e);             // 2^(14 - exponent)
+    u.scale = __uint_as_float(e) * 0x1p-14f;
+  } else {
+    const float amax = fmaxf(__uint_as_float(top), 0x1p-112f);
+    u.inv = 32767.f * __frcp_rn(amax);
+    u.scale = amax * (1.f / 32767.f);
+  }
   if (top >= 0x7f800000u) u.inv = 0.f, u.scale = __uint_as_float(top);
   return u;
 }
@@ -558,7 +570,7 @@ __global__ void __launch_bounds__(kThreads, MT == 1 ? 3 : 2) gemv_dp4a_kernel(co
       top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));
       top = max(top, __shfl_xor_sync(0xffffffffu, top, 2));
       sum += __shfl_xor_sync(0xffffffffu, sum, 1);  // 16-group
-      const XUnit unit = x_unit(top);
+      const XUnit unit = x_unit<!ROWA>(top);
       int xi[8], isum = 0;
 #pragma unroll
       for (int i = 0; i < 8; i++) {
