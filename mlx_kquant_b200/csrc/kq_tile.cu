@@ -1006,7 +1006,18 @@ bool tile_supported(int codec, const uint8_t* w, long long row_bytes, int N, int
 }
 
 double tile_cycles(int codec, bool half_weights, int M, int N, int K) {
-  return pick_shape(half_weights ? kSrcHalf : (codec == Q4_K ? kSrcQ4K : kSrcQ6K), M, N, K).cycles;
+  const TileShape sh = pick_shape(half_weights ? kSrcHalf : (codec == Q4_K ? kSrcQ4K : kSrcQ6K), M, N, K);
+  // Rows that are no whole sixteens leave the accumulator in classes and are put right output by output, 60 cycles a token.
+  // Where the choice between producers and copy left that out, q6_k [28672, 512] x 620 took 78 us with producers (copy 45.5),
+  // [20000, 1024] x 620 69 (47), [8192, 3072] x 1500 88 (69). (In the choice of the shape it does not help: [8192, 3072] x 125
+  // 20.7 -> 23.6.)
+  double sorting = 0.0;
+  if (!half_weights && sh.ks == 1 && row_group((long long)(K >> 8) * bpb_of(codec)) != 0) {
+    const long long tiles = (long long)((N + 128 * sh.cg - 1) / (128 * sh.cg)) * ((M + sh.tn - 1) / sh.tn);
+    const int units = std::max(1, resident_ctas(sh.cg) / sh.cg);
+    sorting = 60.0 * sh.tn * (double)((tiles + units - 1) / units);
+  }
+  return sh.cycles + sorting;
 }
 
 cudaError_t launch_tile(int codec, bool half_weights, bool out_half, const TileArgs& t, cudaStream_t st) {

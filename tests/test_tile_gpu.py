@@ -49,6 +49,16 @@ def test_shapes(codec, m, n, k, dt):
     check(kq.quantized_matmul(x, torch.from_numpy(some[pick]).cuda(), None, codec), ref, dt)
 
 
+# rows in groups of eight, four and two: with producers (few rows) and by the fp16 copy (many)
+@pytest.mark.parametrize("m,n,k", [(70, 6000, 768), (300, 6000, 768), (620, 8200, 512), (130, 8200, 512), (300, 4100, 1536), (700, 4098, 1024)])
+def test_q6k_rows_in_classes(m, n, k):
+    rng, some = some_rows("q6_k", k, m + n + k)
+    pick = rng.integers(0, 64, n)
+    x, _ = x_to_torch(rng.standard_normal((m, k)).astype(np.float32), "bf16")
+    ref = (x.double().cpu().numpy() @ Oracle().dequantize(some, "q6_k", "f32").astype(np.float64).T)[:, pick]
+    check(kq.quantized_matmul(x, torch.from_numpy(some[pick]).cuda(), None, "q6_k"), ref, "bf16")
+
+
 @pytest.mark.parametrize("n", [1001, 1002, 1004])
 def test_q6k_rows_that_do_not_fill_a_class(n):
     """Wire rows in groups of eight, and a number of rows that is no multiple: another kernel, the same result."""
