@@ -58,3 +58,46 @@ def mint_wire(codec: str, W: np.ndarray, imatrix=None) -> np.ndarray:
         im = torch.from_numpy(imatrix) if imatrix is not None else (torch.ones(W.shape[-1]) if GEOMETRY[codec][3] else None)
         return kq.quantize(torch.from_numpy(np.ascontiguousarray(W, np.float32)), codec, im)[0].numpy()
     return synthetic_wire(codec, W.shape[0], W.shape[1], seed=int(abs(W[0, 0]) * 1e6) % 9973)
+
+
+def kernels(call) -> list[str]:
+    """Mangled names of the kernels that `call` launches, in some order: it is captured into a graph, which is not run."""
+    import ctypes as C
+
+    call()   # (what is set up once is no part of a capture)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+        call()
+    cu = C.CDLL("libcuda.so.1")
+
+    def ok(rc):
+        assert rc == 0, f"driver call: {rc}"
+
+    raw, count = C.c_void_p(int(graph.raw_cuda_graph())), C.c_size_t(0)
+    ok(cu.cuGraphGetNodes(raw, None, C.byref(count)))
+    nodes = (C.c_void_p * count.value)()
+    ok(cu.cuGraphGetNodes(raw, nodes, C.byref(count)))
+
+    class Params(C.Structure):   # CUDA_KERNEL_NODE_PARAMS of version 2
+        _fields_ = [("func", C.c_void_p), ("shape", C.c_uint * 7), ("params", C.c_void_p), ("extra", C.c_void_p),
+                    ("kern", C.c_void_p), ("ctx", C.c_void_p), ("room", C.c_uint64 * 8)]
+    names = []
+    for node in nodes:
+        kind = C.c_int()
+        ok(cu.cuGraphNodeGetType(C.c_void_p(node), C.byref(kind)))
+        if kind.value != 0:   # CU_GRAPH_NODE_TYPE_KERNEL
+            continue
+        p, name = Params(), C.c_char_p()
+        ok(cu.cuGraphKernelNodeGetParams_v2(C.c_void_p(node), C.byref(p)))
+        ok(cu.cuFuncGetName(C.byref(name), C.c_void_p(p.func)) if p.func else cu.cuKernelGetName(C.byref(name), C.c_void_p(p.kern)))
+        names.append(name.value.decode())
+    return names
+
+
+def product_kernels(codec: str, m: int, n: int, k: int, dt: str) -> str:
+    """The kernels that x [m, k] . w [n, k]^T launches, one string."""
+    wpb, bpb = GEOMETRY[codec][0], GEOMETRY[codec][1]
+    x = torch.zeros(m, k, dtype=TORCH_DT[dt], device="cuda")
+    w = torch.zeros(n, k // wpb * bpb, dtype=torch.uint8, device="cuda")
+    return " ".join(kernels(lambda: kq.quantized_matmul(x, w, None, codec)))

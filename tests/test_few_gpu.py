@@ -4,7 +4,7 @@ import pytest
 import torch
 
 import mlx_kquant_b200 as kq
-from gpu_util import x_to_torch, y_to_f32
+from gpu_util import product_kernels, x_to_torch, y_to_f32
 from oracle.kq_oracle import Oracle
 
 pytestmark = pytest.mark.gpu
@@ -30,12 +30,15 @@ def check(y, ref, dt):
 # the edges: fewer rows than a tile; a last row block of a few rows; row blocks of several tiles, shares that end inside one;
 # several row blocks a CTA; one and two column tiles, odd columns; activations that need a pair of CTAs, with an odd number of
 # superblocks too; iq4_xs in rows that are no whole sixteens
-@pytest.mark.parametrize("codec,m,n,k", [
+CASES = [
     ("q4_k", 2, 8, 4096), ("q4_k", 3, 1200, 4096), ("q4_k", 8, 2367, 4352), ("q4_k", 9, 4099, 4096), ("q4_k", 16, 2368, 4096),
     ("q4_k", 5, 40001, 1024), ("q4_k", 6, 300, 14336), ("q4_k", 16, 999, 8448), ("q5_k", 7, 2000, 5120), ("q5_k", 13, 150, 4096),
     ("q5_k", 8, 777, 8192), ("q6_k", 2, 4097, 4096), ("q6_k", 4, 1111, 8192), ("q6_k", 8, 9000, 6144), ("q6_k", 2, 500, 14336),
     ("iq4_xs", 1, 100, 4096), ("iq4_xs", 1, 20000, 256), ("iq4_xs", 4, 4001, 2304), ("iq4_xs", 16, 2500, 2304),
-    ("iq4_xs", 15, 1300, 5376), ("iq4_xs", 8, 700, 8448), ("iq4_xs", 2, 60, 16384), ("iq4_xs", 8, 77, 4352)])
+    ("iq4_xs", 15, 1300, 5376), ("iq4_xs", 8, 700, 8448), ("iq4_xs", 2, 60, 16384), ("iq4_xs", 8, 77, 4352)]
+
+
+@pytest.mark.parametrize("codec,m,n,k", CASES)
 @pytest.mark.parametrize("dt", ["f16", "bf16"])
 def test_few_rows(codec, m, n, k, dt):
     x, w, ref = product(codec, m, n, k, dt, n + k)
@@ -73,3 +76,19 @@ def test_rows_too_long_to_count_in_int(dt):
         ref += x[:, k0:k0 + step].double() @ d.double().T
     # half a unit of the output, and float32 sums of 2^26 terms in eight or more parts: 2^-24 sqrt(2^26) of their size at most
     assert float((y - ref).norm() / ref.norm()) < (2.0 ** -11 if dt == "f16" else 2.0 ** -8) + 2.0 ** -11
+
+
+# the longest sixteen rows of q4_k that a pair of CTAs has room for, and fifteen with an odd number of superblocks; one
+# superblock more with sixteen and the rows kernel has them
+@pytest.mark.parametrize("codec,m,n,k,few", [c + (c != ("q4_k", 16, 999, 8448),) for c in CASES] + [("q4_k", 16, 999, 8192, True),
+                                                                                                 ("q4_k", 15, 999, 8448, True)])
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
+def test_which_kernel(codec, m, n, k, few, dt):
+    assert ("few_kernel" if few else "rows_kernel") in product_kernels(codec, m, n, k, dt)
+
+
+@pytest.mark.parametrize("m,k", [(16, 8192), (15, 8448)])
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
+def test_pairs_of_two_column_tiles(m, k, dt):
+    x, w, ref = product("q4_k", m, 999, k, dt, m + k)
+    check(kq.quantized_matmul(x, w, None, "q4_k"), ref, dt)

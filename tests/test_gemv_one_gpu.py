@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import mlx_kquant_b200 as kq
-from gpu_util import x_to_torch, y_to_f32
+from gpu_util import product_kernels, x_to_torch, y_to_f32
 from oracle.kq_oracle import Oracle
 
 pytestmark = pytest.mark.gpu
@@ -32,9 +32,12 @@ def check(y, ref, dt):
 
 # one block and several a CTA, rows that leave the last one short, fewer rows than SMs; superblocks fewer and more than warps
 # x slots, and the longest row; q6_k's K are multiples of 2048 here (whole sixteens)
-@pytest.mark.parametrize("codec,n,k", [("q4_k", 12300, 2048), ("q4_k", 33, 8192), ("q4_k", 1537, 16384), ("q4_k", 20001, 4096),
+CASES = [("q4_k", 12300, 2048), ("q4_k", 33, 8192), ("q4_k", 1537, 16384), ("q4_k", 20001, 4096),
                                        ("q5_k", 1024, 2048), ("q5_k", 5001, 768), ("q5_k", 90, 8448), ("q5_k", 14336, 256),
-                                       ("q6_k", 1025, 2048), ("q6_k", 4800, 4096), ("q6_k", 77, 14336), ("q6_k", 9999, 2048)])
+                                       ("q6_k", 1025, 2048), ("q6_k", 4800, 4096), ("q6_k", 77, 14336), ("q6_k", 9999, 2048)]
+
+
+@pytest.mark.parametrize("codec,n,k", CASES)
 @pytest.mark.parametrize("dt", ["f16", "bf16", "f32"])
 def test_one_row(codec, n, k, dt):
     x, w, ref = product(codec, 1, n, k, dt, n + k)
@@ -55,9 +58,12 @@ def test_not_finite(codec):
 
 
 # rows of 2, 4 and 8 bytes past a sixteen: one to four of them, odd numbers of rows (a last block of one parity alone)
-@pytest.mark.parametrize("codec,m,n,k", [("q6_k", 1, 1001, 2304), ("q6_k", 1, 63, 5120), ("q3_k", 1, 1000, 1280), ("q3_k", 2, 31, 768),
-                                         ("q3_k", 4, 515, 1536), ("q2_k", 1, 400, 1536), ("q2_k", 3, 97, 256), ("iq4_xs", 1, 333, 2304),
-                                         ("iq2_xxs", 1, 20000, 2816), ("q6_k", 3, 129, 1280), ("q3_k", 1, 4100, 256)])
+RAGGED = [("q6_k", 1, 1001, 2304), ("q6_k", 1, 63, 5120), ("q3_k", 1, 1000, 1280), ("q3_k", 2, 31, 768),
+          ("q3_k", 4, 515, 1536), ("q2_k", 1, 400, 1536), ("q2_k", 3, 97, 256), ("iq4_xs", 1, 333, 2304),
+          ("iq2_xxs", 1, 20000, 2816), ("q6_k", 3, 129, 1280), ("q3_k", 1, 4100, 256)]
+
+
+@pytest.mark.parametrize("codec,m,n,k", RAGGED)
 @pytest.mark.parametrize("dt", ["f16", "f32"])
 def test_ragged_rows(codec, m, n, k, dt):
     x, w, ref = product(codec, m, n, k, dt, n + k)
@@ -107,3 +113,16 @@ def test_fp16_rows_of_large_q4_k(n, k):
         beyond += float((y - ref).square().sum() - (ref.half().double() - ref).square().sum())
         size += float(ref.square().sum())
     assert beyond < 3e-5 ** 2 * size
+
+
+@pytest.mark.parametrize("codec,n,k", CASES + [("q4_k", 8192, 8192), ("q4_k", 15400, 4096)])
+@pytest.mark.parametrize("dt", ["f16", "bf16", "f32"])
+def test_which_kernel(codec, n, k, dt):
+    assert "gemv_one_kernel" in product_kernels(codec, 1, n, k, dt)
+
+
+# (three rows of q6_k: the rows kernel takes them, ragged or not)
+@pytest.mark.parametrize("codec,m,n,k", RAGGED)
+@pytest.mark.parametrize("dt", ["f16", "bf16", "f32"])
+def test_which_kernel_has_ragged_rows(codec, m, n, k, dt):
+    assert ("rows_kernel" if (codec, m) == ("q6_k", 3) else "gemv_dp4a_kernel") in product_kernels(codec, m, n, k, dt)

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import mlx_kquant_b200 as kq
-from gpu_util import x_to_torch, y_to_f32
+from gpu_util import product_kernels, x_to_torch, y_to_f32
 from oracle.kq_oracle import Oracle
 
 pytestmark = pytest.mark.gpu
@@ -88,8 +88,11 @@ def test_dot_product_kernels(codec, m, n, k, dt):
 
 
 # kq_gemv_one.cu
-@pytest.mark.parametrize("codec,n,k", [("q4_k", 70, 8192), ("q4_k", 6200, 4096), ("q5_k", 1030, 2048), ("q5_k", 40, 8448),
-                                       ("q6_k", 1030, 2048), ("q6_k", 90, 14336)])
+ONE = [("q4_k", 70, 8192), ("q4_k", 6200, 4096), ("q5_k", 1030, 2048), ("q5_k", 40, 8448),
+       ("q6_k", 1030, 2048), ("q6_k", 90, 14336)]
+
+
+@pytest.mark.parametrize("codec,n,k", ONE)
 @pytest.mark.parametrize("dt", ["f16", "bf16", "f32"])
 def test_one_row(codec, n, k, dt):
     check(codec, 1, n, k, dt)
@@ -113,3 +116,10 @@ def test_task_lists(codec):
         inf = np.isinf(ref)
         assert np.array_equal(np.isnan(y[at]), np.isnan(ref)) and np.array_equal(y[at][inf], ref[inf])
         assert np.isfinite(np.delete(y, at, 0)).all()
+
+
+@pytest.mark.parametrize("codec,m,n,k,name", [c + ("gemv_dp4a_kernel",) for c in RAGGED + WHOLE] +
+                         [(c, 1, n, k, "gemv_one_kernel") for c, n, k in ONE])
+@pytest.mark.parametrize("dt", ["f16", "bf16", "f32"])
+def test_which_kernel(codec, m, n, k, name, dt):
+    assert name in product_kernels(codec, m, n, k, dt)

@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import mlx_kquant_b200 as kq
-from gpu_util import x_to_torch, y_to_f32
+from gpu_util import product_kernels, x_to_torch, y_to_f32
 from mlx_kquant_b200 import _lib
 from oracle.kq_oracle import Oracle
 
@@ -50,7 +50,10 @@ def test_shapes(codec, m, n, k, dt):
 
 
 # rows in groups of eight, four and two: with producers (few rows) and by the fp16 copy (many)
-@pytest.mark.parametrize("m,n,k", [(70, 6000, 768), (300, 6000, 768), (620, 8200, 512), (130, 8200, 512), (300, 4100, 1536), (700, 4098, 1024)])
+CLASSES = [(70, 6000, 768), (300, 6000, 768), (620, 8200, 512), (130, 8200, 512), (300, 4100, 1536), (700, 4098, 1024)]
+
+
+@pytest.mark.parametrize("m,n,k", CLASSES)
 def test_q6k_rows_in_classes(m, n, k):
     rng, some = some_rows("q6_k", k, m + n + k)
     pick = rng.integers(0, 64, n)
@@ -117,3 +120,18 @@ def test_q6k_weights_are_rounded_once(rows):
     bits = lambda v: (v + 0.0).view(torch.int16).int()  # (a weight of zero has the scale's sign or none)
     off = (bits(y) - bits(ref)).abs()
     assert int(off.max()) <= 1 and float((off > 0).float().mean()) < 0.02
+
+
+@pytest.mark.parametrize("codec", ["q4_k", "q6_k"])
+@pytest.mark.parametrize("m,n,k", SHAPES + CLASSES)
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
+def test_which_kernel(codec, m, n, k, dt):
+    names = product_kernels(codec, m, n, k, dt)
+    assert "tile_kernel" in names and (codec != "q4_k" or "dequant_kernel" not in names)
+    if codec == "q6_k" and (m, n, k) in CLASSES:   # few rows: producers, many: the copy
+        assert ("dequant_kernel" in names) == (m > 600)
+
+
+@pytest.mark.parametrize("n", [1001, 1002, 1004])
+def test_which_kernel_has_rows_that_do_not_fill_a_class(n):
+    assert "gemm_kernel" in product_kernels("q6_k", 33, n, 1280, "bf16")
