@@ -104,14 +104,21 @@ KQ_API int kq_quantize_cpu(const void* w, int w_dtype, long long n_weights, long
  *    most 4 M weights whose rows are not whole numbers of 16 bytes: up to several times
  *    faster; values below 2^-32 of their row's largest lose bits), and so do bf16 rows
  *    of q4_k matrices with fewer than eight rows; a call without it still works.
- *  - w: written before the launch that comes ahead of this call in the stream. With one
- *    row, and for some codecs up to sixteen, the kernels start to read weights while
- *    that launch may still be running (programmatic dependent launch). After a kernel
- *    that writes weights, another launch has to come first. */
+ *  - w: written before the launch that comes ahead of this call in the stream. Kernels
+ *    that start to read weights while that launch may still be running (programmatic
+ *    dependent launch): one row of every codec that has an integer kernel (q2_k .. q6_k,
+ *    q4_0, q4_1, q5_0, q5_1, q8_0, iq4_nl, iq4_xs, iq2_xxs), two to four rows of q2_k,
+ *    q3_k, q4_0, q4_1, q5_0, q5_1, q8_0, iq4_nl and of float32 rows of q4_k, q5_k, q6_k
+ *    without a workspace, two to sixteen rows of iq4_xs and iq2_xxs, and of fp16 q4_k
+ *    with fewer than eight weight rows. All others wait first. This matters only for a
+ *    launch that allows its successor to start early: an ordinary kernel, copy or memset
+ *    has ended by then. After one that writes weights and does allow it, another launch
+ *    has to come first. */
 KQ_API size_t kq_quantized_matmul_workspace_bytes(int x_dtype, long long rows, int K);
 /* The same with room for an fp16 copy of (a part of) the weights, of at most 128 MiB or 256 rows, where [N, K] products
- * of that many rows are faster from one: more than 16 rows on matrices of 4 M weights and more of every codec but q4_k
- * (q6_k with K a multiple of 1024: more than 256 rows). A call that is given only the bytes above works without it. */
+ * of that many rows may be faster from one: more than 16 rows on matrices of 4 M weights and more of every codec but q4_k
+ * (q6_k with K a multiple of 1024: more than 256 rows, and there and with other K by an estimate of both ways). A call that
+ * is given only the bytes above works without it. */
 KQ_API size_t kq_quantized_matmul_workspace_bytes_for(const char* kquant_type, int x_dtype, long long rows, int N, int K);
 KQ_API int kq_quantized_matmul(const void* x, int x_dtype, long long rows, int K, long long x_row_stride, const void* w,
                         size_t w_row_bytes, int N, const char* kquant_type, int transpose, void* y,

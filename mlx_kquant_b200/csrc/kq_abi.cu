@@ -447,7 +447,7 @@ int kq_moe_glu_gather(const void* x, int x_dtype, long long T, int K, const void
       return fail(KQ_ERR_INVALID_ARGUMENT,
                   "[mlx_kquant.moe_glu_gather_kq] workspace too small or not 256-byte aligned: %zu bytes given, %zu needed.",
                   workspace_bytes, need);
-    if (kq::moe_grouped_supported(K, (long long)w_row_bytes, false)) {
+    if (kq::moe_grouped_supported(K, false)) {
       e = kq::launch_moe_glu_grouped(x_dtype, x, K, static_cast<const uint8_t*>(gate_w), gate_expert_stride_bytes,
                                      static_cast<const uint8_t*>(up_w), up_expert_stride_bytes, (long long)w_row_bytes, N,
                                      n_experts, indices, n_entries, R, a, limit, y, workspace,
@@ -496,7 +496,7 @@ int kq_gather_qmv_mix(const void* x, int x_dtype, long long T, int S, int K, con
   cudaError_t e;
   const long long n_entries = T * (long long)S;
   if (n_entries > KQ_MOE_DIRECT_MAX_ENTRIES && workspace != nullptr && N % 8 == 0 &&
-      kq::moe_grouped_supported(K, (long long)w_row_bytes, true)) {
+      kq::moe_grouped_supported(K, true)) {
     const size_t need = kq::moe_grouped_workspace_bytes(n_entries, n_experts, n_entries * (long long)N * 2);
     if (workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255) != 0)
       return fail(KQ_ERR_INVALID_ARGUMENT,

@@ -21,6 +21,7 @@
 
 #include "kq_launch.h"
 #include "kq_rows_unit.cuh"
+#include "kq_tma_map.h"
 
 namespace kq {
 
@@ -325,21 +326,6 @@ few_kernel(const GemvArgs a, const FewPlan pl, const __grid_constant__ CUtensorM
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn fw_encode_fn() {
-  static EncodeTiledFn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      p = nullptr;
-    return reinterpret_cast<EncodeTiledFn>(p);
-  }();
-  return fn;
-}
-
 int fw_sm_count() {
   static int sms[16] = {};
   int dev = 0;
@@ -397,7 +383,7 @@ cudaError_t launch_few_t(const GemvArgs& a, const FewPlan& p, cudaStream_t st) {
   if (err == nullptr) return cudaErrorUnknown;
   alignas(64) CUtensorMap map{};
   if (TMA) {
-    EncodeTiledFn enc = fw_encode_fn();
+    EncodeTiledFn enc = encode_tiled_fn();
     if (enc == nullptr) return cudaErrorNotSupported;
     const cuuint64_t dims[2] = {(cuuint64_t)a.row_bytes, (cuuint64_t)a.N};
     const cuuint64_t strides[1] = {(cuuint64_t)a.row_bytes};

@@ -37,6 +37,7 @@
 #include "kq_common.cuh"
 #include "kq_launch.h"
 #include "kq_tcgen05.cuh"
+#include "kq_tma_map.h"
 
 namespace cg = cooperative_groups;
 
@@ -756,22 +757,6 @@ size_t gemm_workspace_bytes(int x_dtype, long long rows, int K) {
 }
 
 // ------------------------------------------------------------------ launch
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda).
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn encode_tiled_fn() {
-  static EncodeTiledFn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      p = nullptr;
-    return reinterpret_cast<EncodeTiledFn>(p);
-  }();
-  return fn;
-}
-
 // Tensor map of an fp16 matrix [M, K] (row stride in elements): boxes of 64 x box_rows, 128B swizzle.
 static cudaError_t make_x_map(CUtensorMap* map, const void* x, long long x_row_stride, int M, int K, int box_rows = 128) {
   EncodeTiledFn fn = encode_tiled_fn();

@@ -7,7 +7,8 @@
 // bytes, in pieces of sixteen with an address each, and read them back word by word. Here one thread of a warp fetches a
 // superblock of the warp's rows as one TMA box, and a thread reads its row's part in 16-byte words (box rows are odd
 // multiples of sixteen bytes: no bank conflicts).
-// One CTA per SM owns N / SM count rows, in blocks of at most 32 (a thread a row); its warps take the (block, superblock)
+// One CTA per SM owns N / SM count rows, in blocks of at most 32 (a thread a row), sixteen blocks at most (beyond 75 776 rows
+// there are more CTAs than SMs); its warps take the (block, superblock)
 // units in turn, several in flight each, and meet in shared memory. Measured, one bf16 row, back to back in a graph, before
 // and after: q6_k [4096, 14336] 29.0 -> 13.4 us, [28672, 8192] 65.8 -> 35.6 (5.4 TB/s), q5_k [8192, 8192] 21.9 -> 12.3, q4_k
 // [28672, 8192] 39.1 -> 25.6 (5.2 TB/s), [14336, 4096] 10.5 -> 9.3. Bound by HBM on large matrices, by the start of a launch
@@ -22,6 +23,7 @@
 #include "kq_common.cuh"
 #include "kq_launch.h"
 #include "kq_tcgen05.cuh"
+#include "kq_tma_map.h"
 
 namespace kq {
 
@@ -346,21 +348,6 @@ gemv_one_kernel(const GemvArgs a, const OnePlan pl, const __grid_constant__ CUte
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn one_encode_fn() {
-  static EncodeTiledFn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      p = nullptr;
-    return reinterpret_cast<EncodeTiledFn>(p);
-  }();
-  return fn;
-}
-
 template <int C, typename XT>
 cudaError_t launch_one_t(const GemvArgs& a, cudaStream_t st) {
   auto kern = gemv_one_kernel<C, XT>;
@@ -376,7 +363,7 @@ cudaError_t launch_one_t(const GemvArgs& a, cudaStream_t st) {
     sms[dev] = n;
   }
   int* err = device_error_word();
-  EncodeTiledFn enc = one_encode_fn();
+  EncodeTiledFn enc = encode_tiled_fn();
   if (err == nullptr || enc == nullptr) return cudaErrorNotSupported;
   OnePlan pl;
   const int per_sm = (a.N + sms[dev] - 1) / sms[dev];

@@ -145,9 +145,9 @@ cudaError_t launch_moe_glu(int x_dtype, const void* x, int K, const uint8_t* wg,
 cudaError_t launch_moe_mix(int x_dtype, const void* x, int K, const uint8_t* w, long long stride_w, long long row_bytes,
                            int N, int n_experts, const uint32_t* idx, const float* scores, long long T, int S, void* y,
                            cudaStream_t st);
-// grouped forms for more entries (tasks of up to four entries per expert); scratch from moe_grouped_workspace_bytes
+// grouped forms for more entries (tasks of eight or sixteen entries of an expert); scratch from moe_grouped_workspace_bytes
 size_t moe_grouped_workspace_bytes(long long n_entries, int n_experts, long long d_bytes);
-bool moe_grouped_supported(int K, long long row_bytes, bool rows_kernel);
+bool moe_grouped_supported(int K, bool rows_kernel);
 cudaError_t launch_moe_grouping_only(const uint32_t* idx, long long n_entries, int n_experts, void* workspace,
                                      cudaStream_t st);
 cudaError_t launch_moe_glu_grouped(int x_dtype, const void* x, int K, const uint8_t* wg, long long stride_g,

@@ -30,6 +30,7 @@
 #include "kq_imma_q4k.cuh"
 #include "kq_launch.h"
 #include "kq_rows_unit.cuh"
+#include "kq_tma_map.h"
 
 namespace kq {
 
@@ -722,23 +723,9 @@ static cudaError_t moe_build_tasks(const uint32_t* idx, long long n_entries, int
                                 reinterpret_cast<int*>(ws + L.tasks), st);
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn md_encode_fn() {
-  static EncodeTiledFn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      p = nullptr;
-    return reinterpret_cast<EncodeTiledFn>(p);
-  }();
-  return fn;
-}
 // all experts' rows of one matrix
 static cudaError_t md_map(CUtensorMap* map, const uint8_t* w, long long row_bytes, int F, int n_experts, long long stride) {
-  EncodeTiledFn enc = md_encode_fn();
+  EncodeTiledFn enc = encode_tiled_fn();
   if (enc == nullptr) return cudaErrorNotSupported;
   const cuuint64_t dims[3] = {(cuuint64_t)row_bytes, (cuuint64_t)F, (cuuint64_t)n_experts};
   const cuuint64_t strides[2] = {(cuuint64_t)row_bytes, (cuuint64_t)stride};
@@ -808,8 +795,11 @@ cudaError_t launch_moe_grouping_only(const uint32_t* idx, long long n_entries, i
   return moe_build_tasks(idx, n_entries, n_experts, static_cast<uint8_t*>(workspace), L, st);
 }
 
-bool moe_grouped_supported(int K, long long row_bytes, bool rows_kernel) {
-  (void)row_bytes;
+// The limits of the kernels before these, whose rows and tiles had to fit twice into shared memory; md_plan has room for longer
+// rows, and the grouped mix is the faster one there too (512 entries of 128 experts, K 1536: 377 us entry by entry, 81 grouped;
+// 32 experts, K 2048, 256 entries: 712 and 77). But it rounds every slot's product to 16 bits before the weighted sum, which the
+// other form does not, so that calls that have had one rounding keep it.
+bool moe_grouped_supported(int K, bool rows_kernel) {
   return K <= (rows_kernel ? 1280 : 2304);
 }
 

@@ -54,36 +54,6 @@ __device__ __forceinline__ bool mbar_wait_err(uint64_t* bar, uint32_t parity, vo
   }
 }
 
-// Non-blocking probe: unlike try_wait the thread is never parked, so a waiter sees the flip at
-// once - for barriers that flip within a microsecond.
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Bounded busy wait on test_wait: same contract as mbar_wait_err.
-__device__ __forceinline__ bool mbar_spin_err(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code,
-                                              int* error_word) {
-  for (int spin = 0; spin < 4096; spin++)
-    if (mbar_test_wait(bar, parity)) return true;
-  const unsigned long long t0 = globaltimer_ns();
-  for (int spin = 0;; spin++) {
-    if (mbar_test_wait(bar, parity)) return true;
-    if ((spin & 1023) == 1023) {
-      if (*abort_flag) return false;
-      if (globaltimer_ns() - t0 > 2000000000ull) {
-        *abort_flag = 1;
-        atomicOr(error_word, code);
-        return false;
-      }
-    }
-  }
-}
-
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
@@ -103,16 +73,6 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
           tmem_d),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Same product with the A operand read from tensor memory (row i of A in lane i, two 16-bit
-// elements per 32-bit column, K running along the columns).
-__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(
-          tmem_d),
-      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // Registers -> tensor memory: thread l of warp w writes 32 consecutive columns of lane 32 (w % 4) + l.

@@ -34,6 +34,7 @@
 #include "kq_common.cuh"
 #include "kq_launch.h"
 #include "kq_tcgen05.cuh"
+#include "kq_tma_map.h"
 
 namespace cg = cooperative_groups;
 
@@ -759,21 +760,6 @@ tile_kernel(const TilePlan a, const __grid_constant__ CUtensorMap map_x, const _
 }
 
 // ------------------------------------------------------------------ host
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn encode_tiled_fn() {
-  static EncodeTiledFn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      p = nullptr;
-    return reinterpret_cast<EncodeTiledFn>(p);
-  }();
-  return fn;
-}
-
 // fp16 matrix [rows, K], row stride in elements: boxes of 64 x box_rows, 128B swizzle
 bool half_map(CUtensorMap* map, const void* p, long long row_stride, long long rows, int K, int box_rows) {
   EncodeTiledFn fn = encode_tiled_fn();
