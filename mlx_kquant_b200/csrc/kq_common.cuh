@@ -463,9 +463,10 @@ __device__ __forceinline__ float plain_dot(const uint8_t* w, const XT* x, int K)
 #pragma unroll
     for (int i = 0; i < 8; i++) {
       float xv;
-      if constexpr (std::is_same<XT, __half>::value) xv = __half2float(x[k + i]);
-      else if constexpr (std::is_same<XT, float>::value) xv = __bfloat162float(__float2bfloat16_rn(x[k + i]));
-      else xv = __bfloat162float(x[k + i]);
+      // (from L2: the kernels start before x is written)
+      if constexpr (std::is_same<XT, __half>::value) xv = __half2float(__ldcg(x + k + i));
+      else if constexpr (std::is_same<XT, float>::value) xv = __bfloat162float(__float2bfloat16_rn(__ldcg(x + k + i)));
+      else xv = __bfloat162float(__ldcg(x + k + i));
       sum = fmaf(xv, v[i], sum);
     }
   }
