@@ -448,6 +448,19 @@ __device__ __forceinline__ IqTables stage_iq_tables(uint8_t* smem, int tid, int 
   return t;
 }
 
+// N words from byte 4 W + odd_bits / 8 of a 16-byte aligned window on
+template <int W, int N>
+__device__ __forceinline__ void window_words(const uint8_t* win, uint32_t odd_bits, uint32_t (&out)[N]) {
+  uint32_t w[(W + N + 4) / 4 * 4];
+#pragma unroll
+  for (int i = 0; i < (W + N + 4) / 4; i++) {
+    const uint4 v = *reinterpret_cast<const uint4*>(win + 16 * i);
+    w[4 * i] = v.x, w[4 * i + 1] = v.y, w[4 * i + 2] = v.z, w[4 * i + 3] = v.w;
+  }
+#pragma unroll
+  for (int i = 0; i < N; i++) out[i] = __funnelshift_r(w[W + i], w[W + i + 1], odd_bits);
+}
+
 // One output by itself: decoded weights times activations in float32 (float32 rows rounded to bf16 first), as the generic
 // kernel has it. For outputs that a split into integers, offsets, sums and scales leaves without a finite value although they
 // may have one, or an infinity: an infinite activation meets an offset's sum (inf - inf) or integers of zero, and a sum can

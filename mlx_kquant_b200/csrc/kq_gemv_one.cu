@@ -114,18 +114,6 @@ __device__ __forceinline__ float one_dot_k4(const uint8_t* blk, const OneX& X) {
   return dd.x * prod - dd.y * mins;
 }
 
-// N words from byte 4 W + odd_bits / 8 of a 16-byte aligned window on
-template <int W, int N>
-__device__ __forceinline__ void one_words(const uint8_t* win, uint32_t odd_bits, uint32_t (&out)[N]) {
-  uint32_t w[(W + N + 4) / 4 * 4];
-#pragma unroll
-  for (int i = 0; i < (W + N + 4) / 4; i++) {
-    const uint4 v = *reinterpret_cast<const uint4*>(win + 16 * i);
-    w[4 * i] = v.x, w[4 * i + 1] = v.y, w[4 * i + 2] = v.z, w[4 * i + 3] = v.w;
-  }
-#pragma unroll
-  for (int i = 0; i < N; i++) out[i] = __funnelshift_r(w[W + i], w[W + i + 1], odd_bits);
-}
 // q6_k: half hf of the superblock is four quarters of 32 weights over the same 64 ql and 32 qh bytes; scales per sixteen
 template <int W>
 __device__ __forceinline__ float one_dot_q6_at(const uint8_t* win, uint32_t odd_bits, const OneX& X) {
@@ -139,11 +127,11 @@ __device__ __forceinline__ float one_dot_q6_at(const uint8_t* win, uint32_t odd_
       sc[0] = __funnelshift_r(v0, v1, odd_bits) ^ 0x80808080u, sc[1] = __funnelshift_r(v1, v2, odd_bits) ^ 0x80808080u;  // biased by 128
     }
     uint32_t H[8];
-    one_words<W, 8>(win + 128 + 32 * hf, odd_bits, H);
+    window_words<W, 8>(win + 128 + 32 * hf, odd_bits, H);
 #pragma unroll
     for (int a = 0; a < 2; a++) {
       uint32_t L[8];
-      one_words<W, 8>(win + 64 * hf + 32 * a, odd_bits, L);
+      window_words<W, 8>(win + 64 * hf + 32 * a, odd_bits, L);
 #pragma unroll
       for (int up = 0; up < 2; up++) {
         const int qd = 2 * up + a;

@@ -302,21 +302,10 @@ template <int UNIT>
 struct Q6kHalf {
   uint32_t ql[16], qh[8], sc[2];
   float d;
-  template <int W, int N>  // N words from byte 4 W + (odd_bits / 8) of a 16-byte aligned window on
-  static __device__ __forceinline__ void words(const uint8_t* win, uint32_t odd_bits, uint32_t (&out)[N]) {
-    uint32_t w[(W + N + 4) / 4 * 4];
-#pragma unroll
-    for (int i = 0; i < (W + N + 4) / 4; i++) {
-      const uint4 v = *reinterpret_cast<const uint4*>(win + 16 * i);
-      w[4 * i] = v.x, w[4 * i + 1] = v.y, w[4 * i + 2] = v.z, w[4 * i + 3] = v.w;
-    }
-#pragma unroll
-    for (int i = 0; i < N; i++) out[i] = __funnelshift_r(w[W + i], w[W + i + 1], odd_bits);
-  }
   template <int W>
   __device__ __forceinline__ void load_at(const uint8_t* win, uint32_t odd_bits, int half) {
-    words<W, 16>(win + 64 * half, odd_bits, ql);
-    words<W, 8>(win + 128 + 32 * half, odd_bits, qh);
+    window_words<W, 16>(win + 64 * half, odd_bits, ql);
+    window_words<W, 8>(win + 128 + 32 * half, odd_bits, qh);
     const uint32_t* s = reinterpret_cast<const uint32_t*>(win + 192 + 8 * half + 4 * W);
     const uint32_t s0 = s[0], s1 = s[1], s2 = s[2];
     sc[0] = __funnelshift_r(s0, s1, odd_bits), sc[1] = __funnelshift_r(s1, s2, odd_bits);
