@@ -60,10 +60,11 @@ __device__ __forceinline__ void dot4(uint32_t q, uint32_t xh, uint32_t xl, int& 
 }
 
 // q4_k / q5_k: 32 quant bytes hold sub-blocks 2 p (low nibbles) and 2 p + 1 (high ones).
-// MID (q4_k, fp16 rows): the integers multiply quants less 8, eight times the activations' float sum makes up for it. An
+// MID (q4_k, fp16 rows of large matrices): the integers multiply quants less 8, eight times the activations' float sum makes up for it. An
 // activation is off by its rounding to an integer, and quants, half their range on average, are twice the weights that they
 // stand for. Errors beyond the output's rounding, [28672, 8192], 5.1e-5 -> 2.2e-5 of the outputs' size: not above the 2.7e-5
-// of the fp16 matrix kernel that had matrices beyond 60 M weights (32.9 us; 25.7 -> 26.5 here).
+// of the fp16 matrix kernel that had matrices beyond 60 M weights (32.9 us; 25.7 -> 26.5 here). Smaller ones had 16-bit integers
+// with a scale per 256 of them (6.3e-5) and are spared the 2 to 3 %.
 template <int C, bool MID>
 __device__ __forceinline__ float one_dot_k4(const uint8_t* blk, const OneX& X) {
   const uint4* b = reinterpret_cast<const uint4*>(blk);
@@ -164,7 +165,7 @@ __device__ __forceinline__ void one_load(uint32_t dst, const CUtensorMap* map, i
       : "memory");
 }
 
-template <int C, typename XT>
+template <int C, typename XT, bool MID>
 __global__ void __launch_bounds__(kOneThreads, 1)
 gemv_one_kernel(const GemvArgs a, const OnePlan pl, const __grid_constant__ CUtensorMap map, int* __restrict__ error_word) {
   using OT = typename std::conditional<std::is_same<XT, __half>::value, __half, __nv_bfloat16>::type;
@@ -307,7 +308,7 @@ gemv_one_kernel(const GemvArgs a, const OnePlan pl, const __grid_constant__ CUte
         default: y += one_dot_q6_at<3>(row, odd, X); break;
       }
     } else {
-      y += one_dot_k4<C, C == Q4_K && std::is_same<XT, __half>::value>(row, X);
+      y += one_dot_k4<C, MID>(row, X);
     }
     __syncwarp();  // the slot has been read
     if (lane == 0 && u + D * kOneWarps < units) issue(u + D * kOneWarps, d);
@@ -336,9 +337,9 @@ gemv_one_kernel(const GemvArgs a, const OnePlan pl, const __grid_constant__ CUte
   }
 }
 
-template <int C, typename XT>
+template <int C, typename XT, bool MID = false>
 cudaError_t launch_one_t(const GemvArgs& a, cudaStream_t st) {
-  auto kern = gemv_one_kernel<C, XT>;
+  auto kern = gemv_one_kernel<C, XT, MID>;
   static int sms[16] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -392,6 +393,7 @@ cudaError_t launch_one_t(const GemvArgs& a, cudaStream_t st) {
 
 template <int C>
 cudaError_t launch_one_c(int x_dtype, const GemvArgs& a, cudaStream_t st) {
+  if (C == Q4_K && x_dtype == F16 && (long long)a.N * a.K > (60ll << 20)) return launch_one_t<C, __half, C == Q4_K>(a, st);
   if (x_dtype == F16) return launch_one_t<C, __half>(a, st);
   if (x_dtype == BF16) return launch_one_t<C, __nv_bfloat16>(a, st);
   return launch_one_t<C, float>(a, st);
