@@ -900,7 +900,9 @@ int resident_ctas(int n) {
 // 128 rows; the copy path's loads) or the tensor pipe (4 cycles a token and 128 of K, the same for a pair as for one CTA of
 // half the rows), whichever is more; a tile its epilogue, most of it in the open where tensor memory holds one accumulator.
 // Constants fitted to a sweep of shapes over 150 sizes (N, K of 1024 to 28672, 17 to 2048 rows; q4_k, q6_k and fp16):
-// the shape taken is within 1-2 % of the best one on average, 25 % at worst.
+// the shape taken is within 1-2 % of the best one on average, 25 % at worst. With K up to 1024 the q4_k producers' work is too short
+// to hide an epilogue that shares the issue slots with it: 50 cycles a token whatever the shape (as 2500 + 8 to 26
+// a token: q4_k x 1500 [28672, 512] 101 us, now 92, [14997, 768] 92 and 77, [19861, 768] 119 and 99).
 double tile_cost(int src, int M, int N, int K, int cg, int tn, int ks, int cap) {
   const bool fused = src != kSrcHalf;
   const long long tiles = (long long)((N + 128 * cg - 1) / (128 * cg)) * ((M + tn - 1) / tn);
@@ -909,7 +911,8 @@ double tile_cost(int src, int M, int N, int K, int cg, int tn, int ks, int cap) 
   const double per_step = fused ? 2.0 : 1.0, steps = std::ceil(K / (kStep * per_step)) / ks;
   const double make = src == kSrcQ4K ? 750.0 : (src == kSrcQ6K ? 830.0 + tn : 200.0 + 1.3 * tn / cg);
   const bool open = turns == 1 || (fused && tn > (cg == 1 ? 128 : 160));
-  const double tile = steps * std::max(make, 2.04 * per_step * tn) + 2500.0 + (open ? 26.0 : 8.0) * tn;
+  const double drain = src == kSrcQ4K && K <= 1024 ? 50.0 * tn : 2500.0 + (open ? 26.0 : 8.0) * tn;
+  const double tile = steps * std::max(make, 2.04 * per_step * tn) + drain;
   return turns * tile + 9000.0 + (ks > 1 ? 3500.0 + 12.0 * ks * tn : 0.0);
 }
 
