@@ -117,7 +117,8 @@ KQ_API int kq_quantize_cpu(const void* w, int w_dtype, long long n_weights, long
 KQ_API size_t kq_quantized_matmul_workspace_bytes(int x_dtype, long long rows, int K);
 /* The same with room for an fp16 copy of (a part of) the weights, of at most 128 MiB or 256 rows, where [N, K] products
  * of that many rows may be faster from one: more than 16 rows on matrices of 4 M weights and more of every codec but q4_k
- * (q6_k with K a multiple of 1024: more than 256 rows, and there and with other K by an estimate of both ways). A call that
+ * (q6_k with K a multiple of 1024: more than 256 rows, and there and with other K by an estimate of both ways), and of q6_k
+ * of any size where N rows are no whole number of groups that start on 16 bytes (of two to eight rows). A call that
  * is given only the bytes above works without it. */
 KQ_API size_t kq_quantized_matmul_workspace_bytes_for(const char* kquant_type, int x_dtype, long long rows, int N, int K);
 KQ_API int kq_quantized_matmul(const void* x, int x_dtype, long long rows, int K, long long x_row_stride, const void* w,

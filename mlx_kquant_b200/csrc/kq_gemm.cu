@@ -849,7 +849,9 @@ static int half_chunk(int N, int K) {
 static size_t half_bytes(int N, int K) { return (2 * (size_t)half_chunk(N, K) * (size_t)K + 255) & ~(size_t)255; }
 // Calls that may use the copy, by size: all codecs without a producer of their own in kq_tile.cu - decode8<> makes a
 // K-step's weights several times slower than the tensor cores use them - once the matrix outweighs the extra launch; q6_k
-// where its rows cannot be fetched there, or with many rows (see launch_gemm).
+// with many rows (see launch_gemm), and whatever its size where its rows cannot be fetched there: beside the general kernel
+// [763, 1024] x 53 16.2 -> 12.8 us, [3001, 1024] x 798 50 -> 23, 144 sizes up to 4 M weights 0.68 of the time on average (one of
+// them, [2047, 256] x 2000, 1.10).
 // With up to 256 rows and short K the lighter decoders keep up: q2_k [4096, 1024] x 128 13.7 / 16.6 us (x 300 22.0 / 19.7),
 // iq4_xs 14.9 / 17.5, q4_0 17.4 / 17.4 there but [16384, 512] 17.8 / 19.8; q5_k and the others gain at every K.
 static int half_min_k(int codec) {
@@ -861,6 +863,7 @@ static int half_min_k(int codec) {
   return 0;
 }
 static bool use_half(int codec, long long M, int N, int K) {
+  if (codec == Q6_K && !tile_rows_fit(codec, N, K)) return true;
   if (codec == Q4_K || (long long)N * K < (4ll << 20)) return false;
   if (codec == Q6_K && (K & 1023) == 0 && ((K & 2047) == 0 || (N & 1) == 0)) return M > 256;
   return M > 256 || K >= half_min_k(codec);

@@ -128,6 +128,7 @@ struct TileArgs {
                       // kernel starts beside it and waits for what it writes
 };
 bool tile_supported(int codec, const uint8_t* w, long long row_bytes, int N, int K, long long expert_stride);
+bool tile_rows_fit(int codec, int N, int K);  // ... that it takes by its sizes
 // estimated cycles of a dense call (half_weights: without the dequantization)
 double tile_cycles(int codec, bool half_weights, int M, int N, int K);
 cudaError_t launch_tile(int codec, bool half_weights, bool out_half, const TileArgs& t, cudaStream_t st);

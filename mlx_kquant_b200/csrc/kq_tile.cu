@@ -983,6 +983,10 @@ bool tile_supported(int codec, const uint8_t* w, long long row_bytes, int N, int
          row_bytes <= (1 << 24);
 }
 
+bool tile_rows_fit(int codec, int N, int K) {
+  return (codec == Q4_K || codec == Q6_K) && (K & 255) == 0 && (N & ((1 << row_group((long long)(K >> 8) * bpb_of(codec))) - 1)) == 0;
+}
+
 double tile_cycles(int codec, bool half_weights, int M, int N, int K) {
   const TileShape sh = pick_shape(half_weights ? kSrcHalf : (codec == Q4_K ? kSrcQ4K : kSrcQ6K), M, N, K);
   // Rows that are no whole sixteens leave the accumulator in classes and are put right output by output, 60 cycles a token.

@@ -134,4 +134,25 @@ def test_which_kernel(codec, m, n, k, dt):
 
 @pytest.mark.parametrize("n", [1001, 1002, 1004])
 def test_which_kernel_has_rows_that_do_not_fill_a_class(n):
-    assert "gemm_kernel" in product_kernels("q6_k", 33, n, 1280, "bf16")
+    names = product_kernels("q6_k", 33, n, 1280, "bf16")
+    assert "dequant_kernel" in names and "tile_kernel" in names
+
+
+@pytest.mark.parametrize("m,n,k", [(17, 9, 256), (53, 763, 1024), (300, 259, 768), (130, 3001, 1280), (65, 1178, 512)])
+@pytest.mark.parametrize("room", [True, False])
+def test_small_q6k_rows_that_do_not_fill_a_class(m, n, k, room):
+    """By the copy, and with the room for the converted activations alone by the general kernel."""
+    rng, some = some_rows("q6_k", k, m + n + k)
+    pick = rng.integers(0, 64, n)
+    x, _ = x_to_torch(rng.standard_normal((m, k)).astype(np.float32), "bf16")
+    ref = (x.double().cpu().numpy() @ Oracle().dequantize(some, "q6_k", "f32").astype(np.float64).T)[:, pick]
+    w = torch.from_numpy(some[pick]).cuda()
+    if room:
+        y = kq.quantized_matmul(x, w, None, "q6_k")
+    else:
+        lib, dt = kq._lib.lib(), kq.ops._DT[x.dtype]
+        ws = torch.empty(lib.kq_quantized_matmul_workspace_bytes(dt, m, k), dtype=torch.uint8, device="cuda")
+        y = torch.empty(m, n, dtype=x.dtype, device="cuda")
+        kq._lib.check(lib.kq_quantized_matmul(x.data_ptr(), dt, m, k, k, w.data_ptr(), w.shape[1], n, b"q6_k", 1, y.data_ptr(), n,
+                                              ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream))
+    check(y, ref, "bf16")
