@@ -1208,7 +1208,9 @@ cudaError_t launch_gemv(int codec, int x_dtype, const GemvArgs& a, cudaStream_t 
   // q4_k: the tensor-pipe kernel up to 24 M weights of short rows, the TMA kernel beyond ([5000, 4096] 5.2 us against 6.2,
   // [5120, 2048] 3.5 / 4.0; [14336, 2048] 6.5 / 5.8, [14336, 4096] 10.5 / 9.3, [2048, 8192] 7.5 / 6.4, [4096, 14336] 16.4 /
   // 10.5, [28672, 8192] 39 / 25.6). q5_k and q6_k: the TMA kernel but for the smallest, which are one chain of latencies
-  // either way ([256, 4096] q6_k 4.1 us there, 4.7 here; [4096, 4096] 8.6 / 5.8, [4096, 14336] 29 / 13.4).
+  // either way ([256, 4096] q6_k 4.1 us there, 4.7 here; [4096, 4096] 8.6 / 5.8, [4096, 14336] 29 / 13.4). All of these take
+  // activations as 16-bit integers; fp16 rows of more than 60 M q4_k weights, which a kernel of fp16 products had, with less of
+  // an error than there (kq_gemv_one.cu, MID).
   const long long weights = (long long)a.N * a.K;
   const bool forced = imma_env && imma_env[0] == '1';
   const bool one = a.K >= 8192 || (codec == Q4_K ? weights >= (24ll << 20) : a.N >= 1024 && weights >= (2ll << 20));
